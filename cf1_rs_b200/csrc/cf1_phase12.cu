@@ -365,69 +365,123 @@ void launch_sk(const SuperkmerArgs &a, int persistent_ctas, cudaStream_t s) {
 // -------------------------------------------------------------- partition ----
 // One CTA.  Boundaries follow the reference's greedy walk: add the bucket,
 // place a boundary when the running count reaches total/num_bins, carry the
-// excess.  When no bucket exceeds the target the walk never lags, so the
-// boundaries after bucket i number min(floor(C(i)/target), num_bins-1) with C
-// the inclusive prefix sum; otherwise one thread walks the buckets.
-__global__ void __launch_bounds__(1024) partition_kernel(const uint32_t *hist, uint32_t B, uint16_t *lut,
-                                                         uint64_t *rec_off, uint32_t *n_bins_eff) {
-  constexpr int BLK = 1024;
-  constexpr int PER = NUM_BUCKETS / BLK;  // 64
-  __shared__ uint64_t sm[BLK / 32];
-  __shared__ unsigned long long s_bin[MAX_BINS];
-  __shared__ uint32_t s_max;
-  const unsigned tid = threadIdx.x;
-  const uint32_t b0 = tid * PER;
-  uint64_t lsum = 0;
-  uint32_t lmax = 0;
-  for (int i = 0; i < PER; i++) {
-    uint32_t h = hist[b0 + i];
-    lsum += h;
-    lmax = h > lmax ? h : lmax;
+// excess.  With C the inclusive prefix sum of the counts and t the target,
+// the boundaries placed after bucket i are
+//   nb(i) = min(nb(i - 1) + 1, floor(C(i) / t)),  nb(-1) = 0,
+// so nb(i) = i + min(1, min over j <= i of floor(C(j) / t) - j): a prefix
+// minimum, capped at num_bins - 1 (a walk that reached the cap stays there).
+// When no bucket exceeds t the walk never lags and nb(i) is floor(C(i) / t)
+// itself, so the pass that carries the minima from warp to warp is skipped.
+// lut[i] = nb(i - 1) grows by at most one from bucket to bucket: a bin is one
+// stretch of buckets, and bin nb(i) starts at C(i) where nb(i) > nb(i - 1).
+//
+// Warp w walks buckets [2048 w, 2048 (w + 1)), 128 at a time, a lane four
+// consecutive ones (one 16-byte load).  Its bound is the latency of these
+// dependent rounds on one SM.
+constexpr int PT_WARPS = 32;
+constexpr uint32_t PT_STEP = 128;                           // buckets a warp takes at once
+constexpr int PT_ITERS = NUM_BUCKETS / PT_WARPS / PT_STEP;  // 16
+
+// Buckets [i0, i0 + 4) of a lane (counts v, c records before them): g[j] =
+// floor(C(i0 + j) / t) - (i0 + j).  The quotient is at most 2 num_bins; the
+// division takes 32 bits when the total does.
+CF1_D void pt_lags(const uint4 &v, uint64_t c, uint64_t t, bool narrow, int i0, int (&g)[4]) {
+  const uint32_t h[4] = {v.x, v.y, v.z, v.w};
+#pragma unroll
+  for (int j = 0; j < 4; j++) {
+    c += h[j];
+    const uint32_t q = t == 0 ? NUM_BUCKETS + 1 : narrow ? (uint32_t)c / (uint32_t)t : (uint32_t)(c / t);
+    g[j] = (int)q - (i0 + j);
   }
-  if (tid == 0) s_max = 0;
-  for (uint32_t b = tid; b < B; b += BLK) s_bin[b] = 0;
+}
+
+__global__ void __launch_bounds__(PT_WARPS * 32) partition_kernel(const uint32_t *hist, uint32_t B, uint16_t *lut,
+                                                                  uint64_t *rec_off, uint32_t *n_bins_eff) {
+  __shared__ uint64_t s_sum[PT_WARPS];
+  __shared__ uint32_t s_max[PT_WARPS];
+  __shared__ int s_min[PT_WARPS];
+  __shared__ int s_last;
+  const unsigned lane = lane_id(), warp = threadIdx.x >> 5;
+  const uint4 *h4 = reinterpret_cast<const uint4 *>(hist) + warp * (PT_ITERS * 32) + lane;
+  ushort4 *lut4 = reinterpret_cast<ushort4 *>(lut) + warp * (PT_ITERS * 32) + lane;
+  uint64_t sum = 0;
+  uint32_t mx = 0;
+#pragma unroll
+  for (int it = 0; it < PT_ITERS; it++) {
+    const uint4 v = h4[it * 32];
+    sum += (uint64_t)v.x + v.y + v.z + v.w;
+    mx = max(mx, max(max(v.x, v.y), max(v.z, v.w)));
+  }
+  sum = warp_sum(sum);
+  mx = __reduce_max_sync(FULL, mx);
+  if (lane == 0) {
+    s_sum[warp] = sum;
+    s_max[warp] = mx;
+  }
   __syncthreads();
-  atomicMax(&s_max, lmax);
-  uint64_t total;
-  uint64_t pre = block_exclusive_scan<BLK>(lsum, sm, total);
-  const uint64_t target = total / B;
-  const uint32_t cap = B - 1;
-  if (target == 0 || (uint64_t)s_max <= target) {
-    uint64_t C = pre;
-    uint64_t j_prev = target == 0 ? min((uint64_t)b0, (uint64_t)cap) : min(C / target, (uint64_t)cap);
-    for (int i = 0; i < PER; i++) {
-      uint32_t bucket = b0 + i;
-      lut[bucket] = (uint16_t)j_prev;
-      C += hist[bucket];
-      j_prev = target == 0 ? min((uint64_t)bucket + 1, (uint64_t)cap) : min(C / target, (uint64_t)cap);
+  const uint64_t ws = s_sum[lane], wx = warp_inclusive_scan(ws);
+  const uint64_t total = __shfl_sync(FULL, wx, 31), c0 = __shfl_sync(FULL, wx - ws, warp);
+  mx = __reduce_max_sync(FULL, s_max[lane]);
+  const uint64_t t = total / B;
+  const int cap = (int)B - 1, first = (int)(warp * PT_ITERS * PT_STEP + lane * 4);
+  const bool narrow = total < (1ull << 32);
+  int lag = 1;  // the minimum of 1 and floor(C(j) / t) - j over the buckets before this warp's
+  if (t != 0 && (uint64_t)mx > t) {
+    uint64_t c = c0;
+    int m = 1;
+    for (int it = 0; it < PT_ITERS; it++) {
+      const uint4 v = h4[it * 32];
+      const uint64_t s4 = (uint64_t)v.x + v.y + v.z + v.w, x = warp_inclusive_scan(s4);
+      int g[4];
+      pt_lags(v, c + x - s4, t, narrow, first + it * (int)PT_STEP, g);
+      m = min(m, min(min(g[0], g[1]), min(g[2], g[3])));
+      c += __shfl_sync(FULL, x, 31);
     }
-  } else if (tid == 0) {
-    uint64_t cur = 0, nb = 0;
-    for (uint32_t bucket = 0; bucket < NUM_BUCKETS; bucket++) {
-      lut[bucket] = (uint16_t)nb;
-      cur += hist[bucket];
-      if (cur >= target && nb < cap) {
-        nb++;
-        cur -= target;
+    m = __reduce_min_sync(FULL, m);
+    if (lane == 0) s_min[warp] = m;
+    __syncthreads();
+    for (unsigned w = 0; w < warp; w++) lag = min(lag, s_min[w]);
+  } else if (t != 0 && warp) {  // no lag: the bucket before this warp's has the smallest
+    lag = min(1, (int)(uint32_t)(c0 / t) - (int)(warp * PT_ITERS * PT_STEP - 1));
+  }
+  uint64_t c = c0;
+  for (int it = 0; it < PT_ITERS; it++) {
+    const int i0 = first + it * (int)PT_STEP;
+    const uint4 v = h4[it * 32];
+    const uint32_t h[4] = {v.x, v.y, v.z, v.w};
+    const uint64_t s4 = (uint64_t)v.x + v.y + v.z + v.w, x = warp_inclusive_scan(s4);
+    uint64_t cb = c + x - s4;
+    int g[4];
+    pt_lags(v, cb, t, narrow, i0, g);
+    int m = min(min(g[0], g[1]), min(g[2], g[3]));
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+      const int y = __shfl_up_sync(FULL, m, o);
+      if (lane >= (unsigned)o) m = min(m, y);
+    }
+    const int upto = __shfl_up_sync(FULL, m, 1);
+    int run = lane ? min(lag, upto) : lag;  // over the buckets before i0
+    uint16_t bin[4];
+#pragma unroll
+    for (int j = 0; j < 4; j++) {
+      const int i = i0 + j, before = max(0, min(i - 1 + run, cap));  // nb(i - 1): 0 for i = 0 (run <= 1)
+      cb += h[j];
+      run = min(run, g[j]);
+      const int after = min(i + run, cap);
+      bin[j] = (uint16_t)before;
+      if (after != before) rec_off[after] = cb;
+      if (i == (int)NUM_BUCKETS - 1) {
+        *n_bins_eff = (uint32_t)before + 1;
+        s_last = after;
       }
     }
+    lut4[it * 32] = make_ushort4(bin[0], bin[1], bin[2], bin[3]);
+    lag = min(lag, __shfl_sync(FULL, m, 31));
+    c += __shfl_sync(FULL, x, 31);
   }
   __syncthreads();
-  for (int i = 0; i < PER; i++) atomicAdd(&s_bin[lut[b0 + i]], (unsigned long long)hist[b0 + i]);
-  __syncthreads();
-  uint64_t carry = 0;
-  for (uint32_t base = 0; base < B; base += BLK) {
-    uint32_t b = base + tid;
-    uint64_t c = b < B ? s_bin[b] : 0;
-    uint64_t tot;
-    uint64_t p = block_exclusive_scan<BLK>(c, sm, tot);
-    if (b < B) rec_off[b] = carry + p;
-    carry += tot;
-  }
-  if (tid == 0) {
-    rec_off[B] = carry;
-    *n_bins_eff = (uint32_t)lut[NUM_BUCKETS - 1] + 1;
-  }
+  if (threadIdx.x == 0) rec_off[0] = 0;
+  for (uint32_t b = (uint32_t)s_last + 1 + threadIdx.x; b <= B; b += PT_WARPS * 32) rec_off[b] = total;
 }
 
 }  // namespace
@@ -460,7 +514,7 @@ void launch_bin_scatter(const uint64_t *rec_tmp, const uint16_t *rec_bucket, uin
 
 void launch_partition(const uint32_t *hist, uint32_t num_bins, uint16_t *lut, uint64_t *rec_off, uint32_t *n_bins_eff,
                       cudaStream_t s) {
-  partition_kernel<<<1, 1024, 0, s>>>(hist, num_bins, lut, rec_off, n_bins_eff);
+  partition_kernel<<<1, PT_WARPS * 32, 0, s>>>(hist, num_bins, lut, rec_off, n_bins_eff);
   CF1_LAUNCH_CHECK();
 }
 
