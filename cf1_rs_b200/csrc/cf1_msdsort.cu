@@ -444,6 +444,7 @@ CF1_D uint32_t cs_sort_unique_range(const KeyT *src, uint32_t m, const CsDigit &
 // u16 of shared memory for the keys' bits in the slices (a slice has at most
 // L0_SW_MAX * 64 < 2^16 - 2 bits).  All threads call it.
 constexpr uint32_t L0_SW_MAX = 768;
+static_assert(L0_SW_MAX * sizeof(uint32_t) <= cs_cap_for(false, false), "l0_slice's pw fits the payload area");
 // With kpay (the keys' joined payload bytes) and o.with_pay, the payloads go
 // out as Level0Out describes; pw: L0_SW_MAX u32 of shared memory.
 CF1_D void l0_slice(const uint64_t *keys, uint32_t n, uint64_t j, int P, const Level0Out &o,
@@ -1268,7 +1269,7 @@ bool msd_sort_unique(KeyT *keys, KeyT *alt, uint64_t n, const uint64_t *seg_off,
   // S, hist, cur, pstart (u32) and the chunk bounds (u16)
   const uint32_t cap = cs_cap_for(KOps<KeyT>::WORDS == 2, sorted);
   size_t smem = cap * sizeof(KeyT) + (3 * CS_BUCKETS + 1) * sizeof(uint32_t) + (CS_BUCKETS + 2) * sizeof(uint16_t) +
-                (pkeys ? cap : 0);
+                (pkeys || !sorted ? cap : 0);  // payloads; without them the unsorted form's l0_slice scratch
   auto kern = sorted ? cs_sort_unique_kernel<KeyT, true> : cs_sort_unique_kernel<KeyT, false>;
   CF1_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
   KeyT *U = T == keys ? alt : keys;
