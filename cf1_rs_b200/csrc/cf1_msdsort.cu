@@ -1,8 +1,8 @@
 // Phase 3a, MSD form: distinct canonical k-mers per bin, sorted or not.
 //
 //   1. one or two multisplit passes on the top P bits of the keys (sorted) or
-//      of key * KEY_SPREAD_MUL (distinct only), segmented by bin (P chosen so
-//      a sub-bucket fits shared memory);
+//      of key * KEY_SPREAD_MUL (distinct only, up to 5 bits less), segmented
+//      by bin (P chosen so a sub-bucket fits shared memory);
 //   2. one CTA per sub-bucket: a shared-memory hash set keeps one copy of
 //      each key; the sorted form then counting-sorts on the next 10 bits,
 //      insertion-sorts the small buckets (bitonic sort of the whole
@@ -12,6 +12,8 @@
 //      array; a bin's first sub-bucket gives its slot offset.
 // A sub-bucket above CAP keys (long homopolymers, huge tandem arrays) makes
 // the caller fall back to the LSD path (cf1_phase3_sort.cu) for the run.
+#include <cstddef>
+
 #include "cf1_device_util.cuh"
 #include "cf1_internal.cuh"
 #include "cf1_mphf.cuh"
@@ -754,8 +756,562 @@ __global__ void __launch_bounds__(CS_BLOCK, SORTED ? 2 : 4) cs_sort_unique_kerne
   }
 }
 
+// ---------------------------------------------------------------- group dedup
+// The unsorted (BBHash) form's dedup: one CTA per group of up to 32
+// consecutive sub-buckets of a bin, whose level-0 slices (and level-1 slices)
+// are consecutive words.  The group's keys sit in the CTA's registers (GD_U
+// per thread) and are told apart by their BBHash bits instead of by a hash
+// set:
+//   1. every occurrence marks its level-0 bit (set; col when it was set
+//      already).  A bit set once is one occurrence of one key: distinct, and
+//      placed by level 0 -- ~88% of the occurrences of unrepeated sequence;
+//   2. the occurrences on a bit set more than once go to a list, and compare
+//      themselves with the first listed one of their bit (the bits numbered
+//      by a popcount of col, no probing): all equal -- copies of one key,
+//      placed, the first owning it and taking the OR of the copies' payload
+//      bytes -- or not: the bit is cleared and its occurrences go to level 1;
+//   3. those mark the group's level-1 slices the same way; the few that share
+//      a level-1 bit (~1%) are compared pairwise, and what level 1 does not
+//      place is listed for level 2.
+// Ranks are popcounts of the placed bits, and the placed keys' bytes leave in
+// rank order.  The keys stay where they are, packed: a bit per occurrence
+// (keep) marks the first copy of every key, and gd_compact_kernel makes the
+// dense array from them when one is asked for.  Nothing is written before the
+// whole group is known to fit; a group that does not (more than GD_MAXN
+// occurrences, long slices, lists too long) is untouched and listed in ov.
+//
+// A group of 32 because the split then needs five bits less (one pass up to 8
+// bits), and because the slices' scans and the barriers are shared by 32
+// sub-buckets: the same passes run by a warp on one sub-bucket of ~120 keys
+// were slower than the warp's hash set below (1 Gbp: 40 against 18 ms).
+// Instruction issue (65% of the slots) and its barriers bound it: ~226 warp
+// instructions per 32 occurrences where the hash set took ~430.  The dedup of
+// 200 Mbp went from 3.77 to 2.08 ms, of 1 Gbp (with tandem arrays) from 18.0
+// to 14.6 ms, of 5 Mbp from 632 to 76 us (the warp kernel's runs of 64
+// sub-buckets left most warps idle); with three occurrences of every key
+// (transcripts) the list is most of the group and it takes 0.81 against 0.59
+// ms, which the split's dropped pass (0.31 ms) makes up for.
+constexpr int GD_BLOCK = 512;
+constexpr int GD_U = 16;                           // keys per thread
+constexpr int GD_BITS = 5;                         // sub-buckets of a group (log2), at most
+constexpr uint32_t GD_MAXN = GD_BLOCK * GD_U;      // occurrences a group may hold
+constexpr uint32_t GD_SWMAX = 32;                  // level-0 words of a slice: one a lane
+constexpr uint32_t GD_WMAX = GD_SWMAX << GD_BITS;  // level-0 words of a group
+constexpr uint32_t GD_W1MAX = (GD_SWMAX / 8) << GD_BITS;  // level-1 words of a group
+constexpr uint32_t GD_MAXL = 5888;                 // occurrences on a level-0 bit set more than once
+constexpr uint32_t GD_MAXC = GD_BLOCK;             // occurrences on a level-1 bit set more than once
+constexpr uint32_t GD_PAIR = 4;                    // threads that compare one of those
+constexpr uint32_t GD_NONE = 0xFFFF, GD_OWN = 0x8000, GD_JOIN = 0x4000;
+struct GdSmem {
+  // cleared at the start, 16 bytes at a time
+  unsigned long long set[GD_WMAX], col[GD_WMAX];   // level 0: bits set (then: placed), bits set more than once
+  unsigned long long set1[GD_W1MAX], col1[GD_W1MAX];
+  uint32_t rp[GD_MAXL / 8];                        // payload bytes beside rk
+  uint32_t rk[GD_MAXL / 2];                        // first listed occurrence of a bit; then the byte stage
+  unsigned long long lk[GD_MAXL];                  // the list (PK: packed words)
+  unsigned long long cid[GD_MAXC];                 // ids of the entries in cq
+  uint32_t cpre[GD_WMAX], fpre[GD_WMAX];           // per half word (16 bits each): col / placed bits before it
+  uint32_t fpre1[GD_W1MAX];
+  uint32_t tot[1 << GD_BITS];                      // placed bits per slice
+  uint32_t cp[GD_MAXC];                            // payloads joined over a key's copies
+  // an entry's bit number (GD_OWN | number when its key is level 0's and it is
+  // the first), its level-1 bit when level 0 leaves it (GD_JOIN: its byte is
+  // in lp), or GD_NONE: a copy
+  uint16_t lx[GD_MAXL];
+  uint16_t cq[GD_MAXC], cb[GD_MAXC];               // entries on a level-1 bit set more than once, and that bit
+  uint8_t lp[GD_MAXL];                             // the list's payload bytes (PK: those joined at level 1)
+  uint8_t lut[64];                                 // payload code -> byte
+  uint32_t nlc, nc, kept, placed1;                 // nlc: list entries | bits set more than once << 16
+};
+static_assert(offsetof(GdSmem, set1) % 16 == 0 && offsetof(GdSmem, rk) % 16 == 0 && offsetof(GdSmem, rp) == offsetof(GdSmem, col1) + sizeof(GdSmem::col1), "cleared in one run");
+static_assert(sizeof(GdSmem) <= 113 * 1024, "two CTAs per SM");
+static_assert(GD_MAXN + 4 <= sizeof(GdSmem::rk), "the byte stage fits rk");
+static_assert(GD_W1MAX * 64 < GD_JOIN && GD_MAXL / 2 < GD_JOIN, "an entry's number, flags and level-1 bit fit 16 bits");
+
+// Popcount prefix of a thread's 64-bit word as its two half words' values
+// (low half first) in one u32.
+CF1_D uint32_t gd_halves(unsigned long long x, uint32_t pre) {
+  return pre | ((pre + (uint32_t)__popc((uint32_t)x)) << 16);
+}
+// A warp's exclusive prefix of v, and the sum.
+CF1_D uint32_t gd_warp_excl(uint32_t v, uint32_t &tot) {
+  const uint32_t x = warp_inclusive_scan(v);
+  tot = __shfl_sync(FULL, x, 31);
+  return x - v;
+}
+// First word of a unit's keep bits: the units' occurrences one after another,
+// every unit from a word of its own.
+CF1_D uint64_t gd_keep_word(uint64_t a, uint64_t q) { return (a >> 5) + q; }
+
+// PK: T holds packed words of a first pass of p1 bits (see pay_code); id(w)
+// = h = key * MS_HASH_MUL without its top p1 bits stands for the key, which
+// is h * KEY_SPREAD_INV.  Group q: bin q >> Pg, the keys whose hash's top Pg
+// bits are q mod 2^Pg, in T[goff[q], goff[q + 1]); it is sub-buckets
+// [q << g, (q + 1) << g), g = P - Pg.
+template <bool PK>
+__global__ void __launch_bounds__(GD_BLOCK, 2) gd_dedup_kernel(const uint64_t *T, const uint8_t *TP,
+                                                              const uint64_t *goff, int Pg, int P, uint32_t *cnt,
+                                                              uint32_t *keep, Level0Out l0, uint32_t *ov,
+                                                              uint32_t *ov_cnt, int p1) {
+  extern __shared__ __align__(16) unsigned char gd_smem[];
+  GdSmem &m = *reinterpret_cast<GdSmem *>(gd_smem);
+  constexpr uint32_t NW = GD_BLOCK / 32, SPW = (1u << GD_BITS) / NW;  // warps; slices a warp takes
+  const unsigned tid = threadIdx.x, lane = lane_id(), warp = tid >> 5;
+  const uint32_t q = blockIdx.x;
+  const uint64_t a = goff[q], n64 = goff[q + 1] - a;
+  const int g = P - Pg;
+  const uint32_t subs = 1u << g, bin = q >> Pg, gi = q & ((1u << Pg) - 1);
+  const bool pay = TP != nullptr, lv0 = l0.AR != nullptr, lpay = lv0 && l0.with_pay && pay;
+  uint32_t sw, sw1;
+  uint64_t first = 0, first1 = 0;
+  if (lv0) {
+    const uint64_t f0 = l0.woff[bin], f1 = l0.woff1[bin];
+    const uint64_t w0 = (l0.woff[bin + 1] - f0) >> P;
+    sw = w0 > GD_SWMAX ? GD_SWMAX + 1 : (uint32_t)w0;
+    sw1 = (sw + 7) / 8;  // as level 1 is sized
+    first = f0 + (uint64_t)(gi << g) * sw;
+    first1 = f1 + (uint64_t)(gi << g) * sw1;
+  } else {  // no levels wanted: the same bits, to tell the keys apart only
+    sw = (uint32_t)min((n64 + 8 * subs - 1) / (8 * subs), (uint64_t)GD_SWMAX);
+    sw1 = (sw + 7) / 8;
+  }
+  if (n64 > GD_MAXN || sw > GD_SWMAX) {
+    if (tid == 0) ov[atomicAdd(ov_cnt, 1u)] = q;
+    return;
+  }
+  const uint32_t n = (uint32_t)n64, gw = sw * subs, gw1 = sw1 * subs;
+  const uint64_t *Tk = T + a + tid;
+  unsigned long long key[GD_U];    // PK: the packed word
+  uint32_t pb[PK ? 1 : GD_U / 4];  // payload bytes, four to a register (PK: inside the word)
+  const uint32_t act = tid < n ? (0xFFFFFFFFu >> (31 - (n - 1 - tid) / GD_BLOCK)) : 0u;  // this thread's keys
+  if constexpr (!PK) {
+#pragma unroll
+    for (int i = 0; i < GD_U / 4; i++) pb[i] = 0;
+  }
+#pragma unroll
+  for (int u = 0; u < GD_U; u++) {
+    key[u] = 0;
+    if (u * GD_BLOCK < n && ((act >> u) & 1)) {  // the first test is uniform, as in every loop over u
+      key[u] = Tk[u * GD_BLOCK];
+      if constexpr (!PK)
+        if (pay) pb[u >> 2] |= (uint32_t)TP[a + tid + u * GD_BLOCK] << (8 * (u & 3));
+    }
+  }
+  if (tid < 64) m.lut[tid] = (uint8_t)pay_byte(tid);
+  if (tid == 0) m.nlc = m.nc = m.kept = 0;
+  {
+    const uint4 z = make_uint4(0, 0, 0, 0), o = make_uint4(~0u, ~0u, ~0u, ~0u);
+    uint4 *s4 = reinterpret_cast<uint4 *>(m.set), *c4 = reinterpret_cast<uint4 *>(m.col);
+    for (uint32_t w = tid; 2 * w < gw; w += GD_BLOCK) s4[w] = c4[w] = z;
+    uint4 *z4 = reinterpret_cast<uint4 *>(m.set1), *r4 = reinterpret_cast<uint4 *>(m.rk);
+    constexpr uint32_t NZ = (2 * sizeof(m.set1) + sizeof(m.rp)) / 16;
+    for (uint32_t w = tid; w < NZ; w += GD_BLOCK) z4[w] = z;
+    for (uint32_t w = tid; w < sizeof(m.rk) / 16; w += GD_BLOCK) r4[w] = o;
+  }
+  const uint64_t hi = PK ? (uint64_t)(gi >> (Pg - p1)) << (64 - p1) : 0;
+  const uint32_t lowP = Pg ? ~((1u << Pg) - 1) : 0xFFFFFFFFu, scale = gw << 6;
+  auto id = [&](unsigned long long w) -> unsigned long long { return PK ? w >> p1 : w; };
+  auto key_of = [&](unsigned long long w) -> uint64_t { return PK ? (hi | (w >> p1)) * KEY_SPREAD_INV : w; };
+  auto pay_of = [&](int u) -> uint32_t {
+    if constexpr (PK) return (uint32_t)m.lut[(uint32_t)key[u] & 63u];
+    else return (pb[u >> 2] >> (8 * (u & 3))) & 0xFFu;
+  };
+  auto list_pay = [&](unsigned long long w, uint32_t i) -> uint32_t {
+    return PK ? (uint32_t)m.lut[(uint32_t)w & 63u] : (uint32_t)m.lp[i];
+  };
+  // the key's level-0 bit in the group: its 32-bit hash scaled to the bin's
+  // sw * 2^P words, minus the group's start, which is the hash without its
+  // top Pg bits scaled to the group's words (exactly: the dropped bits' share
+  // is a whole number of slices)
+  auto bit_of = [&](unsigned long long w) -> uint32_t {
+    const uint32_t x = PK ? (uint32_t)((w << (Pg - p1)) >> 32) & lowP : (uint32_t)((w * MS_HASH_MUL) >> 32) << Pg;
+    return __umulhi(x, scale);
+  };
+  uint32_t *set32 = reinterpret_cast<uint32_t *>(m.set), *col32 = reinterpret_cast<uint32_t *>(m.col);
+  uint32_t *set1w = reinterpret_cast<uint32_t *>(m.set1), *col1w = reinterpret_cast<uint32_t *>(m.col1);
+  const uint16_t *cpre = reinterpret_cast<const uint16_t *>(m.cpre), *fpre = reinterpret_cast<const uint16_t *>(m.fpre),
+                 *fpre1 = reinterpret_cast<const uint16_t *>(m.fpre1);
+  __syncthreads();
+  // 1. mark
+  bool hit = false;
+#pragma unroll
+  for (int u = 0; u < GD_U; u++) {
+    if (u * GD_BLOCK < n && ((act >> u) & 1)) {
+      const uint32_t b = bit_of(key[u]), bm = 1u << (b & 31);
+      if (atomicOr(&set32[b >> 5], bm) & bm) {
+        hit = true;
+        atomicOr(&col32[b >> 5], bm);
+      }
+    }
+  }
+  uint32_t cont = 0, k0 = 0;  // this thread's keys on a bit set more than once, and the first one's list entry
+  uint32_t nl = 0;
+  if (__syncthreads_or((int)hit)) {
+    // 2. the list, and the numbers of those bits (a warp a slice, one
+    //    reservation each)
+#pragma unroll
+    for (int u = 0; u < GD_U; u++) {
+      if (u * GD_BLOCK < n) {  // (lanes past the end test word 0; act drops them)
+        const uint32_t b = bit_of(key[u]);
+        cont |= ((col32[b >> 5] >> (b & 31)) & 1u) << u;
+      }
+    }
+    cont &= act;
+    // one reservation a warp: its list entries and its slices' bits
+    unsigned long long x[SPW];
+    uint32_t v = (uint32_t)__popc(cont), e[SPW];
+#pragma unroll
+    for (uint32_t r = 0; r < SPW; r++) {
+      const uint32_t sl = warp + r * NW;
+      x[r] = sl < subs && lane < sw ? m.col[sl * sw + lane] : 0ull;
+      e[r] = (uint32_t)__popcll(x[r]);
+    }
+    static_assert(SPW == 2, "two slices a warp: one scan with the list, one of its own");
+    uint32_t t0, t1;
+    const uint32_t e0 = gd_warp_excl(v | (e[0] << 16), t0), e1 = gd_warp_excl(e[1], t1);
+    uint32_t base = 0;
+    if (lane == 0 && (t0 | t1)) base = atomicAdd(&m.nlc, t0 + (t1 << 16));
+    base = __shfl_sync(FULL, base, 0);
+    k0 = (base & 0xFFFFu) + (e0 & 0xFFFFu);
+    if (k0 + v <= GD_MAXL) {
+      unsigned long long *lk = m.lk + k0;
+#pragma unroll
+      for (int u = 0; u < GD_U; u++) {
+        const bool c = (cont >> u) & 1;
+        if (c) *lk = key[u];
+        if constexpr (!PK)
+          if (c) m.lp[lk - m.lk] = (uint8_t)pay_of(u);
+        lk += c;
+      }
+    }
+    if (lane < sw) {
+      const uint32_t c0 = base >> 16;
+      if (warp < subs) m.cpre[warp * sw + lane] = gd_halves(x[0], c0 + (e0 >> 16));
+      if (warp + NW < subs) m.cpre[(warp + NW) * sw + lane] = gd_halves(x[1], c0 + (t0 >> 16) + e1);
+    }
+    __syncthreads();
+    nl = m.nlc & 0xFFFFu;
+    if (nl > GD_MAXL) {  // uniform; nothing of the group was written
+      if (tid == 0) ov[atomicAdd(ov_cnt, 1u)] = q;
+      return;
+    }
+    for (uint32_t i = tid; i < nl; i += GD_BLOCK) {
+      const unsigned long long w = m.lk[i];
+      const uint32_t b = bit_of(w), bm = 1u << (b & 31);
+      const uint32_t c = cpre[b >> 5] + (uint32_t)__popc(col32[b >> 5] & (bm - 1));  // below nl / 2
+      m.lx[i] = (uint16_t)c;
+      atomicMin(&m.rk[c], i);
+      if (pay) atomicOr(&m.rp[c >> 2], list_pay(w, i) << (8 * (c & 3)));
+    }
+    __syncthreads();
+    bool lbad = false;
+    for (uint32_t i = tid; i < nl; i += GD_BLOCK) {
+      const unsigned long long w = m.lk[i];
+      const uint32_t f = m.rk[m.lx[i]];
+      if (f != i && id(m.lk[f]) != id(w)) {
+        const uint32_t b = bit_of(w);
+        atomicAnd(&set32[b >> 5], ~(1u << (b & 31)));
+        lbad = true;
+      }
+    }
+    const bool anybad = __syncthreads_or((int)lbad) != 0;
+    // 3. level 1
+    bool hit1 = false;
+    for (uint32_t i = tid; i < nl; i += GD_BLOCK) {
+      const unsigned long long w = m.lk[i];
+      const uint32_t b = bit_of(w);
+      if (!anybad || ((set32[b >> 5] >> (b & 31)) & 1)) {
+        const uint32_t c = m.lx[i];
+        m.lx[i] = (uint16_t)(m.rk[c] == i ? GD_OWN | c : GD_NONE);
+      } else {  // its bit there, from its own hash in its slice
+        const uint32_t x = (uint32_t)((PK ? hi | (w >> p1) : w * MS_HASH_MUL) >> 32) << Pg;
+        const uint32_t b1 = (g ? (x >> (32 - g)) * (sw1 << 6) : 0u) + bb_slice_pos(key_of(w), 1, sw1);
+        const uint32_t bm1 = 1u << (b1 & 31);
+        m.lx[i] = (uint16_t)b1;
+        if (atomicOr(&set1w[b1 >> 5], bm1) & bm1) {
+          hit1 = true;
+          atomicOr(&col1w[b1 >> 5], bm1);
+        }
+      }
+    }
+    if (anybad && __syncthreads_or((int)hit1)) {
+      // the few occurrences on a level-1 bit set more than once, pairwise
+      for (uint32_t i = tid; i < nl; i += GD_BLOCK) {
+        const uint32_t b1 = m.lx[i];
+        if (b1 < GD_OWN && ((col1w[b1 >> 5] >> (b1 & 31)) & 1)) {
+          const uint32_t o = atomicAdd(&m.nc, 1u);
+          if (o < GD_MAXC) {
+            const unsigned long long w = m.lk[i];
+            m.cq[o] = (uint16_t)i;
+            m.cb[o] = (uint16_t)b1;
+            m.cid[o] = id(w);
+            m.cp[o] = pay ? list_pay(w, i) : 0u;
+          }
+        }
+      }
+      __syncthreads();
+      const uint32_t nc = m.nc;
+      if (nc > GD_MAXC) {
+        if (tid == 0) ov[atomicAdd(ov_cnt, 1u)] = q;
+        return;
+      }
+      // (GD_PAIR threads an entry while there are enough)
+      const uint32_t per = nc <= GD_BLOCK / GD_PAIR ? GD_PAIR : 1u, c = tid / per;
+      unsigned long long v = 0;
+      uint32_t b1 = GD_NONE, lead = GD_MAXC;  // the first copy of the entry's key
+      bool bad = false;
+      if (c < nc) {
+        v = m.cid[c];
+        b1 = m.cb[c];
+        for (uint32_t j = tid % per; j < nc; j += per) {
+          const bool on = m.cb[j] == b1, same = m.cid[j] == v;  // (equal keys have equal bits)
+          bad |= on && !same;
+          if (same) lead = min(lead, j);
+        }
+      }
+      if (per > 1) {
+#pragma unroll
+        for (uint32_t o = 1; o < GD_PAIR; o <<= 1) {
+          lead = min(lead, __shfl_xor_sync(FULL, lead, o));
+          bad |= __shfl_xor_sync(FULL, (int)bad, o) != 0;
+        }
+      }
+      if (c < nc && tid % per == 0) {
+        if (bad) atomicAnd(&set1w[b1 >> 5], ~(1u << (b1 & 31)));
+        if (lead != c) {
+          atomicOr(&m.cp[lead], m.cp[c]);
+          m.lx[m.cq[c]] = GD_NONE;
+        } else {
+          m.lx[m.cq[c]] = (uint16_t)(b1 | GD_JOIN);
+        }
+      }
+      __syncthreads();
+      // a key's first copy takes its copies' payloads
+      if (tid < nc) m.lp[m.cq[tid]] = (uint8_t)m.cp[tid];
+    }
+  }
+  // 4. the slices, with the placed bits of the slice before each word (a warp
+  //    two slices, then the slices' bases)
+  unsigned long long fin[SPW];
+  uint32_t loc[SPW], st1 = 0;
+  {
+#pragma unroll
+    for (uint32_t r = 0; r < SPW; r++) {
+      const uint32_t sl = warp + r * NW;
+      fin[r] = sl < subs && lane < sw ? m.set[sl * sw + lane] : 0ull;
+    }
+    uint32_t tot;
+    const uint32_t e = gd_warp_excl((uint32_t)__popcll(fin[0]) | ((uint32_t)__popcll(fin[1]) << 16), tot);
+    loc[0] = e & 0xFFFFu;
+    loc[1] = e >> 16;
+    if (lane == 0) {
+      m.tot[warp] = tot & 0xFFFFu;
+      m.tot[warp + NW] = tot >> 16;
+    }
+    if (lv0 && lane < sw) {
+#pragma unroll
+      for (uint32_t r = 0; r < SPW; r++) {
+        const uint32_t sl = warp + r * NW;
+        if (sl < subs) l0.AR[first + sl * sw + lane] = make_ulonglong2(fin[r], (unsigned long long)loc[r]);
+      }
+    }
+    if (warp == NW - 1 && lane < subs)  // level 1: a slice a lane, its few words one after another
+      for (uint32_t w = 0; w < sw1; w++) {
+        const unsigned long long x = m.set1[lane * sw1 + w];
+        if (lv0) l0.AR1[first1 + lane * sw1 + w] = make_ulonglong2(x, (unsigned long long)st1);
+        m.fpre1[lane * sw1 + w] = gd_halves(x, st1);
+        st1 += (uint32_t)__popcll(x);
+      }
+  }
+  __syncthreads();
+  const uint32_t st = m.tot[lane];
+  uint32_t placed;
+  const uint32_t sbase = gd_warp_excl(st, placed);
+#pragma unroll
+  for (uint32_t r = 0; r < SPW; r++) {
+    const uint32_t sl = warp + r * NW, base = __shfl_sync(FULL, sbase, sl & 31);
+    if (sl < subs && lane < sw) m.fpre[sl * sw + lane] = gd_halves(fin[r], base + loc[r]);
+  }
+  if (warp == NW - 1) {
+    uint32_t p1s;
+    const uint32_t sb1 = placed + gd_warp_excl(st1, p1s);  // level 1's bytes follow level 0's
+    if (lane < subs) {
+      for (uint32_t w = 0; w < sw1; w++) m.fpre1[lane * sw1 + w] += sb1 * 0x10001u;
+      if (lv0) {
+        const uint64_t j = ((uint64_t)q << g) + lane;
+        l0.placed[j] = st;
+        l0.placed1[j] = st1;
+      }
+    }
+    if (lane == 0) {
+      m.placed1 = p1s;
+      if (lv0) {
+        l0.uplaced[q] = placed;
+        l0.uplaced1[q] = p1s;
+      }
+    }
+  }
+  __syncthreads();
+  const uint32_t placed1 = m.placed1;
+  // 5. the first copy of every key kept; each placed key's byte to its rank in
+  //    the stage (rk's area: its last use was before the last barriers)
+  //    from its alignment in l0pay on
+  const uint32_t al = (uint32_t)(a & 3);
+  uint8_t *stage = reinterpret_cast<uint8_t *>(m.rk) + al;
+  uint32_t km = act;
+  for (uint32_t t = cont; t; t &= t - 1)
+    if (m.lx[k0++] == GD_NONE) km &= ~(t & (0u - t));
+  uint32_t word = 0;  // lane u < GD_U: the warp's keep bits of row u
+#pragma unroll
+  for (int u = 0; u < GD_U; u++) {
+    if (u * GD_BLOCK < n) {
+      const unsigned bal = __ballot_sync(FULL, (km >> u) & 1);
+      if (lane == u) word = bal;
+      if (lpay && (((act & ~cont) >> u) & 1)) {
+        const uint32_t b = bit_of(key[u]), bm = 1u << (b & 31);
+        stage[fpre[b >> 5] + (uint32_t)__popc(set32[b >> 5] & (bm - 1))] = (uint8_t)pay_of(u);
+      }
+    }
+  }
+  if (lane < GD_U && word) keep[gd_keep_word(a, q) + lane * NW + warp] = word;
+  const uint32_t kept = __reduce_add_sync(FULL, (uint32_t)__popc(km));
+  if (lane == 0 && kept) atomicAdd(&m.kept, kept);
+  for (uint32_t i = tid; i < nl; i += GD_BLOCK) {
+    const uint32_t x = m.lx[i];
+    if (x == GD_NONE) continue;
+    const unsigned long long w = m.lk[i];
+    if (x & GD_OWN) {
+      const uint32_t b = bit_of(w), bm = 1u << (b & 31);
+      if (lpay)
+        stage[fpre[b >> 5] + (uint32_t)__popc(set32[b >> 5] & (bm - 1))] =
+            reinterpret_cast<const uint8_t *>(m.rp)[x & (GD_OWN - 1)];
+    } else {
+      const uint32_t b1 = x & (GD_JOIN - 1), bm1 = 1u << (b1 & 31), f = set1w[b1 >> 5];
+      const uint8_t p = (x & GD_JOIN) ? m.lp[i] : (uint8_t)list_pay(w, i);
+      if (f & bm1) {
+        if (lpay) stage[fpre1[b1 >> 5] + (uint32_t)__popc(f & (bm1 - 1))] = p;
+      } else if (lv0) {  // to the bin's level-2 list
+        const unsigned long long o = atomicAdd(&l0.surv_cnt[bin], 1ull), s0 = l0.surv_off[bin];
+        if (o < l0.surv_off[bin + 1] - s0) {
+          l0.surv[s0 + o] = key_of(w);
+          if (lpay) l0.surv_pay[s0 + o] = p;
+        } else {
+          atomicOr(l0.err, 1u);
+        }
+      }
+    }
+  }
+  __syncthreads();
+  if (tid == 0) cnt[q] = m.kept;
+  if (lpay) {
+    const uint32_t e = al + placed + placed1;  // bytes [al, e) of the words from a's
+    uint8_t *out = l0.l0pay + (a - al);
+    for (uint32_t w = tid; 4 * w < e; w += GD_BLOCK) {
+      if (4 * w >= al && 4 * w + 4 <= e) reinterpret_cast<uint32_t *>(out)[w] = m.rk[w];
+      else
+        for (uint32_t i = max(4 * w, al); i < min(4 * w + 4, e); i++) out[i] = stage[i - al];
+    }
+  }
+}
+
+// Groups the dedup left: one CTA per listed group moves its keys (unpacked)
+// and bytes from T / TP to the same range of U / UP, sub-bucket by
+// sub-bucket, and writes the sub-buckets' offsets and list entries for the
+// block kernel.
+__global__ void __launch_bounds__(GD_BLOCK) gd_split_kernel(const uint64_t *T, const uint8_t *TP, const uint64_t *goff,
+                                                           const uint32_t *ov, int Pg, int P, int p1, uint64_t *U,
+                                                           uint8_t *UP, uint64_t *sb_off, uint32_t *jlist) {
+  __shared__ unsigned long long s_cnt[1 << GD_BITS], s_cur[1 << GD_BITS];
+  const uint64_t q = ov[blockIdx.x], a = goff[q], e = goff[q + 1];
+  const int g = P - Pg;
+  const uint32_t subs = 1u << g, gi = (uint32_t)(q & ((1ull << Pg) - 1));
+  const uint64_t hi = p1 ? (uint64_t)(gi >> (Pg - p1)) << (64 - p1) : 0;
+  const unsigned tid = threadIdx.x;
+  auto hash = [&](uint64_t x) -> uint64_t { return p1 ? hi | (x >> p1) : x * MS_HASH_MUL; };
+  auto sub = [&](uint64_t h) -> uint32_t { return g ? (uint32_t)(h >> (64 - P)) & (subs - 1) : 0u; };
+  if (tid < subs) s_cnt[tid] = 0;
+  __syncthreads();
+  for (uint64_t i = a + tid; i < e; i += GD_BLOCK) atomicAdd(&s_cnt[sub(hash(T[i]))], 1ull);
+  __syncthreads();
+  if (tid == 0) {
+    uint64_t run = a;
+    for (uint32_t s = 0; s < subs; s++) {
+      s_cur[s] = run;
+      sb_off[(q << g) + s] = run;
+      jlist[((uint64_t)blockIdx.x << g) + s] = (uint32_t)((q << g) + s);
+      run += s_cnt[s];
+    }
+    sb_off[(q + 1) << g] = run;  // the next group's start: the same value if that group is listed too
+  }
+  __syncthreads();
+  for (uint64_t i = a + tid; i < e; i += GD_BLOCK) {
+    const uint64_t x = T[i], h = hash(x), o = atomicAdd(&s_cur[sub(h)], 1ull);
+    U[o] = p1 ? h * KEY_SPREAD_INV : x;
+    if (UP) UP[o] = p1 ? (uint8_t)pay_byte((uint32_t)x) : TP[i];
+  }
+}
+
+// The listed groups' results back in the groups' form, one CTA each: the
+// distinct keys the block kernel left at the sub-buckets' starts in U to the
+// group's start in T (packed again when T is: p1), all of them kept, and the
+// placed bytes it left in lp -- level 0's, then level 1's, sub-bucket by
+// sub-bucket -- to l0pay.
+__global__ void __launch_bounds__(GD_BLOCK) gd_gather_kernel(const uint64_t *U, const uint8_t *lp, const uint64_t *goff,
+                                                            const uint32_t *ov, int g, const uint64_t *sb_off,
+                                                            const uint32_t *scnt, uint64_t *T, uint32_t *cnt,
+                                                            uint32_t *keep, Level0Out l0, int p1) {
+  const uint64_t q = ov[blockIdx.x], a0 = goff[q];
+  uint64_t o = a0;
+  for (uint64_t j = q << g; j < (q + 1) << g; j++) {
+    const uint32_t c = scnt[j];
+    const uint64_t a = sb_off[j];
+    for (uint32_t i = threadIdx.x; i < c; i += GD_BLOCK) T[o + i] = p1 ? (U[a + i] * MS_HASH_MUL) << p1 : U[a + i];
+    o += c;
+  }
+  const uint64_t d = o - a0;
+  if (threadIdx.x == 0) cnt[q] = (uint32_t)d;
+  uint32_t *kw = keep + gd_keep_word(a0, q);
+  for (uint64_t w = threadIdx.x; w * 32 < d; w += GD_BLOCK)
+    kw[w] = d - w * 32 >= 32 ? 0xFFFFFFFFu : (1u << (d - w * 32)) - 1;
+  if (!l0.AR) return;
+  o = a0;
+  for (int l = 0; l < 2; l++) {
+    const uint64_t start = o;
+    for (uint64_t j = q << g; j < (q + 1) << g; j++) {
+      const uint32_t c = l ? l0.placed1[j] : l0.placed[j];
+      const uint64_t a = sb_off[j] + (l ? l0.placed[j] : 0u);
+      if (lp)
+        for (uint32_t i = threadIdx.x; i < c; i += GD_BLOCK) l0.l0pay[o + i] = lp[a + i];
+      o += c;
+    }
+    if (threadIdx.x == 0) (l ? l0.uplaced1 : l0.uplaced)[q] = (uint32_t)(o - start);
+  }
+}
+
+// The dense array of the kept keys, one warp per group.
+__global__ void __launch_bounds__(256) gd_compact_kernel(const uint64_t *T, const uint64_t *goff, const uint32_t *keep,
+                                                        const uint64_t *out_off, uint64_t nunit, int Pg, int p1,
+                                                        uint64_t *dist) {
+  const uint64_t q = ((uint64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
+  if (q >= nunit) return;
+  const uint64_t a = goff[q], n = goff[q + 1] - a, hi = p1 ? ((q & ((1ull << Pg) - 1)) >> (Pg - p1)) << (64 - p1) : 0;
+  const uint32_t *kw = keep + gd_keep_word(a, q);
+  const unsigned lane = lane_id(), lt = lanemask_lt();
+  uint64_t o = out_off[q];
+  for (uint64_t i = 0; i < n; i += 32) {
+    const uint32_t k = kw[i >> 5];
+    if ((k >> lane) & 1) {
+      const uint64_t x = T[a + i + lane];
+      dist[o + __popc(k & lt)] = p1 ? (hi | (x >> p1)) * KEY_SPREAD_INV : x;
+    }
+    o += __popc(k);
+  }
+}
+
 // ---------------------------------------------------------------- warp dedup
-// The unsorted (BBHash) form's dedup, one warp per sub-bucket and no block
+// The unsorted (BBHash) form's dedup where sub-buckets are larger than the
+// width rule's (bins above 12.5 M keys, whose split is capped at 16 bits, or
+// a narrower split from the autotuner): one warp per sub-bucket and no block
 // barriers: sub-buckets of a few hundred keys (the split of key *
 // KEY_SPREAD_MUL spreads them evenly), a private 512-slot open-addressing set
 // per warp in shared memory, and, with level 0 on, the sub-bucket's slice of
@@ -1186,6 +1742,15 @@ void subbuckets_bits(int bits, const uint64_t *seg_off, const uint32_t *tile_off
 template <class KeyT>
 void msd_compact(const KeyT *kept, uint64_t nsub, KeyT *dist, MsdScratch &sc, cudaStream_t s) {
   if (!nsub) return;
+  if constexpr (KOps<KeyT>::WORDS == 1) {
+    if (sc.kept_bits) {
+      gd_compact_kernel<<<(unsigned)ceil_div(nsub * 32, 256), 256, 0, s>>>(
+          kept, sc.sb_off.as<const uint64_t>(), sc.keep.as<const uint32_t>(), sc.out_off.as<const uint64_t>(), nsub,
+          sc.unit_bits, sc.kept_packed, dist);
+      CF1_LAUNCH_CHECK();
+      return;
+    }
+  }
   cs_compact_kernel<KeyT><<<(unsigned)ceil_div(nsub * 32, 256), 256, 0, s>>>(
       kept, sc.sb_off.as<const uint64_t>(), sc.cnt.as<const uint32_t>(), sc.out_off.as<const uint64_t>(), nsub, dist);
   CF1_LAUNCH_CHECK();
@@ -1207,8 +1772,8 @@ int msd_prefix_bits(uint64_t max_bin_keys, bool sorted) {
 }
 
 template <class KeyT>
-bool msd_sort_unique(KeyT *keys, KeyT *alt, uint64_t n, const uint64_t *seg_off, uint32_t nbins, int key_bits, int P,
-                     KeyT *dist, uint64_t *dist_off, MsdScratch &sc, cudaStream_t s, bool sorted,
+bool msd_sort_unique(KeyT *keys, KeyT *alt, uint64_t n, uint64_t max_bin, const uint64_t *seg_off, uint32_t nbins,
+                     int key_bits, int P, KeyT *dist, uint64_t *dist_off, MsdScratch &sc, cudaStream_t s, bool sorted,
                      const Level0Out *l0, KeyT **kept, uint8_t *pkeys, uint8_t *palt, uint8_t **kept_pay,
                      uint8_t **l0pay_buf) {
   uint8_t *PT = pkeys;  // payloads beside T (nullptr: keys carry none)
@@ -1218,14 +1783,23 @@ bool msd_sort_unique(KeyT *keys, KeyT *alt, uint64_t n, const uint64_t *seg_off,
   if (hashed) key_bits = 64;
   // packed passes (see pay_code): the hashed split of keys with payloads
   // whose dedup builds BBHash level 0, with a first pass of >= 6 bits
-  const bool pk = hashed && pkeys && palt && l0 && l0->AR && l0->with_pay && P >= (int)PACK_MIN_BITS;
-  int P1 = P > 8 ? (P + 1) / 2 : P;
+  // Groups of 32 sub-buckets for the group dedup (gd_dedup_kernel), split on
+  // the bits above theirs only, as long as the width rule's aim holds for the
+  // largest bin: 32 sub-buckets of at most WD_MAXD / 2 keys are 6144 of the
+  // group's GD_MAXN.
+  const bool grp = hashed && (max_bin >> P) <= WD_MAXD / 2;
+  const int g = grp ? (P < GD_BITS ? P : GD_BITS) : 0;
+  const int PS = P - g;  // bits split on: a unit is a group, or a sub-bucket
+  sc.unit_bits = PS;
+  sc.kept_bits = false;
+  const bool pk = hashed && pkeys && palt && l0 && l0->AR && l0->with_pay && PS >= (int)PACK_MIN_BITS;
+  int P1 = PS > 8 ? (PS + 1) / 2 : PS;
   if (pk && P1 < (int)PACK_MIN_BITS) P1 = PACK_MIN_BITS;
-  const int P2 = P - P1;
+  const int P2 = PS - P1;
   KeyT *T = keys;
-  uint64_t nsub = (uint64_t)nbins << P;
-  uint64_t *sb_off = sc.sb_off.get<uint64_t>(nsub + 1);
-  if (P == 0) {
+  const uint64_t nsub = (uint64_t)nbins << P, nunit = (uint64_t)nbins << PS;
+  uint64_t *sb_off = sc.sb_off.get<uint64_t>(nunit + 1);  // the units' offsets
+  if (PS == 0) {
     CF1_CUDA(cudaMemcpyAsync(sb_off, seg_off, (nbins + 1) * sizeof(uint64_t), cudaMemcpyDeviceToDevice, s));
   } else if (n) {
     ms_pass_bits<KeyT>(P1, keys, alt, n, seg_off, nbins, key_bits - P1, hashed, sc, s, pkeys, pk ? nullptr : palt,
@@ -1250,9 +1824,9 @@ bool msd_sort_unique(KeyT *keys, KeyT *alt, uint64_t n, const uint64_t *seg_off,
     }
     subbuckets_bits(P2 ? P2 : P1, seg2, sc.tile_off.as<uint32_t>(), nseg2, sc.hscan.as<uint64_t>(), sb_off, s);
   } else {
-    CF1_CUDA(cudaMemsetAsync(sb_off, 0, (nsub + 1) * sizeof(uint64_t), s));
+    CF1_CUDA(cudaMemsetAsync(sb_off, 0, (nunit + 1) * sizeof(uint64_t), s));
   }
-  uint32_t *cnt = sc.cnt.get<uint32_t>(nsub + 1);
+  uint32_t *cnt = sc.cnt.get<uint32_t>(nunit + 1);
   uint32_t *over = sc.flag.get<uint32_t>(1);
   CF1_CUDA(cudaMemsetAsync(over, 0, 4, s));
   int rest = key_bits - P;
@@ -1304,7 +1878,45 @@ bool msd_sort_unique(KeyT *keys, KeyT *alt, uint64_t n, const uint64_t *seg_off,
       coff = co;
     }
     CF1_CUDA(cudaEventRecord(sc.ev[0], s));
-    if (hashed) {
+    if (grp) {
+      // one CTA per group; the groups it cannot hold go to the block kernel
+      // sub-bucket by sub-bucket, through the free buffers
+      uint32_t *ov = sc.ov.get<uint32_t>(nunit + 1);
+      uint32_t *ovc = sc.ovc.get<uint32_t>(2);
+      CF1_CUDA(cudaMemsetAsync(ovc, 0, sizeof(uint32_t), s));
+      auto gkern = pk ? gd_dedup_kernel<true> : gd_dedup_kernel<false>;
+      CF1_CUDA(cudaFuncSetAttribute(gkern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(GdSmem)));
+      uint64_t *T64 = reinterpret_cast<uint64_t *>(T), *U64 = reinterpret_cast<uint64_t *>(U);
+      // a bit per occurrence: the first copy of its key (words of groups
+      // that keep nothing there stay 0)
+      const uint64_t nkeep = n / 32 + nunit + 1;
+      uint32_t *keep = sc.keep.get<uint32_t>(nkeep);
+      CF1_CUDA(cudaMemsetAsync(keep, 0, nkeep * sizeof(uint32_t), s));
+      const int p1 = pk ? P1 : 0;
+      gkern<<<(unsigned)nunit, GD_BLOCK, sizeof(GdSmem), s>>>(T64, PT, sb_off, PS, P, cnt, keep, lo, ov, ovc, p1);
+      CF1_LAUNCH_CHECK();
+      uint32_t h_ov = 0;
+      CF1_CUDA(cudaMemcpyAsync(&h_ov, ovc, sizeof(uint32_t), cudaMemcpyDeviceToHost, s));
+      CF1_CUDA(cudaStreamSynchronize(s));
+      const unsigned nov = h_ov << g;  // sub-buckets
+      sc.last_overflow = nov;
+      sc.kept_packed = p1;
+      sc.kept_bits = true;
+      if (h_ov) {
+        uint64_t *sub_off = sc.sub_off.get<uint64_t>(nsub + 1);
+        uint32_t *scnt = sc.sub_cnt.get<uint32_t>(nsub + 1), *jl = sc.jlist.get<uint32_t>(nov);
+        Level0Out lb = lo;
+        if (lo.with_pay) lb.l0pay = sc.ov_pay.get<uint8_t>(n + 16);
+        gd_split_kernel<<<h_ov, GD_BLOCK, 0, s>>>(T64, PT, sb_off, ov, PS, P, p1, U64, PU, sub_off, jl);
+        CF1_LAUNCH_CHECK();
+        kern<<<nov, CS_BLOCK, smem, s>>>(U, T, sub_off, nsub, shift, rest > 0 ? bits : 0, scnt, over, P, lb, PU, PT,
+                                         nullptr, nullptr, nbins, jl);
+        CF1_LAUNCH_CHECK();
+        gd_gather_kernel<<<h_ov, GD_BLOCK, 0, s>>>(U64, lo.with_pay ? lb.l0pay : nullptr, sb_off, ov, g, sub_off, scnt,
+                                                   T64, cnt, keep, lo, p1);
+        CF1_LAUNCH_CHECK();
+      }
+    } else if (hashed) {
       // the unsorted form: one warp per sub-bucket; the few it cannot hold
       // (more than WD_MAXD distinct keys) go to the block kernel after it
       uint32_t *ov = sc.ov.get<uint32_t>(nsub + 1);
@@ -1344,20 +1956,20 @@ bool msd_sort_unique(KeyT *keys, KeyT *alt, uint64_t n, const uint64_t *seg_off,
   sc.ms_dedup = 0;
   if (nsub) CF1_CUDA(cudaEventElapsedTime(&sc.ms_dedup, sc.ev[0], sc.ev[1]));
   if (h_over) return false;
-  uint64_t *out_off = sc.out_off.get<uint64_t>(nsub + 1);
-  exclusive_scan_u32(cnt, out_off, nsub, sc.scan_tmp, s);
+  uint64_t *out_off = sc.out_off.get<uint64_t>(nunit + 1);
+  exclusive_scan_u32(cnt, out_off, nunit, sc.scan_tmp, s);
   if (kept) *kept = T;
-  if (kept_pay) *kept_pay = PT;
-  if (dist) msd_compact<KeyT>(T, nsub, dist, sc, s);
-  cs_bin_off_kernel<<<(unsigned)ceil_div(nbins + 1, 256), 256, 0, s>>>(out_off, nbins, 1ull << P, dist_off);
+  if (kept_pay) *kept_pay = grp ? nullptr : PT;
+  if (dist) msd_compact<KeyT>(T, nunit, dist, sc, s);
+  cs_bin_off_kernel<<<(unsigned)ceil_div(nbins + 1, 256), 256, 0, s>>>(out_off, nbins, 1ull << PS, dist_off);
   CF1_LAUNCH_CHECK();
   return true;
 }
 
 #define CF1_INST(KT)                                                                                              \
   template int msd_prefix_bits<KT>(uint64_t, bool);                                                                     \
-  template bool msd_sort_unique<KT>(KT *, KT *, uint64_t, const uint64_t *, uint32_t, int, int, KT *, uint64_t *, \
-                                    MsdScratch &, cudaStream_t, bool, const Level0Out *, KT **, uint8_t *,    \
+  template bool msd_sort_unique<KT>(KT *, KT *, uint64_t, uint64_t, const uint64_t *, uint32_t, int, int, KT *,   \
+                                    uint64_t *, MsdScratch &, cudaStream_t, bool, const Level0Out *, KT **, uint8_t *, \
                                     uint8_t *, uint8_t **, uint8_t **);                                       \
   template void msd_compact<KT>(const KT *, uint64_t, KT *, MsdScratch &, cudaStream_t);
 CF1_INST(uint64_t)

@@ -7,7 +7,18 @@ namespace cf1 {
 
 struct MsdScratch {
   DevBuf tile_off, hist, hscan, scan_tmp, sb_off, sb_off1, cnt, out_off, flag, clist, ccount, coff, ov, ovc;
+  // groups the group dedup left: their sub-buckets' offsets, counts, list and placed bytes
+  DevBuf sub_off, sub_cnt, jlist, ov_pay;
   uint32_t last_overflow = 0;  // sub-buckets the last unsorted run left to the block kernel
+  // The last run's units, 2^unit_bits per bin: what sb_off, cnt and out_off
+  // have one entry for.  A unit is a sub-bucket, or a group of sub-buckets
+  // (unsorted form, group dedup).
+  int unit_bits = 0;
+  // Group dedup: the kept keys are the occurrences with a bit in keep, still
+  // words of a first pass of kept_packed bits (0: plain keys).
+  bool kept_bits = false;
+  int kept_packed = 0;
+  DevBuf keep;
   cudaEvent_t ev[2] = {nullptr, nullptr};  // around the last dedup kernel launch
   float ms_dedup = 0;                      // its device time
   ~MsdScratch() {
@@ -61,23 +72,29 @@ struct Level0Out {
   bool with_pay = false;
   uint8_t *l0pay = nullptr;    // filled by msd_sort_unique: the payload buffer the kept bytes are not in
   uint8_t *surv_pay = nullptr; // beside surv
+  // The same per unit: uplaced[q] / uplaced1[q] keys (the arrays above when a
+  // unit is a sub-bucket).  A group's bytes lie at its start: level 0's of
+  // all its sub-buckets in order, then level 1's.
+  uint32_t *uplaced = nullptr, *uplaced1 = nullptr;  // [units]
 };
 
+// max_bin: the keys of the largest bin.
 // With dist = nullptr the distinct keys stay where the dedup left them, at
-// the start of each sub-bucket's range of *kept (keys or alt), and
+// the start of each unit's range of *kept (keys or alt), and
 // msd_compact writes dist later; dist_off is written either way.
 // With pkeys/palt (one payload byte per key, beside keys and alt), each
 // distinct key leaves with the OR of its copies' payloads at the same place
-// of *kept_pay (pkeys or palt, beside *kept).
+// of *kept_pay (pkeys or palt, beside *kept); the group dedup leaves no bytes
+// there (*kept_pay = nullptr: they went to l0's outputs).
 template <class KeyT>
-bool msd_sort_unique(KeyT *keys, KeyT *alt, uint64_t n, const uint64_t *seg_off, uint32_t nbins, int key_bits, int P,
-                     KeyT *dist, uint64_t *dist_off, MsdScratch &sc, cudaStream_t s, bool sorted = true,
-                     const Level0Out *l0 = nullptr, KeyT **kept = nullptr, uint8_t *pkeys = nullptr,
+bool msd_sort_unique(KeyT *keys, KeyT *alt, uint64_t n, uint64_t max_bin, const uint64_t *seg_off, uint32_t nbins,
+                     int key_bits, int P, KeyT *dist, uint64_t *dist_off, MsdScratch &sc, cudaStream_t s,
+                     bool sorted = true, const Level0Out *l0 = nullptr, KeyT **kept = nullptr, uint8_t *pkeys = nullptr,
                      uint8_t *palt = nullptr, uint8_t **kept_pay = nullptr, uint8_t **l0pay_buf = nullptr);
 
-// The deferred copy: distinct keys of the last msd_sort_unique (nsub
-// sub-buckets, left in `kept`) to dist, bins in order.
+// The deferred copy: distinct keys of the last msd_sort_unique (nunit
+// units, left in `kept`) to dist, bins in order.
 template <class KeyT>
-void msd_compact(const KeyT *kept, uint64_t nsub, KeyT *dist, MsdScratch &sc, cudaStream_t s);
+void msd_compact(const KeyT *kept, uint64_t nunit, KeyT *dist, MsdScratch &sc, cudaStream_t s);
 
 }  // namespace cf1

@@ -25,7 +25,7 @@ void launch_classify(const ClassifyArgs<KeyT> &a, int persistent_ctas, cudaStrea
 
 // Phase 4 when phase 3 has joined the occurrences: the side-set byte left
 // beside each distinct key (kept[sb_off[j] + i], i < cnt[j], for the
-// sub-buckets j in [j0, j1) of 2^P per bin) goes to its vertex's slot --
+// dedup's units j in [j0, j1) of 2^P per bin) goes to its vertex's slot --
 // the key's rank (out_off[j] + i) in a bin the learned index serves, its
 // BBHash slot in any other bin.  A slot outside the bin flags DEV_MPHF_MISS.
 // The keys are read from the dense array (dense[out_off[j] + i]) when it is
@@ -36,16 +36,17 @@ void launch_place_sides(const MphfView<KeyT> &m, const KeyT *kept, const KeyT *d
                         int P, uint8_t *sides, uint32_t *err, cudaStream_t s);
 
 // The same for the BBHash form whose levels 0 and 1 the dedup built
-// (Level0Out with payloads): the keys level 0 places in sub-bucket j have
-// the consecutive slots from its level-0 slice's first rank on, those level
-// 1 places the ones from its level-1 slice's first rank on, and their bytes
-// wait in rank order at l0pay[sb_off[j] ...] (level 0's placed[j], then
-// level 1's placed1[j]) -- two contiguous copies each; the keys
-// level 1 left (bin b's at surv[surv_off[b] ...], surv_cnt[b] of them, bytes
-// beside them) walk the levels from 2.  Sub-buckets [j0, j1), bins [b0, b1).
-void launch_place_l0(const BBView &bb, const uint64_t *dist_off, const uint64_t *sb_off, const uint32_t *placed,
-                     const uint32_t *placed1, const uint8_t *l0pay, uint64_t j0, uint64_t j1, int P, uint8_t *sides,
-                     uint32_t *err, cudaStream_t s);
+// (Level0Out with payloads): the keys level 0 places in unit j have the
+// consecutive slots from its first level-0 slice's first rank on, those level
+// 1 places the ones from its first level-1 slice's first rank on, and their
+// bytes wait in rank order at l0pay[uoff[j] ...] (level 0's ucnt0[j], then
+// level 1's ucnt1[j]) -- two contiguous copies each; the keys level 1 left
+// (bin b's at surv[surv_off[b] ...], surv_cnt[b] of them, bytes beside them)
+// walk the levels from 2.  Units [j0, j1) of 2^PU per bin, slices of 2^P per
+// bin; bins [b0, b1).
+void launch_place_l0(const BBView &bb, const uint64_t *dist_off, const uint64_t *uoff, const uint32_t *ucnt0,
+                     const uint32_t *ucnt1, const uint8_t *l0pay, uint64_t j0, uint64_t j1, int PU, int P,
+                     uint8_t *sides, uint32_t *err, cudaStream_t s);
 void launch_place_surv(const BBView &bb, const uint64_t *dist_off, const uint64_t *surv, const uint8_t *surv_pay,
                        const uint64_t *surv_off, const unsigned long long *surv_cnt, uint32_t b0, uint32_t b1,
                        uint8_t *sides, uint32_t *err, cudaStream_t s);

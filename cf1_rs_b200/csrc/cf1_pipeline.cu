@@ -512,8 +512,8 @@ void run_impl(cf1gpu_ctx *c, StreamIO *io = nullptr, Step step = Step::FULL, con
       if (tried != -2) expand_again();  // the previous try consumed the keys
       if (batched) CF1_CUDA(cudaMemsetAsync(&sm->queues[4], 0, sizeof(uint32_t), s));
       CF1_CUDA(cudaEventRecord(c->ev[10], s));
-      const bool ok = msd_sort_unique<KeyT>(keys, alt, NO, seg, B, 2 * k, P, dist_buf(), dist_off, be.msd, s, sorted,
-                                            nullptr, nullptr, pay, pay_alt);
+      const bool ok = msd_sort_unique<KeyT>(keys, alt, NO, max_bin, seg, B, 2 * k, P, dist_buf(), dist_off, be.msd, s,
+                                            sorted, nullptr, nullptr, pay, pay_alt);
       CF1_CUDA(cudaEventRecord(c->ev[11], s));
       CF1_CUDA(cudaEventSynchronize(c->ev[11]));
       const double ms = elapsed(c->ev[10], c->ev[11]);
@@ -567,9 +567,11 @@ void run_impl(cf1gpu_ctx *c, StreamIO *io = nullptr, Step step = Step::FULL, con
     l0.surv_off = room_off;
     l0.surv_cnt = scnt;
     l0.err = &sm->l0_err;
-    uint32_t *placed = c->d_l0placed.get<uint32_t>(2 * (((uint64_t)B << P) + 1));
-    l0.placed = placed;
-    l0.placed1 = placed + ((uint64_t)B << P) + 1;
+    const uint64_t np = ((uint64_t)B << P) + 1;
+    l0.placed = c->d_l0placed.get<uint32_t>(4 * np);
+    l0.placed1 = l0.placed + np;
+    l0.uplaced = l0.placed1 + np;
+    l0.uplaced1 = l0.uplaced + np;
     if (join3) {  // joined side sets: levels 0 and 1 place their keys' bytes by rank (see Level0Out)
       l0.with_pay = true;
       l0.surv_pay = c->d_l0survpay.get<uint8_t>(l0_room + 1);
@@ -580,8 +582,8 @@ void run_impl(cf1gpu_ctx *c, StreamIO *io = nullptr, Step step = Step::FULL, con
   // verification or dump asks for it.
   KeyT *kept = nullptr;
   uint8_t *kept_pay = nullptr, *l0pay = nullptr;
-  bool done = P >= 0 && msd_sort_unique<KeyT>(keys, alt, NO, seg, B, 2 * k, P, l0_fuse ? nullptr : dist_buf(), dist_off,
-                                              be.msd, s, sorted, l0_fuse ? &l0 : nullptr, &kept, pay, pay_alt,
+  bool done = P >= 0 && msd_sort_unique<KeyT>(keys, alt, NO, max_bin, seg, B, 2 * k, P, l0_fuse ? nullptr : dist_buf(),
+                                              dist_off, be.msd, s, sorted, l0_fuse ? &l0 : nullptr, &kept, pay, pay_alt,
                                               &kept_pay, &l0pay);
   c->msd_bits = done ? P : -1;
   if (tune_now) {
@@ -605,15 +607,18 @@ void run_impl(cf1gpu_ctx *c, StreamIO *io = nullptr, Step step = Step::FULL, con
   if (l0_fuse) CF1_CUDA(cudaMemcpyAsync(&l0_err, &sm->l0_err, sizeof(uint32_t), cudaMemcpyDeviceToHost, s));
   CF1_CUDA(cudaStreamSynchronize(s));
   const bool l0_ready = l0_fuse && done && l0_err == 0;
-  const uint64_t nsub = done && P >= 0 ? (uint64_t)B << P : 0;
-  const bool joined = join3 && done && kept_pay != nullptr;  // phase 3 joined the occurrences' side sets
+  const int PU = be.msd.unit_bits;  // the dedup's units (sub-buckets or groups of them), 2^PU per bin
+  const uint64_t nunit = done && P >= 0 ? (uint64_t)B << PU : 0;
+  // phase 3 joined the occurrences' side sets: beside the kept keys, or (group
+  // dedup) in the outputs of levels 0 and 1 only
+  const bool joined = join3 && done && (kept_pay != nullptr || l0_ready);
   if (l0_fuse && done && !l0_ready) {  // level 0 did not fit: the plain build reads the dense keys
     dist = dist_buf();
-    msd_compact<KeyT>(kept, nsub, dist, be.msd, s);
+    msd_compact<KeyT>(kept, nunit, dist, be.msd, s);
   }
   c->dist_pending = l0_ready;
   c->dist_kept = kept;
-  c->dist_nsub = nsub;
+  c->dist_nunit = nunit;
   CF1_CUDA(cudaEventRecord(c->ev[3], s));
 
   // ---- phase 3b: MPHF
@@ -654,14 +659,15 @@ void run_impl(cf1gpu_ctx *c, StreamIO *io = nullptr, Step step = Step::FULL, con
     uint8_t *sb = reinterpret_cast<uint8_t *>(sides);
     const uint64_t *sbo = be.msd.sb_off.template as<const uint64_t>();
     if (joined_l0) {
-      launch_place_l0(be.bb.view(), dist_off, sbo, l0.placed, l0.placed1, l0pay, (uint64_t)b0 << P,
-                      (uint64_t)b1 << P, P, sb, &sm->err, s);
+      launch_place_l0(be.bb.view(), dist_off, sbo, PU == P ? l0.placed : l0.uplaced,
+                      PU == P ? l0.placed1 : l0.uplaced1, l0pay, (uint64_t)b0 << PU, (uint64_t)b1 << PU, PU, P, sb,
+                      &sm->err, s);
       launch_place_surv(be.bb.view(), dist_off, reinterpret_cast<const uint64_t *>(l0.surv), l0.surv_pay, l0.surv_off,
                         l0.surv_cnt, b0, b1, sb, &sm->err, s);
     } else {
       launch_place_sides<KeyT>(make_view<KeyT>(c), kept, c->dist_pending ? nullptr : c->d_dist.as<const KeyT>(),
                                kept_pay, sbo, be.msd.cnt.template as<const uint32_t>(),
-                               be.msd.out_off.template as<const uint64_t>(), (uint64_t)b0 << P, (uint64_t)b1 << P, P, sb,
+                               be.msd.out_off.template as<const uint64_t>(), (uint64_t)b0 << PU, (uint64_t)b1 << PU, PU, sb,
                                &sm->err, s);
     }
   };
@@ -784,7 +790,7 @@ void run_impl(cf1gpu_ctx *c, StreamIO *io = nullptr, Step step = Step::FULL, con
 template <class KeyT>
 void ensure_dist(cf1gpu_ctx *c) {
   if (!c->dist_pending) return;
-  msd_compact<KeyT>(static_cast<const KeyT *>(c->dist_kept), c->dist_nsub, c->d_dist.get<KeyT>(c->n_distinct + 1),
+  msd_compact<KeyT>(static_cast<const KeyT *>(c->dist_kept), c->dist_nunit, c->d_dist.get<KeyT>(c->n_distinct + 1),
                     backend<KeyT>(c).msd, c->stream);
   c->dist_pending = false;
 }

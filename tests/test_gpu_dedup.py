@@ -33,3 +33,39 @@ def test_block_kernel_without_payload_bytes(tmp_path, update):
     g, _ = assert_parity(seq, off, 31, num_bins=1, state_update=update, tuner_cache=_narrow_split(tmp_path, n))
     assert g.stats()["dedup_overflow"] > 0
     g.close()
+
+
+@pytest.mark.parametrize("k", [31, 15])
+@pytest.mark.parametrize("n_bases", [31, 222, 224, 6_170, 6_180, 120_000, 200_000, 3_200_001])
+def test_group_dedup_split_widths(k, n_bases):
+    """One bin of random sequence: no split and one sub-bucket (up to 192
+    k-mers), a group that is the whole bin (up to 32 sub-buckets), one more
+    sub-bucket bit, splits of 5 bits (keys and bytes) and 6 bits (packed
+    words) above the groups, and a two-pass split."""
+    seq, off = o.concat_records([_random(n_bases, n_bases + k)])
+    assert_parity(seq, off, k, num_bins=1)[0].close()
+
+
+@pytest.mark.parametrize("update", ["phase3", "sideset"])
+@pytest.mark.parametrize("n_random", [100, 150_000, 400_000])
+def test_groups_left_to_the_block_kernel(n_random, update):
+    """Tandem arrays and homopolymers put thousands of copies of a k-mer in a
+    group: it passes the group dedup's capacity and goes to the block kernel,
+    beside groups that do not."""
+    s = _random(n_random, n_random)
+    recs = [s, b"A" * 20_000, b"AC" * 9_000, b"ACGTTGC" * 3_000, s[: n_random // 3] * 2, _random(40, 1) * 400]
+    seq, off = o.concat_records(recs)
+    g, _ = assert_parity(seq, off, 31, num_bins=3, state_update=update)
+    assert g.stats()["dedup_overflow"] > 0
+    g.close()
+
+
+def test_repeated_keys_within_a_group():
+    """Every k-mer twice to forty times, in both strands: most level-0 bits
+    are set more than once by copies of one key."""
+    base = _random(30_000, 3)
+    rc = base.translate(bytes.maketrans(b"ACGT", b"TGCA"))[::-1]
+    recs = [base, rc, base[:9_000]] + [base[2_000:4_500]] * 38
+    seq, off = o.concat_records(recs)
+    for bins in (1, 16, 500):
+        assert_parity(seq, off, 31, num_bins=bins)[0].close()
