@@ -45,17 +45,17 @@ constexpr size_t NA_KEYS = 0;                                          // u64 [N
 constexpr size_t NA_ALT = NA_KEYS + NA_MAX_BASES * 8;                  // u64 [NA_MAX_BASES]
 constexpr uint32_t NA_HENTRIES = NA_DIGITS * NA_MAX_TILES;
 constexpr size_t NA_HIST = NA_ALT + NA_MAX_BASES * 8;                  // u32 [NA_HENTRIES]
-constexpr size_t NA_HSCAN = NA_HIST + NA_HENTRIES * 4;                 // u32 [NA_HENTRIES + 1]
-constexpr size_t NA_TCNT = NA_HSCAN + NA_HENTRIES * 4 + 256;           // u32 [NA_MAX_TILES]
-constexpr size_t NA_TOFF = NA_TCNT + NA_MAX_TILES * 4;                 // u32 [NA_MAX_TILES + 1]
-constexpr size_t NA_COUNT = NA_TOFF + (NA_MAX_TILES + 1) * 4 + 252;    // u32 number of keys (256-aligned)
+constexpr size_t NA_HSCAN = NA_HIST + NA_HENTRIES * 4;                 // u32 [NA_HENTRIES]
+constexpr size_t NA_TCNT = NA_HSCAN + NA_HENTRIES * 4;                 // u32 [NA_MAX_TILES]
+constexpr size_t NA_DTOT = NA_TCNT + NA_MAX_TILES * 4;                 // u32 [NA_DIGITS]
+constexpr size_t NA_COUNT = NA_DTOT + NA_DIGITS * 4;                   // u32 number of keys (256-aligned)
 constexpr size_t NA_SCRATCH_BYTES = NA_COUNT + 256;                    // 17.0 MiB in all
 
 static __device__ __align__(256) unsigned char g_noalloc_scratch[NA_SCRATCH_BYTES];
 
 struct Scratch {
   uint64_t *keys, *alt;
-  uint32_t *hist, *hscan, *tcnt, *toff, *count;
+  uint32_t *hist, *hscan, *tcnt, *dtot, *count;
 };
 
 Scratch carve(unsigned char *base) {
@@ -65,33 +65,61 @@ Scratch carve(unsigned char *base) {
   s.hist = reinterpret_cast<uint32_t *>(base + NA_HIST);
   s.hscan = reinterpret_cast<uint32_t *>(base + NA_HSCAN);
   s.tcnt = reinterpret_cast<uint32_t *>(base + NA_TCNT);
-  s.toff = reinterpret_cast<uint32_t *>(base + NA_TOFF);
+  s.dtot = reinterpret_cast<uint32_t *>(base + NA_DTOT);
   s.count = reinterpret_cast<uint32_t *>(base + NA_COUNT);
   return s;
 }
 
+// The bits of x at the even positions of a u64 (a k-mer's low or high code
+// bits, one base after another).
+CF1_D uint64_t na_spread(uint32_t x) {
+  uint64_t v = x;
+  v = (v | (v << 16)) & 0x0000FFFF0000FFFFull;
+  v = (v | (v << 8)) & 0x00FF00FF00FF00FFull;
+  v = (v | (v << 4)) & 0x0F0F0F0F0F0F0F0Full;
+  v = (v | (v << 2)) & 0x3333333333333333ull;
+  return (v | (v << 1)) & 0x5555555555555555ull;
+}
+
 // Canonical k-mer of every placeholder-free window [p, p+k) (src/mphf.rs:
 // 334-343 decode + canonicalise); order does not matter, the sort follows.
-__global__ void na_extract_kernel(const uint8_t *seq, uint64_t len, int k, uint64_t *keys, uint32_t *count) {
-  uint64_t p = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  bool ok = p + (uint64_t)k <= len;
-  uint64_t fw = 0;
-  for (int j = 0; ok && j < k; j++) {
-    uint32_t u = seq[p + j] & 0xDF;
-    ok = (u == 'A') | (u == 'C') | (u == 'G') | (u == 'T');
+// A CTA reads its 256 bases and the 32 after them once and keeps them as
+// three bit planes (code bits, placeholders), a warp vote per word; a window
+// is a funnel shift of each plane, and the reverse complement is the
+// complemented planes in the other bit order.  (One byte load per base of
+// every window and an atomic a warp took 31 us for 1 Mi bases, this 14.)
+__global__ void __launch_bounds__(NA_BLOCK) na_extract_kernel(const uint8_t *seq, uint64_t len, int k, uint64_t *keys,
+                                                              uint32_t *count) {
+  constexpr int NWORDS = NA_BLOCK / 32 + 1;
+  __shared__ uint32_t lo[NWORDS], hi[NWORDS], nm[NWORDS];
+  const uint64_t p0 = (uint64_t)blockIdx.x * NA_BLOCK;
+  const unsigned tid = threadIdx.x, lane = lane_id();
+  auto plane = [&](uint64_t p, uint32_t w) {
+    const uint32_t u = p < len ? seq[p] & 0xDF : 'N';
+    const bool ok = (u == 'A') | (u == 'C') | (u == 'G') | (u == 'T');
     uint32_t b = (u >> 1) & 3;
-    fw = (fw << 2) | (b ^ (b >> 1));
-  }
-  uint64_t can = 0;
-  if (ok) {
-    uint64_t rc = KOps<uint64_t>::rc(fw, k);
-    can = fw < rc ? fw : rc;
-  }
-  unsigned m = __ballot_sync(FULL, ok);
-  uint32_t base = 0;
-  if (lane_id() == 0 && m) base = atomicAdd(count, (uint32_t)__popc(m));
-  base = __shfl_sync(FULL, base, 0);
-  if (ok) keys[base + __popc(m & lanemask_lt())] = can;
+    b ^= b >> 1;
+    const uint32_t l = __ballot_sync(FULL, b & 1), h = __ballot_sync(FULL, b >> 1), n = __ballot_sync(FULL, !ok);
+    if (lane == 0) {
+      lo[w] = l;
+      hi[w] = h;
+      nm[w] = n;
+    }
+  };
+  plane(p0 + tid, tid >> 5);
+  if (tid < 32) plane(p0 + NA_BLOCK + tid, NWORDS - 1);
+  __syncthreads();
+  const uint32_t w = tid >> 5, mask = (1u << k) - 1;  // k <= 31
+  const uint32_t l = __funnelshift_r(lo[w], lo[w + 1], lane) & mask, h = __funnelshift_r(hi[w], hi[w + 1], lane) & mask;
+  const bool ok = (__funnelshift_r(nm[w], nm[w + 1], lane) & mask) == 0;  // (bases past the end are placeholders)
+  const uint64_t fw = na_spread(__brev(l) >> (32 - k)) | (na_spread(__brev(h) >> (32 - k)) << 1);
+  const uint64_t rc = na_spread(~l & mask) | (na_spread(~h & mask) << 1);
+  __shared__ uint32_t sm[NA_NW], s_base;  // one reservation a CTA
+  uint32_t tot;
+  const uint32_t pre = block_exclusive_scan<NA_BLOCK>(ok ? 1u : 0u, sm, tot);
+  if (tid == 0) s_base = tot ? atomicAdd(count, tot) : 0u;
+  __syncthreads();
+  if (ok) keys[s_base + pre] = fw < rc ? fw : rc;
 }
 
 // Per tile digit counts, digit-major (digit d of tile t at d * ntiles + t).
@@ -110,63 +138,83 @@ __global__ void __launch_bounds__(NA_BLOCK) na_hist_kernel(const uint64_t *keys,
   H[threadIdx.x * ntiles + t] = h[threadIdx.x];
 }
 
-// One CTA: exclusive scan of n u32 values (n <= NA_DIGITS * NA_MAX_TILES).
-__global__ void __launch_bounds__(1024) na_scan_kernel(const uint32_t *in, uint32_t *out, uint32_t n) {
-  __shared__ uint32_t sm[32];
-  uint32_t carry = 0;
-  for (uint32_t base = 0; base < n; base += 1024) {
-    uint32_t i = base + threadIdx.x;
-    uint32_t v = i < n ? in[i] : 0, tot;
-    uint32_t pre = block_exclusive_scan<1024>(v, sm, tot);
-    if (i < n) out[i] = carry + pre;
-    carry += tot;
-  }
-  if (threadIdx.x == 0) out[n] = carry;
+// One CTA per digit: exclusive scan of its counts over the tiles (ntiles <=
+// NA_MAX_TILES), and their sum.  The scatter adds the sums of the smaller
+// digits itself.  (One CTA scanning all digits x tiles in 1024-entry rounds
+// took 100 us a pass for 1 Mi bases, of the call's 920.)
+__global__ void __launch_bounds__(NA_BLOCK) na_scan_kernel(const uint32_t *H, uint32_t ntiles, uint32_t *Hs,
+                                                           uint32_t *dtot) {
+  static_assert(NA_MAX_TILES <= 2 * NA_BLOCK, "two tiles a thread");
+  __shared__ uint32_t sm[NA_NW];
+  const uint32_t d = blockIdx.x, t = 2 * threadIdx.x;
+  const uint32_t v0 = t < ntiles ? H[d * ntiles + t] : 0, v1 = t + 1 < ntiles ? H[d * ntiles + t + 1] : 0;
+  uint32_t tot;
+  const uint32_t pre = block_exclusive_scan<NA_BLOCK>(v0 + v1, sm, tot);
+  if (t < ntiles) Hs[d * ntiles + t] = pre;
+  if (t + 1 < ntiles) Hs[d * ntiles + t + 1] = pre + v0;
+  if (threadIdx.x == 0) dtot[d] = tot;
 }
 
-// Stable scatter of one tile (round-major order, warp ranks by match_any,
-// per (round, warp, digit) counts turned into offsets per digit).
+// Stable scatter of one tile.  A warp takes 256 consecutive keys, 32 at a
+// time, and ranks them by its own digit counters (match_any inside a round,
+// the counters between rounds); a prefix over the warps gives tile-local
+// places, the tile is staged in digit order and every digit's run is written
+// by consecutive threads.
 __global__ void __launch_bounds__(NA_BLOCK) na_scatter_kernel(const uint64_t *in, uint64_t *out, const uint32_t *count,
-                                                              int shift, uint32_t ntiles, const uint32_t *Hs) {
-  __shared__ uint16_t cnt[NA_ITEMS * NA_NW * NA_DIGITS];
-  __shared__ uint32_t s_base[NA_DIGITS];
+                                                              int shift, uint32_t ntiles, const uint32_t *Hs,
+                                                              const uint32_t *dtot) {
+  __shared__ uint64_t stage[NA_TILE];
+  __shared__ uint32_t whist[NA_NW][NA_DIGITS];
+  __shared__ uint32_t s_base[NA_DIGITS], sm[NA_NW];
   const uint32_t t = blockIdx.x, n = *count;
-  const unsigned tid = threadIdx.x, warp = tid >> 5;
-  uint64_t start = (uint64_t)t * NA_TILE;
+  const unsigned tid = threadIdx.x, warp = tid >> 5, lane = lane_id(), lt = lanemask_lt();
+  const uint64_t start = (uint64_t)t * NA_TILE;
   if (start >= n) return;
-  uint64_t end = start + NA_TILE < n ? start + NA_TILE : n;
-  uint32_t *c32 = reinterpret_cast<uint32_t *>(cnt);
-  for (uint32_t i = tid; i < NA_ITEMS * NA_NW * NA_DIGITS / 2; i += NA_BLOCK) c32[i] = 0;
-  s_base[tid] = Hs[tid * ntiles + t];
-  __syncthreads();
+  const uint32_t len = (uint32_t)(n - start < NA_TILE ? n - start : NA_TILE);
   uint64_t key[NA_ITEMS];
-  uint32_t dg[NA_ITEMS], wr[NA_ITEMS];
-  const unsigned lt = lanemask_lt();
 #pragma unroll
   for (int r = 0; r < NA_ITEMS; r++) {
-    uint64_t i = start + (uint64_t)r * NA_BLOCK + tid;
-    bool act = i < end;
-    key[r] = act ? in[i] : 0;
-    dg[r] = act ? (uint32_t)(key[r] >> shift) & 0xFF : 0xFFFFFFFFu;
-    unsigned peers = __match_any_sync(FULL, dg[r]);
-    wr[r] = __popc(peers & lt);
-    if (act && wr[r] == 0) cnt[(r * NA_NW + warp) * NA_DIGITS + dg[r]] = (uint16_t)__popc(peers);
+    const uint32_t i = warp * (NA_ITEMS * 32) + r * 32 + lane;
+    key[r] = i < len ? in[start + i] : 0;
+  }
+  for (uint32_t i = tid; i < NA_NW * NA_DIGITS; i += NA_BLOCK) (&whist[0][0])[i] = 0;
+  uint32_t tot;
+  const uint32_t gbase = block_exclusive_scan<NA_BLOCK>(dtot[tid], sm, tot) + Hs[tid * ntiles + t];
+  uint32_t rank[NA_ITEMS];
+#pragma unroll
+  for (int r = 0; r < NA_ITEMS; r++) {
+    const uint32_t i = warp * (NA_ITEMS * 32) + r * 32 + lane;
+    const uint32_t d = i < len ? (uint32_t)(key[r] >> shift) & 0xFF : 0xFFFFFFFFu;
+    const unsigned peers = __match_any_sync(FULL, d);
+    const uint32_t c = d < NA_DIGITS ? whist[warp][d] : 0;
+    rank[r] = c + __popc(peers & lt);
+    __syncwarp();
+    if (d < NA_DIGITS && (peers & lt) == 0) whist[warp][d] = c + __popc(peers);
+    __syncwarp();
   }
   __syncthreads();
-  {
-    uint32_t run = 0;
-    for (int r = 0; r < NA_ITEMS; r++)
-      for (int w = 0; w < NA_NW; w++) {
-        uint16_t &c = cnt[(r * NA_NW + w) * NA_DIGITS + tid];
-        uint32_t v = c;
-        c = (uint16_t)run;
-        run += v;
-      }
+  uint32_t run = 0;
+#pragma unroll
+  for (int w = 0; w < NA_NW; w++) {
+    const uint32_t v = whist[w][tid];
+    whist[w][tid] = run;
+    run += v;
   }
+  const uint32_t first = block_exclusive_scan<NA_BLOCK>(run, sm, tot);  // the digit's tile-local start
+  s_base[tid] = gbase - first;
+#pragma unroll
+  for (int w = 0; w < NA_NW; w++) whist[w][tid] += first;
   __syncthreads();
 #pragma unroll
-  for (int r = 0; r < NA_ITEMS; r++)
-    if (dg[r] != 0xFFFFFFFFu) out[s_base[dg[r]] + cnt[(r * NA_NW + warp) * NA_DIGITS + dg[r]] + wr[r]] = key[r];
+  for (int r = 0; r < NA_ITEMS; r++) {
+    const uint32_t i = warp * (NA_ITEMS * 32) + r * 32 + lane;
+    if (i < len) stage[whist[warp][(uint32_t)(key[r] >> shift) & 0xFF] + rank[r]] = key[r];
+  }
+  __syncthreads();
+  for (uint32_t i = tid; i < len; i += NA_BLOCK) {
+    const uint64_t k = stage[i];
+    out[s_base[(uint32_t)(k >> shift) & 0xFF] + i] = k;
+  }
 }
 
 __global__ void __launch_bounds__(NA_BLOCK) na_unique_count_kernel(const uint64_t *keys, const uint32_t *count,
@@ -181,10 +229,18 @@ __global__ void __launch_bounds__(NA_BLOCK) na_unique_count_kernel(const uint64_
 }
 
 __global__ void __launch_bounds__(NA_BLOCK) na_unique_write_kernel(const uint64_t *keys, const uint32_t *count,
-                                                                   const uint32_t *toff, uint32_t ntiles,
+                                                                   const uint32_t *tcnt, uint32_t ntiles,
                                                                    uint64_t *out, uint64_t *n_out) {
   __shared__ uint32_t sm[NA_NW];
   const uint32_t t = blockIdx.x, n = *count;
+  // the distinct keys of the tiles before this one
+  uint32_t before = 0, all = 0;
+  for (uint32_t i = threadIdx.x; i < ntiles; i += NA_BLOCK) {
+    const uint32_t v = tcnt[i];
+    all += v;
+    before += i < t ? v : 0u;
+  }
+  before = block_sum<NA_BLOCK>(before, sm);
   uint64_t i0 = (uint64_t)t * NA_TILE + (uint64_t)threadIdx.x * NA_ITEMS;
   uint32_t flags = 0, c = 0;
 #pragma unroll
@@ -196,11 +252,14 @@ __global__ void __launch_bounds__(NA_BLOCK) na_unique_write_kernel(const uint64_
   }
   uint32_t tot;
   uint32_t pre = block_exclusive_scan<NA_BLOCK>(c, sm, tot);
-  uint64_t o = toff[t] + pre;
+  uint64_t o = before + pre;
 #pragma unroll
   for (int j = 0; j < NA_ITEMS; j++)
     if ((flags >> j) & 1) out[o++] = keys[i0 + j];
-  if (t == 0 && threadIdx.x == 0) *n_out = toff[ntiles];
+  if (t == 0) {
+    all = block_sum<NA_BLOCK>(all, sm);
+    if (threadIdx.x == 0) *n_out = all;
+  }
 }
 
 std::mutex g_addr_mu;
@@ -249,15 +308,14 @@ extern "C" int cf1gpu_distinct_kmers_noalloc(int device, uint32_t k, const uint8
     uint64_t *src = sc.keys, *dst = sc.alt;
     for (int shift = 0; shift < 2 * (int)k; shift += 8) {
       na_hist_kernel<<<ntiles, NA_BLOCK, 0, s>>>(src, sc.count, shift, ntiles, sc.hist);
-      na_scan_kernel<<<1, 1024, 0, s>>>(sc.hist, sc.hscan, NA_DIGITS * ntiles);
-      na_scatter_kernel<<<ntiles, NA_BLOCK, 0, s>>>(src, dst, sc.count, shift, ntiles, sc.hscan);
+      na_scan_kernel<<<NA_DIGITS, NA_BLOCK, 0, s>>>(sc.hist, ntiles, sc.hscan, sc.dtot);
+      na_scatter_kernel<<<ntiles, NA_BLOCK, 0, s>>>(src, dst, sc.count, shift, ntiles, sc.hscan, sc.dtot);
       uint64_t *t = src;
       src = dst;
       dst = t;
     }
     na_unique_count_kernel<<<ntiles, NA_BLOCK, 0, s>>>(src, sc.count, sc.tcnt);
-    na_scan_kernel<<<1, 1024, 0, s>>>(sc.tcnt, sc.toff, ntiles);
-    na_unique_write_kernel<<<ntiles, NA_BLOCK, 0, s>>>(src, sc.count, sc.toff, ntiles, d_keys_out, d_n_out);
+    na_unique_write_kernel<<<ntiles, NA_BLOCK, 0, s>>>(src, sc.count, sc.tcnt, ntiles, d_keys_out, d_n_out);
     e = cudaGetLastError();
   } else if (e == cudaSuccess) {
     e = cudaMemsetAsync(d_n_out, 0, sizeof(uint64_t), s);
