@@ -9,6 +9,7 @@
 //            marks the collision array instead;
 //   clean  : bits that collided are cleared; a popcount prefix gives ranks;
 //   filter : keys whose bit survived are placed, the rest go to the next level.
+// The last levels, which have few keys, run in one launch (bb_tail_kernel).
 // A bin's local slot of a key placed at level l is the number of keys of the
 // bin placed at earlier levels plus the key's rank inside its level block.
 // All levels live in one array of {bit word, level rank} entries, addressed
@@ -157,28 +158,172 @@ __global__ void bb_meta_kernel(const uint64_t *woff, const uint64_t *R, uint64_t
   base[b] += R[w1] - R[w0];
 }
 
-// A sliced level (levels 0 and 1 of the phase-3 dedup): each entry holds
-// {placed bits, placed bits of its slice before it}; R = the exclusive scan
-// of the slices' placed counts over the whole level (slices of bin b are
-// [b << P, (b + 1) << P)).  srank[j] = the placed keys of slice j's bin
-// before slice j; the bin's metadata takes the keys earlier levels placed as
-// its rank adjustment.
-__global__ void bb_srank_kernel(const uint64_t *R, int P, uint64_t nsub, uint32_t *srank) {
-  const uint64_t j = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  if (j < nsub) srank[j] = (uint32_t)(R[j] - R[(j >> P) << P]);
+// Levels 0 and 1 as the phase-3 dedup left them (sliced, see BBView): each
+// entry holds {placed bits, placed bits of its slice before it}.  One CTA per
+// bin scans the bin's slices' placed counts (slices [b << P, (b + 1) << P))
+// into srank -- the placed keys of the bin's slices before the slice -- and
+// writes the bin's metadata, whose rank adjustment is the keys its earlier
+// levels placed.
+constexpr int BF_BLOCK = 1024;
+__global__ void __launch_bounds__(BF_BLOCK) bb_sliced_kernel(const uint64_t *woff0, const uint64_t *woff1, int P,
+                                                             uint64_t words0, const uint32_t *placed0,
+                                                             const uint32_t *placed1, uint32_t *srank0,
+                                                             uint32_t *srank1, uint64_t *base, BBMeta *meta,
+                                                             uint32_t nbins) {
+  __shared__ uint32_t sm[BF_BLOCK / 32];
+  const uint32_t b = blockIdx.x, tid = threadIdx.x, ns = 1u << P;
+  uint32_t before = 0;  // keys the bin's earlier levels placed (bins hold < 2^32 keys)
+  for (int l = 0; l < 2; l++) {
+    const uint32_t *placed = (l ? placed1 : placed0) + ((uint64_t)b << P);
+    uint32_t *srank = (l ? srank1 : srank0) + ((uint64_t)b << P);
+    const uint64_t *woff = l ? woff1 : woff0;
+    uint32_t carry = 0;
+    for (uint32_t j0 = 0; j0 < ns; j0 += 4 * BF_BLOCK) {  // four consecutive slices a thread
+      const uint32_t j = j0 + 4 * tid;
+      uint32_t v[4], c = 0;
+#pragma unroll
+      for (int i = 0; i < 4; i++) {
+        v[i] = j + i < ns ? placed[j + i] : 0u;
+        c += v[i];
+      }
+      uint32_t tot;
+      uint32_t pre = carry + block_exclusive_scan<BF_BLOCK>(c, sm, tot);
+#pragma unroll
+      for (int i = 0; i < 4; i++) {
+        if (j + i < ns) srank[j + i] = pre;
+        pre += v[i];
+      }
+      carry += tot;
+    }
+    if (tid == 0) {
+      BBMeta m;
+      m.word_off = (l ? words0 : 0) + woff[b];
+      m.nwords = (uint32_t)(woff[b + 1] - woff[b]);
+      m.rank_adj = before;
+      meta[(uint64_t)l * nbins + b] = m;
+    }
+    before += carry;
+  }
+  if (tid == 0) base[b] = before;
 }
 
-__global__ void bb_meta_sliced_kernel(const uint64_t *woff, const uint64_t *R, int P, uint64_t level_base,
-                                      uint64_t *base, BBMeta *meta, uint32_t nbins) {
-  uint32_t b = blockIdx.x * blockDim.x + threadIdx.x;
-  if (b >= nbins) return;
-  const uint64_t r0 = R[(uint64_t)b << P], r1 = R[(uint64_t)(b + 1) << P];
-  BBMeta m;
-  m.word_off = level_base + woff[b];
-  m.nwords = (uint32_t)(woff[b + 1] - woff[b]);
-  m.rank_adj = (uint32_t)base[b];
-  meta[b] = m;
-  base[b] += r1 - r0;
+// The last levels, one CTA per bin, all of them in one launch: per level the
+// bin's keys mark its block, the collided bits are cleared and ranked (ranks
+// count from the block's start, the rank adjustment is the keys earlier levels
+// placed) and the keys left go on.  Level l's keys are rem0 (l = l0), then r0
+// / r1 in turn, at start[b].  Bin b's blocks lie in entries [off[b],
+// off[b + 1]) from ar_base, one level after another; what is left of them is
+// cleared.  Blocks up to BF_WORDS words are marked in shared memory.
+//
+// Launched once the keys left are few (BF_KEYS a bin on average: a level of
+// that many keys takes the CTA ~15 us, and one launch of its own ~55 us with
+// the wait for its size).  A run's MPHF phase, nine launches and a wait per
+// level before: 30 kb 240 -> 20 us, 200 Mbp 590 -> 60 us.
+constexpr uint32_t BF_WORDS = 4096;
+constexpr uint64_t BF_KEYS = 16384;
+// Entries reserved for n keys: the levels' blocks sum up to ~1.14 times the
+// first one's words and a word a level.
+CF1_HD uint64_t bf_room(uint64_t n) {
+  const uint64_t w = (8 * n + 63) / 64;
+  return n ? w + w / 4 + BB_MAX_LEVELS : 0;
+}
+__global__ void bb_room_kernel(const uint64_t *cnt, uint32_t nbins, uint64_t *room) {
+  const uint32_t b = blockIdx.x * blockDim.x + threadIdx.x;
+  if (b < nbins) room[b] = bf_room(cnt[b]);
+}
+template <class KeyT>
+__global__ void __launch_bounds__(BF_BLOCK) bb_tail_kernel(const KeyT *rem0, KeyT *r0, KeyT *r1, const uint64_t *start,
+                                                           const uint64_t *cnt, uint32_t nbins, uint32_t l0,
+                                                           ulonglong2 *AR, const uint64_t *off, uint64_t ar_base,
+                                                           uint64_t ar_cap, const uint64_t *base, BBMeta *meta,
+                                                           uint32_t *levels, uint32_t *err) {
+  extern __shared__ __align__(16) unsigned long long bf_bits[];  // set, col
+  __shared__ uint32_t sm[BF_BLOCK / 32];
+  const uint32_t b = blockIdx.x, tid = threadIdx.x;
+  const uint64_t region = ar_base + off[b], room = off[b + 1] - off[b], s0 = start[b];
+  uint64_t n = cnt[b], used = 0;
+  if (!n) return;
+  if (region + room > ar_cap) {
+    if (tid == 0) atomicOr(err, (uint32_t)DEV_OVERFLOW);
+    return;
+  }
+  uint32_t before = (uint32_t)base[b], l = l0;
+  const KeyT *rem = rem0 + s0;
+  unsigned long long *set = bf_bits, *col = bf_bits + BF_WORDS;
+  for (; n; l++) {
+    const uint64_t nw = (8 * n + 63) / 64;
+    if (l >= BB_MAX_LEVELS || used + nw > room) {
+      if (tid == 0) atomicOr(err, (uint32_t)DEV_BIJECTION);
+      return;
+    }
+    ulonglong2 *E = AR + region + used;
+    const bool local = nw <= BF_WORDS;
+    for (uint64_t w = tid; w < nw; w += BF_BLOCK) {
+      if (local) set[w] = col[w] = 0;
+      else E[w] = make_ulonglong2(0ull, 0ull);
+    }
+    __syncthreads();
+    for (uint64_t i = tid; i < n; i += BF_BLOCK) {
+      const uint64_t pos = bb_pos(bb_key_hash(rem[i]), l, (uint32_t)nw);
+      const uint32_t w = (uint32_t)(pos >> 5), bit = 1u << (pos & 31);  // by half words
+      uint32_t *x = local ? reinterpret_cast<uint32_t *>(set) + w
+                          : reinterpret_cast<uint32_t *>(E + (w >> 1)) + (w & 1);
+      uint32_t *y = local ? reinterpret_cast<uint32_t *>(col) + w
+                          : reinterpret_cast<uint32_t *>(E + (w >> 1)) + 2 + (w & 1);
+      if (atomicOr(x, bit) & bit) atomicOr(y, bit);
+    }
+    __syncthreads();
+    uint32_t placed = 0;
+    for (uint64_t w0 = 0; w0 < nw; w0 += BF_BLOCK) {
+      const uint64_t w = w0 + tid;
+      unsigned long long f = 0;
+      if (w < nw) {
+        if (local) f = set[w] & ~col[w];
+        else {
+          const ulonglong2 e = E[w];
+          f = e.x & ~e.y;
+        }
+      }
+      uint32_t tot;
+      const uint32_t pre = block_exclusive_scan<BF_BLOCK>((uint32_t)__popcll(f), sm, tot);
+      if (w < nw) {
+        E[w] = make_ulonglong2(f, (unsigned long long)(placed + pre));
+        if (local) set[w] = f;
+      }
+      placed += tot;
+    }
+    if (tid == 0) {
+      BBMeta m;
+      m.word_off = region + used;
+      m.nwords = (uint32_t)nw;
+      m.rank_adj = before;
+      meta[(uint64_t)l * nbins + b] = m;
+    }
+    __syncthreads();
+    KeyT *out = ((l & 1) ? r1 : r0) + s0;
+    uint64_t left = 0;
+    for (uint64_t i0 = 0; i0 < n; i0 += BF_BLOCK) {
+      const uint64_t i = i0 + tid;
+      KeyT key{};
+      bool keep = false;
+      if (i < n) {
+        key = rem[i];
+        const uint64_t pos = bb_pos(bb_key_hash(key), l, (uint32_t)nw);
+        keep = !(((local ? set[pos >> 6] : E[pos >> 6].x) >> (pos & 63)) & 1);
+      }
+      uint32_t tot;
+      const uint32_t pre = block_exclusive_scan<BF_BLOCK>(keep ? 1u : 0u, sm, tot);
+      if (keep) out[left + pre] = key;
+      left += tot;
+    }
+    __syncthreads();
+    used += nw;
+    before += placed;
+    n = left;
+    rem = out;
+  }
+  for (uint64_t w = used + tid; w < room; w += BF_BLOCK) AR[region + w] = make_ulonglong2(0ull, 0ull);
+  if (tid == 0) atomicMax(levels, l);
 }
 
 // Keys whose bit did not survive go to the next level: each tile appends its
@@ -224,8 +369,7 @@ __global__ void __launch_bounds__(BB_BLOCK) bb_filter_kernel(const KeyT *rem, co
 
 template <class KeyT>
 void BBHashBuild<KeyT>::clear() {
-  nwords.clear();
-  level_off.clear();
+  tail_words_ = nullptr;
   total_words = 0;
   levels = 0;
   bytes = 0;
@@ -288,8 +432,26 @@ void BBHashBuild<KeyT>::finish_level(uint32_t l, const uint64_t *woff, uint64_t 
 // does not place to r0 / r1 in turn at the same offsets.
 template <class KeyT>
 void BBHashBuild<KeyT>::run_levels(uint32_t l, const KeyT *rem, const uint64_t *start, KeyT *r0, KeyT *r1,
-                                   cudaStream_t s) {
+                                   uint64_t expect, uint32_t *err, cudaStream_t s) {
   KeyT *r[2] = {r0, r1};
+  auto tail = [&] {  // all levels from l in one launch
+    uint64_t *room = wcnt_.as<uint64_t>(), *off = woff_.as<uint64_t>(), *cur = cnt_[l & 1].as<uint64_t>();
+    bb_room_kernel<<<(unsigned)ceil_div(nbins, 256), 256, 0, s>>>(cur, nbins, room);
+    CF1_LAUNCH_CHECK();
+    exclusive_scan_u64(room, off, nbins, scan_tmp_, s);
+    uint32_t *lv = lv_.get<uint32_t>(1);
+    CF1_CUDA(cudaMemcpyAsync(lv, &tail_from_, sizeof(uint32_t), cudaMemcpyHostToDevice, s));
+    const size_t smem = 2 * BF_WORDS * sizeof(unsigned long long);
+    CF1_CUDA(cudaFuncSetAttribute(bb_tail_kernel<KeyT>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    bb_tail_kernel<KeyT><<<nbins, BF_BLOCK, smem, s>>>(rem, r0, r1, start, cur, nbins, l, ar_.as<ulonglong2>(), off,
+                                                       total_words, ar_.cap / sizeof(ulonglong2), base_.as<uint64_t>(),
+                                                       meta_.as<BBMeta>(), lv, err);
+    CF1_LAUNCH_CHECK();
+    tail_words_ = off + nbins;
+    levels = BB_MAX_LEVELS;  // until collect(): a walk ends at the first level a bin does not have
+  };
+  tail_from_ = l;
+  if (expect <= BF_KEYS * nbins) return tail();
   uint64_t *wcnt = wcnt_.as<uint64_t>(), *woff = woff_.as<uint64_t>();
   uint32_t *tile_off = tile_off_.as<uint32_t>();
   unsigned long long *tot = reinterpret_cast<unsigned long long *>(tot_.as<uint64_t>());
@@ -303,11 +465,14 @@ void BBHashBuild<KeyT>::run_levels(uint32_t l, const KeyT *rem, const uint64_t *
     CF1_CUDA(cudaStreamSynchronize(s));
     const uint64_t remaining = ht[0], nw = ht[1];
     if (remaining == 0) break;
+    if (remaining <= BF_KEYS * nbins) {
+      reserve_entries(total_words + bf_room(remaining) + nbins * (bf_room(1) + 1), total_words, s);
+      tail_from_ = l;
+      return tail();
+    }
     if (l >= BB_MAX_LEVELS) throw Error(CF1GPU_ERR_BIJECTION, "BBHash: keys left after the last level");
     exclusive_scan_u64(wcnt, woff, nbins, scan_tmp_, s);
     reserve_entries(total_words + nw, total_words, s);
-    nwords.push_back(nw);
-    level_off.push_back(total_words);
     ulonglong2 *Al = ar_.as<ulonglong2>() + total_words;
     CF1_CUDA(cudaMemsetAsync(Al, 0, nw * sizeof(ulonglong2), s));
     uint32_t ub = (uint32_t)(ceil_div(remaining, BB_TILE) + nbins);
@@ -324,13 +489,33 @@ void BBHashBuild<KeyT>::run_levels(uint32_t l, const KeyT *rem, const uint64_t *
     rem = out;
   }
   levels = l;
-  bytes = total_words * sizeof(ulonglong2) + (size_t)levels * nbins * sizeof(BBMeta);
-  CF1_CUDA(cudaStreamSynchronize(s));
+  set_bytes();
+}
+
+template <class KeyT>
+void BBHashBuild<KeyT>::set_bytes() {
+  bytes = total_words * sizeof(ulonglong2) + (size_t)levels * nbins * sizeof(BBMeta) + 2 * srank_words * sizeof(uint32_t);
+}
+
+template <class KeyT>
+void BBHashBuild<KeyT>::collect_begin(cudaStream_t s) {
+  if (!tail_words_) return;
+  CF1_CUDA(cudaMemcpyAsync(&got_words_, tail_words_, sizeof(uint64_t), cudaMemcpyDeviceToHost, s));
+  CF1_CUDA(cudaMemcpyAsync(&got_levels_, lv_.p, sizeof(uint32_t), cudaMemcpyDeviceToHost, s));
+}
+
+template <class KeyT>
+void BBHashBuild<KeyT>::collect_end() {
+  if (!tail_words_) return;
+  tail_words_ = nullptr;
+  total_words += got_words_;
+  levels = std::max<uint32_t>(got_levels_, l1_slice_bits >= 0 ? 2 : 0);
+  set_bytes();
 }
 
 template <class KeyT>
 void BBHashBuild<KeyT>::build(const KeyT *keys, const uint64_t *seg_off, uint32_t nb, const uint32_t *sel,
-                              cudaStream_t s, KeyT *ws0, KeyT *ws1, uint64_t ws_cap) {
+                              uint32_t *err, cudaStream_t s, KeyT *ws0, KeyT *ws1, uint64_t ws_cap) {
   begin(nb, s);
   std::vector<uint64_t> hoff(nbins + 1);
   CF1_CUDA(cudaMemcpyAsync(hoff.data(), seg_off, (nbins + 1) * sizeof(uint64_t), cudaMemcpyDeviceToHost, s));
@@ -349,52 +534,40 @@ void BBHashBuild<KeyT>::build(const KeyT *keys, const uint64_t *seg_off, uint32_
   // room for the usual level sizes (gamma0 bits per key, then ~12% and
   // fewer keys per level) so that the entry array rarely grows in mid-build
   reserve_entries((BB_GAMMA0 * n_all / 64 + nbins) * 3 / 2 + 64 * nbins + 64, 0, s);
-  run_levels(0, keys, seg_off, r0, r1, s);
+  run_levels(0, keys, seg_off, r0, r1, n_all, err, s);
 }
 
 template <class KeyT>
-ulonglong2 *BBHashBuild<KeyT>::prepare_levels01(uint64_t words0, uint64_t words1, cudaStream_t s) {
+ulonglong2 *BBHashBuild<KeyT>::prepare_levels01(uint32_t nb, uint64_t words0, uint64_t words1, cudaStream_t s) {
+  // with the later levels' room: at most a quarter of the occurrences reach
+  // level 2 (the dedup's list holds no more), bf_room(that) in all
   const uint64_t words = words0 + words1;
-  reserve_entries(words + words / 4 + 64 * 1024, 0, s);
+  reserve_entries(words + words / 3 + (uint64_t)nb * 2 * BB_MAX_LEVELS + 64 * 1024, 0, s);
   return ar_.as<ulonglong2>();
-}
-
-template <class KeyT>
-void BBHashBuild<KeyT>::finish_sliced(uint32_t l, const uint64_t *woff, const uint32_t *placed, int P,
-                                      cudaStream_t s) {
-  const uint64_t nsub = (uint64_t)nbins << P;
-  uint64_t *R = rtmp_.get<uint64_t>(nsub + 1);
-  exclusive_scan_u32(placed, R, nsub, scan_tmp_, s);
-  bb_srank_kernel<<<(unsigned)ceil_div(nsub, 256), 256, 0, s>>>(R, P, nsub, srank_[l].get<uint32_t>(nsub + 1));
-  CF1_LAUNCH_CHECK();
-  bb_meta_sliced_kernel<<<(unsigned)ceil_div(nbins, 256), 256, 0, s>>>(
-      woff, R, P, total_words, base_.as<uint64_t>(), meta_.as<BBMeta>() + (size_t)l * nbins, nbins);
-  CF1_LAUNCH_CHECK();
 }
 
 template <class KeyT>
 void BBHashBuild<KeyT>::build_from_levels01(uint32_t nb, int P, const uint64_t *woff0, uint64_t words0,
                                             const uint32_t *placed0, const uint64_t *woff1, uint64_t words1,
                                             const uint32_t *placed1, const KeyT *surv, const uint64_t *surv_off,
-                                            const uint64_t *surv_cnt, uint64_t surv_total, cudaStream_t s, KeyT *ws0,
-                                            KeyT *ws1, uint64_t ws_cap) {
+                                            const uint64_t *surv_cnt, uint64_t surv_total, uint64_t n_occ,
+                                            uint32_t *err, cudaStream_t s, KeyT *ws0, KeyT *ws1, uint64_t ws_cap) {
   begin(nb, s);
-  nwords.push_back(words0);
-  level_off.push_back(0);
-  finish_sliced(0, woff0, placed0, P, s);
-  total_words = words0;
-  nwords.push_back(words1);
-  level_off.push_back(words0);
-  finish_sliced(1, woff1, placed1, P, s);
-  total_words += words1;
+  const uint64_t nsl = ((uint64_t)nbins << P) + 1;
+  bb_sliced_kernel<<<nbins, BF_BLOCK, 0, s>>>(woff0, woff1, P, words0, placed0, placed1, srank_[0].get<uint32_t>(nsl),
+                                              srank_[1].get<uint32_t>(nsl), base_.as<uint64_t>(), meta_.as<BBMeta>(),
+                                              nbins);
+  CF1_LAUNCH_CHECK();
+  total_words = words0 + words1;
   l1_slice_bits = P;
   srank_words = (uint64_t)nbins << P;
   CF1_CUDA(cudaMemcpyAsync(cnt_[0].as<uint64_t>(), surv_cnt, nbins * sizeof(uint64_t), cudaMemcpyDeviceToDevice, s));
   KeyT *r0 = (ws0 && ws_cap >= surv_total + 1) ? ws0 : rem_[0].get<KeyT>(surv_total + 1);
   KeyT *r1 = (ws1 && ws_cap >= surv_total + 1) ? ws1 : rem_[1].get<KeyT>(surv_total + 1);
-  run_levels(2, surv, surv_off, r0, r1, s);  // level l reads cnt_[l & 1] and writes r[l & 1]
+  // level l reads cnt_[l & 1] and writes r[l & 1]; level 1 leaves ~1% of the keys
+  run_levels(2, surv, surv_off, r0, r1, n_occ / 100, err, s);
   levels = std::max<uint32_t>(levels, 2);
-  bytes = total_words * sizeof(ulonglong2) + (size_t)levels * nbins * sizeof(BBMeta) + 2 * srank_words * sizeof(uint32_t);
+  set_bytes();
 }
 
 template <class KeyT>
@@ -409,11 +582,6 @@ BBView BBHashBuild<KeyT>::view() const {
   v.srank[0] = l1_slice_bits >= 0 ? srank_[0].as<const uint32_t>() : nullptr;
   v.srank[1] = l1_slice_bits >= 0 ? srank_[1].as<const uint32_t>() : nullptr;
   return v;
-}
-
-template <class KeyT>
-uint64_t BBHashBuild<KeyT>::level_words(uint32_t l) const {
-  return l < nwords.size() ? nwords[l] : 0;
 }
 
 template struct BBHashBuild<uint64_t>;

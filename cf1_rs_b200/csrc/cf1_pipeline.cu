@@ -559,7 +559,7 @@ void run_impl(cf1gpu_ctx *c, StreamIO *io = nullptr, Step step = Step::FULL, con
     CF1_CUDA(cudaMemcpyAsync(woff1, hw1.data(), (B + 1) * sizeof(uint64_t), cudaMemcpyHostToDevice, s));
     CF1_CUDA(cudaMemcpyAsync(room_off, hr.data(), (B + 1) * sizeof(uint64_t), cudaMemcpyHostToDevice, s));
     CF1_CUDA(cudaMemsetAsync(scnt, 0, B * sizeof(uint64_t), s));
-    l0.AR = be.bb.prepare_levels01(l0_words, l1_words, s);  // every slice writes all of its entries
+    l0.AR = be.bb.prepare_levels01(B, l0_words, l1_words, s);  // every slice writes all of its entries
     l0.woff = woff0;
     l0.AR1 = l0.AR + l0_words;
     l0.woff1 = woff1;
@@ -629,13 +629,14 @@ void run_impl(cf1gpu_ctx *c, StreamIO *io = nullptr, Step step = Step::FULL, con
   const uint64_t half = (NO + 1) / 2;
   if (c->opts.mphf_mode == CF1GPU_MPHF_LEARNED) {
     be.li.build(dist, dist_off, B, k, c->learned, s);
-    be.bb.build(dist, dist_off, B, be.li.fallback_sel(), s, keys, ws1, NO + 1);
+    be.bb.build(dist, dist_off, B, be.li.fallback_sel(), &sm->err, s, keys, ws1, NO + 1);
   } else if (l0_ready) {
     be.bb.build_from_levels01(B, P, l0.woff, l0_words, l0.placed, l0.woff1, l1_words, l0.placed1,
                               reinterpret_cast<const KeyT *>(l0.surv), l0.surv_off,
-                              reinterpret_cast<const uint64_t *>(l0.surv_cnt), l0_room, s, twin, twin + half, half);
+                              reinterpret_cast<const uint64_t *>(l0.surv_cnt), l0_room, NO, &sm->err, s, twin, twin + half,
+                              half);
   } else {
-    be.bb.build(dist, dist_off, B, nullptr, s, keys, ws1, NO + 1);
+    be.bb.build(dist, dist_off, B, nullptr, &sm->err, s, keys, ws1, NO + 1);
   }
   CF1_CUDA(cudaEventRecord(c->ev[4], s));
 
@@ -746,7 +747,9 @@ void run_impl(cf1gpu_ctx *c, StreamIO *io = nullptr, Step step = Step::FULL, con
   }
   CF1_CUDA(cudaEventRecord(c->ev[7], s));
   CF1_CUDA(cudaMemcpyAsync(&hs, sm, sizeof(Small), cudaMemcpyDeviceToHost, s));
+  be.bb.collect_begin(s);
   CF1_CUDA(cudaStreamSynchronize(s));
+  be.bb.collect_end();
   check_device_errors(hs.err);
   c->cas_retries = hs.cas_retries;
 
