@@ -218,7 +218,7 @@ __global__ void __launch_bounds__(BF_BLOCK) bb_sliced_kernel(const uint64_t *wof
 // Launched once the keys left are few (BF_KEYS a bin on average: a level of
 // that many keys takes the CTA ~15 us, and one launch of its own ~55 us with
 // the wait for its size).  A run's MPHF phase, nine launches and a wait per
-// level before: 30 kb 240 -> 20 us, 200 Mbp 590 -> 60 us.
+// level before: 30 kb 240 -> 49 us, 200 Mbp 586 -> 87 us.
 constexpr uint32_t BF_WORDS = 4096;
 constexpr uint64_t BF_KEYS = 16384;
 // Entries reserved for n keys: the levels' blocks sum up to ~1.14 times the

@@ -34,7 +34,7 @@ namespace {
 
 constexpr int LT_BLOCK = 256;
 constexpr int LT_NW = LT_BLOCK / 32;
-constexpr uint32_t LT_TILE = 4096;
+constexpr uint32_t LT_TILE = 16384;  // keys per CTA: the tile's set-up (segment, root, piece) is a chain of loads
 constexpr uint32_t LT_MAX_SAMPLES = 4096;
 constexpr int H = LI_HIDDEN;
 
@@ -63,7 +63,7 @@ CF1_HD void mlp_accumulate(const float *P, float x, float t, float scale, float 
   }
 }
 
-// Trained parameters Q (2H+1): knot logits theta[H], output weights w2[H],
+// Trained parameters q (2H+1): knot logits theta[H], output weights w2[H],
 // output bias b2.  The first layer is derived from the knots: widths
 // d = softmax(theta), knots t_j = sum_{i<j} d_i, w1_j = 1/d_j,
 // b1_j = -t_j/d_j, so unit j ramps over [t_j, t_j + d_j] and the ramps tile
@@ -71,46 +71,203 @@ CF1_HD void mlp_accumulate(const float *P, float x, float t, float scale, float 
 // every key in it to one leaf).
 constexpr int LI_NQ = 2 * H + 1;
 
-// P (the MLP's w1 b1 w2 b2) from Q; d and t kept for the chain rule.
-CF1_D void derive_params(const float *Q, float *P, float *d, float *t) {
-  float m = Q[0];
-  for (int j = 1; j < H; j++) m = fmaxf(m, Q[j]);
-  float s = 0.f;
-  for (int j = 0; j < H; j++) {
-    d[j] = expf(Q[j] - m);
-    s += d[j];
+// Because the ramps tile [0, 1], a sample x on ramp j has every earlier unit
+// saturated and every later one at 0: its output is base_j + w2_j act(z_j)
+// with base_j = b2 + sum_{i<j} w2_i, and with dy = dLoss/dy its gradient is
+// dy for b2 and the w2 before j, dy act(z_j) for w2_j, dy w2_j (x, 1) for
+// (w1_j, b1_j) inside the ramp.  So a step needs four sums per ramp instead
+// of 16 units per sample:
+//   A_j = sum dy, B_j = sum dy act(z_j), C_j = sum dz, D_j = sum dz x.
+struct LiRamps {
+  float knot[H], w1[H], b1[H], w2[H], base[H];
+};
+
+// Exclusive prefix (from lane 0) and suffix (from lane H - 1) sums, the sum
+// and the maximum over lanes 0 .. H-1 of a warp (H = 16; the upper half warp
+// repeats the lower).
+CF1_D float li_prefix(float v, unsigned j) {
+  float x = v;
+#pragma unroll
+  for (int o = 1; o < H; o <<= 1) {
+    const float y = __shfl_up_sync(FULL, x, o, H);
+    if (j >= (unsigned)o) x += y;
   }
-  float acc = 0.f;
-  for (int j = 0; j < H; j++) {
-    d[j] = d[j] / s;
-    t[j] = acc;
-    acc += d[j];
-    P[j] = 1.f / d[j];
-    P[H + j] = -t[j] / d[j];
-    P[2 * H + j] = Q[H + j];
+  const float e = __shfl_up_sync(FULL, x, 1, H);
+  return j ? e : 0.f;
+}
+CF1_D float li_suffix(float v, unsigned j) {
+  float x = v;
+#pragma unroll
+  for (int o = 1; o < H; o <<= 1) {
+    const float y = __shfl_down_sync(FULL, x, o, H);
+    if (j + o < (unsigned)H) x += y;
   }
-  P[3 * H] = Q[2 * H];
+  const float e = __shfl_down_sync(FULL, x, 1, H);
+  return j + 1 < (unsigned)H ? e : 0.f;
+}
+CF1_D float li_sum(float v) {
+#pragma unroll
+  for (int o = H / 2; o > 0; o >>= 1) v += __shfl_xor_sync(FULL, v, o, H);
+  return v;
+}
+CF1_D float li_max(float v) {
+#pragma unroll
+  for (int o = H / 2; o > 0; o >>= 1) v = fmaxf(v, __shfl_xor_sync(FULL, v, o, H));
+  return v;
 }
 
-// dL/dQ from dL/dP (chain rule through w1 = 1/d, b1 = -t/d, the knot sums
-// and the softmax).
-CF1_D void grad_q(const float *G, const float *d, const float *t, float *GQ) {
-  float gd[H];
-  for (int j = 0; j < H; j++) gd[j] = -G[j] / (d[j] * d[j]) + G[H + j] * t[j] / (d[j] * d[j]);
-  float acc = 0.f;  // t_j = sum_{i<j} d_i: d_i collects dL/dt_j of every j > i
-  for (int j = H - 1; j >= 0; j--) {
-    gd[j] += acc;
-    acc += -G[H + j] / d[j];
+// One warp, lane j (mod H) for unit j: the ramps of (theta_j, w2_j, b2) to s;
+// returns the width d_j and knot t_j.
+CF1_D void li_ramps(float theta, float w2, float b2, LiRamps &s, float &d, float &t) {
+  const unsigned j = lane_id() % H;
+  d = expf(theta - li_max(theta));
+  d = d / li_sum(d);
+  t = li_prefix(d, j);
+  const float before = li_prefix(w2, j);
+  const float w1 = 1.f / d;
+  if (lane_id() < H) {
+    s.knot[j] = t;
+    s.w1[j] = w1;
+    s.b1[j] = -t * w1;
+    s.w2[j] = w2;
+    s.base[j] = b2 + before;
   }
-  float dot = 0.f;
-  for (int j = 0; j < H; j++) dot += d[j] * gd[j];
-  for (int j = 0; j < H; j++) GQ[j] = d[j] * (gd[j] - dot);
-  for (int j = 0; j < H; j++) GQ[H + j] = G[2 * H + j];
-  GQ[2 * H] = G[3 * H];
+}
+
+// The ramp of x: the last knot at or below it (binary search; knot[0] = 0).
+CF1_D uint32_t li_ramp_of(const LiRamps &s, float x) {
+  uint32_t j = 0;
+#pragma unroll
+  for (uint32_t o = H / 2; o > 0; o >>= 1) j += x >= s.knot[j + o] ? o : 0u;
+  return j;
+}
+CF1_D float li_ramp_eval(const LiRamps &s, float x, uint32_t j, float &z) {
+  z = f_fma(s.w1[j], x, s.b1[j]);
+  return f_fma(s.w2[j], li_act(z), s.base[j]);
+}
+
+constexpr int LS_BLOCK = 512;  // training block
+constexpr int LS_NW = LS_BLOCK / 32;
+struct LiSums {
+  float4 w[LS_NW][H];  // per warp and ramp: A, B, C, D
+};
+
+// Sums over a warp of four values a lane:
+// four butterflies in six shuffles (two steps halve the values a lane keeps,
+// three finish its quarter); lane 8 i holds value i.
+CF1_D float li_reduce4(float a, float b, float c, float d) {
+  const unsigned lane = lane_id();
+  const bool hi = lane & 16, hi2 = lane & 8;
+  float s0 = hi ? a : c, s1 = hi ? b : d;  // sent to the other half
+  float k0 = hi ? c : a, k1 = hi ? d : b;  // kept
+  k0 += __shfl_xor_sync(FULL, s0, 16);
+  k1 += __shfl_xor_sync(FULL, s1, 16);
+  float k = hi2 ? k1 : k0;
+  k += __shfl_xor_sync(FULL, hi2 ? k0 : k1, 8);
+#pragma unroll
+  for (int o = 4; o > 0; o >>= 1) k += __shfl_xor_sync(FULL, k, o);
+  return k;
+}
+
+// The block's samples x[0, n), targets t: every warp's sums per ramp.  All
+// threads call it; the caller synchronises around it.  A warp takes 128
+// consecutive samples at a time, four a lane (their searches and evaluations
+// overlap), and reduces once per ramp among them: sorted samples (training)
+// share a ramp or two, any others just take more rounds.
+constexpr int LS_ROWS = 4;
+CF1_D void li_accumulate(const LiRamps &s, const float *x, const float *t, uint32_t n, float scale, LiSums &sums) {
+  const unsigned lane = lane_id(), warp = threadIdx.x >> 5;
+  float *acc = reinterpret_cast<float *>(sums.w[warp]);
+  acc[lane] = 0.f;
+  acc[lane + 32] = 0.f;
+  __syncwarp();
+  for (uint32_t i0 = warp * (32 * LS_ROWS); i0 < n; i0 += LS_BLOCK * LS_ROWS) {
+    float xi[LS_ROWS], dy[LS_ROWS], z[LS_ROWS];
+    uint32_t j[LS_ROWS];
+#pragma unroll
+    for (int r = 0; r < LS_ROWS; r++) {
+      const uint32_t i = i0 + r * 32 + lane;
+      xi[r] = i < n ? x[i] : 0.f;
+      dy[r] = i < n ? t[i] : 0.f;
+      j[r] = li_ramp_of(s, xi[r]);
+    }
+    uint32_t todo = (uint32_t)H;  // the smallest ramp not reduced yet
+#pragma unroll
+    for (int r = 0; r < LS_ROWS; r++) {
+      const float y = li_ramp_eval(s, xi[r], j[r], z[r]);
+      dy[r] = 2.f * (y - dy[r]) * scale;
+      if (i0 + r * 32 + lane >= n) j[r] = (uint32_t)H;
+      todo = min(todo, j[r]);
+    }
+    todo = __reduce_min_sync(FULL, todo);
+    while (todo < (uint32_t)H) {
+      float a = 0.f, b = 0.f, c = 0.f, d = 0.f;
+      const float w2 = s.w2[todo];
+      uint32_t next = (uint32_t)H;
+#pragma unroll
+      for (int r = 0; r < LS_ROWS; r++) {
+        if (j[r] == todo) {
+          const float dz = (z[r] > 0.f && z[r] < 1.f) ? dy[r] * w2 : 0.f;
+          a += dy[r];
+          b += dy[r] * li_act(z[r]);
+          c += dz;
+          d += dz * xi[r];
+        } else if (j[r] > todo) {
+          next = min(next, j[r]);
+        }
+      }
+      const float v = li_reduce4(a, b, c, d);
+      if ((lane & 7) == 0) acc[4 * todo + (lane >> 3)] += v;
+      todo = __reduce_min_sync(FULL, next);
+    }
+  }
+}
+
+// One warp, lane j (mod H): the gradient with respect to (theta_j, w2_j) and
+// b2 from the block's sums, by the chain rule through w1 = 1/d, b1 = -t/d, the
+// knot sums and the softmax.
+CF1_D void li_grad(const LiSums &sums, float d, float t, float &g_theta, float &g_w2, float &g_b2) {
+  const unsigned j = lane_id() % H;
+  float a = 0.f, b = 0.f, c = 0.f, e = 0.f;
+#pragma unroll
+  for (int w = 0; w < LS_NW; w++) {
+    const float4 v = sums.w[w][j];
+    a += v.x;
+    b += v.y;
+    c += v.z;
+    e += v.w;
+  }
+  g_w2 = b + li_suffix(a, j);
+  g_b2 = li_sum(a);
+  const float w1 = 1.f / d;
+  float gd = (c * t - e) * (w1 * w1);
+  gd -= li_suffix(c * w1, j);  // t_j = sum_{i<j} d_i: d_i collects dL/dt_j of every j > i
+  g_theta = d * (gd - li_sum(d * gd));
+}
+
+// Mean squared error of the block's samples, to every thread.
+CF1_D float li_loss(const LiRamps &s, const float *x, const float *t, uint32_t n, float scale, float *sm) {
+  float loss = 0.f;
+  for (uint32_t i = threadIdx.x; i < n; i += LS_BLOCK) {
+    float z;
+    const float e = li_ramp_eval(s, x[i], li_ramp_of(s, x[i]), z) - t[i];
+    loss += e * e * scale;
+  }
+  return block_sum<LS_BLOCK>(loss, sm);
 }
 
 // Adam step size per group: logits O(1), output weights O(1/H).
-CF1_D float lr_scale_q(int q) { return q < H ? 1.f : 1.f / (float)H; }
+struct LiAdam {
+  float m = 0.f, v = 0.f;
+  // One update with gradient g; 1 / (1 - beta^step) come as c1, c2.
+  CF1_D float step(float q, float g, float lr, float c1, float c2) {
+    const float beta1 = 0.9f, beta2 = 0.999f, eps = 1e-8f;
+    m = beta1 * m + (1.f - beta1) * g;
+    v = beta2 * v + (1.f - beta2) * g * g;
+    const float mh = m * c1, vh = v * c2;
+    return q - lr * mh / (sqrtf(vh) + eps);
+  }
+};
 
 // Block reduction of the NPARAM gradient sums and the loss into red/sl.
 CF1_D void reduce_grads(float *g, float loss, float (*red)[LI_NPARAM + 1]) {
@@ -124,16 +281,22 @@ CF1_D void reduce_grads(float *g, float loss, float (*red)[LI_NPARAM + 1]) {
   if (lane == 0) red[warp][LI_NPARAM] = l;
 }
 
+// One CTA per bin: full-batch Adam over the bin's CDF samples.  A step is the
+// sums (all warps), a barrier, the update by one warp with a lane per unit,
+// and a barrier; its latency, not throughput, is what a run of few bins waits
+// for.  With 16 units per sample, the 49 gradient sums reduced one by one and
+// the update on one thread a step took 9.5 us (128 bins of 200 Mbp, 300
+// steps: 2.87 ms), this way 2.3 us (0.70 ms).
 template <class KeyT>
-__global__ void __launch_bounds__(LT_BLOCK) li_train_kernel(const KeyT *keys, const uint64_t *dist_off, LIRoot *roots,
+__global__ void __launch_bounds__(LS_BLOCK) li_train_kernel(const KeyT *keys, const uint64_t *dist_off, LIRoot *roots,
                                                            int k, int steps, float lr, uint32_t max_samples,
                                                            float *loss_out) {
   __shared__ float sx[LT_MAX_SAMPLES], st[LT_MAX_SAMPLES];
-  __shared__ float P[LI_NPARAM], Q[LI_NQ], GQ[LI_NQ], M1[LI_NQ], M2[LI_NQ], sd[H], stk[H];
-  __shared__ float red[LT_NW][LI_NPARAM + 1];
-  __shared__ float s_loss;
+  __shared__ LiRamps ramps;
+  __shared__ LiSums sums;
+  __shared__ float sm[LS_NW];
   const uint32_t b = blockIdx.x;
-  const unsigned tid = threadIdx.x;
+  const unsigned tid = threadIdx.x, j = lane_id() % H;
   const uint64_t base = dist_off[b], n = dist_off[b + 1] - base;
   LIRoot &R = roots[b];
   uint64_t hmin = 0, hmax = 0;
@@ -144,106 +307,69 @@ __global__ void __launch_bounds__(LT_BLOCK) li_train_kernel(const KeyT *keys, co
     inv = hmax > hmin ? __fdiv_rn(1.f, u64_to_f(hmax - hmin)) : 0.f;
   }
   uint32_t S = (uint32_t)(n < max_samples ? n : max_samples);
-  for (uint32_t i = tid; i < S; i += LT_BLOCK) {
+  for (uint32_t i = tid; i < S; i += LS_BLOCK) {
     uint64_t r = (uint64_t)i * n / S;
     uint64_t h = KOps<KeyT>::high64(keys[base + r], k);
     sx[i] = f_mul(u64_to_f(h - hmin), inv);
     st[i] = (float)((double)r / (double)n);
   }
-  if (tid < LI_NQ) {
-    // identity root: equal knot logits (unit j ramps over [j/H, (j+1)/H]),
-    // output weights 1/H, so root(x) = x -- the index without a trained network
-    Q[tid] = tid < H ? 0.f : (tid < 2 * H ? 1.f / (float)H : 0.f);
-    M1[tid] = 0.f;
-    M2[tid] = 0.f;
-  }
-  if (tid == 0) s_loss = 0.f;
-  __syncthreads();
-  if (tid == 0) derive_params(Q, P, sd, stk);
+  // identity root: equal knot logits (unit j ramps over [j/H, (j+1)/H]),
+  // output weights 1/H, so root(x) = x -- the index without a trained network
+  float theta = 0.f, w2 = 1.f / (float)H, b2 = 0.f, d = 0.f, t = 0.f;  // lane j of warp 0: unit j's
+  LiAdam at, aw, ab;
+  if (tid < 32) li_ramps(theta, w2, b2, ramps, d, t);
   __syncthreads();
   const float scale = S ? 1.f / (float)S : 0.f;
-  const float beta1 = 0.9f, beta2 = 0.999f, eps = 1e-8f;
   float b1t = 1.f, b2t = 1.f;
   for (int step = 0; step < steps && S > 0; step++) {
-    float g[LI_NPARAM];
-#pragma unroll
-    for (int p = 0; p < LI_NPARAM; p++) g[p] = 0.f;
-    float loss = 0.f;
-    for (uint32_t i = tid; i < S; i += LT_BLOCK) mlp_accumulate(P, sx[i], st[i], scale, g, loss);
-    reduce_grads(g, loss, red);
+    li_accumulate(ramps, sx, st, S, scale, sums);
     __syncthreads();
-    if (tid == 0) {
-      float G[LI_NPARAM];
-      for (int p = 0; p < LI_NPARAM; p++) {
-        float v = 0.f;
-        for (int w = 0; w < LT_NW; w++) v += red[w][p];
-        G[p] = v;
-      }
-      grad_q(G, sd, stk, GQ);
-      float l = 0.f;
-      for (int w = 0; w < LT_NW; w++) l += red[w][LI_NPARAM];
-      s_loss = l;
-    }
-    __syncthreads();
-    if (tid < LI_NQ) {
-      float G = GQ[tid];
-      b1t *= beta1;
-      b2t *= beta2;
-      M1[tid] = beta1 * M1[tid] + (1.f - beta1) * G;
-      M2[tid] = beta2 * M2[tid] + (1.f - beta2) * G * G;
-      float mh = M1[tid] / (1.f - b1t), vh = M2[tid] / (1.f - b2t);
-      float nq = Q[tid] - lr * lr_scale_q(tid) * mh / (sqrtf(vh) + eps);
+    if (tid < 32) {
+      float g_theta, g_w2, g_b2;
+      li_grad(sums, d, t, g_theta, g_w2, g_b2);
+      b1t *= 0.9f;
+      b2t *= 0.999f;
+      const float c1 = 1.f / (1.f - b1t), c2 = 1.f / (1.f - b2t);
+      theta = at.step(theta, g_theta, lr, c1, c2);
       // projection onto w2 >= 0 (w1 = 1/d > 0 already): non-decreasing root
-      if (tid >= H && tid < 2 * H && nq < 0.f) nq = 0.f;
-      Q[tid] = nq;
+      w2 = fmaxf(aw.step(w2, g_w2, lr / (float)H, c1, c2), 0.f);
+      b2 = ab.step(b2, g_b2, lr / (float)H, c1, c2);
+      li_ramps(theta, w2, b2, ramps, d, t);
     }
-    __syncthreads();
-    if (tid == 0) derive_params(Q, P, sd, stk);
     __syncthreads();
   }
-  // The network on its piecewise-linear form: on [t_j, t_j + d_j) ramps
-  // i < j are saturated and ramps i > j are 0, so the value is
-  // b2 + sum_{i<j} w2_i + (w2_j / d_j) (x - t_j).  Then the output fold: an
-  // affine map with a positive slope sends the bin's smallest key to 0 and
-  // its largest to just below 1, so the leaves cover the keys.
+  // The network on its piecewise-linear form: on [t_j, t_j + d_j) the value is
+  // base_j + (w2_j / d_j) (x - t_j).  Then the output fold: an affine map with
+  // a positive slope sends the bin's smallest key to 0 and its largest to
+  // just below 1, so the leaves cover the keys.
   __shared__ LIRoot s_root;
-  if (tid == 0) {
-    float c = P[3 * H];
-    for (int j = 0; j < H; j++) {
-      s_root.knot[j] = stk[j];
-      s_root.base[j] = c;
-      s_root.slope[j] = P[2 * H + j] / sd[j];
-      c += P[2 * H + j];
+  if (tid < 32) {
+    if (tid < H) {
+      s_root.knot[j] = t;
+      s_root.base[j] = ramps.base[j];
+      s_root.slope[j] = w2 / d;
     }
-    s_root.hmin = hmin;
-    s_root.inv_range = inv;
-    float y0 = li_root_eval(s_root, li_x(s_root, hmin)), y1 = li_root_eval(s_root, li_x(s_root, hmax));
+    if (tid == 0) {
+      s_root.hmin = hmin;
+      s_root.inv_range = inv;
+    }
+    __syncwarp();
+    const float y0 = li_root_eval(s_root, li_x(s_root, hmin)), y1 = li_root_eval(s_root, li_x(s_root, hmax));
+    __syncwarp();
     if (n && y1 > y0) {
-      float a = 0.99999905f / (y1 - y0);
-      for (int j = 0; j < H; j++) {
-        P[2 * H + j] *= a;
+      const float a = 0.99999905f / (y1 - y0);
+      if (tid < H) {
         s_root.base[j] = a * (s_root.base[j] - y0);
         s_root.slope[j] *= a;
       }
-      P[3 * H] = a * P[3 * H] - a * y0;
+      w2 *= a;
+      b2 = a * b2 - a * y0;
+      li_ramps(theta, w2, b2, ramps, d, t);
     }
   }
   __syncthreads();
-  // final loss with the trained parameters
-  {
-    float g[LI_NPARAM];
-#pragma unroll
-    for (int p = 0; p < LI_NPARAM; p++) g[p] = 0.f;
-    float loss = 0.f;
-    for (uint32_t i = tid; i < S; i += LT_BLOCK) mlp_accumulate(P, sx[i], st[i], scale, g, loss);
-    reduce_grads(g, loss, red);
-    __syncthreads();
-    if (tid == 0) {
-      float l = 0.f;
-      for (int w = 0; w < LT_NW; w++) l += red[w][LI_NPARAM];
-      loss_out[b] = l;
-    }
-  }
+  const float loss = li_loss(ramps, sx, st, S, scale, sm);  // with the trained parameters
+  if (tid == 0) loss_out[b] = loss;
   if (tid < H) {
     R.knot[tid] = s_root.knot[tid];
     R.base[tid] = s_root.base[tid];
@@ -255,10 +381,43 @@ __global__ void __launch_bounds__(LT_BLOCK) li_train_kernel(const KeyT *keys, co
   }
 }
 
+// The root of a tile's bin in shared memory, and the piece of it the whole
+// tile lies on, when it does (piece < H).  The tile's keys ascend and li_x
+// does not decrease with the key, so when its first and last key are on one
+// piece, all are: most tiles then skip the 15 comparisons per key, and none
+// reads the root from global memory (200 Mbp, the three passes over the keys:
+// 4.07 -> 2.33 ms with this, larger tiles and the err pass's shared maxima).  (The judge does not assume the order: a tile with keys out of
+// order is reported bad whatever their pieces.)
+struct LiTile {
+  LIRoot r;
+  uint32_t piece;
+};
+CF1_D uint32_t li_piece(const LIRoot &r, float x) {
+  uint32_t j = 0;
+#pragma unroll
+  for (int i = 1; i < H; i++) j += x >= r.knot[i] ? 1u : 0u;
+  return j;
+}
 template <class KeyT>
-CF1_D uint32_t key_leaf(const LIRoot &R, const KeyT &key, int k, uint64_t &h) {
-  h = KOps<KeyT>::high64(key, k);
-  return li_leaf_of(R, li_root_eval(R, li_x(R, h)));
+CF1_D void li_tile(const LIRoot &R, const KeyT *keys, uint64_t start, uint64_t end, int k, LiTile &t) {
+  constexpr uint32_t NWD = sizeof(LIRoot) / 4;
+  static_assert(sizeof(LIRoot) % 4 == 0 && NWD <= LT_BLOCK, "a word a thread");
+  if (threadIdx.x < NWD)
+    reinterpret_cast<uint32_t *>(&t.r)[threadIdx.x] = reinterpret_cast<const uint32_t *>(&R)[threadIdx.x];
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    const uint32_t a = li_piece(t.r, li_x(t.r, KOps<KeyT>::high64(keys[start], k)));
+    const uint32_t b = li_piece(t.r, li_x(t.r, KOps<KeyT>::high64(keys[end - 1], k)));
+    t.piece = a == b ? a : (uint32_t)H;
+  }
+  __syncthreads();
+}
+// Leaf of the key with high bits h: li_leaf_of(li_root_eval(li_x(h))), the
+// piece given by the tile when it has one.
+CF1_D uint32_t li_tile_leaf(const LiTile &t, uint64_t h) {
+  const float x = li_x(t.r, h);
+  const uint32_t j = t.piece < (uint32_t)H ? t.piece : li_piece(t.r, x);
+  return li_leaf_of(t.r, f_fma(t.r.slope[j], f_sub(x, t.r.knot[j]), t.r.base[j]));
 }
 
 // Runs of equal leaves inside a warp (the lanes hold consecutive keys, and a
@@ -285,14 +444,15 @@ __global__ void __launch_bounds__(LT_BLOCK) li_assign_kernel(const KeyT *keys, c
   const uint32_t t = blockIdx.x;
   if (t >= tile_off[nbins]) return;
   TileSpan sp = tile_span(dist_off, tile_off, nbins, t, LT_TILE);
-  const LIRoot &R = roots[sp.seg];
+  __shared__ LiTile s_tile;
+  li_tile(roots[sp.seg], keys, sp.start, sp.end, k, s_tile);
+  const LIRoot &R = s_tile.r;
   const uint64_t base = dist_off[sp.seg];
   const unsigned lane = lane_id();
   for (uint64_t i0 = sp.start; i0 < sp.end; i0 += LT_BLOCK) {
     uint64_t i = i0 + threadIdx.x;
     bool act = i < sp.end;
-    uint64_t h;
-    uint32_t leaf = act ? key_leaf(R, keys[i], k, h) : 0xFFFFFFFFu;
+    uint32_t leaf = act ? li_tile_leaf(s_tile, KOps<KeyT>::high64(keys[i], k)) : 0xFFFFFFFFu;
     uint32_t rank = (uint32_t)(i - base);
     unsigned heads;
     const uint32_t hl = run_head_lane(leaf, lane, heads);
@@ -335,40 +495,37 @@ __global__ void li_fit_kernel(const KeyT *keys, const uint64_t *dist_off, const 
   leaves[g] = L;
 }
 
-// Per leaf: the largest |prediction - rank| over its keys (a segmented max
-// over each warp's runs, one atomic per run).
+// Per leaf: the largest |prediction - rank| over its keys.  A tile's leaves
+// are consecutive (about 512 of them): their maxima are collected in shared
+// memory (leaves outside the window, if any, go to global memory directly).
+constexpr uint32_t LE_WIN = 1024;
 template <class KeyT>
-__global__ void __launch_bounds__(LT_BLOCK) li_err_kernel(const KeyT *keys, const uint64_t *dist_off,
+__global__ void __launch_bounds__(LT_BLOCK, 6) li_err_kernel(const KeyT *keys, const uint64_t *dist_off,
                                                          const uint32_t *tile_off, uint32_t nbins,
                                                          const LIRoot *roots, int k, LILeaf *leaves) {
+  __shared__ LiTile s_tile;
+  __shared__ uint32_t s_err[LE_WIN];
   const uint32_t t = blockIdx.x;
   if (t >= tile_off[nbins]) return;
   TileSpan sp = tile_span(dist_off, tile_off, nbins, t, LT_TILE);
-  const LIRoot &R = roots[sp.seg];
-  const uint64_t base = dist_off[sp.seg];
-  const unsigned lane = lane_id();
-  for (uint64_t i0 = sp.start; i0 < sp.end; i0 += LT_BLOCK) {
-    uint64_t i = i0 + threadIdx.x;
-    bool act = i < sp.end;
-    uint64_t h = 0;
-    uint32_t leaf = act ? key_leaf(R, keys[i], k, h) : 0xFFFFFFFFu;
-    uint32_t e = 0;
-    if (act) {
-      int64_t p = li_predict(leaves[R.leaf_off + leaf], h);
-      int64_t d = p - (int64_t)(i - base);
-      d = d < 0 ? -d : d;
-      e = d > 0xFFFFFFF0ll ? 0xFFFFFFF0u : (uint32_t)d;
-    }
-    unsigned heads;
-    const uint32_t hl = run_head_lane(leaf, lane, heads);
-    const bool tail = run_tail(leaf, lane);
-#pragma unroll
-    for (int d = 1; d < 32; d <<= 1) {
-      const uint32_t v = __shfl_up_sync(FULL, e, d);
-      if (lane >= hl + d) e = v > e ? v : e;
-    }
-    if (act && tail) atomicMax(&leaves[R.leaf_off + leaf].err, e);
+  for (uint32_t i = threadIdx.x; i < LE_WIN; i += LT_BLOCK) s_err[i] = 0;
+  li_tile(roots[sp.seg], keys, sp.start, sp.end, k, s_tile);
+  const uint32_t leaf0 = li_tile_leaf(s_tile, KOps<KeyT>::high64(keys[sp.start], k));
+  LILeaf *bl = leaves + s_tile.r.leaf_off;
+  uint32_t rank = (uint32_t)(sp.start - dist_off[sp.seg]) + threadIdx.x;
+#pragma unroll 4
+  for (uint64_t i = sp.start + threadIdx.x; i < sp.end; i += LT_BLOCK, rank += LT_BLOCK) {
+    const uint64_t h = KOps<KeyT>::high64(keys[i], k);
+    const uint32_t leaf = li_tile_leaf(s_tile, h);
+    int64_t d = li_predict(bl[leaf], h) - (int64_t)rank;
+    d = d < 0 ? -d : d;
+    const uint32_t e = d > 0xFFFFFFF0ll ? 0xFFFFFFF0u : (uint32_t)d;
+    if (leaf - leaf0 < LE_WIN) atomicMax(&s_err[leaf - leaf0], e);
+    else atomicMax(&bl[leaf].err, e);
   }
+  __syncthreads();
+  for (uint32_t i = threadIdx.x; i < LE_WIN; i += LT_BLOCK)
+    if (s_err[i]) atomicMax(&bl[leaf0 + i].err, s_err[i]);
 }
 
 // One CTA per bin: the bin's largest leaf error decides learned vs BBHash.
@@ -413,21 +570,28 @@ __global__ void __launch_bounds__(LT_BLOCK) li_decide_kernel(const uint64_t *dis
 // maps the bin's keys one to one onto [0, n) -- in one streaming read of the
 // keys, with no search.
 template <class KeyT>
-__global__ void __launch_bounds__(LT_BLOCK) li_verify_kernel(const KeyT *keys, const uint64_t *dist_off,
+__global__ void __launch_bounds__(LT_BLOCK, 6) li_verify_kernel(const KeyT *keys, const uint64_t *dist_off,
                                                            const uint32_t *tile_off, uint32_t nbins, LIView v,
                                                            uint32_t *miss) {
   const uint32_t t = blockIdx.x;
   if (t >= tile_off[nbins]) return;
   TileSpan sp = tile_span(dist_off, tile_off, nbins, t, LT_TILE);
   if (!v.roots[sp.seg].use_learned) return;
-  const uint64_t base = dist_off[sp.seg], n = dist_off[sp.seg + 1] - base;
+  const uint64_t base = dist_off[sp.seg];
+  __shared__ LiTile s_tile;
+  li_tile(v.roots[sp.seg], keys, sp.start, sp.end, v.k, s_tile);
+  // the window [p - err, p + err] clamped to the bin's ranks holds the rank r
+  // exactly when |p - r| <= err
+  const LILeaf *leaves = v.leaves + s_tile.r.leaf_off;
   bool bad = false;
+#pragma unroll 4
   for (uint64_t i = sp.start + threadIdx.x; i < sp.end; i += LT_BLOCK) {
     const KeyT key = keys[i];
-    const int64_t r = (int64_t)(i - base);
-    int64_t lo, hi;
-    const bool found = li_window(v, n, sp.seg, key, lo, hi) && lo <= r && r <= hi;
-    bad |= !found || (r > 0 && !(keys[i - 1] < key));
+    const uint64_t h = KOps<KeyT>::high64(key, v.k);
+    const LILeaf lf = leaves[li_tile_leaf(s_tile, h)];
+    int64_t d = li_predict(lf, h) - (int64_t)(i - base);
+    d = d < 0 ? -d : d;
+    bad |= lf.n == 0 || d > (int64_t)lf.err || (i > base && !(keys[i - 1] < key));
   }
   if (__syncthreads_or(bad) && threadIdx.x == 0) miss[sp.seg] = 1;
 }
@@ -462,40 +626,32 @@ __global__ void __launch_bounds__(LT_BLOCK) li_grad_kernel(const float *params, 
   }
 }
 
-// One training step's gradient with respect to the trained parameters Q:
-// the same derive_params, mlp_accumulate, reduce_grads and grad_q calls
-// li_train_kernel makes before its Adam update, over n given samples.
-__global__ void __launch_bounds__(LT_BLOCK) li_grad_q_kernel(const float *q, const float *x, const float *t,
+// One training step's gradient with respect to the trained parameters q:
+// the same li_ramps, li_accumulate and li_grad calls li_train_kernel makes
+// before its Adam update, over n given samples.
+__global__ void __launch_bounds__(LS_BLOCK) li_grad_q_kernel(const float *q, const float *x, const float *t,
                                                             uint32_t n, float *gq_out, float *loss_out) {
-  __shared__ float P[LI_NPARAM], Q[LI_NQ], GQ[LI_NQ], sd[H], stk[H];
-  __shared__ float red[LT_NW][LI_NPARAM + 1];
-  const unsigned tid = threadIdx.x;
-  if (tid < LI_NQ) Q[tid] = q[tid];
+  __shared__ LiRamps ramps;
+  __shared__ LiSums sums;
+  __shared__ float sm[LS_NW];
+  const unsigned tid = threadIdx.x, j = tid % H;
+  float d = 0.f, tk = 0.f;
+  if (tid < 32) li_ramps(q[j], q[H + j], q[2 * H], ramps, d, tk);
   __syncthreads();
-  if (tid == 0) derive_params(Q, P, sd, stk);
-  __syncthreads();
-  float g[LI_NPARAM];
-#pragma unroll
-  for (int p = 0; p < LI_NPARAM; p++) g[p] = 0.f;
-  float loss = 0.f;
   const float scale = n ? 1.f / (float)n : 0.f;
-  for (uint32_t i = tid; i < n; i += LT_BLOCK) mlp_accumulate(P, x[i], t[i], scale, g, loss);
-  reduce_grads(g, loss, red);
+  li_accumulate(ramps, x, t, n, scale, sums);
   __syncthreads();
-  if (tid == 0) {
-    float G[LI_NPARAM];
-    for (int p = 0; p < LI_NPARAM; p++) {
-      float v = 0.f;
-      for (int w = 0; w < LT_NW; w++) v += red[w][p];
-      G[p] = v;
+  if (tid < 32) {
+    float g_theta, g_w2, g_b2;
+    li_grad(sums, d, tk, g_theta, g_w2, g_b2);
+    if (tid < H) {
+      gq_out[tid] = g_theta;
+      gq_out[H + tid] = g_w2;
     }
-    grad_q(G, sd, stk, GQ);
-    float l = 0.f;
-    for (int w = 0; w < LT_NW; w++) l += red[w][LI_NPARAM];
-    *loss_out = l;
+    if (tid == 0) gq_out[2 * H] = g_b2;
   }
-  __syncthreads();
-  if (tid < LI_NQ) gq_out[tid] = GQ[tid];
+  const float loss = li_loss(ramps, x, t, n, scale, sm);
+  if (tid == 0) *loss_out = loss;
 }
 
 }  // namespace
@@ -537,7 +693,7 @@ void LearnedBuild<KeyT>::build(const KeyT *keys, const uint64_t *dist_off, uint3
   CF1_CUDA(cudaMemsetAsync(loss, 0, nbins * sizeof(float), s));
   uint32_t samples = o.max_samples > LT_MAX_SAMPLES ? LT_MAX_SAMPLES : (o.max_samples ? o.max_samples : 1);
   if (nbins) {
-    li_train_kernel<KeyT><<<nbins, LT_BLOCK, 0, s>>>(keys, dist_off, roots, k, o.train_steps < 0 ? 0 : o.train_steps,
+    li_train_kernel<KeyT><<<nbins, LS_BLOCK, 0, s>>>(keys, dist_off, roots, k, o.train_steps < 0 ? 0 : o.train_steps,
                                                      o.lr, samples, loss);
     CF1_LAUNCH_CHECK();
   }
@@ -646,7 +802,7 @@ void learned_grad_q_host(const float *q, const float *x, const float *t, size_t 
     CF1_CUDA(cudaMemcpy(xx, x, n * 4, cudaMemcpyHostToDevice));
     CF1_CUDA(cudaMemcpy(tt, t, n * 4, cudaMemcpyHostToDevice));
   }
-  li_grad_q_kernel<<<1, LT_BLOCK>>>(qq, xx, tt, (uint32_t)n, g, g + LI_NQ);
+  li_grad_q_kernel<<<1, LS_BLOCK>>>(qq, xx, tt, (uint32_t)n, g, g + LI_NQ);
   CF1_LAUNCH_CHECK();
   float out[LI_NQ + 1];
   CF1_CUDA(cudaMemcpy(out, g, (LI_NQ + 1) * 4, cudaMemcpyDeviceToHost));

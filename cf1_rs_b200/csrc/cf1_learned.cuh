@@ -43,10 +43,11 @@ struct LearnedBuild {
   DevBuf roots_, leaves_, lfirst_, llast_, ln_, leaf_off_, tile_off_, sel_, loss_, errsum_;
 };
 
-// Full-batch MSE loss and gradient of the root MLP on the device (the same
-// code the training kernel runs).  params: LI_NPARAM floats.  Host pointers.
+// Full-batch MSE loss and gradient of the root MLP on the device, for any
+// first layer.  params: LI_NPARAM floats.  Host pointers.
 void learned_grad_host(const float *params, const float *x, const float *t, size_t n, float *grad, float *loss);
-// dL/dQ of one training step (Q = knot logits[16], w2[16], b2), on the current device.
+// dL/dq of one training step (q = knot logits[16], w2[16], b2), on the current
+// device, by the code the training kernel runs.
 void learned_grad_q_host(const float *q, const float *x, const float *t, size_t n, float *grad_q, float *loss);
 
 }  // namespace cf1

@@ -3,11 +3,13 @@
 //   1. one or two multisplit passes on the top P bits of the keys (sorted) or
 //      of key * KEY_SPREAD_MUL (distinct only, up to 5 bits less), segmented
 //      by bin (P chosen so a sub-bucket fits shared memory);
-//   2. one CTA per sub-bucket: a shared-memory hash set keeps one copy of
-//      each key; the sorted form then counting-sorts on the next 10 bits,
-//      insertion-sorts the small buckets (bitonic sort of the whole
-//      sub-bucket if any bucket is large); distinct keys are written back at
-//      the sub-bucket's start;
+//   2. one CTA per run of sub-buckets keeps one copy of each key: by rank in
+//      the run's key range (sorted, sr_dedup_kernel) or by the keys' BBHash
+//      bits (distinct only, gd_dedup_kernel); what neither holds goes to one
+//      CTA per sub-bucket with a shared-memory hash set, which in the sorted
+//      form then counting-sorts on the next 10 bits, insertion-sorts the small
+//      buckets (bitonic sort of the whole sub-bucket if any bucket is large);
+//      distinct keys stay at the start;
 //   3. a scan of the per-sub-bucket counts and a copy into the dense distinct
 //      array; a bin's first sub-bucket gives its slot offset.
 // A sub-bucket above CAP keys (long homopolymers, huge tandem arrays) makes
@@ -608,7 +610,7 @@ __global__ void __launch_bounds__(CS_BLOCK, SORTED ? 2 : 4) cs_sort_unique_kerne
                                                                   uint32_t *oversize, int P, Level0Out l0,
                                                                   uint8_t *TP, uint8_t *UP, const uint2 *clist,
                                                                   const uint64_t *coff, uint32_t nbins,
-                                                                  const uint32_t *jlist) {
+                                                                  const uint32_t *jlist, const uint32_t *klist) {
   constexpr uint32_t CAP = cs_cap<KeyT, SORTED>();
   constexpr bool L0 = !SORTED && KOps<KeyT>::WORDS == 1;
   __shared__ unsigned long long s_l0base;
@@ -622,13 +624,14 @@ __global__ void __launch_bounds__(CS_BLOCK, SORTED ? 2 : 4) cs_sort_unique_kerne
   __shared__ uint32_t sm[CS_BLOCK / 32];
   __shared__ int s_big, s_nchunks, s_bad;
   __shared__ uint32_t s_cnt;
-  uint64_t j = blockIdx.x, jend = j + 1;
+  const uint32_t run = klist ? klist[blockIdx.x] : blockIdx.x;  // klist: the runs the rank dedup left
+  uint64_t j = run, jend = j + 1;
   if (jlist) {  // the sub-buckets the warp dedup left
     j = jlist[blockIdx.x];
     jend = j + 1;
   } else if (clist) {
-    const uint32_t bin = upper_segment(coff, nbins, (uint64_t)blockIdx.x);
-    const uint2 r = clist[((uint64_t)bin << P) + (blockIdx.x - coff[bin])];
+    const uint32_t bin = upper_segment(coff, nbins, (uint64_t)run);
+    const uint2 r = clist[((uint64_t)bin << P) + (run - coff[bin])];
     j = ((uint64_t)bin << P) + r.x;
     jend = ((uint64_t)bin << P) + r.y;
   }
@@ -754,6 +757,249 @@ __global__ void __launch_bounds__(CS_BLOCK, SORTED ? 2 : 4) cs_sort_unique_kerne
                SPw);
     }
   }
+}
+
+// ---------------------------------------------------------------- rank dedup
+// The sorted form's dedup: one CTA per run of consecutive sub-buckets of a
+// bin (the plan's chunks), at most SrCfg::CAP keys, held in registers.  A
+// key's position is its distance from the run's start in the key range,
+// scaled by a shift to NP = 8 CAP bits, so positions ascend with the keys:
+//   1. every occurrence marks its position (set; col when it was set
+//      already).  A position marked once is one key, whose rank is the popcount
+//      of set before it, plus
+//   2. what the shared positions before it hold beyond one key: their
+//      occurrences are gathered, position by position (numbered by a popcount
+//      of col, counted by atomics), and one thread per position sorts its few
+//      keys and joins the copies' payload bytes;
+//   3. keys and bytes are staged in shared memory by rank and written out.
+// ~85% of the keys of unrepeated sequence have a position of their own.  A run
+// that does not fit (a sub-bucket above CAP keys, more than SR_MAXD different
+// keys on one position) is untouched and listed for cs_sort_unique_kernel,
+// whose hash set, 1024-bucket counting sort and insertion sorts this replaces
+// for the others: 200 Mbp 6.89 -> 2.86 ms, at k = 63 100 Mbp 3.51 -> 2.13 ms.
+// Its bound is its barriers and instruction issue, as the group dedup's below.
+constexpr int SR_BLOCK = 512;
+constexpr uint32_t SR_MAXD = 48;
+template <class KeyT>
+struct SrCfg {
+  static constexpr int U = KOps<KeyT>::WORDS == 1 ? 8 : 4;  // keys per thread
+  static constexpr uint32_t CAP = SR_BLOCK * U;
+  static constexpr int LOGNP = KOps<KeyT>::WORDS == 1 ? 15 : 14;
+  static constexpr uint32_t NP = 1u << LOGNP, NWORD = NP / 32;
+  static constexpr int WPT = NWORD / SR_BLOCK;  // words of the bitmaps a thread scans
+  static constexpr int CPT = CAP / 2 / SR_BLOCK;  // shared positions a thread scans
+};
+template <class KeyT>
+struct SrSmem {
+  using C = SrCfg<KeyT>;
+  KeyT seg[C::CAP], stage[C::CAP];
+  uint32_t set[C::NWORD], col[C::NWORD];
+  uint32_t cnt[C::CAP / 2];                     // occurrences, then distinct keys, of a shared position
+  uint16_t start[C::CAP / 2], ex[C::CAP / 2 + 2];  // its place in seg; keys beyond one a position before it
+  uint16_t spre[C::NWORD], cpre[C::NWORD];      // set / col bits before a word
+  uint8_t segp[C::CAP], stagep[C::CAP];
+  uint32_t sm[SR_BLOCK / 32];
+};
+
+template <class KeyT>
+__global__ void __launch_bounds__(SR_BLOCK, 2) sr_dedup_kernel(KeyT *T, uint8_t *TP, const uint64_t *sb_off,
+                                                              uint64_t nsub, int P, int rest, uint32_t *cnt,
+                                                              const uint2 *clist, const uint64_t *coff, uint32_t nbins,
+                                                              uint32_t *ov, uint32_t *ov_cnt) {
+  using C = SrCfg<KeyT>;
+  extern __shared__ __align__(16) unsigned char sr_smem[];
+  SrSmem<KeyT> &m = *reinterpret_cast<SrSmem<KeyT> *>(sr_smem);
+  const unsigned tid = threadIdx.x;
+  uint64_t j = blockIdx.x, jend = j + 1;
+  if (clist) {
+    const uint32_t bin = upper_segment(coff, nbins, (uint64_t)blockIdx.x);
+    const uint2 r = clist[((uint64_t)bin << P) + (blockIdx.x - coff[bin])];
+    j = ((uint64_t)bin << P) + r.x;
+    jend = ((uint64_t)bin << P) + r.y;
+  }
+  if (j >= nsub) return;
+  const uint64_t a = sb_off[j], n64 = sb_off[jend] - a;
+  if (n64 > C::CAP) {
+    if (tid == 0) ov[atomicAdd(ov_cnt, 1u)] = blockIdx.x;
+    return;
+  }
+  for (uint64_t q = j + tid; q < jend; q += SR_BLOCK) cnt[q] = 0;
+  if (n64 == 0) return;
+  const uint32_t n = (uint32_t)n64, sub0 = (uint32_t)(j & ((1ull << P) - 1)), span = (uint32_t)(jend - j);
+  int sh = rest - C::LOGNP;  // the run's range, span << rest, in at most NP positions
+  while ((1u << (sh + C::LOGNP - rest)) < span) sh++;
+  if (sh < 0) sh = 0;
+  const uint32_t pos0 = sub0 << (rest - sh);
+  auto pos_of = [&](const KeyT &k) -> uint32_t { return KOps<KeyT>::digit(k, sh, 0xFFFFFFFFu) - pos0; };
+  KeyT key[C::U];
+  uint32_t pb[C::U / 4];
+#pragma unroll
+  for (int i = 0; i < C::U / 4; i++) pb[i] = 0;
+#pragma unroll
+  for (int u = 0; u < C::U; u++) {
+    const uint32_t i = u * SR_BLOCK + tid;
+    if (i < n) {
+      key[u] = T[a + i];
+      if (TP) pb[u >> 2] |= (uint32_t)TP[a + i] << (8 * (u & 3));
+    }
+  }
+  for (uint32_t w = tid; w < C::NWORD; w += SR_BLOCK) m.set[w] = m.col[w] = 0;
+  __syncthreads();
+  // 1. mark
+#pragma unroll
+  for (int u = 0; u < C::U; u++) {
+    if (u * SR_BLOCK + tid < n) {
+      const uint32_t p = pos_of(key[u]), bm = 1u << (p & 31);
+      if (atomicOr(&m.set[p >> 5], bm) & bm) atomicOr(&m.col[p >> 5], bm);
+    }
+  }
+  __syncthreads();
+  uint32_t nset, ncol;
+  {
+    uint32_t v = 0, x[C::WPT];
+#pragma unroll
+    for (int i = 0; i < C::WPT; i++) {
+      const uint32_t w = tid * C::WPT + i;
+      x[i] = (uint32_t)__popc(m.set[w]) | ((uint32_t)__popc(m.col[w]) << 16);
+      v += x[i];
+    }
+    uint32_t tot, pre = block_exclusive_scan<SR_BLOCK>(v, m.sm, tot);
+#pragma unroll
+    for (int i = 0; i < C::WPT; i++) {
+      const uint32_t w = tid * C::WPT + i;
+      m.spre[w] = (uint16_t)pre;
+      m.cpre[w] = (uint16_t)(pre >> 16);
+      pre += x[i];
+    }
+    nset = tot & 0xFFFFu;
+    ncol = tot >> 16;
+  }
+  uint32_t shared = 0, extra = 0;  // this thread's keys on shared positions; keys beyond one a position
+  if (ncol) {  // uniform
+    // 2. the shared positions' occurrences, counted, placed and sorted
+    for (uint32_t c = tid; c < ncol; c += SR_BLOCK) m.cnt[c] = 0;
+    __syncthreads();
+    uint32_t slot[C::U];
+#pragma unroll
+    for (int u = 0; u < C::U; u++) {
+      slot[u] = 0;
+      if (u * SR_BLOCK + tid < n) {
+        const uint32_t p = pos_of(key[u]), bm = 1u << (p & 31), cw = m.col[p >> 5];
+        if (cw & bm) {
+          const uint32_t c = m.cpre[p >> 5] + (uint32_t)__popc(cw & (bm - 1));
+          shared |= 1u << u;
+          slot[u] = c | (atomicAdd(&m.cnt[c], 1u) << 16);
+        }
+      }
+    }
+    __syncthreads();
+    {
+      uint32_t v = 0, x[C::CPT], tot;
+#pragma unroll
+      for (int i = 0; i < C::CPT; i++) {
+        const uint32_t c = tid * C::CPT + i;
+        x[i] = c < ncol ? m.cnt[c] : 0u;
+        v += x[i];
+      }
+      uint32_t pre = block_exclusive_scan<SR_BLOCK>(v, m.sm, tot);
+#pragma unroll
+      for (int i = 0; i < C::CPT; i++) {
+        const uint32_t c = tid * C::CPT + i;
+        if (c < ncol) m.start[c] = (uint16_t)pre;
+        pre += x[i];
+      }
+    }
+    __syncthreads();
+#pragma unroll
+    for (int u = 0; u < C::U; u++) {
+      if ((shared >> u) & 1) {
+        const uint32_t at = m.start[slot[u] & 0xFFFFu] + (slot[u] >> 16);
+        m.seg[at] = key[u];
+        m.segp[at] = (uint8_t)(pb[u >> 2] >> (8 * (u & 3)));
+      }
+    }
+    __syncthreads();
+    bool over = false;
+    for (uint32_t c = tid; c < ncol && !over; c += SR_BLOCK) {
+      // the position's distinct keys, ascending, at the front of its segment
+      KeyT *S = m.seg + m.start[c];
+      uint8_t *SP = m.segp + m.start[c];
+      const uint32_t len = m.cnt[c];
+      uint32_t d = 1;
+      for (uint32_t i = 1; i < len; i++) {
+        const KeyT x = S[i];
+        const uint8_t xp = SP[i];
+        uint32_t q = d;
+        while (q > 0 && x < S[q - 1]) q--;
+        if (q > 0 && S[q - 1] == x) {
+          SP[q - 1] |= xp;
+          continue;
+        }
+        if (d >= SR_MAXD) {
+          over = true;
+          break;
+        }
+        for (uint32_t r = d; r > q; r--) {
+          S[r] = S[r - 1];
+          SP[r] = SP[r - 1];
+        }
+        S[q] = x;
+        SP[q] = xp;
+        d++;
+      }
+      m.cnt[c] = d;
+    }
+    if (__syncthreads_or((int)over)) {  // nothing of the run was written but zero counts
+      if (tid == 0) ov[atomicAdd(ov_cnt, 1u)] = blockIdx.x;
+      return;
+    }
+    uint32_t v = 0, x[C::CPT];
+#pragma unroll
+    for (int i = 0; i < C::CPT; i++) {
+      const uint32_t c = tid * C::CPT + i;
+      x[i] = c < ncol ? m.cnt[c] - 1 : 0u;
+      v += x[i];
+    }
+    uint32_t pre = block_exclusive_scan<SR_BLOCK>(v, m.sm, extra);
+#pragma unroll
+    for (int i = 0; i < C::CPT; i++) {
+      const uint32_t c = tid * C::CPT + i;
+      if (c <= ncol) m.ex[c] = (uint16_t)pre;
+      pre += x[i];
+    }
+    if (tid == 0) m.ex[ncol] = (uint16_t)extra;  // (ncol may be CAP / 2: no thread's)
+    __syncthreads();
+  } else {
+    if (tid == 0) m.ex[0] = 0;
+    __syncthreads();
+  }
+  // 3. by rank
+  auto rank_of = [&](uint32_t p) -> uint32_t {
+    const uint32_t w = p >> 5, lm = (1u << (p & 31)) - 1;
+    return m.spre[w] + (uint32_t)__popc(m.set[w] & lm) + m.ex[m.cpre[w] + (uint32_t)__popc(m.col[w] & lm)];
+  };
+#pragma unroll
+  for (int u = 0; u < C::U; u++) {
+    if (u * SR_BLOCK + tid < n && !((shared >> u) & 1)) {
+      const uint32_t r = rank_of(pos_of(key[u]));
+      m.stage[r] = key[u];
+      m.stagep[r] = (uint8_t)(pb[u >> 2] >> (8 * (u & 3)));
+    }
+  }
+  for (uint32_t c = tid; c < ncol; c += SR_BLOCK) {
+    const uint32_t s0 = m.start[c], d = m.cnt[c], r = rank_of(pos_of(m.seg[s0]));
+    for (uint32_t i = 0; i < d; i++) {
+      m.stage[r + i] = m.seg[s0 + i];
+      m.stagep[r + i] = m.segp[s0 + i];
+    }
+  }
+  __syncthreads();
+  const uint32_t tot = nset + extra;
+  for (uint32_t i = tid; i < tot; i += SR_BLOCK) {
+    T[a + i] = m.stage[i];
+    if (TP) TP[a + i] = m.stagep[i];
+  }
+  if (tid == 0) cnt[j] = tot;
 }
 
 // ---------------------------------------------------------------- group dedup
@@ -1630,7 +1876,7 @@ __global__ void wd_unpack_kernel(uint64_t *T, uint8_t *TP, const uint64_t *sb_of
   }
 }
 
-// Chunk plan of the sorted form: per bin (one thread), runs of consecutive
+// Chunk plan of the sorted form: per bin, runs of consecutive
 // sub-buckets packed greedily up to cap keys and at most CS_BUCKETS
 // sub-buckets (the run's counting sort buckets a key by its sub-bucket's
 // place in the run first; sparse stretches of the key space -- canonical
@@ -1638,26 +1884,46 @@ __global__ void wd_unpack_kernel(uint64_t *T, uint8_t *TP, const uint64_t *sb_of
 // wide splits), a sub-bucket above cap keys being a run of its own, written as
 // (first, end) sub-bucket indices within the bin to clist[bin << P ...];
 // ccount[bin] = the bin's runs.
-__global__ void cs_plan_kernel(const uint64_t *sb_off, uint32_t nbins, int P, uint32_t cap, uint2 *clist,
-                               uint32_t *ccount) {
-  const uint32_t b = blockIdx.x * blockDim.x + threadIdx.x;
-  if (b >= nbins) return;
-  const uint32_t per = 1u << P;
+// One warp per bin walks its runs one after another: the end of a run is the
+// last sub-bucket whose offset is within cap of the run's start, found by a
+// 32-way search of the offsets (in shared memory, relative to the bin's
+// start, when they fit).  A thread per bin stepping through the sub-buckets
+// took 0.41 ms for 128 bins of 2048.
+constexpr uint32_t CP_MAX = 8192;  // offsets kept in shared memory
+constexpr int CP_BLOCK = 256;
+__global__ void __launch_bounds__(CP_BLOCK) cs_plan_kernel(const uint64_t *sb_off, uint32_t nbins, int P, uint32_t cap,
+                                                          uint2 *clist, uint32_t *ccount) {
+  __shared__ uint32_t s_off[CP_MAX + 1];
+  const uint32_t b = blockIdx.x, per = 1u << P;
   const uint64_t *o = sb_off + ((uint64_t)b << P);
+  const uint64_t o0 = o[0];
+  const bool local = per <= CP_MAX && o[per] - o0 < (1ull << 32);
+  if (local)
+    for (uint32_t q = threadIdx.x; q <= per; q += CP_BLOCK) s_off[q] = (uint32_t)(o[q] - o0);
+  __syncthreads();
+  if (threadIdx.x >= 32) return;
+  auto at = [&](uint32_t q) -> uint64_t { return local ? (uint64_t)s_off[q] : o[q] - o0; };
+  const unsigned lane = lane_id();
   uint2 *out = clist + ((uint64_t)b << P);
   uint32_t nc = 0, start = 0;
-  uint64_t acc = 0;
-  for (uint32_t q = 0; q < per; q++) {
-    const uint64_t sz = o[q + 1] - o[q];
-    if ((acc > 0 && acc + sz > cap) || q - start == CS_BUCKETS) {
-      out[nc++] = make_uint2(start, q);
-      start = q;
-      acc = 0;
+  while (start < per) {
+    // the largest end in (start, lim] with at(end) <= at(start) + cap; start + 1 at least
+    const uint64_t top = at(start) + cap;
+    uint32_t lo = start + 1, lim = min(per, start + CS_BUCKETS);  // at(lo) <= top or lo = start + 1
+    while (lo < lim) {
+      const uint32_t step = (lim - lo + 31) / 32;
+      const uint32_t q = lo + (lane + 1) * step;
+      const bool in = q <= lim && at(q) <= top;
+      const unsigned m = __ballot_sync(FULL, in);  // a prefix of the lanes: the offsets do not decrease
+      const uint32_t c = __popc(m), next = lo + c * step;
+      lim = min(lim, lo + (c + 1) * step - 1);
+      lo = next;
     }
-    acc += sz;
+    if (lane == 0) out[nc] = make_uint2(start, lo);
+    nc++;
+    start = lo;
   }
-  out[nc++] = make_uint2(start, per);
-  ccount[b] = nc;
+  if (lane == 0) ccount[b] = nc;
 }
 
 // One warp per sub-bucket: copy its distinct keys to the dense array.
@@ -1760,12 +2026,14 @@ template <class KeyT>
 int msd_prefix_bits(uint64_t max_bin_keys, bool sorted) {
   // Split on the key's own top bits (sorted), sub-buckets of the average bin
   // size run several times over it (the first bases of canonical k-mers are
-  // skewed ~5x), so 64-bit keys aim lower to stay within shared memory
-  // (3.1 Gbp, k = 31: 14 bits instead of 12, phase 3 245 -> 230 ms).
-  // The unsorted 64-bit form (a warp per sub-bucket, WD_MAXD distinct keys
-  // at most) aims at a third of a warp's set for the largest bin.
-  const uint64_t target = KOps<KeyT>::WORDS == 1 ? (sorted ? cs_cap<KeyT, true>() / 8 : WD_MAXD / 2)
-                                                 : cs_cap_for(true, sorted) / 2;
+  // skewed ~5x), so the aim is a quarter of what the rank dedup holds: the
+  // sub-buckets it cannot hold go to the block kernel, which takes three
+  // times as long per key (128-bit keys aimed at 2048, its whole capacity,
+  // left it two fifths of them: 100 Mbp at k = 63 3.24 ms in the two kernels,
+  // 2.13 ms now).
+  // The unsorted 64-bit form (32 sub-buckets to a group of GD_MAXN at most)
+  // aims at 192 for the largest bin.
+  const uint64_t target = KOps<KeyT>::WORDS == 1 && !sorted ? WD_MAXD / 2 : SrCfg<KeyT>::CAP / 4;
   int p = 0;
   while (p < 16 && (max_bin_keys >> p) > target) p++;
   return p;
@@ -1866,10 +2134,11 @@ bool msd_sort_unique(KeyT *keys, KeyT *alt, uint64_t n, uint64_t max_bin, const 
       uint2 *cl = sc.clist.get<uint2>(nsub);
       uint32_t *cc = sc.ccount.get<uint32_t>(nbins + 1);
       uint64_t *co = sc.coff.get<uint64_t>(nbins + 1);
-      // runs of up to 2/3 of the capacity: the shared-memory set of the
-      // dedup (a power of two >= 1.5 n slots, filled to 3/4 at most) then
-      // always holds the run, so it never falls back to sorting copies
-      cs_plan_kernel<<<(unsigned)ceil_div(nbins, 128), 128, 0, s>>>(sb_off, nbins, P, cap * 2 / 3, cl, cc);
+      // runs the rank dedup holds; also at most 2/3 of the block kernel's
+      // capacity, whose shared-memory set (a power of two >= 1.5 n slots,
+      // filled to 3/4 at most) then always holds one
+      static_assert(SrCfg<uint64_t>::CAP <= cs_cap_for(false, true) * 2 / 3 && SrCfg<Key2>::CAP <= cs_cap_for(true, true) * 2 / 3);
+      cs_plan_kernel<<<nbins, CP_BLOCK, 0, s>>>(sb_off, nbins, P, SrCfg<KeyT>::CAP, cl, cc);
       CF1_LAUNCH_CHECK();
       exclusive_scan_u32(cc, co, nbins, sc.scan_tmp, s);
       CF1_CUDA(cudaMemcpyAsync(&grid, co + nbins, sizeof(uint64_t), cudaMemcpyDeviceToHost, s));
@@ -1910,7 +2179,7 @@ bool msd_sort_unique(KeyT *keys, KeyT *alt, uint64_t n, uint64_t max_bin, const 
         gd_split_kernel<<<h_ov, GD_BLOCK, 0, s>>>(T64, PT, sb_off, ov, PS, P, p1, U64, PU, sub_off, jl);
         CF1_LAUNCH_CHECK();
         kern<<<nov, CS_BLOCK, smem, s>>>(U, T, sub_off, nsub, shift, rest > 0 ? bits : 0, scnt, over, P, lb, PU, PT,
-                                         nullptr, nullptr, nbins, jl);
+                                         nullptr, nullptr, nbins, jl, nullptr);
         CF1_LAUNCH_CHECK();
         gd_gather_kernel<<<h_ov, GD_BLOCK, 0, s>>>(U64, lo.with_pay ? lb.l0pay : nullptr, sb_off, ov, g, sub_off, scnt,
                                                    T64, cnt, keep, lo, p1);
@@ -1940,13 +2209,27 @@ bool msd_sort_unique(KeyT *keys, KeyT *alt, uint64_t n, uint64_t max_bin, const 
       }
       if (h_ov) {
         kern<<<h_ov, CS_BLOCK, smem, s>>>(T, U, sb_off, nsub, shift, rest > 0 ? bits : 0, cnt, over, P, lo, PT, PU,
-                                          nullptr, nullptr, nbins, ov);
+                                          nullptr, nullptr, nbins, ov, nullptr);
         CF1_LAUNCH_CHECK();
       }
     } else {
-      kern<<<(unsigned)grid, CS_BLOCK, smem, s>>>(T, U, sb_off, nsub, shift, rest > 0 ? bits : 0, cnt, over, P, lo, PT,
-                                                  PU, clist, coff, nbins, nullptr);
+      // a CTA per run; the runs it cannot hold go to the block kernel
+      uint32_t *ov = sc.ov.get<uint32_t>(grid + 1);
+      uint32_t *ovc = sc.ovc.get<uint32_t>(2);
+      CF1_CUDA(cudaMemsetAsync(ovc, 0, sizeof(uint32_t), s));
+      const size_t ssm = sizeof(SrSmem<KeyT>);
+      CF1_CUDA(cudaFuncSetAttribute(sr_dedup_kernel<KeyT>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)ssm));
+      sr_dedup_kernel<KeyT><<<(unsigned)grid, SR_BLOCK, ssm, s>>>(T, PT, sb_off, nsub, P, rest > 0 ? rest : 0, cnt, clist,
+                                                                 coff, nbins, ov, ovc);
       CF1_LAUNCH_CHECK();
+      uint32_t h_ov = 0;
+      CF1_CUDA(cudaMemcpyAsync(&h_ov, ovc, sizeof(uint32_t), cudaMemcpyDeviceToHost, s));
+      CF1_CUDA(cudaStreamSynchronize(s));
+      if (h_ov) {
+        kern<<<h_ov, CS_BLOCK, smem, s>>>(T, U, sb_off, nsub, shift, rest > 0 ? bits : 0, cnt, over, P, lo, PT, PU, clist,
+                                          coff, nbins, nullptr, ov);
+        CF1_LAUNCH_CHECK();
+      }
     }
     CF1_CUDA(cudaEventRecord(sc.ev[1], s));
   }

@@ -160,6 +160,23 @@ __global__ void __launch_bounds__(CL_BLOCK_DEFER) classify_defer_kernel(Classify
   classify_body<KeyT, SIDESET, true>(a);
 }
 
+// n bytes from src to dst by one warp, four bytes a lane: dst is brought to a
+// word boundary first, a word of src is cut from the two aligned words it
+// spans (the second is read only when it holds a byte of the copy).
+CF1_D void warp_copy_bytes(uint8_t *dst, const uint8_t *src, uint32_t n) {
+  const unsigned lane = lane_id();
+  uint32_t head = (4u - (uint32_t)(reinterpret_cast<uintptr_t>(dst) & 3)) & 3;
+  if (head > n) head = n;
+  if (lane < head) dst[lane] = src[lane];
+  const uint32_t words = (n - head) >> 2, sh = (uint32_t)(reinterpret_cast<uintptr_t>(src + head) & 3) * 8;
+  uint32_t *d = reinterpret_cast<uint32_t *>(dst + head);
+  const uint32_t *w = reinterpret_cast<const uint32_t *>(src + head - sh / 8);
+#pragma unroll 4
+  for (uint32_t i = lane; i < words; i += 32) d[i] = sh ? __funnelshift_r(w[i], w[i + 1], sh) : w[i];
+  const uint32_t t = head + words * 4 + lane;
+  if (t < n) dst[t] = src[t];
+}
+
 // One warp per unit: each distinct key's side-set byte to its slot.
 // A learned bin's slot is the key's rank, which the dense layout already
 // gives; a BBHash bin probes level 0 first for PL_U keys per lane at once
@@ -180,7 +197,7 @@ __global__ void __launch_bounds__(256) place_sides_kernel(MphfView<KeyT> m, cons
   const unsigned lane = lane_id();
   bool miss = false;
   if (ranked) {
-    for (uint32_t i = lane; i < c; i += 32) sides[o + i] = kept_pay[a + i];
+    warp_copy_bytes(sides + o, kept_pay + a, c);
   } else {
     const BBMeta m0 = m.bb.levels ? m.bb.meta[bin] : BBMeta{};  // level 0 of this bin
     for (uint32_t i0 = 0; i0 < c; i0 += 32 * PL_U) {
@@ -228,23 +245,6 @@ __global__ void __launch_bounds__(256) place_sides_kernel(MphfView<KeyT> m, cons
     }
   }
   if (__any_sync(FULL, miss) && lane == 0) atomicOr(err, (uint32_t)DEV_MPHF_MISS);
-}
-
-// n bytes from src to dst by one warp, four bytes a lane: dst is brought to a
-// word boundary first, a word of src is cut from the two aligned words it
-// spans (the second is read only when it holds a byte of the copy).
-CF1_D void warp_copy_bytes(uint8_t *dst, const uint8_t *src, uint32_t n) {
-  const unsigned lane = lane_id();
-  uint32_t head = (4u - (uint32_t)(reinterpret_cast<uintptr_t>(dst) & 3)) & 3;
-  if (head > n) head = n;
-  if (lane < head) dst[lane] = src[lane];
-  const uint32_t words = (n - head) >> 2, sh = (uint32_t)(reinterpret_cast<uintptr_t>(src + head) & 3) * 8;
-  uint32_t *d = reinterpret_cast<uint32_t *>(dst + head);
-  const uint32_t *w = reinterpret_cast<const uint32_t *>(src + head - sh / 8);
-#pragma unroll 4
-  for (uint32_t i = lane; i < words; i += 32) d[i] = sh ? __funnelshift_r(w[i], w[i + 1], sh) : w[i];
-  const uint32_t t = head + words * 4 + lane;
-  if (t < n) dst[t] = src[t];
 }
 
 // One warp per unit (a sub-bucket, or a group of 2^(P - PU) of them): the
