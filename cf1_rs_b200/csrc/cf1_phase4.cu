@@ -14,6 +14,8 @@
 //     streaming pass then packs the bytes into the reference layout;
 //   * CAS: a 64-bit atomicCAS loop directly on the reference layout (12 five-
 //     bit states per word, LSB first), as src/state_vector.rs:47-70 does.
+#include <algorithm>
+
 #include "cf1_device_util.cuh"
 #include "cf1_internal.cuh"
 #include "cf1_mphf.cuh"
@@ -281,17 +283,17 @@ __global__ void __launch_bounds__(256) place_l0_kernel(BBView bb, const uint64_t
   warp_copy_bytes(sides + b1, src + n0, n1);
 }
 
-// The keys levels 0 and 1 left: SV_CTAS CTAs per bin, each key walks from
+// The keys levels 0 and 1 left: `parts` CTAs per bin, each key walks from
 // level 2.
-constexpr uint32_t SV_CTAS = 32;
+constexpr uint32_t SV_CTAS = 32;  // per bin, at most
 __global__ void __launch_bounds__(256) place_surv_kernel(BBView bb, const uint64_t *dist_off, const uint64_t *surv,
                                                          const uint8_t *surv_pay, const uint64_t *surv_off,
                                                          const unsigned long long *surv_cnt, uint32_t b0,
-                                                         uint8_t *sides, uint32_t *err) {
-  const uint32_t bin = b0 + blockIdx.x / SV_CTAS, part = blockIdx.x % SV_CTAS;
+                                                         uint32_t parts, uint8_t *sides, uint32_t *err) {
+  const uint32_t bin = b0 + blockIdx.x / parts, part = blockIdx.x % parts;
   const uint64_t n = surv_cnt[bin], s0 = surv_off[bin], base = dist_off[bin], end = dist_off[bin + 1];
   bool miss = false;
-  for (uint64_t i = (uint64_t)part * blockDim.x + threadIdx.x; i < n; i += (uint64_t)SV_CTAS * blockDim.x) {
+  for (uint64_t i = (uint64_t)part * blockDim.x + threadIdx.x; i < n; i += (uint64_t)parts * blockDim.x) {
     const uint64_t local = bb_walk(bb, bin, bb_key_hash(surv[s0 + i]), 2, bb.levels);
     const uint64_t slot = local == SLOT_NONE ? SLOT_NONE : base + local;
     if (slot >= base && slot < end) sides[slot] = surv_pay[s0 + i];
@@ -411,10 +413,12 @@ void launch_place_l0(const BBView &bb, const uint64_t *dist_off, const uint64_t 
 
 void launch_place_surv(const BBView &bb, const uint64_t *dist_off, const uint64_t *surv, const uint8_t *surv_pay,
                        const uint64_t *surv_off, const unsigned long long *surv_cnt, uint32_t b0, uint32_t b1,
-                       uint8_t *sides, uint32_t *err, cudaStream_t s) {
+                       uint64_t n_occ, uint32_t nbins, uint8_t *sides, uint32_t *err, cudaStream_t s) {
   if (b1 <= b0) return;
-  place_surv_kernel<<<(b1 - b0) * SV_CTAS, 256, 0, s>>>(bb, dist_off, surv, surv_pay, surv_off, surv_cnt, b0, sides,
-                                                        err);
+  // level 1 leaves ~1% of the occurrences: one key a thread
+  const uint32_t parts = (uint32_t)std::min<uint64_t>(SV_CTAS, n_occ / 100 / nbins / 256 + 1);
+  place_surv_kernel<<<(b1 - b0) * parts, 256, 0, s>>>(bb, dist_off, surv, surv_pay, surv_off, surv_cnt, b0, parts,
+                                                      sides, err);
   CF1_LAUNCH_CHECK();
 }
 
