@@ -74,58 +74,78 @@ __global__ void bb_sizes_kernel(const uint64_t *cnt, uint32_t nbins, uint32_t ga
 // unsorted phase-3 output is ordered by the same hash's top bits -- the tile
 // marks a shared-memory copy of that stretch and merges it with one atomicOr
 // per word (and one more per word with a collision) instead of one per key.
+// Each key is hashed once (its position waits in a register for the stretch
+// to be known): 100 M 128-bit keys in hash order, levels 0 and 1, 1.27 ->
+// 0.78 ms; in key order the same keys took 2.84 ms, an atomic each.
 constexpr uint32_t BB_WIN = 2048;  // words of the shared-memory stretch
+constexpr int BB_ITEMS = BB_TILE / BB_BLOCK;
 template <class KeyT>
 __global__ void __launch_bounds__(BB_BLOCK) bb_mark_kernel(const KeyT *rem, const uint64_t *start, const uint64_t *cnt,
                                                            const uint32_t *tile_off, uint32_t nbins,
                                                            const uint64_t *woff, uint32_t level, ulonglong2 *AR) {
   __shared__ unsigned long long s_set[BB_WIN], s_col[BB_WIN];
-  __shared__ unsigned long long s_lo, s_hi;
+  __shared__ uint32_t s_lo, s_hi;
   const uint32_t t = blockIdx.x;
   if (t >= tile_off[nbins]) return;
   TileSpan sp = tile_span_gapped(start, cnt, tile_off, nbins, t, BB_TILE);
   const uint64_t w0 = woff[sp.seg];
   const uint32_t nw = (uint32_t)(woff[sp.seg + 1] - w0);
   if (threadIdx.x == 0) {
-    s_lo = ~0ull;
+    s_lo = ~0u;
     s_hi = 0;
   }
   __syncthreads();
-  unsigned long long lo = ~0ull, hi = 0;
-  for (uint64_t i = sp.start + threadIdx.x; i < sp.end; i += BB_BLOCK) {
-    const unsigned long long wi = bb_pos(bb_key_hash(rem[i]), level, nw) >> 6;
-    lo = wi < lo ? wi : lo;
-    hi = wi > hi ? wi : hi;
+  uint32_t word[BB_ITEMS];  // word of the block
+  uint32_t bits[(BB_ITEMS + 3) / 4];  // the bit in it, four to a register
+  uint32_t lo = ~0u, hi = 0;
+#pragma unroll
+  for (int i = 0; i < (BB_ITEMS + 3) / 4; i++) bits[i] = 0;
+#pragma unroll
+  for (int j = 0; j < BB_ITEMS; j++) {
+    const uint64_t i = sp.start + (uint64_t)j * BB_BLOCK + threadIdx.x;
+    word[j] = ~0u;
+    if (i < sp.end) {
+      const uint64_t pos = bb_pos(bb_key_hash(rem[i]), level, nw);
+      word[j] = (uint32_t)(pos >> 6);
+      bits[j >> 2] |= (uint32_t)(pos & 63) << (8 * (j & 3));
+      lo = min(lo, word[j]);
+      hi = max(hi, word[j]);
+    }
   }
-  atomicMin(&s_lo, lo);
-  atomicMax(&s_hi, hi);
+  lo = __reduce_min_sync(FULL, lo);
+  hi = __reduce_max_sync(FULL, hi);
+  if (lane_id() == 0) {
+    atomicMin(&s_lo, lo);
+    atomicMax(&s_hi, hi);
+  }
   __syncthreads();
-  const uint64_t wlo = s_lo, span = s_hi >= s_lo ? s_hi - s_lo + 1 : 0;
-  if (span > 0 && span <= BB_WIN) {
+  const uint32_t wlo = s_lo, span = s_hi >= s_lo ? s_hi - s_lo + 1 : 0;
+  const bool local = span > 0 && span <= BB_WIN;
+  if (local) {
     for (uint32_t j = threadIdx.x; j < span; j += BB_BLOCK) s_set[j] = s_col[j] = 0;
     __syncthreads();
-    for (uint64_t i = sp.start + threadIdx.x; i < sp.end; i += BB_BLOCK) {
-      const uint64_t pos = bb_pos(bb_key_hash(rem[i]), level, nw);
-      const uint32_t j = (uint32_t)((pos >> 6) - wlo);
-      const unsigned long long bit = 1ull << (pos & 63);
-      if (atomicOr(&s_set[j], bit) & bit) atomicOr(&s_col[j], bit);
-    }
-    __syncthreads();
-    for (uint32_t j = threadIdx.x; j < span; j += BB_BLOCK) {
-      const unsigned long long set = s_set[j];
-      if (!set) continue;
-      ulonglong2 *e = AR + w0 + wlo + j;
-      const unsigned long long col = s_col[j] | (atomicOr(&e->x, set) & set);
-      if (col) atomicOr(&e->y, col);
-    }
-    return;
   }
-  for (uint64_t i = sp.start + threadIdx.x; i < sp.end; i += BB_BLOCK) {
-    uint64_t pos = bb_pos(bb_key_hash(rem[i]), level, nw);
-    ulonglong2 *e = AR + w0 + (pos >> 6);
-    unsigned long long bit = 1ull << (pos & 63);
-    unsigned long long old = atomicOr(&e->x, bit);
-    if (old & bit) atomicOr(&e->y, bit);
+#pragma unroll
+  for (int j = 0; j < BB_ITEMS; j++) {
+    if (word[j] == ~0u) continue;
+    const uint32_t b = (bits[j >> 2] >> (8 * (j & 3))) & 63, half = b >> 5, bit = 1u << (b & 31);
+    if (local) {
+      const uint32_t x = 2 * (word[j] - wlo) + half;
+      if (atomicOr(reinterpret_cast<uint32_t *>(s_set) + x, bit) & bit)
+        atomicOr(reinterpret_cast<uint32_t *>(s_col) + x, bit);
+    } else {
+      uint32_t *e = reinterpret_cast<uint32_t *>(AR + w0 + word[j]) + half;
+      if (atomicOr(e, bit) & bit) atomicOr(e + 2, bit);
+    }
+  }
+  if (!local) return;
+  __syncthreads();
+  for (uint32_t j = threadIdx.x; j < span; j += BB_BLOCK) {
+    const unsigned long long set = s_set[j];
+    if (!set) continue;
+    ulonglong2 *e = AR + w0 + wlo + j;
+    const unsigned long long col = s_col[j] | (atomicOr(&e->x, set) & set);
+    if (col) atomicOr(&e->y, col);
   }
 }
 
@@ -334,7 +354,6 @@ __global__ void __launch_bounds__(BB_BLOCK) bb_filter_kernel(const KeyT *rem, co
                                                              const uint32_t *tile_off, uint32_t nbins,
                                                              const uint64_t *woff, uint32_t level, const ulonglong2 *AR,
                                                              unsigned long long *cnt_next, KeyT *out) {
-  constexpr int ITEMS = BB_TILE / BB_BLOCK;
   __shared__ uint32_t sm[BB_BLOCK / 32];
   __shared__ unsigned long long s_base;
   const uint32_t t = blockIdx.x;
@@ -342,27 +361,25 @@ __global__ void __launch_bounds__(BB_BLOCK) bb_filter_kernel(const KeyT *rem, co
   TileSpan sp = tile_span_gapped(start, cnt, tile_off, nbins, t, BB_TILE);
   const uint64_t w0 = woff[sp.seg];
   const uint32_t nw = (uint32_t)(woff[sp.seg + 1] - w0);
-  uint64_t i0 = sp.start + (uint64_t)threadIdx.x * ITEMS;
-  uint32_t flags = 0, c = 0;
-#pragma unroll
-  for (int j = 0; j < ITEMS; j++) {
-    uint64_t i = i0 + j;
-    bool keep = false;
+  // consecutive threads on consecutive keys (sixteen consecutive ones a thread
+  // touched a line per lane: 1.13 against 0.59 ms for those keys)
+  uint32_t flags = 0;
+#pragma unroll 4
+  for (int j = 0; j < BB_ITEMS; j++) {
+    const uint64_t i = sp.start + (uint64_t)j * BB_BLOCK + threadIdx.x;
     if (i < sp.end) {
-      uint64_t pos = bb_pos(bb_key_hash(rem[i]), level, nw);
-      keep = ((AR[w0 + (pos >> 6)].x >> (pos & 63)) & 1) == 0;
+      const uint64_t pos = bb_pos(bb_key_hash(rem[i]), level, nw);
+      flags |= (uint32_t)(((AR[w0 + (pos >> 6)].x >> (pos & 63)) & 1) ^ 1) << j;
     }
-    flags |= (uint32_t)keep << j;
-    c += keep;
   }
   uint32_t tot;
-  uint32_t pre = block_exclusive_scan<BB_BLOCK>(c, sm, tot);
+  uint32_t pre = block_exclusive_scan<BB_BLOCK>((uint32_t)__popc(flags), sm, tot);
   if (threadIdx.x == 0) s_base = tot ? atomicAdd(&cnt_next[sp.seg], (unsigned long long)tot) : 0;
   __syncthreads();
   uint64_t o = start[sp.seg] + s_base + pre;
 #pragma unroll
-  for (int j = 0; j < ITEMS; j++)
-    if ((flags >> j) & 1) out[o++] = rem[i0 + j];
+  for (int j = 0; j < BB_ITEMS; j++)
+    if ((flags >> j) & 1) out[o++] = rem[sp.start + (uint64_t)j * BB_BLOCK + threadIdx.x];
 }
 
 }  // namespace

@@ -47,9 +47,11 @@ constexpr uint32_t cs_cap() { return cs_cap_for(KOps<KeyT>::WORDS == 2, SORTED);
 
 // Digit of a key in a multisplit pass: bits [shift, shift + width) of the key
 // or, when only the distinct keys and not their order are needed (hashed),
-// of key * MS_HASH_MUL.  The product's top bits spread any key set evenly,
-// where the key's own top bits -- the first bases of a canonical k-mer --
-// are skewed several-fold.  (64-bit keys; wider keys always sort.)
+// of H * MS_HASH_MUL, H the key's BBHash hash (the key itself for 64-bit
+// keys).  The product's top bits spread any key set evenly, where the key's
+// own top bits -- the first bases of a canonical k-mer -- are skewed
+// several-fold, and they are BBHash level 0's: keys that end up side by side
+// have their level-0 bits side by side.
 constexpr uint64_t MS_HASH_MUL = KEY_SPREAD_MUL;
 template <class KeyT>
 CF1_D uint32_t ms_digit(const KeyT &k, int shift, uint32_t mask, bool hashed);
@@ -58,7 +60,8 @@ CF1_D uint32_t ms_digit<uint64_t>(const uint64_t &k, int shift, uint32_t mask, b
   return (uint32_t)((hashed ? k * MS_HASH_MUL : k) >> shift) & mask;
 }
 template <>
-CF1_D uint32_t ms_digit<Key2>(const Key2 &k, int shift, uint32_t mask, bool) {
+CF1_D uint32_t ms_digit<Key2>(const Key2 &k, int shift, uint32_t mask, bool hashed) {
+  if (hashed) return (uint32_t)((bb_key_hash(k) * MS_HASH_MUL) >> shift) & mask;
   return KOps<Key2>::digit(k, shift, mask);
 }
 
@@ -643,7 +646,7 @@ __global__ void __launch_bounds__(CS_BLOCK, SORTED ? 2 : 4) cs_sort_unique_kerne
     if (n == 0) return 0;
     CsShared sh{hist, cur, sm, &s_big, TP ? reinterpret_cast<uint8_t *>(SPw) : nullptr};
     CsDigit plain{shift, bits, 0, 0, 0u};
-    if (jend - j > 1) {  // a packed run: bucket = place of the sub-bucket in the run, then the next bits
+    if (SORTED && jend - j > 1) {  // a packed run: bucket = place of the sub-bucket in the run, then the next bits
       const uint32_t span = (uint32_t)(jend - j);
       if (span > CS_BUCKETS) return ~0u;  // the plan never makes one; refused (LSD path) rather than mis-bucketed
       int g = 0;
@@ -760,10 +763,12 @@ __global__ void __launch_bounds__(CS_BLOCK, SORTED ? 2 : 4) cs_sort_unique_kerne
 }
 
 // ---------------------------------------------------------------- rank dedup
-// The sorted form's dedup: one CTA per run of consecutive sub-buckets of a
-// bin (the plan's chunks), at most SrCfg::CAP keys, held in registers.  A
-// key's position is its distance from the run's start in the key range,
-// scaled by a shift to NP = 8 CAP bits, so positions ascend with the keys:
+// The sorted form's dedup, and that of 128-bit keys in the BBHash form
+// (HASHED): one CTA per run of consecutive sub-buckets of a bin (the plan's
+// chunks), at most SrCfg::CAP keys, held in registers.  A key's position is
+// its distance from the run's start in the key range (HASHED: in the range of
+// the level-0 hash), scaled by a shift to NP = 8 CAP bits, so positions ascend
+// with the keys (with the hash):
 //   1. every occurrence marks its position (set; col when it was set
 //      already).  A position marked once is one key, whose rank is the popcount
 //      of set before it, plus
@@ -801,7 +806,7 @@ struct SrSmem {
   uint32_t sm[SR_BLOCK / 32];
 };
 
-template <class KeyT>
+template <class KeyT, bool HASHED>
 __global__ void __launch_bounds__(SR_BLOCK, 2) sr_dedup_kernel(KeyT *T, uint8_t *TP, const uint64_t *sb_off,
                                                               uint64_t nsub, int P, int rest, uint32_t *cnt,
                                                               const uint2 *clist, const uint64_t *coff, uint32_t nbins,
@@ -830,8 +835,12 @@ __global__ void __launch_bounds__(SR_BLOCK, 2) sr_dedup_kernel(KeyT *T, uint8_t 
   while ((1u << (sh + C::LOGNP - rest)) < span) sh++;
   if (sh < 0) sh = 0;
   const uint32_t pos0 = sub0 << (rest - sh);
-  auto pos_of = [&](const KeyT &k) -> uint32_t { return KOps<KeyT>::digit(k, sh, 0xFFFFFFFFu) - pos0; };
+  auto pos_of = [&](const KeyT &k) -> uint32_t {
+    if constexpr (HASHED) return ((uint32_t)((bb_key_hash(k) * MS_HASH_MUL) >> 32) >> sh) - pos0;
+    else return KOps<KeyT>::digit(k, sh, 0xFFFFFFFFu) - pos0;
+  };
   KeyT key[C::U];
+  uint32_t pos[C::U];
   uint32_t pb[C::U / 4];
 #pragma unroll
   for (int i = 0; i < C::U / 4; i++) pb[i] = 0;
@@ -843,13 +852,15 @@ __global__ void __launch_bounds__(SR_BLOCK, 2) sr_dedup_kernel(KeyT *T, uint8_t 
       if (TP) pb[u >> 2] |= (uint32_t)TP[a + i] << (8 * (u & 3));
     }
   }
+#pragma unroll
+  for (int u = 0; u < C::U; u++) pos[u] = u * SR_BLOCK + tid < n ? pos_of(key[u]) : 0u;
   for (uint32_t w = tid; w < C::NWORD; w += SR_BLOCK) m.set[w] = m.col[w] = 0;
   __syncthreads();
   // 1. mark
 #pragma unroll
   for (int u = 0; u < C::U; u++) {
     if (u * SR_BLOCK + tid < n) {
-      const uint32_t p = pos_of(key[u]), bm = 1u << (p & 31);
+      const uint32_t p = pos[u], bm = 1u << (p & 31);
       if (atomicOr(&m.set[p >> 5], bm) & bm) atomicOr(&m.col[p >> 5], bm);
     }
   }
@@ -884,7 +895,7 @@ __global__ void __launch_bounds__(SR_BLOCK, 2) sr_dedup_kernel(KeyT *T, uint8_t 
     for (int u = 0; u < C::U; u++) {
       slot[u] = 0;
       if (u * SR_BLOCK + tid < n) {
-        const uint32_t p = pos_of(key[u]), bm = 1u << (p & 31), cw = m.col[p >> 5];
+        const uint32_t p = pos[u], bm = 1u << (p & 31), cw = m.col[p >> 5];
         if (cw & bm) {
           const uint32_t c = m.cpre[p >> 5] + (uint32_t)__popc(cw & (bm - 1));
           shared |= 1u << u;
@@ -981,7 +992,7 @@ __global__ void __launch_bounds__(SR_BLOCK, 2) sr_dedup_kernel(KeyT *T, uint8_t 
 #pragma unroll
   for (int u = 0; u < C::U; u++) {
     if (u * SR_BLOCK + tid < n && !((shared >> u) & 1)) {
-      const uint32_t r = rank_of(pos_of(key[u]));
+      const uint32_t r = rank_of(pos[u]);
       m.stage[r] = key[u];
       m.stagep[r] = (uint8_t)(pb[u >> 2] >> (8 * (u & 3)));
     }
@@ -2033,7 +2044,9 @@ int msd_prefix_bits(uint64_t max_bin_keys, bool sorted) {
   // 2.13 ms now).
   // The unsorted 64-bit form (32 sub-buckets to a group of GD_MAXN at most)
   // aims at 192 for the largest bin.
-  const uint64_t target = KOps<KeyT>::WORDS == 1 && !sorted ? WD_MAXD / 2 : SrCfg<KeyT>::CAP / 4;
+  // 128-bit keys split by their hash are spread evenly: three quarters.
+  const uint64_t target = sorted ? SrCfg<KeyT>::CAP / 4
+                                 : KOps<KeyT>::WORDS == 1 ? WD_MAXD / 2 : SrCfg<KeyT>::CAP * 3 / 4;
   int p = 0;
   while (p < 16 && (max_bin_keys >> p) > target) p++;
   return p;
@@ -2047,7 +2060,8 @@ bool msd_sort_unique(KeyT *keys, KeyT *alt, uint64_t n, uint64_t max_bin, const 
   uint8_t *PT = pkeys;  // payloads beside T (nullptr: keys carry none)
   // passes on the top P bits: P1 then P2 (P2 may be 0) -- of the key, or of
   // its hash when only distinct keys are wanted (64-bit keys)
-  const bool hashed = !sorted && KOps<KeyT>::WORDS == 1;
+  const bool hashed = !sorted;
+  constexpr bool W1 = KOps<KeyT>::WORDS == 1;
   if (hashed) key_bits = 64;
   // packed passes (see pay_code): the hashed split of keys with payloads
   // whose dedup builds BBHash level 0, with a first pass of >= 6 bits
@@ -2055,12 +2069,12 @@ bool msd_sort_unique(KeyT *keys, KeyT *alt, uint64_t n, uint64_t max_bin, const 
   // the bits above theirs only, as long as the width rule's aim holds for the
   // largest bin: 32 sub-buckets of at most WD_MAXD / 2 keys are 6144 of the
   // group's GD_MAXN.
-  const bool grp = hashed && (max_bin >> P) <= WD_MAXD / 2;
+  const bool grp = W1 && hashed && (max_bin >> P) <= WD_MAXD / 2;
   const int g = grp ? (P < GD_BITS ? P : GD_BITS) : 0;
   const int PS = P - g;  // bits split on: a unit is a group, or a sub-bucket
   sc.unit_bits = PS;
   sc.kept_bits = false;
-  const bool pk = hashed && pkeys && palt && l0 && l0->AR && l0->with_pay && PS >= (int)PACK_MIN_BITS;
+  const bool pk = W1 && hashed && pkeys && palt && l0 && l0->AR && l0->with_pay && PS >= (int)PACK_MIN_BITS;
   int P1 = PS > 8 ? (PS + 1) / 2 : PS;
   if (pk && P1 < (int)PACK_MIN_BITS) P1 = PACK_MIN_BITS;
   const int P2 = PS - P1;
@@ -2124,13 +2138,13 @@ bool msd_sort_unique(KeyT *keys, KeyT *alt, uint64_t n, uint64_t max_bin, const 
     lo.l0pay = PU;
     for (auto &e : sc.ev)
       if (!e) CF1_CUDA(cudaEventCreate(&e));
-    // sorted form: consecutive small sub-buckets of a bin are packed into
+    // sorted form (and 128-bit keys): consecutive small sub-buckets of a bin are packed into
     // one CTA's run (the top bits of canonical k-mers are skewed, so most
     // sub-buckets are far below the capacity the largest ones need)
     const uint2 *clist = nullptr;
     const uint64_t *coff = nullptr;
     uint64_t grid = nsub;
-    if (sorted && P > 0) {
+    if ((sorted || !W1) && P > 0) {
       uint2 *cl = sc.clist.get<uint2>(nsub);
       uint32_t *cc = sc.ccount.get<uint32_t>(nbins + 1);
       uint64_t *co = sc.coff.get<uint64_t>(nbins + 1);
@@ -2185,7 +2199,7 @@ bool msd_sort_unique(KeyT *keys, KeyT *alt, uint64_t n, uint64_t max_bin, const 
                                                    T64, cnt, keep, lo, p1);
         CF1_LAUNCH_CHECK();
       }
-    } else if (hashed) {
+    } else if (W1 && hashed) {
       // the unsorted form: one warp per sub-bucket; the few it cannot hold
       // (more than WD_MAXD distinct keys) go to the block kernel after it
       uint32_t *ov = sc.ov.get<uint32_t>(nsub + 1);
@@ -2218,9 +2232,10 @@ bool msd_sort_unique(KeyT *keys, KeyT *alt, uint64_t n, uint64_t max_bin, const 
       uint32_t *ovc = sc.ovc.get<uint32_t>(2);
       CF1_CUDA(cudaMemsetAsync(ovc, 0, sizeof(uint32_t), s));
       const size_t ssm = sizeof(SrSmem<KeyT>);
-      CF1_CUDA(cudaFuncSetAttribute(sr_dedup_kernel<KeyT>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)ssm));
-      sr_dedup_kernel<KeyT><<<(unsigned)grid, SR_BLOCK, ssm, s>>>(T, PT, sb_off, nsub, P, rest > 0 ? rest : 0, cnt, clist,
-                                                                 coff, nbins, ov, ovc);
+      auto skern = hashed && !W1 ? sr_dedup_kernel<KeyT, !W1> : sr_dedup_kernel<KeyT, false>;
+      CF1_CUDA(cudaFuncSetAttribute(skern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)ssm));
+      skern<<<(unsigned)grid, SR_BLOCK, ssm, s>>>(T, PT, sb_off, nsub, P, hashed ? 32 - P : rest > 0 ? rest : 0, cnt, clist,
+                                                 coff, nbins, ov, ovc);
       CF1_LAUNCH_CHECK();
       uint32_t h_ov = 0;
       CF1_CUDA(cudaMemcpyAsync(&h_ov, ovc, sizeof(uint32_t), cudaMemcpyDeviceToHost, s));

@@ -249,8 +249,8 @@ void run_impl(cf1gpu_ctx *c, StreamIO *io = nullptr, Step step = Step::FULL, con
   c->dist_pending = false;  // the sort buffers are about to be reused
   const uint64_t launches0 = step == Step::XFINISH ? c->x_launches0 : g_launches.load();
   // The learned index needs each bin's keys sorted; BBHash needs them
-  // distinct (128-bit keys always take the sorted path).
-  const bool sorted = c->opts.mphf_mode == CF1GPU_MPHF_LEARNED || c->opts.sort_mode == 1 || KOps<KeyT>::WORDS == 2;
+  // distinct.
+  const bool sorted = c->opts.mphf_mode == CF1GPU_MPHF_LEARNED || c->opts.sort_mode == 1;
   // autotuner: parameters of this input class from the cache, or measured
   // in this run and stored
   bool tune_now = false;  // (streamed runs do not measure: their phase 1 waits on the input)
