@@ -31,6 +31,7 @@ SOURCES = [
     "cf1_pipeline.cu",
     "cf1_export.cu",
     "cf1_fasta.cu",
+    "cf1_hostio.cu",
     "cf1_capi.cu",
     "cf1_noalloc.cu",
     "cf1_tuner.cu",

@@ -515,18 +515,18 @@ void BBHashBuild<KeyT>::set_bytes() {
 }
 
 template <class KeyT>
-void BBHashBuild<KeyT>::collect_begin(cudaStream_t s) {
+void BBHashBuild<KeyT>::collect_begin(uint64_t *got, cudaStream_t s) {
   if (!tail_words_) return;
-  CF1_CUDA(cudaMemcpyAsync(&got_words_, tail_words_, sizeof(uint64_t), cudaMemcpyDeviceToHost, s));
-  CF1_CUDA(cudaMemcpyAsync(&got_levels_, lv_.p, sizeof(uint32_t), cudaMemcpyDeviceToHost, s));
+  CF1_CUDA(cudaMemcpyAsync(&got[0], tail_words_, sizeof(uint64_t), cudaMemcpyDeviceToHost, s));
+  CF1_CUDA(cudaMemcpyAsync(&got[1], lv_.p, sizeof(uint32_t), cudaMemcpyDeviceToHost, s));
 }
 
 template <class KeyT>
-void BBHashBuild<KeyT>::collect_end() {
+void BBHashBuild<KeyT>::collect_end(const uint64_t *got) {
   if (!tail_words_) return;
   tail_words_ = nullptr;
-  total_words += got_words_;
-  levels = std::max<uint32_t>(got_levels_, l1_slice_bits >= 0 ? 2 : 0);
+  total_words += got[0];
+  levels = std::max<uint32_t>((uint32_t)got[1], l1_slice_bits >= 0 ? 2 : 0);
   set_bytes();
 }
 

@@ -41,8 +41,8 @@ struct BBHashBuild {
                            const uint64_t *woff1, uint64_t words1, const uint32_t *placed1, const KeyT *surv,
                            const uint64_t *surv_off, const uint64_t *surv_cnt, uint64_t surv_total, uint64_t n_occ,
                            uint32_t *err, cudaStream_t s, KeyT *ws0 = nullptr, KeyT *ws1 = nullptr, uint64_t ws_cap = 0);
-  void collect_begin(cudaStream_t s);
-  void collect_end();
+  void collect_begin(uint64_t *got, cudaStream_t s);  // got: two words of page-locked memory
+  void collect_end(const uint64_t *got);
   BBView view() const;
   void clear();
   const BBMeta *meta_device() const { return meta_.as<const BBMeta>(); }
@@ -66,8 +66,7 @@ struct BBHashBuild {
   DevBuf ar_, meta_, base_, rem_[2], cnt_[2], tot_, tile_off_, wcnt_, woff_, pc_, rtmp_, scan_tmp_, srank_[2], lv_;
   uint32_t tail_from_ = 0;                  // first level of the one-launch tail (copied from here)
   const uint64_t *tail_words_ = nullptr;    // device: its entries; nullptr: none pending
-  uint64_t got_words_ = 0;
-  uint32_t got_levels_ = 0;
+
 };
 
 }  // namespace cf1

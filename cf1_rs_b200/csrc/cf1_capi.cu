@@ -4,6 +4,7 @@
 #include <string>
 
 #include "cf1_context.cuh"
+#include "cf1_hostio.cuh"
 #include "cf1_learned.cuh"
 #include "cf1_pipeline.cuh"
 
@@ -102,6 +103,7 @@ int cf1gpu_create(const cf1gpu_opts *opts, cf1gpu_ctx **out) {
     CF1_CUDA(cudaStreamCreateWithFlags(&c->copy_stream, cudaStreamNonBlocking));
     for (auto &e : c->ev) CF1_CUDA(cudaEventCreate(&e));
     for (auto &e : c->stage_ev) CF1_CUDA(cudaEventCreateWithFlags(&e, cudaEventDisableTiming));
+    for (auto &e : c->io_ev) CF1_CUDA(cudaEventCreateWithFlags(&e, cudaEventDisableTiming));
     if (opts->sk_tile) c->tune.sk_tile = opts->sk_tile;
     if (opts->learned_max_err) c->learned.max_err = opts->learned_max_err;
     if (opts->learned_train_steps > 0) c->learned.train_steps = opts->learned_train_steps;
@@ -242,10 +244,7 @@ int cf1gpu_copy_states(cf1gpu_ctx *c, uint64_t *dst, size_t n_words) {
     c->last_error = "n_words must be ceil(total_kmers / 12) = " + std::to_string(nw);
     return CF1GPU_ERR_INVALID_ARG;
   }
-  return guard(c, [&] {
-    if (nw) CF1_CUDA(cudaMemcpyAsync(dst, c->d_states.p, nw * 8, cudaMemcpyDeviceToHost, c->stream));
-    CF1_CUDA(cudaStreamSynchronize(c->stream));
-  });
+  return guard(c, [&] { cf1::copy_out(c, dst, c->d_states.p, nw * 8); });
 }
 
 int cf1gpu_query(cf1gpu_ctx *c, const uint64_t *keys, size_t n, uint64_t *slots) {
@@ -361,6 +360,8 @@ void cf1gpu_destroy(cf1gpu_ctx *c) {
   for (auto &e : c->ev)
     if (e) cudaEventDestroy(e);
   for (auto &e : c->stage_ev)
+    if (e) cudaEventDestroy(e);
+  for (auto &e : c->io_ev)
     if (e) cudaEventDestroy(e);
   if (c->stream) cudaStreamDestroy(c->stream);
   if (c->copy_stream) cudaStreamDestroy(c->copy_stream);

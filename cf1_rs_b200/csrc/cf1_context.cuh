@@ -53,12 +53,15 @@ struct cf1gpu_ctx {
   cudaStream_t copy_stream = nullptr;  // streamed runs: host<->device copies beside the kernels
   cudaEvent_t ev[12] = {};
   cudaEvent_t stage_ev[8] = {};        // streamed runs: a phase-4 stage's words are packed
+  cudaEvent_t io_ev[4] = {};           // staged copies: a chunk in (2), a chunk out (2) has arrived
   int num_sms = 148;
   cf1::Tuning tune;
   cf1::LearnedOpts learned;
 
   // host input: records concatenated, one placeholder after each
   cf1::PinnedBuf host;
+  cf1::PinnedBuf stage_in, stage_out;  // chunks of copies to and from pageable memory
+  cf1::PinnedBuf readback;             // small results a run waits for (page-locked: one wait for several)
   uint64_t L = 0;
   uint64_t n_records = 0;
   uint64_t n_bases = 0;

@@ -2054,8 +2054,8 @@ int msd_prefix_bits(uint64_t max_bin_keys, bool sorted) {
 
 template <class KeyT>
 bool msd_sort_unique(KeyT *keys, KeyT *alt, uint64_t n, uint64_t max_bin, const uint64_t *seg_off, uint32_t nbins,
-                     int key_bits, int P, KeyT *dist, uint64_t *dist_off, MsdScratch &sc, cudaStream_t s, bool sorted,
-                     const Level0Out *l0, KeyT **kept, uint8_t *pkeys, uint8_t *palt, uint8_t **kept_pay,
+                     int key_bits, int P, KeyT *dist, uint64_t *dist_off, MsdScratch &sc, MsdRead &rd,
+                     cudaStream_t s, bool sorted, const Level0Out *l0, KeyT **kept, uint8_t *pkeys, uint8_t *palt, uint8_t **kept_pay,
                      uint8_t **l0pay_buf) {
   uint8_t *PT = pkeys;  // payloads beside T (nullptr: keys carry none)
   // passes on the top P bits: P1 then P2 (P2 may be 0) -- of the key, or of
@@ -2131,6 +2131,21 @@ bool msd_sort_unique(KeyT *keys, KeyT *alt, uint64_t n, uint64_t max_bin, const 
   KeyT *U = T == keys ? alt : keys;
   uint8_t *PU = pkeys ? (PT == pkeys ? palt : pkeys) : nullptr;
   if (l0pay_buf) *l0pay_buf = PU;
+  uint32_t *ovc = sc.ovc.get<uint32_t>(2);  // overflow count, work counter
+  CF1_CUDA(cudaMemsetAsync(ovc, 0, 2 * sizeof(uint32_t), s));
+  // the units' counts scanned and all results read back with one wait; once
+  // more when the block kernel had to take what the dedup left
+  uint64_t *out_off = sc.out_off.get<uint64_t>(nunit + 1);
+  auto finish = [&] {
+    exclusive_scan_u32(cnt, out_off, nunit, sc.scan_tmp, s);
+    cs_bin_off_kernel<<<(unsigned)ceil_div(nbins + 1, 256), 256, 0, s>>>(out_off, nbins, 1ull << PS, dist_off);
+    CF1_LAUNCH_CHECK();
+    CF1_CUDA(cudaMemcpyAsync(&rd.n_distinct, dist_off + nbins, sizeof(uint64_t), cudaMemcpyDeviceToHost, s));
+    CF1_CUDA(cudaMemcpyAsync(&rd.overflow, ovc, sizeof(uint32_t), cudaMemcpyDeviceToHost, s));
+    CF1_CUDA(cudaMemcpyAsync(&rd.oversize, over, sizeof(uint32_t), cudaMemcpyDeviceToHost, s));
+    if (l0 && l0->AR) CF1_CUDA(cudaMemcpyAsync(&rd.l0_err, l0->err, sizeof(uint32_t), cudaMemcpyDeviceToHost, s));
+    CF1_CUDA(cudaStreamSynchronize(s));
+  };
   if (nsub) {
     Level0Out lo;
     if (l0 && hashed) lo = *l0;
@@ -2155,8 +2170,9 @@ bool msd_sort_unique(KeyT *keys, KeyT *alt, uint64_t n, uint64_t max_bin, const 
       cs_plan_kernel<<<nbins, CP_BLOCK, 0, s>>>(sb_off, nbins, P, SrCfg<KeyT>::CAP, cl, cc);
       CF1_LAUNCH_CHECK();
       exclusive_scan_u32(cc, co, nbins, sc.scan_tmp, s);
-      CF1_CUDA(cudaMemcpyAsync(&grid, co + nbins, sizeof(uint64_t), cudaMemcpyDeviceToHost, s));
+      CF1_CUDA(cudaMemcpyAsync(&rd.runs, co + nbins, sizeof(uint64_t), cudaMemcpyDeviceToHost, s));
       CF1_CUDA(cudaStreamSynchronize(s));
+      grid = rd.runs;
       clist = cl;
       coff = co;
     }
@@ -2165,8 +2181,6 @@ bool msd_sort_unique(KeyT *keys, KeyT *alt, uint64_t n, uint64_t max_bin, const 
       // one CTA per group; the groups it cannot hold go to the block kernel
       // sub-bucket by sub-bucket, through the free buffers
       uint32_t *ov = sc.ov.get<uint32_t>(nunit + 1);
-      uint32_t *ovc = sc.ovc.get<uint32_t>(2);
-      CF1_CUDA(cudaMemsetAsync(ovc, 0, sizeof(uint32_t), s));
       auto gkern = pk ? gd_dedup_kernel<true> : gd_dedup_kernel<false>;
       CF1_CUDA(cudaFuncSetAttribute(gkern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(GdSmem)));
       uint64_t *T64 = reinterpret_cast<uint64_t *>(T), *U64 = reinterpret_cast<uint64_t *>(U);
@@ -2178,9 +2192,9 @@ bool msd_sort_unique(KeyT *keys, KeyT *alt, uint64_t n, uint64_t max_bin, const 
       const int p1 = pk ? P1 : 0;
       gkern<<<(unsigned)nunit, GD_BLOCK, sizeof(GdSmem), s>>>(T64, PT, sb_off, PS, P, cnt, keep, lo, ov, ovc, p1);
       CF1_LAUNCH_CHECK();
-      uint32_t h_ov = 0;
-      CF1_CUDA(cudaMemcpyAsync(&h_ov, ovc, sizeof(uint32_t), cudaMemcpyDeviceToHost, s));
-      CF1_CUDA(cudaStreamSynchronize(s));
+      CF1_CUDA(cudaEventRecord(sc.ev[1], s));
+      finish();
+      const uint32_t h_ov = rd.overflow;
       const unsigned nov = h_ov << g;  // sub-buckets
       sc.last_overflow = nov;
       sc.kept_packed = p1;
@@ -2198,13 +2212,13 @@ bool msd_sort_unique(KeyT *keys, KeyT *alt, uint64_t n, uint64_t max_bin, const 
         gd_gather_kernel<<<h_ov, GD_BLOCK, 0, s>>>(U64, lo.with_pay ? lb.l0pay : nullptr, sb_off, ov, g, sub_off, scnt,
                                                    T64, cnt, keep, lo, p1);
         CF1_LAUNCH_CHECK();
+        CF1_CUDA(cudaEventRecord(sc.ev[1], s));
+        finish();
       }
     } else if (W1 && hashed) {
       // the unsorted form: one warp per sub-bucket; the few it cannot hold
       // (more than WD_MAXD distinct keys) go to the block kernel after it
       uint32_t *ov = sc.ov.get<uint32_t>(nsub + 1);
-      uint32_t *ovc = sc.ovc.get<uint32_t>(2);  // overflow count, work counter
-      CF1_CUDA(cudaMemsetAsync(ovc, 0, 2 * sizeof(uint32_t), s));
       const size_t wsm = WD_WARPS * sizeof(WdSmem);
       auto wkern = pk ? wd_dedup_kernel<true> : wd_dedup_kernel<false>;
       CF1_CUDA(cudaFuncSetAttribute(wkern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)wsm));
@@ -2212,9 +2226,9 @@ bool msd_sort_unique(KeyT *keys, KeyT *alt, uint64_t n, uint64_t max_bin, const 
       wkern<<<wgrid, WD_WARPS * 32, wsm, s>>>(reinterpret_cast<uint64_t *>(T), PT, sb_off, nsub, P, cnt, lo, ov, ovc,
                                               ovc + 1, pk ? P1 : 0);
       CF1_LAUNCH_CHECK();
-      uint32_t h_ov = 0;
-      CF1_CUDA(cudaMemcpyAsync(&h_ov, ovc, sizeof(uint32_t), cudaMemcpyDeviceToHost, s));
-      CF1_CUDA(cudaStreamSynchronize(s));
+      CF1_CUDA(cudaEventRecord(sc.ev[1], s));
+      finish();
+      const uint32_t h_ov = rd.overflow;
       sc.last_overflow = h_ov;
       if (h_ov && pk) {  // the block kernel takes keys and bytes
         wd_unpack_kernel<<<(unsigned)ceil_div((uint64_t)h_ov * 32, 256), 256, 0, s>>>(
@@ -2225,49 +2239,45 @@ bool msd_sort_unique(KeyT *keys, KeyT *alt, uint64_t n, uint64_t max_bin, const 
         kern<<<h_ov, CS_BLOCK, smem, s>>>(T, U, sb_off, nsub, shift, rest > 0 ? bits : 0, cnt, over, P, lo, PT, PU,
                                           nullptr, nullptr, nbins, ov, nullptr);
         CF1_LAUNCH_CHECK();
+        CF1_CUDA(cudaEventRecord(sc.ev[1], s));
+        finish();
       }
     } else {
       // a CTA per run; the runs it cannot hold go to the block kernel
       uint32_t *ov = sc.ov.get<uint32_t>(grid + 1);
-      uint32_t *ovc = sc.ovc.get<uint32_t>(2);
-      CF1_CUDA(cudaMemsetAsync(ovc, 0, sizeof(uint32_t), s));
       const size_t ssm = sizeof(SrSmem<KeyT>);
       auto skern = hashed && !W1 ? sr_dedup_kernel<KeyT, !W1> : sr_dedup_kernel<KeyT, false>;
       CF1_CUDA(cudaFuncSetAttribute(skern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)ssm));
       skern<<<(unsigned)grid, SR_BLOCK, ssm, s>>>(T, PT, sb_off, nsub, P, hashed ? 32 - P : rest > 0 ? rest : 0, cnt, clist,
                                                  coff, nbins, ov, ovc);
       CF1_LAUNCH_CHECK();
-      uint32_t h_ov = 0;
-      CF1_CUDA(cudaMemcpyAsync(&h_ov, ovc, sizeof(uint32_t), cudaMemcpyDeviceToHost, s));
-      CF1_CUDA(cudaStreamSynchronize(s));
+      CF1_CUDA(cudaEventRecord(sc.ev[1], s));
+      finish();
+      const uint32_t h_ov = rd.overflow;
       if (h_ov) {
         kern<<<h_ov, CS_BLOCK, smem, s>>>(T, U, sb_off, nsub, shift, rest > 0 ? bits : 0, cnt, over, P, lo, PT, PU, clist,
                                           coff, nbins, nullptr, ov);
         CF1_LAUNCH_CHECK();
+        CF1_CUDA(cudaEventRecord(sc.ev[1], s));
+        finish();
       }
     }
-    CF1_CUDA(cudaEventRecord(sc.ev[1], s));
+  } else {
+    finish();
   }
-  uint32_t h_over = 0;
-  CF1_CUDA(cudaMemcpyAsync(&h_over, over, 4, cudaMemcpyDeviceToHost, s));
-  CF1_CUDA(cudaStreamSynchronize(s));
   sc.ms_dedup = 0;
   if (nsub) CF1_CUDA(cudaEventElapsedTime(&sc.ms_dedup, sc.ev[0], sc.ev[1]));
-  if (h_over) return false;
-  uint64_t *out_off = sc.out_off.get<uint64_t>(nunit + 1);
-  exclusive_scan_u32(cnt, out_off, nunit, sc.scan_tmp, s);
+  if (rd.oversize) return false;
   if (kept) *kept = T;
   if (kept_pay) *kept_pay = grp ? nullptr : PT;
   if (dist) msd_compact<KeyT>(T, nunit, dist, sc, s);
-  cs_bin_off_kernel<<<(unsigned)ceil_div(nbins + 1, 256), 256, 0, s>>>(out_off, nbins, 1ull << PS, dist_off);
-  CF1_LAUNCH_CHECK();
   return true;
 }
 
 #define CF1_INST(KT)                                                                                              \
   template int msd_prefix_bits<KT>(uint64_t, bool);                                                                     \
   template bool msd_sort_unique<KT>(KT *, KT *, uint64_t, uint64_t, const uint64_t *, uint32_t, int, int, KT *,   \
-                                    uint64_t *, MsdScratch &, cudaStream_t, bool, const Level0Out *, KT **, uint8_t *, \
+                                    uint64_t *, MsdScratch &, MsdRead &, cudaStream_t, bool, const Level0Out *, KT **, uint8_t *, \
                                     uint8_t *, uint8_t **, uint8_t **);                                       \
   template void msd_compact<KT>(const KT *, uint64_t, KT *, MsdScratch &, cudaStream_t);
 CF1_INST(uint64_t)

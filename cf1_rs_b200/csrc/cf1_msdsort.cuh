@@ -5,6 +5,15 @@
 
 namespace cf1 {
 
+// What a run of msd_sort_unique reads back, in page-locked memory of the
+// caller's.
+struct MsdRead {
+  uint64_t n_distinct, runs;
+  uint32_t overflow;  // units (unsorted) or runs (sorted) left to the block kernel
+  uint32_t oversize;  // a sub-bucket fits nowhere
+  uint32_t l0_err;    // Level0Out::err
+};
+
 struct MsdScratch {
   DevBuf tile_off, hist, hscan, scan_tmp, sb_off, sb_off1, cnt, out_off, flag, clist, ccount, coff, ov, ovc;
   // groups the group dedup left: their sub-buckets' offsets, counts, list and placed bytes
@@ -88,8 +97,8 @@ struct Level0Out {
 // there (*kept_pay = nullptr: they went to l0's outputs).
 template <class KeyT>
 bool msd_sort_unique(KeyT *keys, KeyT *alt, uint64_t n, uint64_t max_bin, const uint64_t *seg_off, uint32_t nbins,
-                     int key_bits, int P, KeyT *dist, uint64_t *dist_off, MsdScratch &sc, cudaStream_t s,
-                     bool sorted = true, const Level0Out *l0 = nullptr, KeyT **kept = nullptr, uint8_t *pkeys = nullptr,
+                     int key_bits, int P, KeyT *dist, uint64_t *dist_off, MsdScratch &sc, MsdRead &rd,
+                     cudaStream_t s, bool sorted = true, const Level0Out *l0 = nullptr, KeyT **kept = nullptr, uint8_t *pkeys = nullptr,
                      uint8_t *palt = nullptr, uint8_t **kept_pay = nullptr, uint8_t **l0pay_buf = nullptr);
 
 // The deferred copy: distinct keys of the last msd_sort_unique (nunit

@@ -6,6 +6,7 @@
 
 #include "cf1_context.cuh"
 #include "cf1_device_util.cuh"
+#include "cf1_hostio.cuh"
 #include "cf1_mphf.cuh"
 #include "cf1_phase4.cuh"
 #include "cf1_pipeline.cuh"
@@ -30,6 +31,17 @@ void PinnedBuf::reserve(size_t bytes, size_t keep) {
 }
 
 namespace {
+
+// Results a run reads back while it goes, in the context's page-locked block:
+// copies to it queue without a wait of their own.
+struct Readback {
+  struct Counters {
+    uint64_t n_super, n_occ, n_kept;
+  } u;
+  cf1::MsdRead msd;
+  uint64_t bb[2];  // entries and deepest level of BBHash's last levels
+  uint64_t bins[3][MAX_BINS + 1];  // k-mer, record and slot offsets of the bins
+};
 
 // Small device counters of one run.
 struct Small {
@@ -312,6 +324,9 @@ void run_impl(cf1gpu_ctx *c, StreamIO *io = nullptr, Step step = Step::FULL, con
   // The list lives in the key buffer, which phase 3 only fills after phase 2
   // has routed the list.
   Small hs;
+  c->readback.reserve(sizeof(Readback) + sizeof(Small), 0);
+  Readback *rb = reinterpret_cast<Readback *>(c->readback.p);
+  Small *rsm = reinterpret_cast<Small *>(c->readback.p + sizeof(Readback));
   const bool xscan = step == Step::XSCAN;
   auto phase1 = [&](uint32_t tile) {
     a.tile = tile;
@@ -331,9 +346,11 @@ void run_impl(cf1gpu_ctx *c, StreamIO *io = nullptr, Step step = Step::FULL, con
       CF1_CUDA(cudaMemsetAsync(sm, 0, sizeof(Small), s));
       launch_superkmer_scan(a, xscan ? 0 : pctas, s);
       if (!xscan) launch_partition(hist, B, lut, rec_off, &sm->n_bins_eff, s);
-      CF1_CUDA(cudaMemcpyAsync(&hs, sm, sizeof(Small), cudaMemcpyDeviceToHost, s));
-      if (!xscan) CF1_CUDA(cudaMemcpyAsync(&c->n_super, rec_off + B, sizeof(uint64_t), cudaMemcpyDeviceToHost, s));
+      CF1_CUDA(cudaMemcpyAsync(rsm, sm, sizeof(Small), cudaMemcpyDeviceToHost, s));
+      if (!xscan) CF1_CUDA(cudaMemcpyAsync(&rb->u.n_super, rec_off + B, sizeof(uint64_t), cudaMemcpyDeviceToHost, s));
       CF1_CUDA(cudaStreamSynchronize(s));
+      hs = *rsm;
+      if (!xscan) c->n_super = rb->u.n_super;
       if (!xscan && hs.rec_count != c->n_super)
         throw Error(CF1GPU_ERR_QUEUE_OVERRUN, "phase 1: record count != histogram total");
       if (hs.rec_count <= a.rec_cap) break;
@@ -392,9 +409,11 @@ void run_impl(cf1gpu_ctx *c, StreamIO *io = nullptr, Step step = Step::FULL, con
     }
     a.tile_begin = 0;
     launch_partition(hist, B, lut, rec_off, &sm->n_bins_eff, s);
-    CF1_CUDA(cudaMemcpyAsync(&hs, sm, sizeof(Small), cudaMemcpyDeviceToHost, s));
-    CF1_CUDA(cudaMemcpyAsync(&c->n_super, rec_off + B, sizeof(uint64_t), cudaMemcpyDeviceToHost, s));
+    CF1_CUDA(cudaMemcpyAsync(rsm, sm, sizeof(Small), cudaMemcpyDeviceToHost, s));
+    CF1_CUDA(cudaMemcpyAsync(&rb->u.n_super, rec_off + B, sizeof(uint64_t), cudaMemcpyDeviceToHost, s));
     CF1_CUDA(cudaStreamSynchronize(s));
+    hs = *rsm;
+    c->n_super = rb->u.n_super;
     if (hs.rec_count != c->n_super) throw Error(CF1GPU_ERR_QUEUE_OVERRUN, "phase 1: record count != histogram total");
     if (hs.rec_count > a.rec_cap) {  // the list overflowed: all bases are in place now, scan again
       c->rec_cap_hint = hs.rec_count;
@@ -509,8 +528,8 @@ void run_impl(cf1gpu_ctx *c, StreamIO *io = nullptr, Step step = Step::FULL, con
   // the dense distinct-key array, allocated when a step writes it
   auto dist_buf = [&]() { return c->d_dist.get<KeyT>(NO + 1); };
   uint64_t *dist_off = c->d_dist_off.get<uint64_t>(B + 1);
-  std::vector<uint64_t> hseg(B + 1);
-  CF1_CUDA(cudaMemcpyAsync(hseg.data(), seg, (B + 1) * sizeof(uint64_t), cudaMemcpyDeviceToHost, s));
+  const uint64_t *hseg = rb->bins[0];
+  CF1_CUDA(cudaMemcpyAsync(rb->bins[0], seg, (B + 1) * sizeof(uint64_t), cudaMemcpyDeviceToHost, s));
   CF1_CUDA(cudaStreamSynchronize(s));
   uint64_t max_bin = 0;
   for (uint32_t b = 0; b < B; b++) max_bin = std::max(max_bin, hseg[b + 1] - hseg[b]);
@@ -530,8 +549,8 @@ void run_impl(cf1gpu_ctx *c, StreamIO *io = nullptr, Step step = Step::FULL, con
       if (tried != -2) expand_again();  // the previous try consumed the keys
       if (batched) CF1_CUDA(cudaMemsetAsync(&sm->queues[4], 0, sizeof(uint32_t), s));
       CF1_CUDA(cudaEventRecord(c->ev[10], s));
-      const bool ok = msd_sort_unique<KeyT>(keys, alt, NO, max_bin, seg, B, 2 * k, P, dist_buf(), dist_off, be.msd, s,
-                                            sorted, nullptr, nullptr, pay, pay_alt);
+      const bool ok = msd_sort_unique<KeyT>(keys, alt, NO, max_bin, seg, B, 2 * k, P, dist_buf(), dist_off, be.msd, rb->msd,
+                                            s, sorted, nullptr, nullptr, pay, pay_alt);
       CF1_CUDA(cudaEventRecord(c->ev[11], s));
       CF1_CUDA(cudaEventSynchronize(c->ev[11]));
       const double ms = elapsed(c->ev[10], c->ev[11]);
@@ -601,7 +620,7 @@ void run_impl(cf1gpu_ctx *c, StreamIO *io = nullptr, Step step = Step::FULL, con
   KeyT *kept = nullptr;
   uint8_t *kept_pay = nullptr, *l0pay = nullptr;
   bool done = P >= 0 && msd_sort_unique<KeyT>(keys, alt, NO, max_bin, seg, B, 2 * k, P, l0_fuse ? nullptr : dist_buf(),
-                                              dist_off, be.msd, s, sorted, l0_fuse ? &l0 : nullptr, &kept, pay, pay_alt,
+                                              dist_off, be.msd, rb->msd, s, sorted, l0_fuse ? &l0 : nullptr, &kept, pay, pay_alt,
                                               &kept_pay, &l0pay);
   c->msd_bits = done ? P : -1;
   if (tune_now) {
@@ -620,11 +639,12 @@ void run_impl(cf1gpu_ctx *c, StreamIO *io = nullptr, Step step = Step::FULL, con
     segmented_unique<KeyT>(keys, NO, seg, B, dist_buf(), dist_off, be.sort, s);
   }
   KeyT *dist = c->d_dist.as<KeyT>();
-  CF1_CUDA(cudaMemcpyAsync(&c->n_distinct, dist_off + B, sizeof(uint64_t), cudaMemcpyDeviceToHost, s));
-  uint32_t l0_err = 1;
-  if (l0_fuse) CF1_CUDA(cudaMemcpyAsync(&l0_err, &sm->l0_err, sizeof(uint32_t), cudaMemcpyDeviceToHost, s));
-  CF1_CUDA(cudaStreamSynchronize(s));
-  const bool l0_ready = l0_fuse && done && l0_err == 0;
+  if (!done) {  // (the MSD path read the count back with its own results)
+    CF1_CUDA(cudaMemcpyAsync(&rb->msd.n_distinct, dist_off + B, sizeof(uint64_t), cudaMemcpyDeviceToHost, s));
+    CF1_CUDA(cudaStreamSynchronize(s));
+  }
+  c->n_distinct = rb->msd.n_distinct;
+  const bool l0_ready = l0_fuse && done && rb->msd.l0_err == 0;
   const int PU = be.msd.unit_bits;  // the dedup's units (sub-buckets or groups of them), 2^PU per bin
   const uint64_t nunit = done && P >= 0 ? (uint64_t)B << PU : 0;
   // phase 3 joined the occurrences' side sets: beside the kept keys, or (group
@@ -721,12 +741,13 @@ void run_impl(cf1gpu_ctx *c, StreamIO *io = nullptr, Step step = Step::FULL, con
     // group classifies.  Small results go in one stage: a stage is three
     // launches and a copy (30 kb: 120 us of kernels in eight).
     const int stages = (int)std::max<uint64_t>(1, std::min<uint64_t>(STREAM_STAGES, nwords * 8 / STREAM_STAGE_BYTES));
-    std::vector<uint64_t> hro(B + 1), hdo(B + 1);
+    uint64_t *hro = rb->bins[1], *hdo = rb->bins[2];
     if (stages > 1) {
-      CF1_CUDA(cudaMemcpyAsync(hro.data(), rec_off, (B + 1) * sizeof(uint64_t), cudaMemcpyDeviceToHost, s));
-      CF1_CUDA(cudaMemcpyAsync(hdo.data(), dist_off, (B + 1) * sizeof(uint64_t), cudaMemcpyDeviceToHost, s));
+      CF1_CUDA(cudaMemcpyAsync(hro, rec_off, (B + 1) * sizeof(uint64_t), cudaMemcpyDeviceToHost, s));
+      CF1_CUDA(cudaMemcpyAsync(hdo, dist_off, (B + 1) * sizeof(uint64_t), cudaMemcpyDeviceToHost, s));
       CF1_CUDA(cudaStreamSynchronize(s));
     } else {
+      hro[0] = hdo[0] = 0;
       hro[B] = NS;
     }
     uint32_t b0 = 0;
@@ -770,10 +791,11 @@ void run_impl(cf1gpu_ctx *c, StreamIO *io = nullptr, Step step = Step::FULL, con
     if (sideset) launch_sideset_pack(sides, 0, nwords, states, s);
   }
   CF1_CUDA(cudaEventRecord(c->ev[7], s));
-  CF1_CUDA(cudaMemcpyAsync(&hs, sm, sizeof(Small), cudaMemcpyDeviceToHost, s));
-  be.bb.collect_begin(s);
+  CF1_CUDA(cudaMemcpyAsync(rsm, sm, sizeof(Small), cudaMemcpyDeviceToHost, s));
+  be.bb.collect_begin(rb->bb, s);
   CF1_CUDA(cudaStreamSynchronize(s));
-  be.bb.collect_end();
+  be.bb.collect_end(rb->bb);
+  hs = *rsm;
   check_device_errors(hs.err);
   c->cas_retries = hs.cas_retries;
 
@@ -830,9 +852,8 @@ void dump_impl(cf1gpu_ctx *c, uint64_t *keys, uint8_t *states) {
   uint64_t *dk = c->d_qout.get<uint64_t>(n * cf1::KOps<KeyT>::WORDS + 1);
   uint8_t *ds = c->d_qin.get<uint8_t>(n + 1);
   launch_dump<KeyT>(make_view<KeyT>(c), c->nbins, n, c->d_states.as<const unsigned long long>(), dk, ds, s);
-  CF1_CUDA(cudaMemcpyAsync(keys, dk, n * cf1::KOps<KeyT>::WORDS * 8, cudaMemcpyDeviceToHost, s));
-  CF1_CUDA(cudaMemcpyAsync(states, ds, n, cudaMemcpyDeviceToHost, s));
-  CF1_CUDA(cudaStreamSynchronize(s));
+  copy_out(c, keys, dk, n * cf1::KOps<KeyT>::WORDS * 8);
+  copy_out(c, states, ds, n);
 }
 
 template <class KeyT>
@@ -856,6 +877,42 @@ void query_impl(cf1gpu_ctx *c, const uint64_t *keys, size_t n, uint64_t *slots) 
   constexpr int KW = cf1::KOps<KeyT>::WORDS;
   uint64_t *din = c->d_qin.get<uint64_t>(n * KW + 1);
   uint64_t *dout = c->d_qout.get<uint64_t>(n + 1);
+  const bool in_p = pageable(keys), out_p = pageable(slots);
+  if (n * 8 >= IO_STAGE_MIN && (in_p || out_p)) {
+    // In chunks: while one is looked up and its slots come back, the next
+    // one's keys go over and the previous one's slots are handed to the
+    // caller (8 M k-mers of pageable arrays in one piece each way: 20 ms).
+    const size_t per = IO_CHUNK / (KW * 8), chunks = (n + per - 1) / per;
+    c->stage_in.reserve(2 * IO_CHUNK, 0);
+    c->stage_out.reserve(2 * IO_CHUNK, 0);
+    HostCopier cp(n * (KW + 1) * 8);
+    auto len = [&](size_t i) { return std::min(per, n - i * per); };
+    auto drain = [&](size_t i) {
+      CF1_CUDA(cudaEventSynchronize(c->io_ev[2 + (i & 1)]));
+      cp.copy(slots + i * per, c->stage_out.p + (i & 1) * IO_CHUNK, len(i) * 8);
+    };
+    for (size_t i = 0; i < chunks; i++) {
+      const size_t b = i & 1, at = i * per;
+      const void *src = keys + at * KW;
+      if (in_p) {
+        if (i >= 2) CF1_CUDA(cudaEventSynchronize(c->io_ev[b]));  // the chunk's last keys have gone over
+        cp.copy(c->stage_in.p + b * IO_CHUNK, src, len(i) * KW * 8);
+        src = c->stage_in.p + b * IO_CHUNK;
+      }
+      CF1_CUDA(cudaMemcpyAsync(din + at * KW, src, len(i) * KW * 8, cudaMemcpyHostToDevice, c->copy_stream));
+      CF1_CUDA(cudaEventRecord(c->io_ev[b], c->copy_stream));
+      CF1_CUDA(cudaStreamWaitEvent(s, c->io_ev[b], 0));
+      launch_query<KeyT>(make_view<KeyT>(c), c->d_lut.as<const uint16_t>(), c->k, c->m, din + at * KW, len(i), dout + at,
+                         s);
+      CF1_CUDA(cudaMemcpyAsync(out_p ? static_cast<void *>(c->stage_out.p + b * IO_CHUNK) : slots + at, dout + at,
+                               len(i) * 8, cudaMemcpyDeviceToHost, s));
+      CF1_CUDA(cudaEventRecord(c->io_ev[2 + b], s));
+      if (out_p && i) drain(i - 1);
+    }
+    if (out_p) drain(chunks - 1);
+    CF1_CUDA(cudaStreamSynchronize(s));
+    return;
+  }
   CF1_CUDA(cudaMemcpyAsync(din, keys, n * KW * 8, cudaMemcpyHostToDevice, s));
   launch_query<KeyT>(make_view<KeyT>(c), c->d_lut.as<const uint16_t>(), c->k, c->m, din, n, dout, s);
   CF1_CUDA(cudaMemcpyAsync(slots, dout, n * 8, cudaMemcpyDeviceToHost, s));
@@ -1136,7 +1193,8 @@ void add_records(cf1gpu_ctx *c, const uint8_t *seqs, const uint64_t *off, size_t
   c->host.reserve(pos + 1, c->L);
   uint8_t *h = c->host.p;
   uint64_t total = pos - c->L;
-  unsigned nt = total > (64ull << 20) ? std::max(1u, std::min(16u, std::thread::hardware_concurrency())) : 1;
+  // a thread per 8 MB: one copies ~10 GB/s, and starting one takes ~100 us
+  unsigned nt = (unsigned)std::max<uint64_t>(1, std::min<uint64_t>({16, std::thread::hardware_concurrency(), total >> 23}));
   auto work = [&](unsigned t) {
     // record i goes to thread t when its destination start falls in t's share
     uint64_t lo = c->L + total * t / nt, hi = c->L + total * (t + 1) / nt;
