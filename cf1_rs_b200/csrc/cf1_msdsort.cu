@@ -25,10 +25,14 @@ namespace cf1 {
 
 namespace {
 
-constexpr int MS_BLOCK = 256;
-constexpr int MS_ITEMS = 16;
-constexpr uint32_t MS_TILE = MS_BLOCK * MS_ITEMS;  // 4096 keys per pass tile
-constexpr int MS_NW = MS_BLOCK / 32;
+constexpr int MS_BLOCK = 512;
+constexpr int MS_BITS = 11;  // most bits of a pass
+// Keys a thread of a multisplit pass holds: 128 bytes of them.
+template <class KeyT>
+constexpr int ms_items() { return KOps<KeyT>::WORDS == 1 ? 16 : 8; }
+template <class KeyT>
+constexpr uint32_t ms_tile() { return MS_BLOCK * ms_items<KeyT>(); }
+constexpr uint32_t MS_RUN = 8;  // tiles a CTA of the counting kernel takes
 constexpr int CS_BLOCK = 512;  // 16 warps: shared memory allows 2 CTAs per SM
 constexpr int CS_BITS = 10;
 constexpr uint32_t CS_BUCKETS = 1u << CS_BITS;
@@ -67,159 +71,131 @@ CF1_D uint32_t ms_digit<Key2>(const Key2 &k, int shift, uint32_t mask, bool hash
 
 
 // ---------------------------------------------------------------- multisplit pass
-template <class KeyT, int BITS>
+// One pass splits every segment on a digit of up to 11 bits:
+//   ms_hist_kernel    counts the segments' digits (a CTA takes MS_RUN tiles,
+//                     in shared memory, and adds its counts to the totals);
+//   a scan of the totals, which gives the sub-segments' offsets;
+//   ms_scatter_kernel moves the tiles.
+// Up to 11 bits in one pass because a pass is bound by its traffic: a tile of
+// 8192 keys still gives 1024 digits runs of 64 bytes, whose partial sectors L2
+// merges.  (1 Gbp, 10 bits: passes of 6 and 4 bits 4.63 + 3.95 ms and their
+// counts 1.18 + 1.15, one pass 5.71 and 1.13; 100 Mbp of 128-bit keys, 9 bits:
+// 2.72 and 0.51, now 1.40 and 0.25.)
+
+// Segment and stretch [start, end) of run t: tiles of `tile` keys, MS_RUN at a
+// time (tile_off counts tiles; a run never crosses a segment's edge).
+template <class KeyT>
 __global__ void __launch_bounds__(MS_BLOCK) ms_hist_kernel(const KeyT *keys, const uint64_t *seg_off,
-                                                           const uint32_t *tile_off, uint32_t nseg, int shift,
-                                                           bool hashed, uint32_t *H) {
-  constexpr uint32_t DIG = 1u << BITS;
-  __shared__ uint32_t h[DIG];
-  const uint32_t t = blockIdx.x;
-  if (t >= tile_off[nseg]) {
-    for (uint32_t d = threadIdx.x; d < DIG; d += MS_BLOCK) H[(uint64_t)t * DIG + d] = 0;
-    return;
-  }
-  for (uint32_t d = threadIdx.x; d < DIG; d += MS_BLOCK) h[d] = 0;
+                                                           const uint32_t *run_off, uint32_t nseg, int shift, int bits,
+                                                           bool hashed, uint32_t *tot) {
+  extern __shared__ uint32_t ms_h[];  // [1 << bits]
+  const uint32_t t = blockIdx.x, dig = 1u << bits;
+  if (t >= run_off[nseg]) return;
+  for (uint32_t d = threadIdx.x; d < dig; d += MS_BLOCK) ms_h[d] = 0;
   __syncthreads();
-  TileSpan sp = tile_span(seg_off, tile_off, nseg, t, MS_TILE);
+  const TileSpan sp = tile_span(seg_off, run_off, nseg, t, ms_tile<KeyT>() * MS_RUN);
+#pragma unroll 4
   for (uint64_t i = sp.start + threadIdx.x; i < sp.end; i += MS_BLOCK)
-    atomicAdd(&h[ms_digit(keys[i], shift, DIG - 1, hashed)], 1u);
+    atomicAdd(&ms_h[ms_digit(keys[i], shift, dig - 1, hashed)], 1u);
   __syncthreads();
-  for (uint32_t d = threadIdx.x; d < DIG; d += MS_BLOCK)
-    H[(uint64_t)sp.first_tile * DIG + (uint64_t)d * sp.ntiles + (t - sp.first_tile)] = h[d];
+  uint32_t *g = tot + ((uint64_t)sp.seg << bits);
+  for (uint32_t d = threadIdx.x; d < dig; d += MS_BLOCK)
+    if (ms_h[d]) atomicAdd(&g[d], ms_h[d]);
 }
 
-// Multisplit of one tile: warp w ranks the keys of the w-th 512-key slice of
-// the tile by a shared-memory atomic add on its per-warp digit count (the
-// order inside a digit does not matter: every sub-bucket is sorted or
-// deduplicated whole afterwards), a per-digit prefix over warps gives
-// tile-local positions, the tile is staged in shared memory in digit order,
-// and each digit's run is written out with consecutive threads on
-// consecutive addresses.  Four CTAs per SM (64 registers): at 3.1 Gbp the
-// two 64-bit passes took 3.3 ms less than with three CTAs and 80 registers.
+// Multisplit of one tile: every key takes its place among the tile's keys of
+// its digit from a shared-memory counter (the order inside a digit does not
+// matter: every sub-bucket is sorted or deduplicated whole afterwards), a scan
+// of the counters gives tile-local starts, one atomic a digit reserves the
+// tile's run in the digit's sub-segment, the tile is staged in shared memory in
+// digit order, and the runs are written out with consecutive threads on
+// consecutive addresses.  All of a thread's loads are issued before the first
+// is used, and the keys stay in registers for the staging step.
 // With pin/pout, each key's payload byte (its side-set byte) moves with it;
 // with PACK (pin, no pout; hashed 64-bit keys, pack = the pass's bits) the
 // byte goes into the key's packed output word (see pay_code).
-template <class KeyT, int BITS, bool PACK>
-__global__ void __launch_bounds__(MS_BLOCK, 4) ms_scatter_kernel(const KeyT *in, KeyT *out, const uint64_t *seg_off,
+template <class KeyT, bool PACK>
+__global__ void __launch_bounds__(MS_BLOCK, 2) ms_scatter_kernel(const KeyT *in, KeyT *out, const uint64_t *seg_off,
                                                                  const uint32_t *tile_off, uint32_t nseg, int shift,
-                                                                 bool hashed, const uint64_t *Hs, const uint8_t *pin,
-                                                                 uint8_t *pout, int pack) {
-  constexpr uint32_t DIG = 1u << BITS;
+                                                                 int bits, bool hashed, const uint64_t *sub_off,
+                                                                 uint32_t *cursor, const uint8_t *pin, uint8_t *pout,
+                                                                 int pack) {
+  constexpr int ITEMS = ms_items<KeyT>();
+  constexpr uint32_t TILE = ms_tile<KeyT>();
+  constexpr uint32_t PER = (1u << MS_BITS) / MS_BLOCK;  // digits a thread scans, at most
   extern __shared__ __align__(16) unsigned char ms_smem[];
-  KeyT *stage = reinterpret_cast<KeyT *>(ms_smem);                            // [MS_TILE]
-  uint32_t *whist = reinterpret_cast<uint32_t *>(stage + MS_TILE);           // [MS_NW][DIG]
-  uint32_t *lstart = whist + MS_NW * DIG;                                     // [DIG]
-  uint64_t *base = reinterpret_cast<uint64_t *>(lstart + DIG);                // [DIG]
-  uint8_t *pstage = reinterpret_cast<uint8_t *>(base + DIG);                  // [MS_TILE] when pin
+  const uint32_t dig = 1u << bits;
+  KeyT *stage = reinterpret_cast<KeyT *>(ms_smem);             // [TILE]
+  uint64_t *base = reinterpret_cast<uint64_t *>(stage + TILE);  // [dig] out index of a digit's key, less its stage index
+  uint32_t *cnt = reinterpret_cast<uint32_t *>(base + dig);     // [dig] counts, then tile-local starts
+  uint8_t *pstage = reinterpret_cast<uint8_t *>(cnt + dig);     // [TILE] when pin
   __shared__ uint32_t sm[MS_BLOCK / 32];
   const uint32_t t = blockIdx.x;
   if (t >= tile_off[nseg]) return;
-  TileSpan sp = tile_span(seg_off, tile_off, nseg, t, MS_TILE);
+  const TileSpan sp = tile_span(seg_off, tile_off, nseg, t, TILE);
   const unsigned tid = threadIdx.x, lane = lane_id(), warp = tid >> 5;
-  for (uint32_t i = tid; i < MS_NW * DIG; i += MS_BLOCK) whist[i] = 0;
-  for (uint32_t d = tid; d < DIG; d += MS_BLOCK)
-    base[d] = Hs[(uint64_t)sp.first_tile * DIG + (uint64_t)d * sp.ntiles + (t - sp.first_tile)];
-  __syncthreads();
-  const uint32_t n = (uint32_t)(sp.end - sp.start);
-  // per key: (rank in the warp's slice for its digit) << 8 | digit, or ~0
-  // for lanes past the tile (128-bit keys are read again when staged, which
-  // keeps their register count down)
-  uint32_t pk[MS_ITEMS];
-  uint32_t *wh = whist + warp * DIG;
-  // 64-bit keys: all of the thread's loads are issued before the first is
-  // used, and the keys stay in registers for the staging step
-  constexpr bool HOLD = KOps<KeyT>::WORDS == 1;
-  KeyT kk[HOLD ? MS_ITEMS : 1];
-  // the payload bytes are loaded with the keys, four to a register, so their
-  // latency is not paid again when the tile is staged
-  uint32_t pb[MS_ITEMS / 4];
+  const uint32_t n = (uint32_t)(sp.end - sp.start), i0 = warp * (ITEMS * 32) + lane;
+  KeyT key[ITEMS];
+  uint32_t pb[ITEMS / 4];  // payload bytes, four to a register
 #pragma unroll
-  for (int q = 0; q < MS_ITEMS / 4; q++) pb[q] = 0;
-  if constexpr (HOLD) {
+  for (int q = 0; q < ITEMS / 4; q++) pb[q] = 0;
 #pragma unroll
-    for (int r = 0; r < MS_ITEMS; r++) {
-      uint32_t li = warp * (MS_ITEMS * 32) + r * 32 + lane;
-      kk[r] = li < n ? in[sp.start + li] : KeyT{};
-      if (pin && li < n) pb[r >> 2] |= (uint32_t)pin[sp.start + li] << (8 * (r & 3));
-    }
+  for (int r = 0; r < ITEMS; r++) {
+    const uint32_t li = i0 + r * 32;
+    key[r] = li < n ? in[sp.start + li] : KeyT{};
+    if (pin && li < n) pb[r >> 2] |= (uint32_t)pin[sp.start + li] << (8 * (r & 3));
   }
+  for (uint32_t d = tid; d < dig; d += MS_BLOCK) cnt[d] = 0;
+  __syncthreads();
+  uint32_t pk[ITEMS];  // rank << MS_BITS | digit
 #pragma unroll
-  for (int r = 0; r < MS_ITEMS; r++) {
-    uint32_t li = warp * (MS_ITEMS * 32) + r * 32 + lane;
-    pk[r] = 0xFFFFFFFFu;
-    if (li < n) {
-      uint32_t d = ms_digit(HOLD ? kk[HOLD ? r : 0] : in[sp.start + li], shift, DIG - 1, hashed);
-      pk[r] = (atomicAdd(&wh[d], 1u) << 8) | d;
+  for (int r = 0; r < ITEMS; r++) {
+    if (i0 + r * 32 < n) {
+      const uint32_t d = ms_digit(key[r], shift, dig - 1, hashed);
+      pk[r] = (atomicAdd(&cnt[d], 1u) << MS_BITS) | d;
     }
   }
   __syncthreads();
-  // per digit: exclusive prefix over warps; tile total per digit
-  uint32_t tot_d = 0;
-  for (uint32_t d = tid; d < DIG; d += MS_BLOCK) {
-    uint32_t run = 0;
-    for (int w = 0; w < MS_NW; w++) {
-      uint32_t v = whist[w * DIG + d];
-      whist[w * DIG + d] = run;
-      run += v;
+  {
+    const uint32_t per = dig > MS_BLOCK ? dig / MS_BLOCK : 1u, d0 = tid * per;
+    uint32_t c[PER], own = 0;
+#pragma unroll
+    for (uint32_t i = 0; i < PER; i++) {
+      c[i] = i < per && d0 + i < dig ? cnt[d0 + i] : 0u;
+      own += c[i];
     }
-    if (DIG <= MS_BLOCK) tot_d = run;
-    else lstart[d] = run;
-  }
-  __syncthreads();
-  // tile-local start of each digit: exclusive scan over digits (one digit a
-  // thread; the threads past the digits add nothing)
-  if (DIG <= MS_BLOCK) {
-    uint32_t tot;
-    uint32_t pre = block_exclusive_scan<MS_BLOCK>(tot_d, sm, tot);
-    if (tid < DIG) lstart[tid] = pre;
-  } else if (tid == 0) {
-    uint32_t run = 0;
-    for (uint32_t d = 0; d < DIG; d++) {
-      uint32_t v = lstart[d];
-      lstart[d] = run;
-      run += v;
+    uint32_t tot, run = block_exclusive_scan<MS_BLOCK>(own, sm, tot);
+    const uint64_t g = ((uint64_t)sp.seg << bits) + d0;
+#pragma unroll
+    for (uint32_t i = 0; i < PER; i++) {
+      if (i < per && d0 + i < dig) {
+        cnt[d0 + i] = run;
+        if (c[i]) base[d0 + i] = sub_off[g + i] + atomicAdd(&cursor[g + i], c[i]) - run;
+        run += c[i];
+      }
     }
   }
   __syncthreads();
 #pragma unroll
-  for (int r = 0; r < MS_ITEMS; r++) {
-    if (pk[r] != 0xFFFFFFFFu) {
-      uint32_t d = pk[r] & 0xFF, li = warp * (MS_ITEMS * 32) + r * 32 + lane;
-      const uint32_t at = lstart[d] + wh[d] + (pk[r] >> 8);
-      stage[at] = HOLD ? kk[HOLD ? r : 0] : in[sp.start + li];
-      if (pin) pstage[at] = HOLD ? (uint8_t)(pb[r >> 2] >> (8 * (r & 3))) : pin[sp.start + li];
+  for (int r = 0; r < ITEMS; r++) {
+    if (i0 + r * 32 < n) {
+      const uint32_t at = cnt[pk[r] & ((1u << MS_BITS) - 1)] + (pk[r] >> MS_BITS);
+      stage[at] = key[r];
+      if (pin) pstage[at] = (uint8_t)(pb[r >> 2] >> (8 * (r & 3)));
     }
   }
   __syncthreads();
+#pragma unroll 4
   for (uint32_t i = tid; i < n; i += MS_BLOCK) {
-    KeyT kk = stage[i];
-    uint32_t d = ms_digit(kk, shift, DIG - 1, hashed);
-    const uint64_t o = base[d] + (i - lstart[d]);
+    const KeyT k = stage[i];
+    const uint64_t o = base[ms_digit(k, shift, dig - 1, hashed)] + i;
     if constexpr (PACK) {  // hashed 64-bit keys with payloads: the packed word (see pay_code)
-      out[o] = ((kk * MS_HASH_MUL) << pack) | pay_code(pstage[i]);
+      out[o] = ((k * MS_HASH_MUL) << pack) | pay_code(pstage[i]);
     } else {
-      out[o] = kk;
+      out[o] = k;
       if (pout) pout[o] = pstage[i];
     }
   }
-}
-
-// Sub-bucket starts after the last pass: sub-bucket (segment s, digit d)
-// begins at the scanned histogram entry of its first tile.
-template <int BITS>
-__global__ void ms_subbucket_kernel(const uint64_t *seg_off, const uint32_t *tile_off, uint32_t nseg,
-                                    const uint64_t *Hs, uint64_t *sb_off) {
-  constexpr uint32_t DIG = 1u << BITS;
-  uint64_t j = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  uint64_t nsub = (uint64_t)nseg * DIG;
-  if (j > nsub) return;
-  if (j == nsub) {
-    sb_off[j] = seg_off[nseg];
-    return;
-  }
-  uint32_t s = (uint32_t)(j / DIG), d = (uint32_t)(j % DIG);
-  uint32_t ft = tile_off[s], nt = tile_off[s + 1] - ft;
-  sb_off[j] = nt ? Hs[(uint64_t)ft * DIG + (uint64_t)d * nt] : seg_off[s];
 }
 
 // ---------------------------------------------------------------- chunk sort
@@ -1953,65 +1929,33 @@ __global__ void cs_bin_off_kernel(const uint64_t *out_off, uint32_t nbins, uint6
   if (b <= nbins) dist_off[b] = out_off[(uint64_t)b * per_bin];
 }
 
-template <class KeyT, int BITS>
-void ms_pass(const KeyT *in, KeyT *out, uint64_t n, const uint64_t *seg_off, uint32_t nseg, int shift, bool hashed,
-             MsdScratch &sc, cudaStream_t s, const uint8_t *pin, uint8_t *pout, int pack) {
-  constexpr uint32_t DIG = 1u << BITS;
-  uint32_t ub = (uint32_t)(ceil_div(n, MS_TILE) + nseg);
-  uint32_t *tile_off = sc.tile_off.get<uint32_t>(nseg + 1);
-  segment_tiles(seg_off, nseg, MS_TILE, tile_off, s);
-  uint32_t *H = sc.hist.get<uint32_t>((uint64_t)ub * DIG);
-  uint64_t *Hs = sc.hscan.get<uint64_t>((uint64_t)ub * DIG + 1);
-  ms_hist_kernel<KeyT, BITS><<<ub, MS_BLOCK, 0, s>>>(in, seg_off, tile_off, nseg, shift, hashed, H);
-  CF1_LAUNCH_CHECK();
-  exclusive_scan_u32(H, Hs, (uint64_t)ub * DIG, sc.scan_tmp, s);
-  size_t smem = MS_TILE * sizeof(KeyT) + (MS_NW + 1) * DIG * sizeof(uint32_t) + DIG * sizeof(uint64_t) +
-                (pin ? MS_TILE : 0);
-  auto kern = ms_scatter_kernel<KeyT, BITS, false>;
-  if constexpr (KOps<KeyT>::WORDS == 1)
-    if (pack) kern = ms_scatter_kernel<KeyT, BITS, true>;
-  CF1_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-  kern<<<ub, MS_BLOCK, smem, s>>>(in, out, seg_off, tile_off, nseg, shift, hashed, Hs, pin, pout, pack);
-  CF1_LAUNCH_CHECK();
-}
-
+// Splits the segments of `in` into `out` on `bits` bits; sub_off[0 .. nseg <<
+// bits] gets the sub-segments' offsets.
 template <class KeyT>
-void ms_pass_bits(int bits, const KeyT *in, KeyT *out, uint64_t n, const uint64_t *seg_off, uint32_t nseg, int shift,
-                  bool hashed, MsdScratch &sc, cudaStream_t s, const uint8_t *pin, uint8_t *pout, int pack = 0) {
-  switch (bits) {
-    case 1: ms_pass<KeyT, 1>(in, out, n, seg_off, nseg, shift, hashed, sc, s, pin, pout, pack); break;
-    case 2: ms_pass<KeyT, 2>(in, out, n, seg_off, nseg, shift, hashed, sc, s, pin, pout, pack); break;
-    case 3: ms_pass<KeyT, 3>(in, out, n, seg_off, nseg, shift, hashed, sc, s, pin, pout, pack); break;
-    case 4: ms_pass<KeyT, 4>(in, out, n, seg_off, nseg, shift, hashed, sc, s, pin, pout, pack); break;
-    case 5: ms_pass<KeyT, 5>(in, out, n, seg_off, nseg, shift, hashed, sc, s, pin, pout, pack); break;
-    case 6: ms_pass<KeyT, 6>(in, out, n, seg_off, nseg, shift, hashed, sc, s, pin, pout, pack); break;
-    case 7: ms_pass<KeyT, 7>(in, out, n, seg_off, nseg, shift, hashed, sc, s, pin, pout, pack); break;
-    case 8: ms_pass<KeyT, 8>(in, out, n, seg_off, nseg, shift, hashed, sc, s, pin, pout, pack); break;
-    default: throw Error(-1, "MSD pass width must be 1..8 bits");
-  }
-}
-
-template <int BITS>
-void subbuckets(const uint64_t *seg_off, const uint32_t *tile_off, uint32_t nseg, const uint64_t *Hs,
-                uint64_t *sb_off, cudaStream_t s) {
-  uint64_t nsub = (uint64_t)nseg << BITS;
-  ms_subbucket_kernel<BITS><<<(unsigned)ceil_div(nsub + 1, 256), 256, 0, s>>>(seg_off, tile_off, nseg, Hs, sb_off);
+void ms_pass(int bits, const KeyT *in, KeyT *out, uint64_t n, const uint64_t *seg_off, uint32_t nseg, int shift,
+             bool hashed, uint64_t *sub_off, MsdScratch &sc, cudaStream_t s, const uint8_t *pin, uint8_t *pout,
+             int pack = 0) {
+  constexpr uint32_t TILE = ms_tile<KeyT>();
+  if (bits < 1 || bits > MS_BITS) throw Error(-1, "MSD pass width must be 1..11 bits");
+  const uint64_t nsub = (uint64_t)nseg << bits;
+  uint32_t *tile_off = sc.tile_off.get<uint32_t>(2 * (nseg + 1)), *run_off = tile_off + nseg + 1;
+  segment_tiles(seg_off, nseg, TILE, tile_off, s);
+  segment_tiles(seg_off, nseg, TILE * MS_RUN, run_off, s);
+  uint32_t *tot = sc.hist.get<uint32_t>(2 * nsub), *cursor = tot + nsub;
+  CF1_CUDA(cudaMemsetAsync(tot, 0, 2 * nsub * sizeof(uint32_t), s));
+  const size_t hsm = sizeof(uint32_t) << bits;
+  ms_hist_kernel<KeyT><<<(unsigned)(ceil_div(n, TILE * MS_RUN) + nseg), MS_BLOCK, hsm, s>>>(in, seg_off, run_off, nseg,
+                                                                                         shift, bits, hashed, tot);
   CF1_LAUNCH_CHECK();
-}
-
-void subbuckets_bits(int bits, const uint64_t *seg_off, const uint32_t *tile_off, uint32_t nseg, const uint64_t *Hs,
-                     uint64_t *sb_off, cudaStream_t s) {
-  switch (bits) {
-    case 1: subbuckets<1>(seg_off, tile_off, nseg, Hs, sb_off, s); break;
-    case 2: subbuckets<2>(seg_off, tile_off, nseg, Hs, sb_off, s); break;
-    case 3: subbuckets<3>(seg_off, tile_off, nseg, Hs, sb_off, s); break;
-    case 4: subbuckets<4>(seg_off, tile_off, nseg, Hs, sb_off, s); break;
-    case 5: subbuckets<5>(seg_off, tile_off, nseg, Hs, sb_off, s); break;
-    case 6: subbuckets<6>(seg_off, tile_off, nseg, Hs, sb_off, s); break;
-    case 7: subbuckets<7>(seg_off, tile_off, nseg, Hs, sb_off, s); break;
-    case 8: subbuckets<8>(seg_off, tile_off, nseg, Hs, sb_off, s); break;
-    default: throw Error(-1, "MSD pass width must be 1..8 bits");
-  }
+  exclusive_scan_u32(tot, sub_off, nsub, sc.scan_tmp, s);
+  const size_t smem = TILE * sizeof(KeyT) + ((sizeof(uint64_t) + sizeof(uint32_t)) << bits) + (pin ? TILE : 0);
+  auto kern = ms_scatter_kernel<KeyT, false>;
+  if constexpr (KOps<KeyT>::WORDS == 1)
+    if (pack) kern = ms_scatter_kernel<KeyT, true>;
+  CF1_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+  kern<<<(unsigned)(ceil_div(n, TILE) + nseg), MS_BLOCK, smem, s>>>(in, out, seg_off, tile_off, nseg, shift, bits, hashed,
+                                                                   sub_off, cursor, pin, pout, pack);
+  CF1_LAUNCH_CHECK();
 }
 
 }  // namespace
@@ -2063,6 +2007,7 @@ bool msd_sort_unique(KeyT *keys, KeyT *alt, uint64_t n, uint64_t max_bin, const 
   const bool hashed = !sorted;
   constexpr bool W1 = KOps<KeyT>::WORDS == 1;
   if (hashed) key_bits = 64;
+  else P = P < key_bits ? P : key_bits;  // short keys (k <= 7) have no more prefix bits than that
   // packed passes (see pay_code): the hashed split of keys with payloads
   // whose dedup builds BBHash level 0, with a first pass of >= 6 bits
   // Groups of 32 sub-buckets for the group dedup (gd_dedup_kernel), split on
@@ -2075,7 +2020,7 @@ bool msd_sort_unique(KeyT *keys, KeyT *alt, uint64_t n, uint64_t max_bin, const 
   sc.unit_bits = PS;
   sc.kept_bits = false;
   const bool pk = W1 && hashed && pkeys && palt && l0 && l0->AR && l0->with_pay && PS >= (int)PACK_MIN_BITS;
-  int P1 = PS > 8 ? (PS + 1) / 2 : PS;
+  int P1 = PS > MS_BITS ? (PS + 1) / 2 : PS;
   if (pk && P1 < (int)PACK_MIN_BITS) P1 = PACK_MIN_BITS;
   const int P2 = PS - P1;
   KeyT *T = keys;
@@ -2084,27 +2029,22 @@ bool msd_sort_unique(KeyT *keys, KeyT *alt, uint64_t n, uint64_t max_bin, const 
   if (PS == 0) {
     CF1_CUDA(cudaMemcpyAsync(sb_off, seg_off, (nbins + 1) * sizeof(uint64_t), cudaMemcpyDeviceToDevice, s));
   } else if (n) {
-    ms_pass_bits<KeyT>(P1, keys, alt, n, seg_off, nbins, key_bits - P1, hashed, sc, s, pkeys, pk ? nullptr : palt,
-                       pk ? P1 : 0);
-    const uint64_t *seg2 = seg_off;
-    uint32_t nseg2 = nbins;
+    // sub-segments of pass 1: (bin, first digit), the segments of pass 2
+    uint64_t *sb1 = P2 ? sc.sb_off1.get<uint64_t>(((uint64_t)nbins << P1) + 1) : sb_off;
+    ms_pass<KeyT>(P1, keys, alt, n, seg_off, nbins, key_bits - P1, hashed, sb1, sc, s, pkeys, pk ? nullptr : palt,
+                  pk ? P1 : 0);
     if (P2) {
-      // segments of pass 2: (bin, first digit), from pass 1's scanned histogram
-      uint64_t *sb1 = sc.sb_off1.get<uint64_t>(((uint64_t)nbins << P1) + 1);
-      subbuckets_bits(P1, seg_off, sc.tile_off.as<uint32_t>(), nbins, sc.hscan.as<uint64_t>(), sb1, s);
-      nseg2 = (uint32_t)((uint64_t)nbins << P1);
-      seg2 = sb1;
+      const uint32_t nseg2 = (uint32_t)((uint64_t)nbins << P1);
       if (pk)  // packed words: their own top bits are the next digit, the bytes travel inside
-        ms_pass_bits<KeyT>(P2, alt, keys, n, seg2, nseg2, 64 - P2, false, sc, s, nullptr, nullptr);
+        ms_pass<KeyT>(P2, alt, keys, n, sb1, nseg2, 64 - P2, false, sb_off, sc, s, nullptr, nullptr);
       else
-        ms_pass_bits<KeyT>(P2, alt, keys, n, seg2, nseg2, key_bits - P1 - P2, hashed, sc, s, palt, pkeys);
+        ms_pass<KeyT>(P2, alt, keys, n, sb1, nseg2, key_bits - P1 - P2, hashed, sb_off, sc, s, palt, pkeys);
       T = keys;
       PT = pkeys;
     } else {
       T = alt;
       PT = palt;
     }
-    subbuckets_bits(P2 ? P2 : P1, seg2, sc.tile_off.as<uint32_t>(), nseg2, sc.hscan.as<uint64_t>(), sb_off, s);
   } else {
     CF1_CUDA(cudaMemsetAsync(sb_off, 0, (nunit + 1) * sizeof(uint64_t), s));
   }
