@@ -229,8 +229,8 @@ static_assert(KEY_SPREAD_MUL * KEY_SPREAD_INV == 1, "KEY_SPREAD_INV inverts KEY_
 // Packed words of the phase-3 multisplit (hashed split of 64-bit keys with
 // payload bytes, pass 1 of at least 6 bits): after the first pass a key's
 // top p1 bits of h = key * KEY_SPREAD_MUL are its segment's, so the word
-// keeps the other 64 - p1 bits of h, shifted up, and the payload byte's
-// 6-bit code in the p1 bits freed.
+// keeps the other 64 - p1 bits of h, shifted up, and the payload's 6-bit code
+// (contribution_code) in the p1 bits freed.
 // The next pass splits on the word's own top bits; the dedup rebuilds h from
 // the sub-bucket's index and the key as h * KEY_SPREAD_INV.  A single
 // occurrence's side-set byte has nibbles in {3, 5, 6, 9, F} (sideset_byte):
@@ -245,7 +245,7 @@ constexpr uint64_t pay_nib_codes() {
   return t;
 }
 constexpr uint64_t PAY_NIB_CODE = pay_nib_codes();  // nibble -> code, 3 bits each
-constexpr uint32_t PAY_NIB_OF = 0x0F9653u;            // code -> nibble, 4 bits each (codes 0..5)
+constexpr uint32_t PAY_NIB_OF = 0xF00F9653u;          // code -> nibble, 4 bits each (codes 0..5; 7 is M too)
 CF1_HD uint32_t pay_code(uint32_t byte) {
   return (uint32_t)((PAY_NIB_CODE >> (3 * (byte & 0xF))) & 7) | ((uint32_t)((PAY_NIB_CODE >> (3 * (byte >> 4))) & 7) << 3);
 }
@@ -437,6 +437,23 @@ CF1_HD uint32_t contribution_sideset_rolled(KeyT fw, KeyT rcv, KeyT nf, KeyT nr,
   const KeyT can = kmin(fw, rcv);
   return sideset_byte(fw == can, has_prev, prev, has_next, next, has_next && kmin(nf, nr) == can,
                       has_next && nf == fw);
+}
+
+// The same as the byte's 6-bit code (see pay_code; pay_byte gives the byte),
+// which is what travels with a key until its occurrences are joined.  A side's
+// code is its base, or 4 for M: read forward the front is x, the base before,
+// and the back y, the base after; read backward they swap and complement (4
+// becomes 7, which also reads back as M).  prev and next are 4 where there is
+// no base; nf and nr are only looked at when has_next.
+template <class KeyT>
+CF1_HD uint32_t contribution_code(KeyT fw, KeyT rcv, KeyT nf, uint32_t prev, bool has_next, uint32_t next) {
+  uint32_t x = prev, y = has_next ? next : 4u;
+  const bool loop = nf == fw;
+  if (has_next && (loop || nf == rcv)) {  // the next k-mer is the same vertex
+    y = 4;
+    if (loop) x = 4;
+  }
+  return rcv < fw ? ((x << 3) | y) ^ 27u : (y << 3) | x;
 }
 
 template <class KeyT>

@@ -111,9 +111,9 @@ __global__ void __launch_bounds__(MS_BLOCK) ms_hist_kernel(const KeyT *keys, con
 // digit order, and the runs are written out with consecutive threads on
 // consecutive addresses.  All of a thread's loads are issued before the first
 // is used, and the keys stay in registers for the staging step.
-// With pin/pout, each key's payload byte (its side-set byte) moves with it;
+// With pin/pout, each key's payload (its side-set code) moves with it;
 // with PACK (pin, no pout; hashed 64-bit keys, pack = the pass's bits) the
-// byte goes into the key's packed output word (see pay_code).
+// code goes into the key's packed output word (see pay_code).
 template <class KeyT, bool PACK>
 __global__ void __launch_bounds__(MS_BLOCK, 2) ms_scatter_kernel(const KeyT *in, KeyT *out, const uint64_t *seg_off,
                                                                  const uint32_t *tile_off, uint32_t nseg, int shift,
@@ -190,7 +190,7 @@ __global__ void __launch_bounds__(MS_BLOCK, 2) ms_scatter_kernel(const KeyT *in,
     const KeyT k = stage[i];
     const uint64_t o = base[ms_digit(k, shift, dig - 1, hashed)] + i;
     if constexpr (PACK) {  // hashed 64-bit keys with payloads: the packed word (see pay_code)
-      out[o] = ((k * MS_HASH_MUL) << pack) | pay_code(pstage[i]);
+      out[o] = ((k * MS_HASH_MUL) << pack) | pstage[i];
     } else {
       out[o] = k;
       if (pout) pout[o] = pstage[i];
@@ -589,7 +589,8 @@ __global__ void __launch_bounds__(CS_BLOCK, SORTED ? 2 : 4) cs_sort_unique_kerne
                                                                   uint32_t *oversize, int P, Level0Out l0,
                                                                   uint8_t *TP, uint8_t *UP, const uint2 *clist,
                                                                   const uint64_t *coff, uint32_t nbins,
-                                                                  const uint32_t *jlist, const uint32_t *klist) {
+                                                                  const uint32_t *jlist, const uint32_t *klist,
+                                                                  bool codes) {
   constexpr uint32_t CAP = cs_cap<KeyT, SORTED>();
   constexpr bool L0 = !SORTED && KOps<KeyT>::WORDS == 1;
   __shared__ unsigned long long s_l0base;
@@ -617,6 +618,10 @@ __global__ void __launch_bounds__(CS_BLOCK, SORTED ? 2 : 4) cs_sort_unique_kerne
   if (j >= nsub) return;
   const uint64_t a = sb_off[j], n = sb_off[jend] - a;
   const unsigned tid = threadIdx.x;
+  if (codes && TP) {  // payloads as they travel: the bytes they stand for
+    for (uint64_t i = a + tid; i < a + n; i += CS_BLOCK) TP[i] = (uint8_t)pay_byte(TP[i]);
+    __syncthreads();
+  }
   // the sub-bucket's distinct keys end at T[a, a + result); ~0u: oversized
   auto body = [&]() -> uint32_t {
     if (n == 0) return 0;
@@ -825,7 +830,7 @@ __global__ void __launch_bounds__(SR_BLOCK, 2) sr_dedup_kernel(KeyT *T, uint8_t 
     const uint32_t i = u * SR_BLOCK + tid;
     if (i < n) {
       key[u] = T[a + i];
-      if (TP) pb[u >> 2] |= (uint32_t)TP[a + i] << (8 * (u & 3));
+      if (TP) pb[u >> 2] |= pay_byte(TP[a + i]) << (8 * (u & 3));
     }
   }
 #pragma unroll
@@ -1072,6 +1077,24 @@ CF1_D uint32_t gd_warp_excl(uint32_t v, uint32_t &tot) {
   tot = __shfl_sync(FULL, x, 31);
   return x - v;
 }
+// Shared-memory ORs under a predicate, as predicated instructions: written as
+// `if`, each became a branch with its reconvergence in the unrolled loops.
+CF1_D uint32_t gd_shared(const void *p) { return (uint32_t)__cvta_generic_to_shared(p); }
+CF1_D uint32_t gd_or_if(uint32_t pred, uint32_t addr, uint32_t v) {  // returns the old word, 0 without pred
+  uint32_t old;
+  asm volatile(
+      "{\n .reg .pred p;\n setp.ne.u32 p, %1, 0;\n mov.u32 %0, 0;\n @p atom.shared.or.b32 %0, [%2], %3;\n}"
+      : "=r"(old)
+      : "r"(pred), "r"(addr), "r"(v)
+      : "memory");
+  return old;
+}
+CF1_D void gd_red_or_if(uint32_t pred, uint32_t addr, uint32_t v) {
+  asm volatile("{\n .reg .pred p;\n setp.ne.u32 p, %0, 0;\n @p red.shared.or.b32 [%1], %2;\n}"
+               :
+               : "r"(pred), "r"(addr), "r"(v)
+               : "memory");
+}
 // First word of a unit's keep bits: the units' occurrences one after another,
 // every unit from a word of its own.
 CF1_D uint64_t gd_keep_word(uint64_t a, uint64_t q) { return (a >> 5) + q; }
@@ -1115,7 +1138,7 @@ __global__ void __launch_bounds__(GD_BLOCK, 2) gd_dedup_kernel(const uint64_t *T
   const uint32_t n = (uint32_t)n64, gw = sw * subs, gw1 = sw1 * subs;
   const uint64_t *Tk = T + a + tid;
   unsigned long long key[GD_U];    // PK: the packed word
-  uint32_t pb[PK ? 1 : GD_U / 4];  // payload bytes, four to a register (PK: inside the word)
+  uint32_t pb[PK ? 1 : GD_U / 4];  // payload codes, four to a register (PK: inside the word)
   const uint32_t act = tid < n ? (0xFFFFFFFFu >> (31 - (n - 1 - tid) / GD_BLOCK)) : 0u;  // this thread's keys
   if constexpr (!PK) {
 #pragma unroll
@@ -1147,7 +1170,7 @@ __global__ void __launch_bounds__(GD_BLOCK, 2) gd_dedup_kernel(const uint64_t *T
   auto key_of = [&](unsigned long long w) -> uint64_t { return PK ? (hi | (w >> p1)) * KEY_SPREAD_INV : w; };
   auto pay_of = [&](int u) -> uint32_t {
     if constexpr (PK) return (uint32_t)m.lut[(uint32_t)key[u] & 63u];
-    else return (pb[u >> 2] >> (8 * (u & 3))) & 0xFFu;
+    else return (uint32_t)m.lut[(pb[u >> 2] >> (8 * (u & 3))) & 63u];
   };
   auto list_pay = [&](unsigned long long w, uint32_t i) -> uint32_t {
     return PK ? (uint32_t)m.lut[(uint32_t)w & 63u] : (uint32_t)m.lp[i];
@@ -1166,20 +1189,20 @@ __global__ void __launch_bounds__(GD_BLOCK, 2) gd_dedup_kernel(const uint64_t *T
                  *fpre1 = reinterpret_cast<const uint16_t *>(m.fpre1);
   __syncthreads();
   // 1. mark
-  bool hit = false;
+  const uint32_t set_at = gd_shared(m.set), col_at = gd_shared(m.col);
+  uint32_t hit = 0;
 #pragma unroll
   for (int u = 0; u < GD_U; u++) {
-    if (u * GD_BLOCK < n && ((act >> u) & 1)) {
-      const uint32_t b = bit_of(key[u]), bm = 1u << (b & 31);
-      if (atomicOr(&set32[b >> 5], bm) & bm) {
-        hit = true;
-        atomicOr(&col32[b >> 5], bm);
-      }
+    if (u * GD_BLOCK < n) {
+      const uint32_t b = bit_of(key[u]), bm = 1u << (b & 31), w = (b >> 5) * 4;
+      const uint32_t h = gd_or_if(act & (1u << u), set_at + w, bm) & bm;
+      gd_red_or_if(h, col_at + w, bm);
+      hit |= h;
     }
   }
   uint32_t cont = 0, k0 = 0;  // this thread's keys on a bit set more than once, and the first one's list entry
   uint32_t nl = 0;
-  if (__syncthreads_or((int)hit)) {
+  if (__syncthreads_or(hit != 0)) {
     // 2. the list, and the numbers of those bits (a warp a slice, one
     //    reservation each)
 #pragma unroll
@@ -1207,14 +1230,14 @@ __global__ void __launch_bounds__(GD_BLOCK, 2) gd_dedup_kernel(const uint64_t *T
     base = __shfl_sync(FULL, base, 0);
     k0 = (base & 0xFFFFu) + (e0 & 0xFFFFu);
     if (k0 + v <= GD_MAXL) {
-      unsigned long long *lk = m.lk + k0;
+      uint32_t k = k0;
 #pragma unroll
       for (int u = 0; u < GD_U; u++) {
         const bool c = (cont >> u) & 1;
-        if (c) *lk = key[u];
+        if (c) m.lk[k] = key[u];
         if constexpr (!PK)
-          if (c) m.lp[lk - m.lk] = (uint8_t)pay_of(u);
-        lk += c;
+          if (c) m.lp[k] = (uint8_t)pay_of(u);
+        k += c;
       }
     }
     if (lane < sw) {
@@ -1394,16 +1417,17 @@ __global__ void __launch_bounds__(GD_BLOCK, 2) gd_dedup_kernel(const uint64_t *T
   uint32_t km = act;
   for (uint32_t t = cont; t; t &= t - 1)
     if (m.lx[k0++] == GD_NONE) km &= ~(t & (0u - t));
+  const uint32_t own = lpay ? act & ~cont : 0u;
   uint32_t word = 0;  // lane u < GD_U: the warp's keep bits of row u
 #pragma unroll
   for (int u = 0; u < GD_U; u++) {
     if (u * GD_BLOCK < n) {
       const unsigned bal = __ballot_sync(FULL, (km >> u) & 1);
       if (lane == u) word = bal;
-      if (lpay && (((act & ~cont) >> u) & 1)) {
-        const uint32_t b = bit_of(key[u]), bm = 1u << (b & 31);
-        stage[fpre[b >> 5] + (uint32_t)__popc(set32[b >> 5] & (bm - 1))] = (uint8_t)pay_of(u);
-      }
+      // (every lane's rank is in range; only keys with a bit of their own store)
+      const uint32_t b = bit_of(key[u]), bm = 1u << (b & 31);
+      const uint32_t r = fpre[b >> 5] + (uint32_t)__popc(set32[b >> 5] & (bm - 1));
+      if ((own >> u) & 1) stage[r] = (uint8_t)pay_of(u);
     }
   }
   if (lane < GD_U && word) keep[gd_keep_word(a, q) + lane * NW + warp] = word;
@@ -1480,7 +1504,7 @@ __global__ void __launch_bounds__(GD_BLOCK) gd_split_kernel(const uint64_t *T, c
   for (uint64_t i = a + tid; i < e; i += GD_BLOCK) {
     const uint64_t x = T[i], h = hash(x), o = atomicAdd(&s_cur[sub(h)], 1ull);
     U[o] = p1 ? h * KEY_SPREAD_INV : x;
-    if (UP) UP[o] = p1 ? (uint8_t)pay_byte((uint32_t)x) : TP[i];
+    if (UP) UP[o] = (uint8_t)pay_byte(p1 ? (uint32_t)x : TP[i]);
   }
 }
 
@@ -1640,7 +1664,7 @@ __global__ void __launch_bounds__(WD_WARPS * 32, 4) wd_dedup_kernel(uint64_t *T,
             p[u] = i < n ? pay_byte((uint32_t)w) : 0u;
           } else {
             key[u] = i < n ? T[a + i] : EMPTY;
-            p[u] = (pay && i < n) ? TP[a + i] : 0u;
+            p[u] = (pay && i < n) ? pay_byte(TP[a + i]) : 0u;
           }
         }
   #pragma unroll
@@ -2147,7 +2171,7 @@ bool msd_sort_unique(KeyT *keys, KeyT *alt, uint64_t n, uint64_t max_bin, const 
         gd_split_kernel<<<h_ov, GD_BLOCK, 0, s>>>(T64, PT, sb_off, ov, PS, P, p1, U64, PU, sub_off, jl);
         CF1_LAUNCH_CHECK();
         kern<<<nov, CS_BLOCK, smem, s>>>(U, T, sub_off, nsub, shift, rest > 0 ? bits : 0, scnt, over, P, lb, PU, PT,
-                                         nullptr, nullptr, nbins, jl, nullptr);
+                                         nullptr, nullptr, nbins, jl, nullptr, false);
         CF1_LAUNCH_CHECK();
         gd_gather_kernel<<<h_ov, GD_BLOCK, 0, s>>>(U64, lo.with_pay ? lb.l0pay : nullptr, sb_off, ov, g, sub_off, scnt,
                                                    T64, cnt, keep, lo, p1);
@@ -2177,7 +2201,7 @@ bool msd_sort_unique(KeyT *keys, KeyT *alt, uint64_t n, uint64_t max_bin, const 
       }
       if (h_ov) {
         kern<<<h_ov, CS_BLOCK, smem, s>>>(T, U, sb_off, nsub, shift, rest > 0 ? bits : 0, cnt, over, P, lo, PT, PU,
-                                          nullptr, nullptr, nbins, ov, nullptr);
+                                          nullptr, nullptr, nbins, ov, nullptr, !pk);
         CF1_LAUNCH_CHECK();
         CF1_CUDA(cudaEventRecord(sc.ev[1], s));
         finish();
@@ -2196,7 +2220,7 @@ bool msd_sort_unique(KeyT *keys, KeyT *alt, uint64_t n, uint64_t max_bin, const 
       const uint32_t h_ov = rd.overflow;
       if (h_ov) {
         kern<<<h_ov, CS_BLOCK, smem, s>>>(T, U, sb_off, nsub, shift, rest > 0 ? bits : 0, cnt, over, P, lo, PT, PU, clist,
-                                          coff, nbins, nullptr, ov);
+                                          coff, nbins, nullptr, ov, true);
         CF1_LAUNCH_CHECK();
         CF1_CUDA(cudaEventRecord(sc.ev[1], s));
         finish();

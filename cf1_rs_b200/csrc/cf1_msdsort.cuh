@@ -91,8 +91,8 @@ struct Level0Out {
 // With dist = nullptr the distinct keys stay where the dedup left them, at
 // the start of each unit's range of *kept (keys or alt), and
 // msd_compact writes dist later; dist_off is written either way.
-// With pkeys/palt (one payload byte per key, beside keys and alt), each
-// distinct key leaves with the OR of its copies' payloads at the same place
+// With pkeys/palt (one side-set code per key, beside keys and alt), each
+// distinct key leaves with the OR of its copies' side-set bytes at the same place
 // of *kept_pay (pkeys or palt, beside *kept); the group dedup leaves no bytes
 // there (*kept_pay = nullptr: they went to l0's outputs).
 template <class KeyT>

@@ -25,7 +25,7 @@ __global__ void record_len_kernel(const uint64_t *records, uint64_t n, uint32_t 
 // Warp-cooperative expansion: a warp takes 32 records, and its lanes walk the
 // records' k-mers in one flattened index space, so output stores are
 // contiguous whatever the record lengths.  With `sides` (and NM), each
-// occurrence also writes its side-set byte: the (front, back) contribution
+// occurrence also writes its side-set code: the (front, back) contribution
 // its true neighbours in the sequence give the vertex (src/classify.rs:
 // 65-518 as the per-side join), so phase 3 can join a vertex's occurrences
 // while it removes their duplicate keys.
@@ -84,9 +84,10 @@ __global__ void __launch_bounds__(256) expand_kernel(const uint64_t *records, ui
             const bool hn = t + 1 < onrec || (oends & 2u);
             uint32_t pb, nb;
             KeyT fw = KOps<KeyT>::extract_nb(W, p, k, hp, pb, nb);
-            KeyT rc = KOps<KeyT>::rc(fw, k);
+            KeyT rc = KOps<KeyT>::rc(fw, k), nf = fw, nr = rc;
+            KOps<KeyT>::roll(nf, nr, nb, k);
             keys[ooff + t] = kmin(fw, rc);
-            sides[ooff + t] = (uint8_t)contribution_sideset(fw, rc, hp, pb, hn, hn ? nb : 0u, k);
+            sides[ooff + t] = (uint8_t)contribution_code(fw, rc, nf, hp ? pb : 4u, hn, nb);
           } else {
             KeyT fw = KOps<KeyT>::extract(W, p, k);
             KeyT rc = KOps<KeyT>::rc(fw, k);
@@ -111,8 +112,10 @@ __global__ void __launch_bounds__(256) expand_kernel(const uint64_t *records, ui
 // word; when its run crosses into the next record it takes that record's
 // first k-mer, look-ahead and preceding base, prepared once per record by
 // the record's own lane, through shuffles.  The rolled k-mer is also the
-// "next k-mer" the side-set byte needs for its self-loop test.  Keys and
-// bytes are staged per warp in shared memory and written out contiguously.
+// "next k-mer" the side-set code needs for its self-loop test.  Keys and
+// codes are staged per warp in shared memory and written out contiguously.
+// Integer ALU bound.  The code in place of the byte (four table nibbles and
+// their selects) took 1 Gbp from 7.06 to 6.34 ms.
 constexpr int XR_E = 16;                       // most occurrences a lane takes per round
 constexpr int XR_WARPS = 8;
 constexpr uint32_t XR_SPAN = 32 * XR_E;        // occurrences a warp takes per round at most
@@ -180,8 +183,8 @@ __global__ void __launch_bounds__(XR_WARPS * 32) expand_roll_kernel(const uint64
       rc0 = KOps<uint64_t>::rc(fw0, k);
     }
     // n (13 bits), whether the record has a base before / after (2), the
-    // base before it (2), whether its bases may be read (1)
-    const uint32_t info0 = n | (ends << 16) | (pb0 << 18) | ((uint32_t)inb << 20);
+    // base before it or 4 (3), whether its bases may be read (1)
+    const uint32_t info0 = n | (ends << 16) | ((ends & 1u ? pb0 : 4u) << 18) | ((uint32_t)inb << 21);
     const uint32_t incl = warp_inclusive_scan(n);
     const uint32_t total = __shfl_sync(FULL, incl, 31);
     for (uint32_t base = 0; base < total;) {
@@ -201,8 +204,10 @@ __global__ void __launch_bounds__(XR_WARPS * 32) expand_roll_kernel(const uint64
       uint32_t t = j0 - (rec_end - (info & 0x1FFFu));
       uint64_t fw = 0, rc = 0, ah = 0;
       uint32_t prevb = 0;
-      if (j0 < total && (info >> 20 & 1u)) {
-        xr_window(W, cpos + t, k, t > 0 || (info >> 16 & 1u), fw, ah, prevb);
+      if (j0 < total && (info >> 21 & 1u)) {
+        const bool hp = t > 0 || (info >> 16 & 1u);
+        xr_window(W, cpos + t, k, hp, fw, ah, prevb);
+        if (!hp) prevb = 4;
         rc = KOps<uint64_t>::rc(fw, k);
       }
       for (uint32_t e = 0; e < er; e++) {
@@ -220,9 +225,8 @@ __global__ void __launch_bounds__(XR_WARPS * 32) expand_roll_kernel(const uint64
           info = infoN;
           rec_end = endN;
           t = 0;
-          prevb = (infoN >> 18) & 3u;
+          prevb = (infoN >> 18) & 7u;
         }
-        const bool hp = t > 0 || (info >> 16 & 1u);
         const bool hn = t + 1 < (info & 0x1FFFu) || (info >> 17 & 1u);
         const uint32_t nb = (uint32_t)(ah >> 62);
         const uint64_t nf = ((fw << 2) | nb) & kmask;
@@ -230,7 +234,7 @@ __global__ void __launch_bounds__(XR_WARPS * 32) expand_roll_kernel(const uint64
         if (j < total) {
           const uint32_t i = lane * er + e;
           sk[xr_slot(i)] = kmin(fw, rc);
-          ss[xr_bslot(i)] = (uint8_t)contribution_sideset_rolled(fw, rc, nf, nr, hp, prevb, hn, nb);
+          ss[xr_bslot(i)] = (uint8_t)contribution_code(fw, rc, nf, prevb, hn, nb);
         }
         prevb = (uint32_t)(fw >> top);  // this k-mer's first base precedes the next one
         fw = nf;

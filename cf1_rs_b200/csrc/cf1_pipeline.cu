@@ -513,7 +513,7 @@ void run_impl(cf1gpu_ctx *c, StreamIO *io = nullptr, Step step = Step::FULL, con
   // ---- phase 3a: expand, sort per bin, unique
   const uint64_t NO = c->n_occ;
   KeyT *keys = c->d_keys.get<KeyT>(NO + 1);
-  // state_update 0: every occurrence's side-set byte travels with its key
+  // state_update 0: every occurrence's side-set code travels with its key
   // through the MSD sort, whose dedup joins a vertex's occurrences, so phase
   // 4 only places each distinct key's byte in its slot (the LSD fallback has
   // no payloads: phase 4 then classifies the occurrences as before)
