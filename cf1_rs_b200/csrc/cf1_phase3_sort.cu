@@ -111,21 +111,25 @@ __global__ void __launch_bounds__(256) expand_kernel(const uint64_t *records, ui
 // forms one base at a time (src/kmer.rs:240-262) from a 32-base look-ahead
 // word; when its run crosses into the next record it takes that record's
 // first k-mer, look-ahead and preceding base, prepared once per record by
-// the record's own lane, through shuffles.  The rolled k-mer is also the
+// the record's own lane, from shared memory (a branch a lane takes once in
+// its ~9 occurrences, where shuffles cost every lane eight instructions and a
+// dozen selects an occurrence).  The rolled k-mer is also the
 // "next k-mer" the side-set code needs for its self-loop test.  Keys and
 // codes are staged per warp in shared memory and written out contiguously.
-// Integer ALU bound.  The code in place of the byte (four table nibbles and
-// their selects) took 1 Gbp from 7.06 to 6.34 ms.
+// Integer ALU bound while the packed sequence stays in L2: 159 instructions
+// per 32 occurrences with the shuffles, and without them 200 Mbp went from
+// 1.20 to 1.08 ms and 40 Mb of transcripts from 0.25 to 0.20.  At 1 Gbp (6.4
+// ms both ways) the records' scattered reads bound it.  The code in place of
+// the byte (four table nibbles and their selects) took 1 Gbp from 7.06 to 6.34.
 constexpr int XR_E = 16;                       // most occurrences a lane takes per round
 constexpr int XR_WARPS = 8;
 constexpr uint32_t XR_SPAN = 32 * XR_E;        // occurrences a warp takes per round at most
-constexpr uint32_t XR_PAD = XR_SPAN + XR_SPAN / 16;
-constexpr uint32_t XR_BPAD = XR_SPAN + XR_SPAN / 4;
-// Staging slots of key i and byte i: a pad word per 16 keys and four pad
-// bytes per 16 bytes, so that the lanes' runs (stride er) fall on different
-// shared-memory banks.
-CF1_D uint32_t xr_slot(uint32_t i) { return i + (i >> 4); }
-CF1_D uint32_t xr_bslot(uint32_t i) { return i + ((i >> 4) << 2); }
+// Strides of the lanes' runs of er keys and er codes in the staging: an odd
+// number of 8-byte words, and an odd number of 4-byte words, so that the lanes
+// fall on different shared-memory banks.
+CF1_D uint32_t xr_key_stride(uint32_t er) { return er | 1; }
+CF1_D uint32_t xr_code_stride(uint32_t er) { return (((er + 3) / 4) | 1) * 4; }
+constexpr uint32_t XR_PAD = 32 * (XR_E | 1), XR_BPAD = 32 * (((XR_E + 3) / 4) | 1) * 4;
 
 // The k-mer starting at base p (k <= 31), the 32 bases after it (p + k ...,
 // most significant first) and, with want_prev, the base before it.  Reads
@@ -150,9 +154,11 @@ __global__ void __launch_bounds__(XR_WARPS * 32) expand_roll_kernel(const uint64
                                                                     const uint64_t *NM, uint8_t *sides) {
   __shared__ uint64_t skey[XR_WARPS][XR_PAD];
   __shared__ uint8_t sside[XR_WARPS][XR_BPAD];
+  __shared__ ulonglong2 srec[XR_WARPS][2][32];
   const unsigned lane = lane_id(), warp = threadIdx.x >> 5;
   uint64_t *sk = skey[warp];
   uint8_t *ss = sside[warp];
+  ulonglong2 *rec_fr = srec[warp][0], *rec_ai = srec[warp][1];
   const uint64_t n_chunks = ceil_div_dev(n_rec);
   const uint64_t kmask = KOps<uint64_t>::mask(k);
   const int top = 2 * k - 2;
@@ -187,9 +193,13 @@ __global__ void __launch_bounds__(XR_WARPS * 32) expand_roll_kernel(const uint64
     const uint32_t info0 = n | (ends << 16) | ((ends & 1u ? pb0 : 4u) << 18) | ((uint32_t)inb << 21);
     const uint32_t incl = warp_inclusive_scan(n);
     const uint32_t total = __shfl_sync(FULL, incl, 31);
+    rec_fr[lane] = make_ulonglong2(fw0, rc0);
+    rec_ai[lane] = make_ulonglong2(ah0, info0 | ((uint64_t)incl << 32));
+    __syncwarp();
     for (uint32_t base = 0; base < total;) {
       const uint32_t rem = total - base;
       const uint32_t er = rem >= XR_SPAN ? (uint32_t)XR_E : (rem + 31) / 32;
+      const uint32_t kstr = xr_key_stride(er), bstr = xr_code_stride(er);
       const uint32_t j0 = base + lane * er;
       // the record holding j0: the number of records ending at or before it
       int cur = 0;
@@ -198,62 +208,63 @@ __global__ void __launch_bounds__(XR_WARPS * 32) expand_roll_kernel(const uint64
         const uint32_t v = __shfl_sync(FULL, incl, cur + step - 1);
         if (v <= j0) cur += step;
       }
-      uint32_t info = __shfl_sync(FULL, info0, cur);
-      uint32_t rec_end = __shfl_sync(FULL, incl, cur);
+      const uint64_t ie = rec_ai[cur].y;
       const uint64_t cpos = __shfl_sync(FULL, pos, cur);
-      uint32_t t = j0 - (rec_end - (info & 0x1FFFu));
+      uint32_t info = (uint32_t)ie;
+      uint32_t left = (uint32_t)(ie >> 32) - j0;  // occurrences up to the record's end
       uint64_t fw = 0, rc = 0, ah = 0;
       uint32_t prevb = 0;
       if (j0 < total && (info >> 21 & 1u)) {
+        const uint32_t t = (info & 0x1FFFu) - left;
         const bool hp = t > 0 || (info >> 16 & 1u);
         xr_window(W, cpos + t, k, hp, fw, ah, prevb);
         if (!hp) prevb = 4;
         rc = KOps<uint64_t>::rc(fw, k);
       }
-      for (uint32_t e = 0; e < er; e++) {
-        const uint32_t j = j0 + e;
-        // the next record's first k-mer, taken when the run crosses into it
-        const int nx = cur < 31 ? cur + 1 : 31;
-        const uint64_t fwN = __shfl_sync(FULL, fw0, nx), rcN = __shfl_sync(FULL, rc0, nx),
-                       ahN = __shfl_sync(FULL, ah0, nx);
-        const uint32_t infoN = __shfl_sync(FULL, info0, nx), endN = __shfl_sync(FULL, incl, nx);
-        if (j == rec_end && j < total) {
-          cur = nx;
-          fw = fwN;
-          rc = rcN;
-          ah = ahN;
-          info = infoN;
-          rec_end = endN;
-          t = 0;
-          prevb = (infoN >> 18) & 7u;
+      const uint32_t mine = j0 < total ? min(er, total - j0) : 0u;
+      uint64_t *kp = sk + lane * kstr;
+      uint8_t *bp = ss + lane * bstr;
+      for (uint32_t e = 0; e < mine; e++) {
+        if (left == 0) {  // the run crosses into the next record
+          cur++;
+          const ulonglong2 fr = rec_fr[cur], ai = rec_ai[cur];
+          fw = fr.x;
+          rc = fr.y;
+          ah = ai.x;
+          info = (uint32_t)ai.y;
+          left = info & 0x1FFFu;
+          prevb = (info >> 18) & 7u;
         }
-        const bool hn = t + 1 < (info & 0x1FFFu) || (info >> 17 & 1u);
+        left--;
+        const bool hn = left > 0 || (info >> 17 & 1u);
         const uint32_t nb = (uint32_t)(ah >> 62);
         const uint64_t nf = ((fw << 2) | nb) & kmask;
         const uint64_t nr = (rc >> 2) | ((uint64_t)(3 - nb) << top);
-        if (j < total) {
-          const uint32_t i = lane * er + e;
-          sk[xr_slot(i)] = kmin(fw, rc);
-          ss[xr_bslot(i)] = (uint8_t)contribution_code(fw, rc, nf, prevb, hn, nb);
-        }
+        kp[e] = kmin(fw, rc);
+        bp[e] = (uint8_t)contribution_code(fw, rc, nf, prevb, hn, nb);
         prevb = (uint32_t)(fw >> top);  // this k-mer's first base precedes the next one
         fw = nf;
         rc = nr;
         ah <<= 2;
-        t++;
       }
       __syncwarp();
       const uint32_t span = 32 * er;
-      for (uint32_t i = lane; i < span; i += 32) {
-        const uint64_t o = out0 + base + i;
-        if (base + i < total) {
-          if (o < n_keys) {
-            keys[o] = sk[xr_slot(i)];
-            sides[o] = ss[xr_bslot(i)];
-          } else {
-            atomicOr(err, (uint32_t)DEV_OVERFLOW);
-          }
-        }
+      // out0 + base + i below n_keys: always, unless the records disagree with
+      // their prefix sums
+      const uint64_t o0 = out0 + base, room = n_keys > o0 ? n_keys - o0 : 0;
+      uint32_t lim = min(span, rem);
+      if (lim > room) {
+        if (lane == 0) atomicOr(err, (uint32_t)DEV_OVERFLOW);
+        lim = (uint32_t)room;
+      }
+      uint64_t *ko = keys + o0;
+      uint8_t *so = sides + o0;
+      const uint32_t inv = 65536u / er + 1, kpad = kstr - er, bpad = bstr - er;  // i / er for i < 512
+#pragma unroll 4
+      for (uint32_t i = lane; i < lim; i += 32) {
+        const uint32_t q = (i * inv) >> 16;  // the lane that wrote it
+        ko[i] = sk[i + q * kpad];
+        so[i] = ss[i + q * bpad];
       }
       __syncwarp();
       base += span;
