@@ -297,17 +297,29 @@ CF1_HD uint64_t kmer_minimizer(KeyT key, int k, int m) {
 }
 
 // ------------------------------------------------------------ super k-mers ----
-// A routed super k-mer: first k-mer position (40 bits), k-mer count - 1
-// (12 bits), bin (12 bits).
+// A routed super k-mer: first k-mer position (38 bits: the bases of an input
+// that fits the GPU), k-mer count - 1 (12 bits), bin (12 bits), and in the two
+// top bits its ends: whether a base (no placeholder) precedes its first k-mer,
+// and whether one follows its last k-mer.  Records exchanged between shards
+// have no ends (rec_bare); phase 2 looks theirs up (rec_ends_of).
 constexpr uint32_t MAX_TILE = 4096;
 constexpr uint32_t MAX_BINS = 4096;
 constexpr uint32_t NUM_BUCKETS = 65536;
 CF1_HD uint64_t rec_pack(uint64_t pos, uint32_t n, uint32_t bin) {
   return (pos << 24) | ((uint64_t)(n - 1) << 12) | bin;
 }
-CF1_HD uint64_t rec_pos(uint64_t r) { return r >> 24; }
+constexpr uint32_t REC_PREV = 1, REC_NEXT = 2;
+CF1_HD uint64_t rec_pos(uint64_t r) { return (r >> 24) & ((1ull << 38) - 1); }
+CF1_HD uint32_t rec_ends(uint64_t r) { return (uint32_t)(r >> 62); }
+CF1_HD uint64_t rec_with_ends(uint64_t r, uint32_t ends) { return (r << 2 >> 2) | ((uint64_t)ends << 62); }
+CF1_HD uint64_t rec_with_bin(uint64_t r, uint32_t bin) { return (r & ~0xFFFull) | bin; }
+CF1_HD uint64_t rec_bare(uint64_t r) { return r << 2 >> 2; }
 CF1_HD uint32_t rec_n(uint64_t r) { return (uint32_t)((r >> 12) & 0xFFF) + 1; }
 CF1_HD uint32_t rec_bin(uint64_t r) { return (uint32_t)(r & 0xFFF); }
+CF1_HD uint32_t rec_ends_of(uint64_t r, const uint64_t *NM, uint64_t L, int k) {
+  const uint64_t p = rec_pos(r), e = p + rec_n(r) - 1 + k;  // e: the base after the last k-mer
+  return (p > 0 && p <= L && !is_n(NM, p - 1) ? REC_PREV : 0u) | (e < L && !is_n(NM, e) ? REC_NEXT : 0u);
+}
 
 // ------------------------------------------------------------------ states ----
 // 5-bit codes (src/state.rs:80-146): 0 unvisited, 3 MIMO, 4|b MISO(back b),

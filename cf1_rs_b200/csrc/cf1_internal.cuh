@@ -146,10 +146,11 @@ constexpr int K_FIXED = 31, M_FIXED = 15, W_FIXED = 17;
 // Phase 1: minimizer histogram + unordered super k-mer list.
 void launch_superkmer_scan(const SuperkmerArgs &a, int persistent_ctas, cudaStream_t s);
 // Phase 2: route the list into per-bin ranges rec_off[0..num_bins] of records
-// (rec_bucket nullptr: the records already carry their bin).
+// (rec_bucket nullptr: the records already carry their bin, and get their ends
+// from NM).
 void launch_bin_scatter(const uint64_t *rec_tmp, const uint16_t *rec_bucket, uint64_t n, const uint16_t *lut,
                         uint32_t num_bins, const uint64_t *rec_off, uint32_t *cursor, uint64_t *records, uint32_t *err,
-                        cudaStream_t s);
+                        const uint64_t *NM, uint64_t L, int k, cudaStream_t s);
 // Greedy partition of the histogram (src/minimizer.rs:116-172) into the
 // bucket->bin table, plus per-bin record offsets rec_off[0..num_bins].
 void launch_partition(const uint32_t *hist, uint32_t num_bins, uint16_t *lut, uint64_t *rec_off, uint32_t *n_bins_eff,
@@ -170,7 +171,7 @@ void record_kmer_prefix(const uint64_t *records, uint64_t n_rec, uint64_t *kpre,
 template <class KeyT>
 void launch_expand(const uint64_t *records, uint64_t n_rec, const uint64_t *kpre, const uint64_t *W, int k, KeyT *keys,
                    uint64_t n_keys, uint64_t L, uint32_t *queue, uint32_t *err, int persistent_ctas, cudaStream_t s,
-                   const uint64_t *NM = nullptr, uint8_t *sides = nullptr);
+                   uint8_t *sides = nullptr);
 
 // Sorts each segment [seg_off[b], seg_off[b+1]) of keys ascending (LSD radix,
 // segmented).  The result is in `keys` on return.

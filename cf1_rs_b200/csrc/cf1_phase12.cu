@@ -253,13 +253,19 @@ __global__ void __launch_bounds__(BLOCK) superkmer_kernel(SuperkmerArgs a) {
     for (uint32_t sg = tid; sg < nseg; sg += BLOCK) {
       const uint32_t st = starts[sg], rn = st >> 16;
       if (rn == 0xFFFFu) continue;
-      const uint32_t p = st & 0xFFFFu, n = (starts[sg + 1] & 0xFFFFu) - p;
+      const uint32_t nx = starts[sg + 1], p = st & 0xFFFFu, n = (nx & 0xFFFFu) - p;
+      // the record's ends: a neighbouring segment of the tile is a record
+      // exactly where the base on that side is no placeholder (the windows of
+      // this one are clean, so a placeholder in the next window is its new base)
+      const uint64_t e = P0 + p + n - 1 + k;
+      const bool hp = sg > 0 ? (starts[sg - 1] >> 16) != 0xFFFFu : P0 > 0 && !is_n(a.NM, P0 - 1);
+      const bool hn = sg + 1 < nseg ? (nx >> 16) != 0xFFFFu : e < a.L && !is_n(a.NM, e);
       const uint32_t bk = mix_bucket(mix_order_inv(zrow[p]));
       atomicAdd(&a.hist[bk], 1u);
       my_kmers += n;
       const uint64_t o = s_base + rn;
       if (o < a.rec_cap) {
-        a.rec_tmp[o] = rec_pack(P0 + p, n, 0);
+        a.rec_tmp[o] = rec_with_ends(rec_pack(P0 + p, n, 0), (hp ? REC_PREV : 0u) | (hn ? REC_NEXT : 0u));
         a.rec_bucket[o] = (uint16_t)bk;
       }
     }
@@ -286,7 +292,8 @@ constexpr uint32_t BS_TILE = BS_BLOCK * BS_ITEMS;
 __global__ void __launch_bounds__(BS_BLOCK, 3) bin_scatter_kernel(const uint64_t *rec_tmp, const uint16_t *rec_bucket,
                                                                uint64_t n, const uint16_t *lut, uint32_t num_bins,
                                                                const uint64_t *rec_off, uint32_t *cursor,
-                                                               uint64_t *records, uint32_t *err) {
+                                                               uint64_t *records, uint32_t *err, const uint64_t *NM,
+                                                               uint64_t L, int k) {
   extern __shared__ __align__(16) uint64_t bs_smem[];
   uint64_t *stage = bs_smem;                                           // [BS_TILE]
   uint32_t *s_cnt = reinterpret_cast<uint32_t *>(bs_smem + BS_TILE);  // [num_bins]
@@ -306,8 +313,9 @@ __global__ void __launch_bounds__(BS_BLOCK, 3) bin_scatter_kernel(const uint64_t
     li[i] = 0xFFFFFFFFu;
     if (j < nt) {
       const uint64_t t = rec_tmp[r0 + j];
-      const uint32_t b = rec_bucket ? lut[rec_bucket[r0 + j]] : rec_bin(t);  // no buckets: the records carry their bin
-      rec[i] = rec_pack(rec_pos(t), rec_n(t), b);
+      // no buckets: records of other shards, which carry their bin and no ends
+      const uint32_t b = rec_bucket ? lut[rec_bucket[r0 + j]] : rec_bin(t);
+      rec[i] = rec_bucket ? rec_with_bin(t, b) : rec_with_ends(t, rec_ends_of(t, NM, L, k));
       li[i] = atomicAdd(&s_cnt[b], 1u);
     }
   }
@@ -505,12 +513,12 @@ void launch_superkmer_scan(const SuperkmerArgs &a, int persistent_ctas, cudaStre
 
 void launch_bin_scatter(const uint64_t *rec_tmp, const uint16_t *rec_bucket, uint64_t n, const uint16_t *lut,
                         uint32_t num_bins, const uint64_t *rec_off, uint32_t *cursor, uint64_t *records, uint32_t *err,
-                        cudaStream_t s) {
+                        const uint64_t *NM, uint64_t L, int k, cudaStream_t s) {
   if (n == 0) return;
   size_t smem = BS_TILE * sizeof(uint64_t) + 3 * num_bins * sizeof(uint32_t);
   CF1_CUDA(cudaFuncSetAttribute(bin_scatter_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
   bin_scatter_kernel<<<(unsigned)ceil_div(n, (uint64_t)BS_TILE), BS_BLOCK, smem, s>>>(
-      rec_tmp, rec_bucket, n, lut, num_bins, rec_off, cursor, records, err);
+      rec_tmp, rec_bucket, n, lut, num_bins, rec_off, cursor, records, err, NM, L, k);
   CF1_LAUNCH_CHECK();
 }
 

@@ -24,7 +24,7 @@ __global__ void record_len_kernel(const uint64_t *records, uint64_t n, uint32_t 
 
 // Warp-cooperative expansion: a warp takes 32 records, and its lanes walk the
 // records' k-mers in one flattened index space, so output stores are
-// contiguous whatever the record lengths.  With `sides` (and NM), each
+// contiguous whatever the record lengths.  With `sides`, each
 // occurrence also writes its side-set code: the (front, back) contribution
 // its true neighbours in the sequence give the vertex (src/classify.rs:
 // 65-518 as the per-side join), so phase 3 can join a vertex's occurrences
@@ -32,8 +32,7 @@ __global__ void record_len_kernel(const uint64_t *records, uint64_t n, uint32_t 
 template <class KeyT>
 __global__ void __launch_bounds__(256) expand_kernel(const uint64_t *records, uint64_t n_rec, const uint64_t *kpre,
                                                      const uint64_t *W, int k, KeyT *keys, uint64_t n_keys,
-                                                     uint64_t L, uint32_t *queue, uint32_t *err, const uint64_t *NM,
-                                                     uint8_t *sides) {
+                                                     uint64_t L, uint32_t *queue, uint32_t *err, uint8_t *sides) {
   const unsigned lane = lane_id();
   const uint64_t n_chunks = ceil_div_dev(n_rec);
   uint64_t chunk = ((uint64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
@@ -50,15 +49,9 @@ __global__ void __launch_bounds__(256) expand_kernel(const uint64_t *records, ui
     uint32_t n = valid ? rec_n(rec) : 0;
     uint64_t pos = rec_pos(rec);
     uint64_t off = valid ? kpre[r] : 0;
-    // whether the record's first k-mer has a base before it and its last one
-    // a base after it (inside a super k-mer the windows before and after are
-    // valid, so only these two can lack a neighbour): read once per record,
-    // not in the k-mer loop
-    uint32_t ends = 0;
-    if (sides && valid) {
-      const uint64_t q = pos + n - 1;  // the last k-mer
-      ends = (uint32_t)(pos > 0 && !is_n(NM, pos - 1)) | ((uint32_t)(q + k < L && !is_n(NM, q + k)) << 1);
-    }
+    // inside a super k-mer the windows before and after are valid, so only its
+    // first and last k-mers can lack a neighbour
+    const uint32_t ends = rec_ends(rec) & (pos > 0 ? 3u : REC_NEXT);
     uint32_t incl = warp_inclusive_scan(n);
     uint32_t total = __shfl_sync(FULL, incl, 31);
     uint32_t excl = incl - n;
@@ -116,11 +109,13 @@ __global__ void __launch_bounds__(256) expand_kernel(const uint64_t *records, ui
 // dozen selects an occurrence).  The rolled k-mer is also the
 // "next k-mer" the side-set code needs for its self-loop test.  Keys and
 // codes are staged per warp in shared memory and written out contiguously.
-// Integer ALU bound while the packed sequence stays in L2: 159 instructions
-// per 32 occurrences with the shuffles, and without them 200 Mbp went from
-// 1.20 to 1.08 ms and 40 Mb of transcripts from 0.25 to 0.20.  At 1 Gbp (6.4
-// ms both ways) the records' scattered reads bound it.  The code in place of
-// the byte (four table nibbles and their selects) took 1 Gbp from 7.06 to 6.34.
+// Integer ALU bound while the packed sequence stays in L2 (159 instructions
+// per 32 occurrences with the shuffles; without them 200 Mbp went from 1.20 to
+// 1.08 ms, 40 Mb of transcripts from 0.25 to 0.20); at 1 Gbp the records'
+// scattered reads bound it.  Taking a record's ends from the record, instead
+// of two more scattered reads of the placeholder mask, took 1 Gbp from 6.41 to
+// 4.69 ms and 200 Mbp to 0.91.  The code in place of the byte (four table
+// nibbles and their selects) had taken 1 Gbp from 7.06 to 6.34.
 constexpr int XR_E = 16;                       // most occurrences a lane takes per round
 constexpr int XR_WARPS = 8;
 constexpr uint32_t XR_SPAN = 32 * XR_E;        // occurrences a warp takes per round at most
@@ -150,8 +145,7 @@ CF1_D void xr_window(const uint64_t *W, uint64_t p, int k, bool want_prev, uint6
 __global__ void __launch_bounds__(XR_WARPS * 32) expand_roll_kernel(const uint64_t *records, uint64_t n_rec,
                                                                     const uint64_t *kpre, const uint64_t *W, int k,
                                                                     uint64_t *keys, uint64_t n_keys, uint64_t L,
-                                                                    uint32_t *queue, uint32_t *err,
-                                                                    const uint64_t *NM, uint8_t *sides) {
+                                                                    uint32_t *queue, uint32_t *err, uint8_t *sides) {
   __shared__ uint64_t skey[XR_WARPS][XR_PAD];
   __shared__ uint8_t sside[XR_WARPS][XR_BPAD];
   __shared__ ulonglong2 srec[XR_WARPS][2][32];
@@ -183,8 +177,7 @@ __global__ void __launch_bounds__(XR_WARPS * 32) expand_roll_kernel(const uint64
     uint32_t ends = 0, pb0 = 0;
     uint64_t fw0 = 0, rc0 = 0, ah0 = 0;
     if (inb) {
-      const uint64_t q = pos + n - 1;  // the last k-mer
-      ends = (uint32_t)(pos > 0 && !is_n(NM, pos - 1)) | ((uint32_t)(q + k < L && !is_n(NM, q + k)) << 1);
+      ends = rec_ends(rec) & (pos > 0 ? 3u : REC_NEXT);
       xr_window(W, pos, k, ends & 1u, fw0, ah0, pb0);
       rc0 = KOps<uint64_t>::rc(fw0, k);
     }
@@ -420,7 +413,7 @@ void record_kmer_prefix(const uint64_t *records, uint64_t n_rec, uint64_t *kpre,
 template <class KeyT>
 void launch_expand(const uint64_t *records, uint64_t n_rec, const uint64_t *kpre, const uint64_t *W, int k, KeyT *keys,
                    uint64_t n_keys, uint64_t L, uint32_t *queue, uint32_t *err, int persistent_ctas, cudaStream_t s,
-                   const uint64_t *NM, uint8_t *sides) {
+                   uint8_t *sides) {
   if (n_rec == 0) return;
   uint64_t warps = ceil_div(n_rec, 32);
   if constexpr (KOps<KeyT>::WORDS == 1) {
@@ -429,7 +422,7 @@ void launch_expand(const uint64_t *records, uint64_t n_rec, const uint64_t *kpre
                                                         ceil_div(warps, XR_WARPS))
                                       : (unsigned)ceil_div(warps, XR_WARPS);
       expand_roll_kernel<<<grid, XR_WARPS * 32, 0, s>>>(records, n_rec, kpre, W, k, keys, n_keys, L,
-                                                        persistent_ctas ? queue : nullptr, err, NM, sides);
+                                                        persistent_ctas ? queue : nullptr, err, sides);
       CF1_LAUNCH_CHECK();
       return;
     }
@@ -437,7 +430,7 @@ void launch_expand(const uint64_t *records, uint64_t n_rec, const uint64_t *kpre
   unsigned grid = persistent_ctas ? persistent_grid(expand_kernel<KeyT>, 256, 0, persistent_ctas, ceil_div(warps, 8))
                                   : (unsigned)ceil_div(warps, 8);
   expand_kernel<KeyT><<<grid, 256, 0, s>>>(records, n_rec, kpre, W, k, keys, n_keys, L,
-                                           persistent_ctas ? queue : nullptr, err, NM, sides);
+                                           persistent_ctas ? queue : nullptr, err, sides);
   CF1_LAUNCH_CHECK();
 }
 
@@ -490,8 +483,7 @@ void segmented_unique(const KeyT *keys, uint64_t n, const uint64_t *seg_off, uin
 
 #define CF1_INST(KT)                                                                                                 \
   template void launch_expand<KT>(const uint64_t *, uint64_t, const uint64_t *, const uint64_t *, int, KT *,        \
-                                  uint64_t, uint64_t, uint32_t *, uint32_t *, int, cudaStream_t, const uint64_t *,  \
-                                  uint8_t *);                                                                       \
+                                  uint64_t, uint64_t, uint32_t *, uint32_t *, int, cudaStream_t, uint8_t *);        \
   template void segmented_sort<KT>(KT *, uint64_t, const uint64_t *, uint32_t, int, SortScratch<KT> &, cudaStream_t); \
   template void segmented_unique<KT>(const KT *, uint64_t, const uint64_t *, uint32_t, KT *, uint64_t *,            \
                                      SortScratch<KT> &, cudaStream_t);

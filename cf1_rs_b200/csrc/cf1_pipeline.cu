@@ -125,7 +125,7 @@ __global__ void __launch_bounds__(XR_BLOCK) xroute_scatter_kernel(const uint64_t
     if (bin[i] == 0xFFFFFFFFu) continue;
     const uint32_t d = bin[i] % shards;
     const uint64_t r = r0 + (uint64_t)i * XR_BLOCK + threadIdx.x, t = rec[r], idx = xr_base[d] + li[i];
-    if (idx < off[d + 1]) out[idx] = rec_pack(rec_pos(t), rec_n(t), bin[i]);
+    if (idx < off[d + 1]) out[idx] = rec_with_bin(rec_bare(t), bin[i]);
     else atomicOr(err, (uint32_t)DEV_OVERFLOW);
   }
 }
@@ -141,7 +141,7 @@ __global__ void __launch_bounds__(XR_BLOCK) xrecv_count_kernel(const uint64_t *r
   for (uint64_t r = (uint64_t)blockIdx.x * XR_BLOCK + threadIdx.x; r < n; r += (uint64_t)gridDim.x * XR_BLOCK) {
     const uint64_t x = rec[r];
     const uint32_t b = rec_bin(x);
-    if (b >= nbins || b % shards != idx || rec_pos(x) + rec_n(x) + (uint64_t)k - 1 > L) atomicOr(err, (uint32_t)DEV_FOREIGN);
+    if (b >= nbins || b % shards != idx || (x >> 24) + rec_n(x) + (uint64_t)k - 1 > L) atomicOr(err, (uint32_t)DEV_FOREIGN);
     else atomicAdd(&xr_cnt[b], 1u);
   }
   __syncthreads();
@@ -481,7 +481,7 @@ void run_impl(cf1gpu_ctx *c, StreamIO *io = nullptr, Step step = Step::FULL, con
   CF1_CUDA(cudaMemsetAsync(records, 0, (NS + 1) * sizeof(uint64_t), s));
   uint32_t *cursor = c->d_cursor.get<uint32_t>(B);
   CF1_CUDA(cudaMemsetAsync(cursor, 0, B * sizeof(uint32_t), s));
-  launch_bin_scatter(a.rec_tmp, a.rec_bucket, NS, lut, B, rec_off, cursor, records, &sm->err, s);
+  launch_bin_scatter(a.rec_tmp, a.rec_bucket, NS, lut, B, rec_off, cursor, records, &sm->err, NM, L, k, s);
   if (shards > 1 && step == Step::FULL) {
     // Keep this shard's bins: their records, moved to the front through the
     // free key buffer (the phase-1 list in it has been routed); the other
@@ -520,7 +520,7 @@ void run_impl(cf1gpu_ctx *c, StreamIO *io = nullptr, Step step = Step::FULL, con
   const bool join3 = c->opts.state_update == 0 && !c->force_lsd;
   uint8_t *pay = join3 ? c->d_pay.get<uint8_t>(NO + 16) : nullptr;
   uint8_t *pay_alt = join3 ? c->d_pay_alt.get<uint8_t>(NO + 16) : nullptr;
-  launch_expand<KeyT>(records, NS, kpre, W, k, keys, NO, L, batched ? &sm->queues[2] : nullptr, &sm->err, pctas, s, NM,
+  launch_expand<KeyT>(records, NS, kpre, W, k, keys, NO, L, batched ? &sm->queues[2] : nullptr, &sm->err, pctas, s,
                       pay);
   uint64_t *seg = c->d_seg.get<uint64_t>(B + 1);
   seg_gather_kernel<<<(unsigned)ceil_div(B + 1, 256), 256, 0, s>>>(kpre, rec_off, B, seg);
@@ -538,7 +538,7 @@ void run_impl(cf1gpu_ctx *c, StreamIO *io = nullptr, Step step = Step::FULL, con
   auto msd_width = [&](int delta) { return P0 < 0 ? -1 : std::min(16, std::max(0, P0 + delta)); };
   auto expand_again = [&]() {
     launch_expand<KeyT>(records, NS, kpre, W, k, keys, NO, L, batched ? &sm->queues[4] : nullptr, &sm->err, pctas, s,
-                        NM, pay);
+                        pay);
   };
   if (tune_now && P0 >= 0) {  // autotuner: time each MSD width, keep the fastest
     double best = 1e30;
