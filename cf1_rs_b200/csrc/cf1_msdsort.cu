@@ -995,7 +995,7 @@ __global__ void __launch_bounds__(SR_BLOCK, 2) sr_dedup_kernel(KeyT *T, uint8_t 
 }
 
 // ---------------------------------------------------------------- group dedup
-// The unsorted (BBHash) form's dedup: one CTA per group of up to 32
+// The unsorted (BBHash) form's dedup: one CTA per group of up to 16 or 32
 // consecutive sub-buckets of a bin, whose level-0 slices (and level-1 slices)
 // are consecutive words.  The group's keys sit in the CTA's registers (GD_U
 // per thread) and are told apart by their BBHash bits instead of by a hash
@@ -1015,56 +1015,77 @@ __global__ void __launch_bounds__(SR_BLOCK, 2) sr_dedup_kernel(KeyT *T, uint8_t 
 // rank order.  The keys stay where they are, packed: a bit per occurrence
 // (keep) marks the first copy of every key, and gd_compact_kernel makes the
 // dense array from them when one is asked for.  Nothing is written before the
-// whole group is known to fit; a group that does not (more than GD_MAXN
+// whole group is known to fit; a group that does not (more than MAXN
 // occurrences, long slices, lists too long) is untouched and listed in ov.
 //
-// A group of 32 because the split then needs five bits less (one pass up to 8
-// bits), and because the slices' scans and the barriers are shared by 32
+// Groups because the split then needs four or five bits less (one pass up to
+// 11 bits), and because the slices' scans and the barriers are shared by their
 // sub-buckets: the same passes run by a warp on one sub-bucket of ~120 keys
 // were slower than the warp's hash set below (1 Gbp: 40 against 18 ms).
-// Instruction issue (65% of the slots) and its barriers bound it: ~226 warp
-// instructions per 32 occurrences where the hash set took ~430.  The dedup of
-// 200 Mbp went from 3.77 to 2.08 ms, of 1 Gbp (with tandem arrays) from 18.0
-// to 14.6 ms, of 5 Mbp from 632 to 76 us (the warp kernel's runs of 64
-// sub-buckets left most warps idle); with three occurrences of every key
-// (transcripts) the list is most of the group and it takes 0.81 against 0.59
-// ms, which the split's dropped pass (0.31 ms) makes up for.
-constexpr int GD_BLOCK = 512;
-constexpr int GD_U = 16;                           // keys per thread
-constexpr int GD_BITS = 5;                         // sub-buckets of a group (log2), at most
-constexpr uint32_t GD_MAXN = GD_BLOCK * GD_U;      // occurrences a group may hold
-constexpr uint32_t GD_SWMAX = 32;                  // level-0 words of a slice: one a lane
-constexpr uint32_t GD_WMAX = GD_SWMAX << GD_BITS;  // level-0 words of a group
-constexpr uint32_t GD_W1MAX = (GD_SWMAX / 8) << GD_BITS;  // level-1 words of a group
-constexpr uint32_t GD_MAXL = 5888;                 // occurrences on a level-0 bit set more than once
-constexpr uint32_t GD_MAXC = GD_BLOCK;             // occurrences on a level-1 bit set more than once
-constexpr uint32_t GD_PAIR = 4;                    // threads that compare one of those
+// Instruction issue (65% of the slots) and its barriers bound it: ~220 warp
+// instructions per 32 occurrences where the hash set took ~430.  Groups of 16,
+// in CTAs half the size, four to an SM, wait less at the barriers (200 Mbp
+// 2.00 against 1.88 ms, 40 Mb of transcripts 0.81 and 0.72, 1 Gbp 14.1 and
+// 13.7) but need one more split bit, so they are taken while the split has at
+// most GD_SPLIT bits all the same (its scatter of 1 Gbp: 5.6 ms on 10 bits,
+// 7.2 on 11; of 200 Mbp 1.00 on 8 and 1.04 on 9), and not for a bin that one
+// group of 32 holds unsplit.  The dedup of 200 Mbp went from 3.77 to 1.88 ms,
+// of 1 Gbp (with tandem arrays) from 18.0 to 14.1 ms, of 5 Mbp from 632 to 74
+// us (the warp kernel's runs of 64 sub-buckets left most warps idle); with
+// three occurrences of every key (transcripts) the list is most of the group
+// and it takes 0.72 against 0.59 ms, which the split's dropped pass (0.31 ms)
+// makes up for.
+constexpr int GD_U = 16;                 // keys per thread
+constexpr int GD_BITS = 5;               // sub-buckets of a group (log2), at most
+constexpr int GD_SPLIT = 10;             // most split bits that groups of 16 sub-buckets are worth
+constexpr int GD_MOVE = 512;             // threads of the kernels that move a listed group
+constexpr uint32_t GD_SWMAX = 32;        // level-0 words of a slice: one a lane
+constexpr uint32_t GD_PAIR = 4;          // threads that compare one occurrence of a shared level-1 bit
 constexpr uint32_t GD_NONE = 0xFFFF, GD_OWN = 0x8000, GD_JOIN = 0x4000;
+template <int BITS>
+struct GdCfg {
+  static constexpr int BLOCK = 16 << BITS;
+  static constexpr uint32_t MAXN = BLOCK * GD_U;          // occurrences a group may hold
+  static constexpr uint32_t WMAX = GD_SWMAX << BITS;      // level-0 words of a group
+  static constexpr uint32_t W1MAX = (GD_SWMAX / 8) << BITS;  // level-1 words of a group
+  static constexpr uint32_t MAXL = BITS == 5 ? 5888 : 2816;  // occurrences on a level-0 bit set more than once
+  static constexpr uint32_t MAXC = BLOCK;                 // occurrences on a level-1 bit set more than once
+};
+template <int BITS>
 struct GdSmem {
+  using C = GdCfg<BITS>;
   // cleared at the start, 16 bytes at a time
-  unsigned long long set[GD_WMAX], col[GD_WMAX];   // level 0: bits set (then: placed), bits set more than once
-  unsigned long long set1[GD_W1MAX], col1[GD_W1MAX];
-  uint32_t rp[GD_MAXL / 8];                        // payload bytes beside rk
-  uint32_t rk[GD_MAXL / 2];                        // first listed occurrence of a bit; then the byte stage
-  unsigned long long lk[GD_MAXL];                  // the list (PK: packed words)
-  unsigned long long cid[GD_MAXC];                 // ids of the entries in cq
-  uint32_t cpre[GD_WMAX], fpre[GD_WMAX];           // per half word (16 bits each): col / placed bits before it
-  uint32_t fpre1[GD_W1MAX];
-  uint32_t tot[1 << GD_BITS];                      // placed bits per slice
-  uint32_t cp[GD_MAXC];                            // payloads joined over a key's copies
+  unsigned long long set[C::WMAX], col[C::WMAX];   // level 0: bits set (then: placed), bits set more than once
+  unsigned long long set1[C::W1MAX], col1[C::W1MAX];
+  uint32_t rp[C::MAXL / 8];                        // payload bytes beside rk
+  uint32_t rk[C::MAXL / 2];                        // first listed occurrence of a bit; then the byte stage
+  unsigned long long lk[C::MAXL];                  // the list (PK: packed words)
+  unsigned long long cid[C::MAXC];                 // ids of the entries in cq
+  uint32_t cpre[C::WMAX], fpre[C::WMAX];           // per half word (16 bits each): col / placed bits before it
+  uint32_t fpre1[C::W1MAX];
+  uint32_t tot[1 << BITS];                      // placed bits per slice
+  uint32_t cp[C::MAXC];                            // payloads joined over a key's copies
   // an entry's bit number (GD_OWN | number when its key is level 0's and it is
   // the first), its level-1 bit when level 0 leaves it (GD_JOIN: its byte is
   // in lp), or GD_NONE: a copy
-  uint16_t lx[GD_MAXL];
-  uint16_t cq[GD_MAXC], cb[GD_MAXC];               // entries on a level-1 bit set more than once, and that bit
-  uint8_t lp[GD_MAXL];                             // the list's payload bytes (PK: those joined at level 1)
+  uint16_t lx[C::MAXL];
+  uint16_t cq[C::MAXC], cb[C::MAXC];               // entries on a level-1 bit set more than once, and that bit
+  uint8_t lp[C::MAXL];                             // the list's payload bytes (PK: those joined at level 1)
   uint8_t lut[64];                                 // payload code -> byte
   uint32_t nlc, nc, kept, placed1;                 // nlc: list entries | bits set more than once << 16
 };
-static_assert(offsetof(GdSmem, set1) % 16 == 0 && offsetof(GdSmem, rk) % 16 == 0 && offsetof(GdSmem, rp) == offsetof(GdSmem, col1) + sizeof(GdSmem::col1), "cleared in one run");
-static_assert(sizeof(GdSmem) <= 113 * 1024, "two CTAs per SM");
-static_assert(GD_MAXN + 4 <= sizeof(GdSmem::rk), "the byte stage fits rk");
-static_assert(GD_W1MAX * 64 < GD_JOIN && GD_MAXL / 2 < GD_JOIN, "an entry's number, flags and level-1 bit fit 16 bits");
+template <int BITS>
+constexpr bool gd_layout_ok() {
+  using S = GdSmem<BITS>;
+  using C = GdCfg<BITS>;
+  return offsetof(S, set1) % 16 == 0 && offsetof(S, rk) % 16 == 0 &&
+         offsetof(S, rp) == offsetof(S, col1) + sizeof(S::col1) &&  // cleared in one run
+         (2 * sizeof(S::set1) + sizeof(S::rp)) % 16 == 0 &&
+         sizeof(S) <= (BITS == 5 ? 113 : 56) * 1024 &&  // two CTAs per SM, or four
+         C::MAXN + 4 <= sizeof(S::rk) &&                 // the byte stage
+         C::W1MAX * 64 < GD_JOIN && C::MAXL / 2 < GD_JOIN;  // an entry's number, flags and level-1 bit in 16 bits
+}
+static_assert(gd_layout_ok<4>() && gd_layout_ok<5>());
 
 // Popcount prefix of a thread's 64-bit word as its two half words' values
 // (low half first) in one u32.
@@ -1104,14 +1125,18 @@ CF1_D uint64_t gd_keep_word(uint64_t a, uint64_t q) { return (a >> 5) + q; }
 // is h * KEY_SPREAD_INV.  Group q: bin q >> Pg, the keys whose hash's top Pg
 // bits are q mod 2^Pg, in T[goff[q], goff[q + 1]); it is sub-buckets
 // [q << g, (q + 1) << g), g = P - Pg.
-template <bool PK>
-__global__ void __launch_bounds__(GD_BLOCK, 2) gd_dedup_kernel(const uint64_t *T, const uint8_t *TP,
+template <bool PK, int BITS>
+__global__ void __launch_bounds__(GdCfg<BITS>::BLOCK, BITS == 5 ? 2 : 4)
+    gd_dedup_kernel(const uint64_t *T, const uint8_t *TP,
                                                               const uint64_t *goff, int Pg, int P, uint32_t *cnt,
                                                               uint32_t *keep, Level0Out l0, uint32_t *ov,
                                                               uint32_t *ov_cnt, int p1) {
+  using C = GdCfg<BITS>;
+  constexpr int GD_BLOCK = C::BLOCK;
+  constexpr uint32_t GD_MAXN = C::MAXN, GD_MAXL = C::MAXL, GD_MAXC = C::MAXC;
   extern __shared__ __align__(16) unsigned char gd_smem[];
-  GdSmem &m = *reinterpret_cast<GdSmem *>(gd_smem);
-  constexpr uint32_t NW = GD_BLOCK / 32, SPW = (1u << GD_BITS) / NW;  // warps; slices a warp takes
+  GdSmem<BITS> &m = *reinterpret_cast<GdSmem<BITS> *>(gd_smem);
+  constexpr uint32_t NW = GD_BLOCK / 32, SPW = (1u << BITS) / NW;  // warps; slices a warp takes
   const unsigned tid = threadIdx.x, lane = lane_id(), warp = tid >> 5;
   const uint32_t q = blockIdx.x;
   const uint64_t a = goff[q], n64 = goff[q + 1] - a;
@@ -1380,7 +1405,7 @@ __global__ void __launch_bounds__(GD_BLOCK, 2) gd_dedup_kernel(const uint64_t *T
       }
   }
   __syncthreads();
-  const uint32_t st = m.tot[lane];
+  const uint32_t st = lane < (1u << BITS) ? m.tot[lane] : 0u;
   uint32_t placed;
   const uint32_t sbase = gd_warp_excl(st, placed);
 #pragma unroll
@@ -1475,7 +1500,7 @@ __global__ void __launch_bounds__(GD_BLOCK, 2) gd_dedup_kernel(const uint64_t *T
 // and bytes from T / TP to the same range of U / UP, sub-bucket by
 // sub-bucket, and writes the sub-buckets' offsets and list entries for the
 // block kernel.
-__global__ void __launch_bounds__(GD_BLOCK) gd_split_kernel(const uint64_t *T, const uint8_t *TP, const uint64_t *goff,
+__global__ void __launch_bounds__(GD_MOVE) gd_split_kernel(const uint64_t *T, const uint8_t *TP, const uint64_t *goff,
                                                            const uint32_t *ov, int Pg, int P, int p1, uint64_t *U,
                                                            uint8_t *UP, uint64_t *sb_off, uint32_t *jlist) {
   __shared__ unsigned long long s_cnt[1 << GD_BITS], s_cur[1 << GD_BITS];
@@ -1488,7 +1513,7 @@ __global__ void __launch_bounds__(GD_BLOCK) gd_split_kernel(const uint64_t *T, c
   auto sub = [&](uint64_t h) -> uint32_t { return g ? (uint32_t)(h >> (64 - P)) & (subs - 1) : 0u; };
   if (tid < subs) s_cnt[tid] = 0;
   __syncthreads();
-  for (uint64_t i = a + tid; i < e; i += GD_BLOCK) atomicAdd(&s_cnt[sub(hash(T[i]))], 1ull);
+  for (uint64_t i = a + tid; i < e; i += GD_MOVE) atomicAdd(&s_cnt[sub(hash(T[i]))], 1ull);
   __syncthreads();
   if (tid == 0) {
     uint64_t run = a;
@@ -1501,7 +1526,7 @@ __global__ void __launch_bounds__(GD_BLOCK) gd_split_kernel(const uint64_t *T, c
     sb_off[(q + 1) << g] = run;  // the next group's start: the same value if that group is listed too
   }
   __syncthreads();
-  for (uint64_t i = a + tid; i < e; i += GD_BLOCK) {
+  for (uint64_t i = a + tid; i < e; i += GD_MOVE) {
     const uint64_t x = T[i], h = hash(x), o = atomicAdd(&s_cur[sub(h)], 1ull);
     U[o] = p1 ? h * KEY_SPREAD_INV : x;
     if (UP) UP[o] = (uint8_t)pay_byte(p1 ? (uint32_t)x : TP[i]);
@@ -1513,7 +1538,7 @@ __global__ void __launch_bounds__(GD_BLOCK) gd_split_kernel(const uint64_t *T, c
 // group's start in T (packed again when T is: p1), all of them kept, and the
 // placed bytes it left in lp -- level 0's, then level 1's, sub-bucket by
 // sub-bucket -- to l0pay.
-__global__ void __launch_bounds__(GD_BLOCK) gd_gather_kernel(const uint64_t *U, const uint8_t *lp, const uint64_t *goff,
+__global__ void __launch_bounds__(GD_MOVE) gd_gather_kernel(const uint64_t *U, const uint8_t *lp, const uint64_t *goff,
                                                             const uint32_t *ov, int g, const uint64_t *sb_off,
                                                             const uint32_t *scnt, uint64_t *T, uint32_t *cnt,
                                                             uint32_t *keep, Level0Out l0, int p1) {
@@ -1522,13 +1547,13 @@ __global__ void __launch_bounds__(GD_BLOCK) gd_gather_kernel(const uint64_t *U, 
   for (uint64_t j = q << g; j < (q + 1) << g; j++) {
     const uint32_t c = scnt[j];
     const uint64_t a = sb_off[j];
-    for (uint32_t i = threadIdx.x; i < c; i += GD_BLOCK) T[o + i] = p1 ? (U[a + i] * MS_HASH_MUL) << p1 : U[a + i];
+    for (uint32_t i = threadIdx.x; i < c; i += GD_MOVE) T[o + i] = p1 ? (U[a + i] * MS_HASH_MUL) << p1 : U[a + i];
     o += c;
   }
   const uint64_t d = o - a0;
   if (threadIdx.x == 0) cnt[q] = (uint32_t)d;
   uint32_t *kw = keep + gd_keep_word(a0, q);
-  for (uint64_t w = threadIdx.x; w * 32 < d; w += GD_BLOCK)
+  for (uint64_t w = threadIdx.x; w * 32 < d; w += GD_MOVE)
     kw[w] = d - w * 32 >= 32 ? 0xFFFFFFFFu : (1u << (d - w * 32)) - 1;
   if (!l0.AR) return;
   o = a0;
@@ -1538,7 +1563,7 @@ __global__ void __launch_bounds__(GD_BLOCK) gd_gather_kernel(const uint64_t *U, 
       const uint32_t c = l ? l0.placed1[j] : l0.placed[j];
       const uint64_t a = sb_off[j] + (l ? l0.placed[j] : 0u);
       if (lp)
-        for (uint32_t i = threadIdx.x; i < c; i += GD_BLOCK) l0.l0pay[o + i] = lp[a + i];
+        for (uint32_t i = threadIdx.x; i < c; i += GD_MOVE) l0.l0pay[o + i] = lp[a + i];
       o += c;
     }
     if (threadIdx.x == 0) (l ? l0.uplaced1 : l0.uplaced)[q] = (uint32_t)(o - start);
@@ -2010,7 +2035,7 @@ int msd_prefix_bits(uint64_t max_bin_keys, bool sorted) {
   // times as long per key (128-bit keys aimed at 2048, its whole capacity,
   // left it two fifths of them: 100 Mbp at k = 63 3.24 ms in the two kernels,
   // 2.13 ms now).
-  // The unsorted 64-bit form (32 sub-buckets to a group of GD_MAXN at most)
+  // The unsorted 64-bit form (16 or 32 sub-buckets to a group)
   // aims at 192 for the largest bin.
   // 128-bit keys split by their hash are spread evenly: three quarters.
   const uint64_t target = sorted ? SrCfg<KeyT>::CAP / 4
@@ -2034,12 +2059,12 @@ bool msd_sort_unique(KeyT *keys, KeyT *alt, uint64_t n, uint64_t max_bin, const 
   else P = P < key_bits ? P : key_bits;  // short keys (k <= 7) have no more prefix bits than that
   // packed passes (see pay_code): the hashed split of keys with payloads
   // whose dedup builds BBHash level 0, with a first pass of >= 6 bits
-  // Groups of 32 sub-buckets for the group dedup (gd_dedup_kernel), split on
+  // Groups of 16 or 32 sub-buckets for the group dedup (see there), split on
   // the bits above theirs only, as long as the width rule's aim holds for the
-  // largest bin: 32 sub-buckets of at most WD_MAXD / 2 keys are 6144 of the
-  // group's GD_MAXN.
+  // largest bin: sub-buckets of at most WD_MAXD / 2 keys are three quarters of
+  // what a group holds.
   const bool grp = W1 && hashed && (max_bin >> P) <= WD_MAXD / 2;
-  const int g = grp ? (P < GD_BITS ? P : GD_BITS) : 0;
+  const int g = !grp ? 0 : P <= GD_BITS ? P : P - 4 <= GD_SPLIT ? 4 : GD_BITS;
   const int PS = P - g;  // bits split on: a unit is a group, or a sub-bucket
   sc.unit_bits = PS;
   sc.kept_bits = false;
@@ -2145,8 +2170,12 @@ bool msd_sort_unique(KeyT *keys, KeyT *alt, uint64_t n, uint64_t max_bin, const 
       // one CTA per group; the groups it cannot hold go to the block kernel
       // sub-bucket by sub-bucket, through the free buffers
       uint32_t *ov = sc.ov.get<uint32_t>(nunit + 1);
-      auto gkern = pk ? gd_dedup_kernel<true> : gd_dedup_kernel<false>;
-      CF1_CUDA(cudaFuncSetAttribute(gkern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(GdSmem)));
+      const bool small = g <= 4;
+      auto gkern = small ? (pk ? gd_dedup_kernel<true, 4> : gd_dedup_kernel<false, 4>)
+                         : (pk ? gd_dedup_kernel<true, 5> : gd_dedup_kernel<false, 5>);
+      const size_t gsm = small ? sizeof(GdSmem<4>) : sizeof(GdSmem<5>);
+      const int gblock = small ? GdCfg<4>::BLOCK : GdCfg<5>::BLOCK;
+      CF1_CUDA(cudaFuncSetAttribute(gkern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)gsm));
       uint64_t *T64 = reinterpret_cast<uint64_t *>(T), *U64 = reinterpret_cast<uint64_t *>(U);
       // a bit per occurrence: the first copy of its key (words of groups
       // that keep nothing there stay 0)
@@ -2154,7 +2183,7 @@ bool msd_sort_unique(KeyT *keys, KeyT *alt, uint64_t n, uint64_t max_bin, const 
       uint32_t *keep = sc.keep.get<uint32_t>(nkeep);
       CF1_CUDA(cudaMemsetAsync(keep, 0, nkeep * sizeof(uint32_t), s));
       const int p1 = pk ? P1 : 0;
-      gkern<<<(unsigned)nunit, GD_BLOCK, sizeof(GdSmem), s>>>(T64, PT, sb_off, PS, P, cnt, keep, lo, ov, ovc, p1);
+      gkern<<<(unsigned)nunit, gblock, gsm, s>>>(T64, PT, sb_off, PS, P, cnt, keep, lo, ov, ovc, p1);
       CF1_LAUNCH_CHECK();
       CF1_CUDA(cudaEventRecord(sc.ev[1], s));
       finish();
@@ -2168,12 +2197,12 @@ bool msd_sort_unique(KeyT *keys, KeyT *alt, uint64_t n, uint64_t max_bin, const 
         uint32_t *scnt = sc.sub_cnt.get<uint32_t>(nsub + 1), *jl = sc.jlist.get<uint32_t>(nov);
         Level0Out lb = lo;
         if (lo.with_pay) lb.l0pay = sc.ov_pay.get<uint8_t>(n + 16);
-        gd_split_kernel<<<h_ov, GD_BLOCK, 0, s>>>(T64, PT, sb_off, ov, PS, P, p1, U64, PU, sub_off, jl);
+        gd_split_kernel<<<h_ov, GD_MOVE, 0, s>>>(T64, PT, sb_off, ov, PS, P, p1, U64, PU, sub_off, jl);
         CF1_LAUNCH_CHECK();
         kern<<<nov, CS_BLOCK, smem, s>>>(U, T, sub_off, nsub, shift, rest > 0 ? bits : 0, scnt, over, P, lb, PU, PT,
                                          nullptr, nullptr, nbins, jl, nullptr, false);
         CF1_LAUNCH_CHECK();
-        gd_gather_kernel<<<h_ov, GD_BLOCK, 0, s>>>(U64, lo.with_pay ? lb.l0pay : nullptr, sb_off, ov, g, sub_off, scnt,
+        gd_gather_kernel<<<h_ov, GD_MOVE, 0, s>>>(U64, lo.with_pay ? lb.l0pay : nullptr, sb_off, ov, g, sub_off, scnt,
                                                    T64, cnt, keep, lo, p1);
         CF1_LAUNCH_CHECK();
         CF1_CUDA(cudaEventRecord(sc.ev[1], s));

@@ -69,3 +69,13 @@ def test_repeated_keys_within_a_group():
     seq, off = o.concat_records(recs)
     for bins in (1, 16, 500):
         assert_parity(seq, off, 31, num_bins=bins)[0].close()
+
+
+@pytest.mark.parametrize("n_bases,copies", [(3_145_700, 1), (3_145_800, 1), (15_870, 3), (15_600, 3), (1_060_000, 3)])
+def test_group_size_change_over(n_bases, copies):
+    """Both sides of the split width where groups go from 16 to 32 sub-buckets
+    (192 * 2^14 k-mers in a bin), and groups of 16 and 32 whose occurrences,
+    three of every key, pass or just fit the list."""
+    seq, off = o.concat_records([_random(n_bases, n_bases)] * copies)
+    g, _ = assert_parity(seq, off, 31, num_bins=1)
+    g.close()
