@@ -163,7 +163,7 @@ struct SortScratch {
 };
 
 // Per record k-mer offsets: kpre[i] = sum of n over records < i (kpre[n_rec] = total).
-void record_kmer_prefix(const uint64_t *records, uint64_t n_rec, uint64_t *kpre, DevBuf &lens, DevBuf &scratch,
+void record_kmer_prefix(const uint64_t *records, uint64_t n_rec, uint64_t *kpre, DevBuf &scratch,
                         cudaStream_t s);
 
 // Writes each k-mer's canonical form; keys[kpre[i] + j] is k-mer j of record

@@ -17,11 +17,6 @@ constexpr int RS_NW = RS_BLOCK / 32;
 
 CF1_D uint64_t ceil_div_dev(uint64_t n) { return (n + 31) / 32; }
 
-__global__ void record_len_kernel(const uint64_t *records, uint64_t n, uint32_t *len) {
-  uint64_t i = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  if (i < n) len[i] = rec_n(records[i]);
-}
-
 // Warp-cooperative expansion: a warp takes 32 records, and its lanes walk the
 // records' k-mers in one flattened index space, so output stores are
 // contiguous whatever the record lengths.  With `sides`, each
@@ -399,16 +394,6 @@ __global__ void seg_out_off_kernel(const uint32_t *tile_off, uint32_t nseg, cons
 }
 
 }  // namespace
-
-void record_kmer_prefix(const uint64_t *records, uint64_t n_rec, uint64_t *kpre, DevBuf &lens, DevBuf &scratch,
-                        cudaStream_t s) {
-  uint32_t *len = lens.get<uint32_t>(n_rec + 1);
-  if (n_rec) {
-    record_len_kernel<<<(unsigned)ceil_div(n_rec, 256), 256, 0, s>>>(records, n_rec, len);
-    CF1_LAUNCH_CHECK();
-  }
-  exclusive_scan_u32(len, kpre, n_rec, scratch, s);
-}
 
 template <class KeyT>
 void launch_expand(const uint64_t *records, uint64_t n_rec, const uint64_t *kpre, const uint64_t *W, int k, KeyT *keys,

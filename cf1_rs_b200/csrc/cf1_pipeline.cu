@@ -503,7 +503,7 @@ void run_impl(cf1gpu_ctx *c, StreamIO *io = nullptr, Step step = Step::FULL, con
     CF1_CUDA(cudaMemcpyAsync(rec_off, new_off, (B + 1) * sizeof(uint64_t), cudaMemcpyDeviceToDevice, s));
   }
   uint64_t *kpre = c->d_kpre.get<uint64_t>(NS + 1);
-  record_kmer_prefix(records, NS, kpre, c->d_lens, c->d_scan, s);
+  record_kmer_prefix(records, NS, kpre, c->d_scan, s);
   if (shards > 1 || step == Step::XFINISH) {  // the k-mer windows of this shard's records
     CF1_CUDA(cudaMemcpyAsync(&c->n_occ, kpre + NS, sizeof(uint64_t), cudaMemcpyDeviceToHost, s));
     CF1_CUDA(cudaStreamSynchronize(s));
