@@ -233,7 +233,7 @@ static_assert(KEY_SPREAD_MUL * KEY_SPREAD_INV == 1, "KEY_SPREAD_INV inverts KEY_
 // (contribution_code) in the p1 bits freed.
 // The next pass splits on the word's own top bits; the dedup rebuilds h from
 // the sub-bucket's index and the key as h * KEY_SPREAD_INV.  A single
-// occurrence's side-set byte has nibbles in {3, 5, 6, 9, F} (sideset_byte):
+// occurrence's side-set byte has nibbles in {3, 5, 6, 9, F}:
 // each nibble is a 3-bit code (0 also has one; anything else, which no
 // occurrence gives, reads as F).
 constexpr uint64_t pay_nib_codes() {
@@ -421,42 +421,14 @@ CF1_HD uint32_t contribution(KeyT fw, KeyT rcv, bool has_prev, uint32_t prev, bo
   return fwd ? encode_sides(prev, next) : encode_sides(3 - next, 3 - prev);
 }
 
-// sideset_lookup(contribution(...)) computed directly: the side-set byte of
-// one occurrence (front nibble low, back nibble high; M = 0xF), from what it
-// depends on: whether the k-mer is read forward (fwd), whether it has a base
-// before / after it (and which), whether the next k-mer is the same vertex
-// (next_same) and, if so, the same oriented k-mer (next_same_fw).  prev is
-// not read without has_prev, nor next, next_same, next_same_fw without
-// has_next.
-CF1_HD uint32_t sideset_byte(bool fwd, bool has_prev, uint32_t prev, bool has_next, uint32_t next, bool next_same,
-                             bool next_same_fw) {
-  if (!has_prev && !has_next) return 0xFFu;
-  const uint32_t cp = side_code(prev), cpc = side_code(3 - prev);
-  const uint32_t right = fwd ? (cp | 0xF0u) : (0x0Fu | (cpc << 4));
-  if (!has_next) return right;
-  if (next_same) return (!has_prev || next_same_fw) ? 0xFFu : right;
-  const uint32_t cn = side_code(next), cnc = side_code(3 - next);
-  if (!has_prev) return fwd ? (0x0Fu | (cn << 4)) : (cnc | 0xF0u);
-  return fwd ? (cp | (cn << 4)) : (cnc | (cpc << 4));
-}
-
-// The same from the k-mer's forward and reverse-complement values and the
-// next k-mer's (nf, nr: the k-mer rolled by `next`), which a caller walking
-// the sequence has already; with !has_next nf and nr are not read.
-template <class KeyT>
-CF1_HD uint32_t contribution_sideset_rolled(KeyT fw, KeyT rcv, KeyT nf, KeyT nr, bool has_prev, uint32_t prev,
-                                            bool has_next, uint32_t next) {
-  const KeyT can = kmin(fw, rcv);
-  return sideset_byte(fw == can, has_prev, prev, has_next, next, has_next && kmin(nf, nr) == can,
-                      has_next && nf == fw);
-}
-
-// The same as the byte's 6-bit code (see pay_code; pay_byte gives the byte),
-// which is what travels with a key until its occurrences are joined.  A side's
-// code is its base, or 4 for M: read forward the front is x, the base before,
-// and the back y, the base after; read backward they swap and complement (4
-// becomes 7, which also reads back as M).  prev and next are 4 where there is
-// no base; nf and nr are only looked at when has_next.
+// sideset_lookup(contribution(...)) computed directly, from the k-mer's forward
+// and reverse-complement values and the next k-mer's forward value nf (the
+// k-mer rolled by `next`), as the byte's 6-bit code (see pay_code; pay_byte
+// gives the byte), which is what travels with a key until its occurrences are
+// joined.  A side's code is its base, or 4 for M: read forward the front is x,
+// the base before, and the back y, the base after; read backward they swap and
+// complement (4 becomes 7, which also reads back as M).  prev and next are 4
+// where there is no base; nf is only looked at when has_next.
 template <class KeyT>
 CF1_HD uint32_t contribution_code(KeyT fw, KeyT rcv, KeyT nf, uint32_t prev, bool has_next, uint32_t next) {
   uint32_t x = prev, y = has_next ? next : 4u;
@@ -466,14 +438,6 @@ CF1_HD uint32_t contribution_code(KeyT fw, KeyT rcv, KeyT nf, uint32_t prev, boo
     if (loop) x = 4;
   }
   return rcv < fw ? ((x << 3) | y) ^ 27u : (y << 3) | x;
-}
-
-template <class KeyT>
-CF1_HD uint32_t contribution_sideset(KeyT fw, KeyT rcv, bool has_prev, uint32_t prev, bool has_next, uint32_t next,
-                                     int k) {
-  KeyT nf = fw, nr = rcv;
-  KOps<KeyT>::roll(nf, nr, next, k);
-  return contribution_sideset_rolled(fw, rcv, nf, nr, has_prev, prev, has_next, next);
 }
 
 // ------------------------------------------------------------- error flags ----
