@@ -1037,6 +1037,8 @@ __global__ void __launch_bounds__(SR_BLOCK, 2) sr_dedup_kernel(KeyT *T, uint8_t 
 // makes up for.
 constexpr int GD_U = 16;                 // keys per thread
 constexpr int GD_BITS = 5;               // sub-buckets of a group (log2), at most
+constexpr int MSD_MAX_BITS = 16;         // widest split
+constexpr uint32_t GD_MAXSUB = 224;      // occurrences of a sub-bucket a group of 32 has room for, on average
 constexpr int GD_SPLIT = 10;             // most split bits that groups of 16 sub-buckets are worth
 constexpr int GD_MOVE = 512;             // threads of the kernels that move a listed group
 constexpr uint32_t GD_SWMAX = 32;        // level-0 words of a slice: one a lane
@@ -2041,7 +2043,7 @@ int msd_prefix_bits(uint64_t max_bin_keys, bool sorted) {
   const uint64_t target = sorted ? SrCfg<KeyT>::CAP / 4
                                  : KOps<KeyT>::WORDS == 1 ? WD_MAXD / 2 : SrCfg<KeyT>::CAP * 3 / 4;
   int p = 0;
-  while (p < 16 && (max_bin_keys >> p) > target) p++;
+  while (p < MSD_MAX_BITS && (max_bin_keys >> p) > target) p++;
   return p;
 }
 
@@ -2063,7 +2065,10 @@ bool msd_sort_unique(KeyT *keys, KeyT *alt, uint64_t n, uint64_t max_bin, const 
   // the bits above theirs only, as long as the width rule's aim holds for the
   // largest bin: sub-buckets of at most WD_MAXD / 2 keys are three quarters of
   // what a group holds.
-  const bool grp = W1 && hashed && (max_bin >> P) <= WD_MAXD / 2;
+  // (At the widest split, bins of 12.6 to 14.7 M keys, up to 224: 32 of them
+  // are 7168 of a group's 8192.  3.1 Gbp in 256 bins: 127 ms a run with the
+  // warp sets, 106 with groups.)
+  const bool grp = W1 && hashed && (max_bin >> P) <= (P == MSD_MAX_BITS ? GD_MAXSUB : WD_MAXD / 2);
   const int g = !grp ? 0 : P <= GD_BITS ? P : P - 4 <= GD_SPLIT ? 4 : GD_BITS;
   const int PS = P - g;  // bits split on: a unit is a group, or a sub-bucket
   sc.unit_bits = PS;
