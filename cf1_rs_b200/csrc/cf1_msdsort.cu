@@ -756,7 +756,10 @@ __global__ void __launch_bounds__(CS_BLOCK, SORTED ? 2 : 4) cs_sort_unique_kerne
 //   2. what the shared positions before it hold beyond one key: their
 //      occurrences are gathered, position by position (numbered by a popcount
 //      of col, counted by atomics), and one thread per position sorts its few
-//      keys and joins the copies' payload bytes;
+//      keys and joins the copies' payload bytes.  In a run with more than
+//      SR_MANY occurrences on a position, the copies of every position's
+//      first key join it before that, all at once: one thread walking tandem
+//      arrays' hundreds of copies took 3.1 Gbp with them 180 ms, now 133;
 //   3. keys and bytes are staged in shared memory by rank and written out.
 // ~85% of the keys of unrepeated sequence have a position of their own.  A run
 // that does not fit (a sub-bucket above CAP keys, more than SR_MAXD different
@@ -766,6 +769,7 @@ __global__ void __launch_bounds__(CS_BLOCK, SORTED ? 2 : 4) cs_sort_unique_kerne
 // Its bound is its barriers and instruction issue, as the group dedup's below.
 constexpr int SR_BLOCK = 512;
 constexpr uint32_t SR_MAXD = 48;
+constexpr uint32_t SR_MANY = 8;
 template <class KeyT>
 struct SrCfg {
   static constexpr int U = KOps<KeyT>::WORDS == 1 ? 8 : 4;  // keys per thread
@@ -786,6 +790,8 @@ struct SrSmem {
   uint8_t segp[C::CAP], stagep[C::CAP];
   uint32_t sm[SR_BLOCK / 32];
 };
+
+static_assert(offsetof(SrSmem<uint64_t>, stagep) % 4 == 0 && offsetof(SrSmem<Key2>, stagep) % 4 == 0, "joined in words");
 
 template <class KeyT, bool HASHED>
 __global__ void __launch_bounds__(SR_BLOCK, 2) sr_dedup_kernel(KeyT *T, uint8_t *TP, const uint64_t *sb_off,
@@ -866,12 +872,16 @@ __global__ void __launch_bounds__(SR_BLOCK, 2) sr_dedup_kernel(KeyT *T, uint8_t 
     nset = tot & 0xFFFFu;
     ncol = tot >> 16;
   }
-  uint32_t shared = 0, extra = 0;  // this thread's keys on shared positions; keys beyond one a position
+  uint32_t shared = 0, extra = 0;    // this thread's keys on shared positions; keys beyond one a position
+  uint32_t copies = 0;               // copies of the first key that reached their position
+  bool join = false;
   if (ncol) {  // uniform
     // 2. the shared positions' occurrences, counted, placed and sorted
+    uint32_t *joined = reinterpret_cast<uint32_t *>(m.stagep);  // a position's first key's copies' payloads
     for (uint32_t c = tid; c < ncol; c += SR_BLOCK) m.cnt[c] = 0;
     __syncthreads();
-    uint32_t slot[C::U];
+    bool many = false;
+    uint32_t slot[C::U];  // position | place among the position's occurrences << 16
 #pragma unroll
     for (int u = 0; u < C::U; u++) {
       slot[u] = 0;
@@ -880,11 +890,37 @@ __global__ void __launch_bounds__(SR_BLOCK, 2) sr_dedup_kernel(KeyT *T, uint8_t 
         if (cw & bm) {
           const uint32_t c = m.cpre[p >> 5] + (uint32_t)__popc(cw & (bm - 1));
           shared |= 1u << u;
-          slot[u] = c | (atomicAdd(&m.cnt[c], 1u) << 16);
+          const uint32_t at = atomicAdd(&m.cnt[c], 1u);
+          slot[u] = c | (at << 16);
+          many |= at >= SR_MANY;
         }
       }
     }
-    __syncthreads();
+    join = __syncthreads_or((int)many) != 0;
+    if (join) {
+      // copies of a position's first key join it here, all at once; what is
+      // sorted below are the other keys
+      for (uint32_t w = tid; 4 * w < ncol; w += SR_BLOCK) joined[w] = 0;
+#pragma unroll
+      for (int u = 0; u < C::U; u++)
+        if (((shared >> u) & 1) && slot[u] < 0x10000u) m.stage[slot[u]] = key[u];
+      __syncthreads();
+#pragma unroll
+      for (int u = 0; u < C::U; u++) {
+        if (((shared >> u) & 1) && slot[u] >= 0x10000u) {
+          const uint32_t c = slot[u] & 0xFFFFu;
+          if (m.stage[c] == key[u]) {
+            copies |= 1u << u;
+            if (TP) atomicOr(&joined[c >> 2], ((pb[u >> 2] >> (8 * (u & 3))) & 0xFFu) << (8 * (c & 3)));
+          } else {
+            slot[u] = c | (((atomicAdd(&m.cnt[c], 0x10000u) >> 16) + 1) << 16);
+          }
+        }
+      }
+      __syncthreads();
+      for (uint32_t c = tid; c < ncol; c += SR_BLOCK) m.cnt[c] = (m.cnt[c] >> 16) + 1;
+      __syncthreads();
+    }
     {
       uint32_t v = 0, x[C::CPT], tot;
 #pragma unroll
@@ -904,10 +940,12 @@ __global__ void __launch_bounds__(SR_BLOCK, 2) sr_dedup_kernel(KeyT *T, uint8_t 
     __syncthreads();
 #pragma unroll
     for (int u = 0; u < C::U; u++) {
-      if ((shared >> u) & 1) {
-        const uint32_t at = m.start[slot[u] & 0xFFFFu] + (slot[u] >> 16);
+      if (((shared & ~copies) >> u) & 1) {
+        const uint32_t c = slot[u] & 0xFFFFu, at = m.start[c] + (slot[u] >> 16);
+        uint32_t p = pb[u >> 2] >> (8 * (u & 3));
+        if (join && slot[u] < 0x10000u) p |= joined[c >> 2] >> (8 * (c & 3));
         m.seg[at] = key[u];
-        m.segp[at] = (uint8_t)(pb[u >> 2] >> (8 * (u & 3)));
+        m.segp[at] = (uint8_t)p;
       }
     }
     __syncthreads();

@@ -52,3 +52,18 @@ def test_copies_and_close_keys(k):
     close = [head + ACGT[rng.integers(0, 4, k - len(head))].tobytes() for _ in range(700)]
     _check(close + [base], k, num_bins=1)
     _check(close + [base], k, num_bins=1, state_update="sideset")
+
+
+@pytest.mark.parametrize("mode,k", [("learned", 31), ("learned", 63), ("bbhash", 63)])
+@pytest.mark.parametrize("copies", [3, 40, 700])
+def test_tandem_array(mode, k, copies):
+    """A 171-base unit repeated, every copy with one substitution: positions
+    with up to hundreds of copies of their first key, and other keys beside."""
+    rng = np.random.default_rng(copies + k)
+    unit = rng.integers(0, 4, 171)
+    rows = np.tile(unit, (copies, 1))
+    rows[np.arange(copies), rng.integers(0, 171, copies)] = rng.integers(0, 4, copies)
+    seq, off = o.concat_records([np.frombuffer(b"ACGT", np.uint8)[rows.ravel()].tobytes(),
+                                 np.frombuffer(b"ACGT", np.uint8)[rng.integers(0, 4, 20_000)].tobytes()])
+    g, _ = assert_parity(seq, off, k, mode=mode, num_bins=2)
+    g.close()
