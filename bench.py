@@ -108,8 +108,8 @@ def traffic_md(form: str, kernel: str) -> str:
     if kernel == "classify":
         return os.path.join(ROOT, "profiles", "classify_traffic_workload5_full.md")
     if form == "bbhash":
-        return os.path.join(ROOT, "profiles", "wd_dedup_kernel_workload5_scale0.05.md")
-    return os.path.join(ROOT, "profiles", "cs_sort_unique_kernel_workload5_scale0.05.md")
+        return os.path.join(ROOT, "profiles", "gd_dedup_kernel_workload5_scale0.05.md")
+    return os.path.join(ROOT, "profiles", "sr_dedup_kernel_workload5_scale0.05.md")
 
 
 def committed_traffic(workload: int, scale: float, form: str, kernel: str = "classify"):
@@ -472,12 +472,16 @@ def gpu_arm(args):
         # multisplit on packed words (the byte inside the key's word), so the
         # dedup reads w bytes per occurrence there
         packed = head_name == "bbhash" and w == 8 and 6 <= int(s["sort_msd_bits"]) <= 64
-        b_dd = (w if packed else w + 1.0) * n_occ + (w + 1.0) * n_dist + (2.0 * n_occ if head_name == "bbhash" else 0.0)
+        # the group dedup leaves the keys where they are and writes a byte per
+        # distinct key, the others write the distinct keys too
+        grouped = head_name == "bbhash" and w == 8
+        b_dd = ((w if packed else w + 1.0) * n_occ + (1.0 if grouped else w + 1.0) * n_dist
+                + (2.0 * n_occ if head_name == "bbhash" else 0.0))
         ach = b_dd / (head["ms_dedup_kernel"] / 1e3) / 1e9
-        # BBHash form: the warp dedup, with the block kernel for the few
-        # sub-buckets it leaves (timed together); learned form: the sorted
-        # chunk dedup
-        kname = "wd_dedup_kernel" if head_name == "bbhash" else "cs_sort_unique_kernel"
+        # BBHash form: the group dedup (128-bit keys: the rank dedup), with
+        # the block kernel for what it leaves (timed together); learned form:
+        # the rank dedup
+        kname = "gd_dedup_kernel" if grouped else "sr_dedup_kernel"
         roofline = {"kernel": kname, "bound": "hbm", "achieved": ach, "peak": peaks["hbm_gbs"],
                     "unit": "GB/s", "frac": ach / peaks["hbm_gbs"], "peak_kind": peak_kind,
                     "traffic": committed_traffic(args.workload, args.scale, head_name, "dedup"),
