@@ -769,7 +769,7 @@ __global__ void __launch_bounds__(CS_BLOCK, SORTED ? 2 : 4) cs_sort_unique_kerne
 // Its bound is its barriers and instruction issue, as the group dedup's below.
 constexpr int SR_BLOCK = 512;
 constexpr uint32_t SR_MAXD = 48;
-constexpr uint32_t SR_MANY = 8;
+constexpr uint32_t SR_MANY = 32;  // (8 sent repeats of ordinary genomes there too: 200 Mbp 3.21 ms, 3.17 now)
 template <class KeyT>
 struct SrCfg {
   static constexpr int U = KOps<KeyT>::WORDS == 1 ? 8 : 4;  // keys per thread
