@@ -242,7 +242,10 @@ __global__ void __launch_bounds__(BF_BLOCK) bb_sliced_kernel(const uint64_t *wof
 constexpr uint32_t BF_WORDS = 4096;
 constexpr uint64_t BF_KEYS = 16384;
 // Entries reserved for n keys: the levels' blocks sum up to ~1.14 times the
-// first one's words and a word a level.
+// first one's words and a word a level.  Keys that a level's hash crowds
+// together -- thousands of one sub-bucket, which share level 0's top bits --
+// pass most of them on and need more: DEV_BB_ROOM, and the run is repeated
+// with a launch a level (one_launch off), each sized by its keys.
 CF1_HD uint64_t bf_room(uint64_t n) {
   const uint64_t w = (8 * n + 63) / 64;
   return n ? w + w / 4 + BB_MAX_LEVELS : 0;
@@ -273,7 +276,7 @@ __global__ void __launch_bounds__(BF_BLOCK) bb_tail_kernel(const KeyT *rem0, Key
   for (; n; l++) {
     const uint64_t nw = (8 * n + 63) / 64;
     if (l >= BB_MAX_LEVELS || used + nw > room) {
-      if (tid == 0) atomicOr(err, (uint32_t)DEV_BIJECTION);
+      if (tid == 0) atomicOr(err, (uint32_t)(l >= BB_MAX_LEVELS ? DEV_BIJECTION : DEV_BB_ROOM));
       return;
     }
     ulonglong2 *E = AR + region + used;
@@ -468,7 +471,7 @@ void BBHashBuild<KeyT>::run_levels(uint32_t l, const KeyT *rem, const uint64_t *
     levels = BB_MAX_LEVELS;  // until collect(): a walk ends at the first level a bin does not have
   };
   tail_from_ = l;
-  if (expect <= BF_KEYS * nbins) return tail();
+  if (one_launch && expect <= BF_KEYS * nbins) return tail();
   uint64_t *wcnt = wcnt_.as<uint64_t>(), *woff = woff_.as<uint64_t>();
   uint32_t *tile_off = tile_off_.as<uint32_t>();
   unsigned long long *tot = reinterpret_cast<unsigned long long *>(tot_.as<uint64_t>());
@@ -482,7 +485,7 @@ void BBHashBuild<KeyT>::run_levels(uint32_t l, const KeyT *rem, const uint64_t *
     CF1_CUDA(cudaStreamSynchronize(s));
     const uint64_t remaining = ht[0], nw = ht[1];
     if (remaining == 0) break;
-    if (remaining <= BF_KEYS * nbins) {
+    if (one_launch && remaining <= BF_KEYS * nbins) {
       reserve_entries(total_words + bf_room(remaining) + nbins * (bf_room(1) + 1), total_words, s);
       tail_from_ = l;
       return tail();

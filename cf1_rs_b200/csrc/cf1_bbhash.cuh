@@ -11,6 +11,7 @@ struct BBHashBuild {
   uint64_t bytes = 0;
   int l1_slice_bits = -1;          // see BBView
   uint64_t srank_words = 0;        // entries of each sliced level's srank table
+  bool one_launch = true;          // the last levels in one launch (off: a launch a level, after DEV_BB_ROOM)
 
   BBHashBuild() = default;
   BBHashBuild(const BBHashBuild &) = delete;

@@ -449,6 +449,7 @@ enum DeviceError : uint32_t {
   DEV_BIJECTION = 1u << 3,     // slot seen twice or never
   DEV_WAIT_LIMIT = 1u << 4,    // a bounded spin wait gave up
   DEV_FOREIGN = 1u << 5,       // a received record is not this shard's to process
+  DEV_BB_ROOM = 1u << 6,       // a bin's last BBHash levels outgrew their room
 };
 
 }  // namespace cf1

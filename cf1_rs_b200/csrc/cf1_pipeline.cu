@@ -168,6 +168,7 @@ void check_device_errors(uint32_t err) {
   if (err & DEV_CAS_LIMIT) throw Error(CF1GPU_ERR_DEVICE_TIMEOUT, "phase 4: a state CAS loop passed its bound");
   if (err & DEV_WAIT_LIMIT) throw Error(CF1GPU_ERR_DEVICE_TIMEOUT, "a bounded device wait gave up");
   if (err & DEV_OVERFLOW) throw Error(CF1GPU_ERR_QUEUE_OVERRUN, "a device buffer bound was hit");
+  if (err & DEV_BB_ROOM) throw Error(CF1GPU_ERR_BIJECTION, "BBHash: a bin's last levels outgrew their room");
   if (err & DEV_MPHF_MISS) throw Error(CF1GPU_ERR_BIJECTION, "phase 4: a k-mer was not found by the MPHF");
   if (err & DEV_BIJECTION) throw Error(CF1GPU_ERR_BIJECTION, "MPHF is not a bijection onto [0, n)");
   if (err & DEV_FOREIGN)
@@ -800,6 +801,16 @@ void run_impl(cf1gpu_ctx *c, StreamIO *io = nullptr, Step step = Step::FULL, con
   CF1_CUDA(cudaStreamSynchronize(s));
   be.bb.collect_end(rb->bb);
   hs = *rsm;
+  if ((hs.err & DEV_BB_ROOM) && be.bb.one_launch) {  // once more, with BBHash's last levels launched one by one
+    struct OneByOne {
+      bool &one_launch;
+      explicit OneByOne(bool &f) : one_launch(f) { one_launch = false; }
+      ~OneByOne() { one_launch = true; }
+    } one_by_one(be.bb.one_launch);
+    run_impl<KeyT>(c, io, step, xs);
+    if (tune_now) c->stats.tuner_state = (uint64_t)(c->tuner_state = 2);
+    return;
+  }
   check_device_errors(hs.err);
   c->cas_retries = hs.cas_retries;
 
