@@ -733,7 +733,9 @@ __global__ void __launch_bounds__(CS_BLOCK, SORTED ? 2 : 4) cs_sort_unique_kerne
   }
   for (uint64_t q = j + 1 + tid; q < jend; q += CS_BLOCK) cnt[q] = 0;
   if constexpr (L0) {
-    if (l0.AR && res != ~0u) {
+    if (l0.AR && res == ~0u) {  // no slice: its placed counts are read all the same (gd_gather_kernel)
+      if (tid == 0) l0.placed[j] = l0.placed1[j] = 0;
+    } else if (l0.AR) {
       __syncthreads();
       unsigned long long *h64 = reinterpret_cast<unsigned long long *>(hist);
       l0_slice(reinterpret_cast<const uint64_t *>(T) + a, res, j, P, l0, h64, h64 + L0_SW_MAX,
