@@ -2043,7 +2043,10 @@ void ms_pass(int bits, const KeyT *in, KeyT *out, uint64_t n, const uint64_t *se
   auto kern = ms_scatter_kernel<KeyT, false>;
   if constexpr (KOps<KeyT>::WORDS == 1)
     if (pack) kern = ms_scatter_kernel<KeyT, true>;
-  CF1_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+  // (the largest pass's, not this one's: the attribute is the function's on
+  // the device, and another context may launch it at any width meanwhile)
+  constexpr size_t MOST = TILE * sizeof(KeyT) + ((sizeof(uint64_t) + sizeof(uint32_t)) << MS_BITS) + TILE;
+  CF1_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)MOST));
   kern<<<(unsigned)(ceil_div(n, TILE) + nseg), MS_BLOCK, smem, s>>>(in, out, seg_off, tile_off, nseg, shift, bits, hashed,
                                                                    sub_off, cursor, pin, pout, pack);
   CF1_LAUNCH_CHECK();
@@ -2158,10 +2161,11 @@ bool msd_sort_unique(KeyT *keys, KeyT *alt, uint64_t n, uint64_t max_bin, const 
   }
   // S, hist, cur, pstart (u32) and the chunk bounds (u16)
   const uint32_t cap = cs_cap_for(KOps<KeyT>::WORDS == 2, sorted);
-  size_t smem = cap * sizeof(KeyT) + (3 * CS_BUCKETS + 1) * sizeof(uint32_t) + (CS_BUCKETS + 2) * sizeof(uint16_t) +
-                (pkeys || !sorted ? cap : 0);  // payloads; without them the unsorted form's l0_slice scratch
+  const size_t smem_keys = cap * sizeof(KeyT) + (3 * CS_BUCKETS + 1) * sizeof(uint32_t) + (CS_BUCKETS + 2) * sizeof(uint16_t);
+  const size_t smem = smem_keys + (pkeys || !sorted ? cap : 0);  // payloads; without them the unsorted form's l0_slice scratch
   auto kern = sorted ? cs_sort_unique_kernel<KeyT, true> : cs_sort_unique_kernel<KeyT, false>;
-  CF1_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+  // (with the payloads in any case, as ms_pass sets its own)
+  CF1_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)(smem_keys + cap)));
   KeyT *U = T == keys ? alt : keys;
   uint8_t *PU = pkeys ? (PT == pkeys ? palt : pkeys) : nullptr;
   if (l0pay_buf) *l0pay_buf = PU;

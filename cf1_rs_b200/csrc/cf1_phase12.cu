@@ -529,7 +529,10 @@ void launch_bin_scatter(const uint64_t *rec_tmp, const uint16_t *rec_bucket, uin
                         const uint64_t *NM, uint64_t L, int k, cudaStream_t s) {
   if (n == 0) return;
   size_t smem = BS_TILE * sizeof(uint64_t) + 3 * num_bins * sizeof(uint32_t);
-  CF1_CUDA(cudaFuncSetAttribute(bin_scatter_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+  // (the largest bin count's: the attribute is the function's on the device,
+  // and another context may launch it with other bins meanwhile)
+  constexpr size_t MOST = BS_TILE * sizeof(uint64_t) + 3 * MAX_BINS * sizeof(uint32_t);
+  CF1_CUDA(cudaFuncSetAttribute(bin_scatter_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)MOST));
   bin_scatter_kernel<<<(unsigned)ceil_div(n, (uint64_t)BS_TILE), BS_BLOCK, smem, s>>>(
       rec_tmp, rec_bucket, n, lut, num_bins, rec_off, cursor, records, err, NM, L, k);
   CF1_LAUNCH_CHECK();
