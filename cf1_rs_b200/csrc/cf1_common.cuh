@@ -64,6 +64,26 @@ CF1_HD uint64_t mulhi64(uint64_t a, uint64_t b) {
 #endif
 }
 
+// A copy of n bytes between any two addresses, four bytes a thread: `head`
+// bytes bring the destination to a word boundary, then `words` words are cut
+// from the aligned source words they span, shifted by `shift` bits, and the
+// rest (up to six bytes) are copied one by one.  Every aligned source word
+// but the first ends inside the source, so nothing after it is read: the
+// bytes there may be past their allocation, or still arriving.  (The first
+// starts up to three bytes before the source, in the same aligned word.)
+struct ByteCopy {
+  uint32_t head, words, shift;
+};
+CF1_HD ByteCopy byte_copy(uintptr_t dst, uintptr_t src, uint32_t n) {
+  ByteCopy c;
+  c.head = (4u - (uint32_t)(dst & 3)) & 3;
+  if (c.head > n) c.head = n;
+  const uint32_t into = (uint32_t)(src + c.head) & 3, left = n - c.head, over = into ? 4 - into : 0;
+  c.words = left > over ? (left - over) >> 2 : 0;
+  c.shift = into * 8;
+  return c;
+}
+
 // --------------------------------------------------------- k-mer algebra ----
 // KOps<KeyT> collects what the path needs of Kmer<K> (src/kmer.rs): extraction
 // from the packed sequence, reverse complement (src/kmer.rs:161-200, computed

@@ -162,20 +162,16 @@ __global__ void __launch_bounds__(CL_BLOCK_DEFER) classify_defer_kernel(Classify
   classify_body<KeyT, SIDESET, true>(a);
 }
 
-// n bytes from src to dst by one warp, four bytes a lane: dst is brought to a
-// word boundary first, a word of src is cut from the two aligned words it
-// spans (the second is read only when it holds a byte of the copy).
+// n bytes from src to dst by one warp, four bytes a lane (see ByteCopy).
 CF1_D void warp_copy_bytes(uint8_t *dst, const uint8_t *src, uint32_t n) {
   const unsigned lane = lane_id();
-  uint32_t head = (4u - (uint32_t)(reinterpret_cast<uintptr_t>(dst) & 3)) & 3;
-  if (head > n) head = n;
-  if (lane < head) dst[lane] = src[lane];
-  const uint32_t words = (n - head) >> 2, sh = (uint32_t)(reinterpret_cast<uintptr_t>(src + head) & 3) * 8;
-  uint32_t *d = reinterpret_cast<uint32_t *>(dst + head);
-  const uint32_t *w = reinterpret_cast<const uint32_t *>(src + head - sh / 8);
+  const ByteCopy c = byte_copy(reinterpret_cast<uintptr_t>(dst), reinterpret_cast<uintptr_t>(src), n);
+  if (lane < c.head) dst[lane] = src[lane];
+  uint32_t *d = reinterpret_cast<uint32_t *>(dst + c.head);
+  const uint32_t *w = reinterpret_cast<const uint32_t *>(src + c.head - c.shift / 8);
 #pragma unroll 4
-  for (uint32_t i = lane; i < words; i += 32) d[i] = sh ? __funnelshift_r(w[i], w[i + 1], sh) : w[i];
-  const uint32_t t = head + words * 4 + lane;
+  for (uint32_t i = lane; i < c.words; i += 32) d[i] = c.shift ? __funnelshift_r(w[i], w[i + 1], c.shift) : w[i];
+  const uint32_t t = c.head + c.words * 4 + lane;
   if (t < n) dst[t] = src[t];
 }
 
