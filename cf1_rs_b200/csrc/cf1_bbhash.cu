@@ -47,7 +47,8 @@ __global__ void bb_init_counts_kernel(const uint64_t *seg_off, const uint32_t *s
 constexpr uint32_t BB_GAMMA0 = 8, BB_GAMMA = 8;
 
 // Words of each bin's block at this level (gamma bits per key, at least one
-// word for a non-empty bin) and the level's totals {keys, words}.
+// word for a non-empty bin), the level's totals {keys, words} and the keys of
+// its largest bin.
 __global__ void bb_sizes_kernel(const uint64_t *cnt, uint32_t nbins, uint32_t gamma, uint64_t *wcnt,
                                 unsigned long long *tot) {
   uint32_t b = blockIdx.x * blockDim.x + threadIdx.x;
@@ -57,9 +58,11 @@ __global__ void bb_sizes_kernel(const uint64_t *cnt, uint32_t nbins, uint32_t ga
     words = n ? (gamma * n + 63) / 64 : 0;
     wcnt[b] = words;
   }
+  const uint32_t largest = __reduce_max_sync(FULL, (uint32_t)n);  // (bins hold < 2^32 keys)
   n = warp_sum(n);
   words = warp_sum(words);
   if (lane_id() == 0 && (n | words)) {
+    atomicMax(&tot[2], (unsigned long long)largest);
     atomicAdd(&tot[0], (unsigned long long)n);
     atomicAdd(&tot[1], (unsigned long long)words);
   }
@@ -237,10 +240,13 @@ __global__ void __launch_bounds__(BF_BLOCK) bb_sliced_kernel(const uint64_t *wof
 //
 // Launched once the keys left are few (BF_KEYS a bin on average: a level of
 // that many keys takes the CTA ~15 us, and one launch of its own ~55 us with
-// the wait for its size).  A run's MPHF phase, nine launches and a wait per
-// level before: 30 kb 240 -> 49 us, 200 Mbp 586 -> 87 us.
+// the wait for its size) and no bin has more than four times that, which its
+// CTA would walk alone while the device idles (20 M 63-mers in one of 2048
+// bins: 61 ms, the MPHF phase 0.7 ms with their large levels launched apart).
+// A run's MPHF phase, nine launches and a wait per level before: 30 kb 240 ->
+// 49 us, 200 Mbp 586 -> 87 us.
 constexpr uint32_t BF_WORDS = 4096;
-constexpr uint64_t BF_KEYS = 16384;
+constexpr uint64_t BF_KEYS = 16384, BF_LARGEST = 4 * BF_KEYS;
 // Entries reserved for n keys: the levels' blocks sum up to ~1.14 times the
 // first one's words and a word a level.  Keys that a level's hash crowds
 // together -- thousands of one sub-bucket, which share level 0's top bits --
@@ -426,7 +432,7 @@ void BBHashBuild<KeyT>::begin(uint32_t nb, cudaStream_t s) {
   wcnt_.get<uint64_t>(nbins + 1);
   woff_.get<uint64_t>(nbins + 1);
   tile_off_.get<uint32_t>(nbins + 1);
-  tot_.get<uint64_t>(2);
+  tot_.get<uint64_t>(3);
 }
 
 // Ranks and metadata of a level whose cleaned bits are in place: AR =
@@ -452,7 +458,7 @@ void BBHashBuild<KeyT>::finish_level(uint32_t l, const uint64_t *woff, uint64_t 
 // does not place to r0 / r1 in turn at the same offsets.
 template <class KeyT>
 void BBHashBuild<KeyT>::run_levels(uint32_t l, const KeyT *rem, const uint64_t *start, KeyT *r0, KeyT *r1,
-                                   uint64_t expect, uint32_t *err, cudaStream_t s) {
+                                   uint64_t expect, uint64_t largest, uint32_t *err, cudaStream_t s) {
   KeyT *r[2] = {r0, r1};
   auto tail = [&] {  // all levels from l in one launch
     uint64_t *room = wcnt_.as<uint64_t>(), *off = woff_.as<uint64_t>(), *cur = cnt_[l & 1].as<uint64_t>();
@@ -471,21 +477,21 @@ void BBHashBuild<KeyT>::run_levels(uint32_t l, const KeyT *rem, const uint64_t *
     levels = BB_MAX_LEVELS;  // until collect(): a walk ends at the first level a bin does not have
   };
   tail_from_ = l;
-  if (one_launch && expect <= BF_KEYS * nbins) return tail();
+  if (one_launch && expect <= BF_KEYS * nbins && largest <= BF_LARGEST) return tail();
   uint64_t *wcnt = wcnt_.as<uint64_t>(), *woff = woff_.as<uint64_t>();
   uint32_t *tile_off = tile_off_.as<uint32_t>();
   unsigned long long *tot = reinterpret_cast<unsigned long long *>(tot_.as<uint64_t>());
   for (;; l++) {
     uint64_t *cur = cnt_[l & 1].as<uint64_t>(), *nxt_cnt = cnt_[(l + 1) & 1].as<uint64_t>();
-    CF1_CUDA(cudaMemsetAsync(tot, 0, 2 * sizeof(unsigned long long), s));
+    CF1_CUDA(cudaMemsetAsync(tot, 0, 3 * sizeof(unsigned long long), s));
     bb_sizes_kernel<<<(unsigned)ceil_div(nbins, 256), 256, 0, s>>>(cur, nbins, l ? BB_GAMMA : BB_GAMMA0, wcnt, tot);
     CF1_LAUNCH_CHECK();
-    uint64_t ht[2] = {0, 0};
+    uint64_t ht[3] = {0, 0, 0};
     CF1_CUDA(cudaMemcpyAsync(ht, tot, sizeof(ht), cudaMemcpyDeviceToHost, s));
     CF1_CUDA(cudaStreamSynchronize(s));
     const uint64_t remaining = ht[0], nw = ht[1];
     if (remaining == 0) break;
-    if (one_launch && remaining <= BF_KEYS * nbins) {
+    if (one_launch && remaining <= BF_KEYS * nbins && ht[2] <= BF_LARGEST) {
       reserve_entries(total_words + bf_room(remaining) + nbins * (bf_room(1) + 1), total_words, s);
       tail_from_ = l;
       return tail();
@@ -540,9 +546,10 @@ void BBHashBuild<KeyT>::build(const KeyT *keys, const uint64_t *seg_off, uint32_
   std::vector<uint64_t> hoff(nbins + 1);
   CF1_CUDA(cudaMemcpyAsync(hoff.data(), seg_off, (nbins + 1) * sizeof(uint64_t), cudaMemcpyDeviceToHost, s));
   CF1_CUDA(cudaStreamSynchronize(s));
-  for (uint32_t b = 0; b < nbins; b++)  // local slots are 32-bit
-    if (hoff[b + 1] - hoff[b] >= (1ull << 32))
-      throw Error(CF1GPU_ERR_INVALID_ARG, "BBHash: a bin holds 2^32 or more distinct keys; use more bins");
+  uint64_t largest = 0;
+  for (uint32_t b = 0; b < nbins; b++) largest = std::max(largest, hoff[b + 1] - hoff[b]);
+  if (largest >= (1ull << 32))  // local slots are 32-bit
+    throw Error(CF1GPU_ERR_INVALID_ARG, "BBHash: a bin holds 2^32 or more distinct keys; use more bins");
   const uint64_t n_all = hoff[nbins];
   // Keys of bin b at every level sit at [seg_off[b], seg_off[b] + cnt[b]) of
   // the level's key array: the distinct keys at level 0, then the two
@@ -554,7 +561,7 @@ void BBHashBuild<KeyT>::build(const KeyT *keys, const uint64_t *seg_off, uint32_
   // room for the usual level sizes (gamma0 bits per key, then ~12% and
   // fewer keys per level) so that the entry array rarely grows in mid-build
   reserve_entries((BB_GAMMA0 * n_all / 64 + nbins) * 3 / 2 + 64 * nbins + 64, 0, s);
-  run_levels(0, keys, seg_off, r0, r1, n_all, err, s);
+  run_levels(0, keys, seg_off, r0, r1, n_all, largest, err, s);
 }
 
 template <class KeyT>
@@ -571,7 +578,7 @@ void BBHashBuild<KeyT>::build_from_levels01(uint32_t nb, int P, const uint64_t *
                                             const uint32_t *placed0, const uint64_t *woff1, uint64_t words1,
                                             const uint32_t *placed1, const KeyT *surv, const uint64_t *surv_off,
                                             const uint64_t *surv_cnt, uint64_t surv_total, uint64_t n_occ,
-                                            uint32_t *err, cudaStream_t s, KeyT *ws0, KeyT *ws1, uint64_t ws_cap) {
+                                            uint64_t max_bin, uint32_t *err, cudaStream_t s, KeyT *ws0, KeyT *ws1, uint64_t ws_cap) {
   begin(nb, s);
   const uint64_t nsl = ((uint64_t)nbins << P) + 1;
   bb_sliced_kernel<<<nbins, BF_BLOCK, 0, s>>>(woff0, woff1, P, words0, placed0, placed1, srank_[0].get<uint32_t>(nsl),
@@ -585,7 +592,7 @@ void BBHashBuild<KeyT>::build_from_levels01(uint32_t nb, int P, const uint64_t *
   KeyT *r0 = (ws0 && ws_cap >= surv_total + 1) ? ws0 : rem_[0].get<KeyT>(surv_total + 1);
   KeyT *r1 = (ws1 && ws_cap >= surv_total + 1) ? ws1 : rem_[1].get<KeyT>(surv_total + 1);
   // level l reads cnt_[l & 1] and writes r[l & 1]; level 1 leaves ~1% of the keys
-  run_levels(2, surv, surv_off, r0, r1, n_occ / 100, err, s);
+  run_levels(2, surv, surv_off, r0, r1, n_occ / 100, max_bin / 100, err, s);
   levels = std::max<uint32_t>(levels, 2);
   set_bytes();
 }

@@ -36,12 +36,12 @@ struct BBHashBuild {
   // sub-bucket) and builds the later levels over the keys level 1 left (bin
   // b's at surv[surv_off[b] + [0, surv_cnt[b])]).  woff0 / woff1: the bins'
   // block offsets [nbins + 1] of levels 0 and 1; P: the slice bits; n_occ: the
-  // k-mer occurrences.
+  // k-mer occurrences, max_bin: those of the largest bin.
   ulonglong2 *prepare_levels01(uint32_t nbins, uint64_t words0, uint64_t words1, cudaStream_t s);
   void build_from_levels01(uint32_t nbins, int P, const uint64_t *woff0, uint64_t words0, const uint32_t *placed0,
                            const uint64_t *woff1, uint64_t words1, const uint32_t *placed1, const KeyT *surv,
                            const uint64_t *surv_off, const uint64_t *surv_cnt, uint64_t surv_total, uint64_t n_occ,
-                           uint32_t *err, cudaStream_t s, KeyT *ws0 = nullptr, KeyT *ws1 = nullptr, uint64_t ws_cap = 0);
+                           uint64_t max_bin, uint32_t *err, cudaStream_t s, KeyT *ws0 = nullptr, KeyT *ws1 = nullptr, uint64_t ws_cap = 0);
   void collect_begin(uint64_t *got, cudaStream_t s);  // got: two words of page-locked memory
   void collect_end(const uint64_t *got);
   BBView view() const;
@@ -57,9 +57,9 @@ struct BBHashBuild {
   void reserve_entries(uint64_t words, uint64_t keep, cudaStream_t s);
   void begin(uint32_t nbins, cudaStream_t s);
   void finish_level(uint32_t l, const uint64_t *woff, uint64_t nw, cudaStream_t s);
-  // expect: about how many keys level l has
+  // expect: about how many keys level l has, largest: in its largest bin
   void run_levels(uint32_t l, const KeyT *rem, const uint64_t *start, KeyT *r0, KeyT *r1, uint64_t expect,
-                  uint32_t *err, cudaStream_t s);
+                  uint64_t largest, uint32_t *err, cudaStream_t s);
   void set_bytes();
 
   // The entry array and the level buffers are kept across builds and grown on

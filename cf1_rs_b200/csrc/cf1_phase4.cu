@@ -435,10 +435,10 @@ void launch_place_l0(const BBView &bb, const uint64_t *dist_off, const uint64_t 
 
 void launch_place_surv(const BBView &bb, const uint64_t *dist_off, const uint64_t *surv, const uint8_t *surv_pay,
                        const uint64_t *surv_off, const unsigned long long *surv_cnt, uint32_t b0, uint32_t b1,
-                       uint64_t n_occ, uint32_t nbins, uint8_t *sides, uint32_t *err, cudaStream_t s) {
+                       uint64_t max_bin, uint8_t *sides, uint32_t *err, cudaStream_t s) {
   if (b1 <= b0) return;
-  // level 1 leaves ~1% of the occurrences: one key a thread
-  const uint32_t parts = (uint32_t)std::min<uint64_t>(SV_CTAS, n_occ / 100 / nbins / 256 + 1);
+  // level 1 leaves ~1% of the occurrences: one key a thread in the largest bin
+  const uint32_t parts = (uint32_t)std::min<uint64_t>(SV_CTAS, max_bin / 100 / 256 + 1);
   place_surv_kernel<<<(b1 - b0) * parts, 256, 0, s>>>(bb, dist_off, surv, surv_pay, surv_off, surv_cnt, b0, parts,
                                                       sides, err);
   CF1_LAUNCH_CHECK();

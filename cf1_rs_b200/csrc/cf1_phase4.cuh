@@ -43,13 +43,13 @@ void launch_place_sides(const MphfView<KeyT> &m, const KeyT *kept, const KeyT *d
 // level 1's ucnt1[j]) -- two contiguous copies each; the keys level 1 left
 // (bin b's at surv[surv_off[b] ...], surv_cnt[b] of them, bytes beside them)
 // walk the levels from 2.  Units [j0, j1) of 2^PU per bin, slices of 2^P per
-// bin; bins [b0, b1); n_occ: the k-mer occurrences of the nbins bins.
+// bin; bins [b0, b1); max_bin: the k-mer occurrences of the largest bin.
 void launch_place_l0(const BBView &bb, const uint64_t *dist_off, const uint64_t *uoff, const uint32_t *ucnt0,
                      const uint32_t *ucnt1, const uint8_t *l0pay, uint64_t j0, uint64_t j1, int PU, int P,
                      uint8_t *sides, uint32_t *err, cudaStream_t s);
 void launch_place_surv(const BBView &bb, const uint64_t *dist_off, const uint64_t *surv, const uint8_t *surv_pay,
                        const uint64_t *surv_off, const unsigned long long *surv_cnt, uint32_t b0, uint32_t b1,
-                       uint64_t n_occ, uint32_t nbins, uint8_t *sides, uint32_t *err, cudaStream_t s);
+                       uint64_t max_bin, uint8_t *sides, uint32_t *err, cudaStream_t s);
 
 // Packs side-set bytes (3 u32 per state word) into state words [w0, w1).
 void launch_sideset_pack(const uint32_t *sides, uint64_t w0, uint64_t w1, unsigned long long *states,

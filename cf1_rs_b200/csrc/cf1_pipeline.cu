@@ -672,7 +672,7 @@ void run_impl(cf1gpu_ctx *c, StreamIO *io = nullptr, Step step = Step::FULL, con
   } else if (l0_ready) {
     be.bb.build_from_levels01(B, P, l0.woff, l0_words, l0.placed, l0.woff1, l1_words, l0.placed1,
                               reinterpret_cast<const KeyT *>(l0.surv), l0.surv_off,
-                              reinterpret_cast<const uint64_t *>(l0.surv_cnt), l0_room, NO, &sm->err, s, twin, twin + half,
+                              reinterpret_cast<const uint64_t *>(l0.surv_cnt), l0_room, NO, max_bin, &sm->err, s, twin, twin + half,
                               half);
   } else {
     be.bb.build(dist, dist_off, B, nullptr, &sm->err, s, keys, ws1, NO + 1);
@@ -703,7 +703,7 @@ void run_impl(cf1gpu_ctx *c, StreamIO *io = nullptr, Step step = Step::FULL, con
                       PU == P ? l0.placed1 : l0.uplaced1, l0pay, (uint64_t)b0 << PU, (uint64_t)b1 << PU, PU, P, sb,
                       &sm->err, s);
       launch_place_surv(be.bb.view(), dist_off, reinterpret_cast<const uint64_t *>(l0.surv), l0.surv_pay, l0.surv_off,
-                        l0.surv_cnt, b0, b1, NO, B, sb, &sm->err, s);
+                        l0.surv_cnt, b0, b1, max_bin, sb, &sm->err, s);
     } else {
       launch_place_sides<KeyT>(make_view<KeyT>(c), kept, c->dist_pending ? nullptr : c->d_dist.as<const KeyT>(),
                                kept_pay, sbo, be.msd.cnt.template as<const uint32_t>(),
