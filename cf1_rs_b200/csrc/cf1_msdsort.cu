@@ -14,6 +14,7 @@
 //      array; a bin's first sub-bucket gives its slot offset.
 // A sub-bucket above CAP keys (long homopolymers, huge tandem arrays) makes
 // the caller fall back to the LSD path (cf1_phase3_sort.cu) for the run.
+#include <cmath>
 #include <cstddef>
 
 #include "cf1_device_util.cuh"
@@ -1538,6 +1539,54 @@ __global__ void __launch_bounds__(GdCfg<BITS>::BLOCK, BITS == 5 ? 2 : 4)
   }
 }
 
+// Group bits of a split of P bits: groups of 16 while the split has at most
+// GD_SPLIT bits then, else of 32; the whole bin where 32 hold it.
+int gd_group_bits(int P) { return P <= GD_BITS ? P : P - 4 <= GD_SPLIT ? 4 : GD_BITS; }
+
+// ---------------------------------------------------------------- repeats
+// How much of the input repeats, for the group dedup's list: it has room for
+// 72% (69%) of a group's occurrences, and copies of a key always share their
+// bit, so groups near their capacity overflow it when most keys occur twice or
+// more (reads at any coverage, assemblies of one species).  One to four bins,
+// evenly spaced: their keys in one 64th of the hash range mark a bitmap of 8
+// bits an occurrence -- level 0's own density -- in global memory.  got: the
+// keys marked, the bits set, the keys that share their bit.
+constexpr uint32_t RP_CTAS = 512;  // of all bins
+constexpr int RP_BITS = 6, RP_BLOCK = 512;
+constexpr uint64_t RP_RANGE = 37;  // any of the 64
+// Occurrences from which a look is taken: it costs ~10 us, and below that a run
+// with most of its groups left to the block kernel takes under a millisecond.
+constexpr uint64_t RP_MIN = 8u << 20;
+CF1_HD uint32_t rp_bins(uint32_t nbins) { return nbins < 32 ? 1 : nbins < 64 ? 2 : 4; }  // at most 1/16 of the keys
+CF1_HD uint64_t rp_words(uint64_t occ) { return (occ >> (RP_BITS + 2)) + 1; }  // u32 words of occ keys' bits
+__global__ void __launch_bounds__(RP_BLOCK) rp_sample_kernel(const uint64_t *keys, const uint64_t *seg_off, uint32_t nbins,
+                                                            uint32_t *set, uint32_t *col, unsigned long long *got) {
+  const uint32_t nb = rp_bins(nbins), per = RP_CTAS / nb, i = blockIdx.x / per, part = blockIdx.x % per;
+  const uint32_t bin = (uint32_t)((2ull * i + 1) * nbins / (2 * nb));
+  const uint64_t a = seg_off[bin], e = seg_off[bin + 1];
+  const uint32_t words = (uint32_t)((e - a) >> (RP_BITS + 2));
+  if (!words) return;
+  uint32_t *s = set + (a >> (RP_BITS + 2)), *c = col + (a >> (RP_BITS + 2));
+  uint32_t n = 0, bits = 0, shared = 0;
+#pragma unroll 8
+  for (uint64_t j = a + part * RP_BLOCK + threadIdx.x; j < e; j += per * RP_BLOCK) {
+    const uint64_t h = keys[j] * MS_HASH_MUL;
+    if (h >> (64 - RP_BITS) != RP_RANGE) continue;
+    const uint32_t b = (uint32_t)(((h << RP_BITS >> 32) * (uint64_t)words) >> 27), bm = 1u << (b & 31);
+    n++;
+    if (!(atomicOr(&s[b >> 5], bm) & bm)) bits++;
+    else shared += atomicOr(&c[b >> 5], bm) & bm ? 1 : 2;
+  }
+  n = warp_sum(n);
+  bits = warp_sum(bits);
+  shared = warp_sum(shared);
+  if (lane_id() == 0 && n) {
+    atomicAdd(&got[0], (unsigned long long)n);
+    atomicAdd(&got[1], (unsigned long long)bits);
+    atomicAdd(&got[2], (unsigned long long)shared);
+  }
+}
+
 // Groups the dedup left: one CTA per listed group moves its keys (unpacked)
 // and bytes from T / TP to the same range of U / UP, sub-bucket by
 // sub-bucket, and writes the sub-buckets' offsets and list entries for the
@@ -2105,11 +2154,33 @@ int msd_prefix_bits(uint64_t max_bin_keys, bool sorted) {
   return p;
 }
 
+void msd_look_for_repeats(const uint64_t *keys, uint64_t n, const uint64_t *seg_off, uint32_t nbins, MsdScratch &sc,
+                          MsdRead &rd, cudaStream_t s) {
+  rd.repeats[0] = 0;
+  // (bins past the widest split, on average, go without the group dedup anyway)
+  if (n < RP_MIN || n / nbins > ((uint64_t)(GD_MAXSUB + 1) << MSD_MAX_BITS)) return;
+  const uint64_t words = rp_words(n);
+  uint32_t *set = sc.hist.get<uint32_t>(2 * words + 8);  // free until the split
+  unsigned long long *got = reinterpret_cast<unsigned long long *>(set);
+  CF1_CUDA(cudaMemsetAsync(set, 0, (2 * words + 8) * sizeof(uint32_t), s));
+  rp_sample_kernel<<<RP_CTAS, RP_BLOCK, 0, s>>>(keys, seg_off, nbins, set + 8, set + 8 + words, got);
+  CF1_LAUNCH_CHECK();
+  CF1_CUDA(cudaMemcpyAsync(rd.repeats, got, sizeof(rd.repeats), cudaMemcpyDeviceToHost, s));
+}
+
+bool msd_lists_overflow(uint64_t max_bin, int P, const MsdRead &rd) {
+  if (!rd.repeats[0]) return false;
+  const int g = gd_group_bits(P);
+  const double keys = (double)rd.repeats[0], copies = keys / (double)rd.repeats[1];
+  const double list = (double)rd.repeats[2] / keys * std::ldexp((double)max_bin, g - P);
+  return list + 1.5 * std::sqrt(list * copies) > (g <= 4 ? GdCfg<4>::MAXL : GdCfg<5>::MAXL);
+}
+
 template <class KeyT>
 bool msd_sort_unique(KeyT *keys, KeyT *alt, uint64_t n, uint64_t max_bin, const uint64_t *seg_off, uint32_t nbins,
                      int key_bits, int P, KeyT *dist, uint64_t *dist_off, MsdScratch &sc, MsdRead &rd,
                      cudaStream_t s, bool sorted, const Level0Out *l0, KeyT **kept, uint8_t *pkeys, uint8_t *palt, uint8_t **kept_pay,
-                     uint8_t **l0pay_buf) {
+                     uint8_t **l0pay_buf, bool groups) {
   uint8_t *PT = pkeys;  // payloads beside T (nullptr: keys carry none)
   // passes on the top P bits: P1 then P2 (P2 may be 0) -- of the key, or of
   // its hash when only distinct keys are wanted (64-bit keys)
@@ -2126,8 +2197,8 @@ bool msd_sort_unique(KeyT *keys, KeyT *alt, uint64_t n, uint64_t max_bin, const 
   // (At the widest split, bins of 12.6 to 14.7 M keys, up to 224: 32 of them
   // are 7168 of a group's 8192.  3.1 Gbp in 256 bins: 127 ms a run with the
   // warp sets, 106 with groups.)
-  const bool grp = W1 && hashed && (max_bin >> P) <= (P == MSD_MAX_BITS ? GD_MAXSUB : WD_MAXD / 2);
-  const int g = !grp ? 0 : P <= GD_BITS ? P : P - 4 <= GD_SPLIT ? 4 : GD_BITS;
+  const bool grp = W1 && hashed && groups && (max_bin >> P) <= (P == MSD_MAX_BITS ? GD_MAXSUB : WD_MAXD / 2);
+  const int g = grp ? gd_group_bits(P) : 0;
   const int PS = P - g;  // bits split on: a unit is a group, or a sub-bucket
   sc.unit_bits = PS;
   sc.kept_bits = false;
@@ -2335,7 +2406,7 @@ bool msd_sort_unique(KeyT *keys, KeyT *alt, uint64_t n, uint64_t max_bin, const 
   template int msd_prefix_bits<KT>(uint64_t, bool);                                                                     \
   template bool msd_sort_unique<KT>(KT *, KT *, uint64_t, uint64_t, const uint64_t *, uint32_t, int, int, KT *,   \
                                     uint64_t *, MsdScratch &, MsdRead &, cudaStream_t, bool, const Level0Out *, KT **, uint8_t *, \
-                                    uint8_t *, uint8_t **, uint8_t **);                                       \
+                                    uint8_t *, uint8_t **, uint8_t **, bool);                                 \
   template void msd_compact<KT>(const KT *, uint64_t, KT *, MsdScratch &, cudaStream_t);
 CF1_INST(uint64_t)
 CF1_INST(Key2)

@@ -9,6 +9,7 @@ namespace cf1 {
 // caller's.
 struct MsdRead {
   uint64_t n_distinct, runs;
+  uint64_t repeats[3];  // msd_look_for_repeats: keys looked at, bits they set, keys that share theirs
   uint32_t overflow;  // units (unsorted) or runs (sorted) left to the block kernel
   uint32_t oversize;  // a sub-bucket fits nowhere
   uint32_t l0_err;    // Level0Out::err
@@ -87,6 +88,14 @@ struct Level0Out {
   uint32_t *uplaced = nullptr, *uplaced1 = nullptr;  // [units]
 };
 
+// How much the keys of the unsorted 64-bit form repeat, from a few bins, to
+// rd.repeats by the stream's next wait (repeats[0] = 0: not looked at), and whether the group dedup's lists then overflow on a split of P
+// bits: mean and 1.5 standard deviations of the largest bin's lists, the keys'
+// copies coming together.
+void msd_look_for_repeats(const uint64_t *keys, uint64_t n, const uint64_t *seg_off, uint32_t nbins, MsdScratch &sc,
+                          MsdRead &rd, cudaStream_t s);
+bool msd_lists_overflow(uint64_t max_bin, int P, const MsdRead &rd);
+
 // max_bin: the keys of the largest bin.
 // With dist = nullptr the distinct keys stay where the dedup left them, at
 // the start of each unit's range of *kept (keys or alt), and
@@ -94,12 +103,13 @@ struct Level0Out {
 // With pkeys/palt (one side-set code per key, beside keys and alt), each
 // distinct key leaves with the OR of its copies' side-set bytes at the same place
 // of *kept_pay (pkeys or palt, beside *kept); the group dedup leaves no bytes
-// there (*kept_pay = nullptr: they went to l0's outputs).
+// there (*kept_pay = nullptr: they went to l0's outputs).  groups = false:
+// the unsorted 64-bit form goes without the group dedup.
 template <class KeyT>
 bool msd_sort_unique(KeyT *keys, KeyT *alt, uint64_t n, uint64_t max_bin, const uint64_t *seg_off, uint32_t nbins,
                      int key_bits, int P, KeyT *dist, uint64_t *dist_off, MsdScratch &sc, MsdRead &rd,
                      cudaStream_t s, bool sorted = true, const Level0Out *l0 = nullptr, KeyT **kept = nullptr, uint8_t *pkeys = nullptr,
-                     uint8_t *palt = nullptr, uint8_t **kept_pay = nullptr, uint8_t **l0pay_buf = nullptr);
+                     uint8_t *palt = nullptr, uint8_t **kept_pay = nullptr, uint8_t **l0pay_buf = nullptr, bool groups = true);
 
 // The deferred copy: distinct keys of the last msd_sort_unique (nunit
 // units, left in `kept`) to dist, bins in order.

@@ -526,12 +526,25 @@ void run_impl(cf1gpu_ctx *c, StreamIO *io = nullptr, Step step = Step::FULL, con
   auto dist_buf = [&]() { return c->d_dist.get<KeyT>(NO + 1); };
   uint64_t *dist_off = c->d_dist_off.get<uint64_t>(B + 1);
   const uint64_t *hseg = rb->bins[0];
+  const bool grouped = !sorted && !c->wide && c->opts.mphf_mode == CF1GPU_MPHF_BBHASH;
+  if constexpr (KOps<KeyT>::WORDS == 1)
+    if (grouped) msd_look_for_repeats(keys, NO, seg, B, be.msd, rb->msd, s);
   CF1_CUDA(cudaMemcpyAsync(rb->bins[0], seg, (B + 1) * sizeof(uint64_t), cudaMemcpyDeviceToHost, s));
   CF1_CUDA(cudaStreamSynchronize(s));
   uint64_t max_bin = 0;
   for (uint32_t b = 0; b < B; b++) max_bin = std::max(max_bin, hseg[b + 1] - hseg[b]);
   KeyT *alt = be.sort.alt.template get<KeyT>(NO + 1);
-  const int P0 = c->force_lsd ? -1 : msd_prefix_bits<KeyT>(max_bin, sorted);
+  int P0 = c->force_lsd ? -1 : msd_prefix_bits<KeyT>(max_bin, sorted);
+  // Repeated sequence that would overflow the group dedup's lists: one split
+  // bit more, so groups of half the size, and the warp sets where the split is
+  // at its widest.  (98 Mb of 64 bins, every key 2 / 8 / 30 times: 11.1 / 9.2 /
+  // 8.9 ms with most groups left to the block kernel, 4.3 / 3.7 / 3.4 on one bit
+  // more; sequence that does not repeat loses by it, 2.97 against 3.35.)
+  bool groups = true;
+  if (grouped && P0 >= 0 && msd_lists_overflow(max_bin, P0, rb->msd)) {
+    if (P0 < 16) P0++;
+    else groups = false;
+  }
   auto msd_width = [&](int delta) { return P0 < 0 ? -1 : std::min(16, std::max(0, P0 + delta)); };
   auto expand_again = [&]() {
     launch_expand<KeyT>(records, NS, kpre, W, k, keys, NO, L, batched ? &sm->queues[4] : nullptr, &sm->err, pctas, s,
@@ -551,7 +564,7 @@ void run_impl(cf1gpu_ctx *c, StreamIO *io = nullptr, Step step = Step::FULL, con
       if (batched) CF1_CUDA(cudaMemsetAsync(&sm->queues[4], 0, sizeof(uint32_t), s));
       CF1_CUDA(cudaEventRecord(c->ev[10], s));
       const bool ok = msd_sort_unique<KeyT>(keys, alt, NO, max_bin, seg, B, 2 * k, P, dist_buf(), dist_off, be.msd, rb->msd,
-                                            s, sorted, nullptr, nullptr, pay, pay_alt);
+                                            s, sorted, nullptr, nullptr, pay, pay_alt, nullptr, nullptr, groups);
       CF1_CUDA(cudaEventRecord(c->ev[11], s));
       CF1_CUDA(cudaEventSynchronize(c->ev[11]));
       const double ms = elapsed(c->ev[10], c->ev[11]);
@@ -622,7 +635,7 @@ void run_impl(cf1gpu_ctx *c, StreamIO *io = nullptr, Step step = Step::FULL, con
   uint8_t *kept_pay = nullptr, *l0pay = nullptr;
   bool done = P >= 0 && msd_sort_unique<KeyT>(keys, alt, NO, max_bin, seg, B, 2 * k, P, l0_fuse ? nullptr : dist_buf(),
                                               dist_off, be.msd, rb->msd, s, sorted, l0_fuse ? &l0 : nullptr, &kept, pay, pay_alt,
-                                              &kept_pay, &l0pay);
+                                              &kept_pay, &l0pay, groups);
   c->msd_bits = done ? P : -1;
   if (tune_now) {
     tuned.sk_tile = c->tune.sk_tile;
