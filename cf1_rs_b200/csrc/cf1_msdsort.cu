@@ -579,17 +579,15 @@ CF1_D void l0_slice(const uint64_t *keys, uint32_t n, uint64_t j, int P, const L
 // makes the kernel report the sub-bucket as oversized.
 // With TP/UP (payload bytes parallel to T and U), every distinct key leaves
 // with the OR of its copies' payloads beside it in TP.
-// Chunks (sorted form): with clist, CTA c takes the run of consecutive
-// sub-buckets [j0, j1) of one bin that the plan packed together (coff: the
-// plan's chunks per bin, scanned), sorts the run as one range -- its bucket is
-// the sub-bucket's place in the run, then the next key bits -- and credits
-// all its distinct keys to sub-bucket j0.
+// Runs (sorted form): with runs, CTA c takes the consecutive sub-buckets
+// [j0, j1) of one bin that the plan packed together, sorts the run as one
+// range -- its bucket is the sub-bucket's place in the run, then the next key
+// bits -- and credits all its distinct keys to sub-bucket j0.
 template <class KeyT, bool SORTED>
 __global__ void __launch_bounds__(CS_BLOCK, SORTED ? 2 : 4) cs_sort_unique_kernel(KeyT *T, KeyT *U, const uint64_t *sb_off,
                                                                   uint64_t nsub, int shift, int bits, uint32_t *cnt,
                                                                   uint32_t *oversize, int P, Level0Out l0,
-                                                                  uint8_t *TP, uint8_t *UP, const uint2 *clist,
-                                                                  const uint64_t *coff, uint32_t nbins,
+                                                                  uint8_t *TP, uint8_t *UP, const uint2 *runs,
                                                                   const uint32_t *jlist, const uint32_t *klist,
                                                                   bool codes) {
   constexpr uint32_t CAP = cs_cap<KeyT, SORTED>();
@@ -610,11 +608,9 @@ __global__ void __launch_bounds__(CS_BLOCK, SORTED ? 2 : 4) cs_sort_unique_kerne
   if (jlist) {  // the sub-buckets the warp dedup left
     j = jlist[blockIdx.x];
     jend = j + 1;
-  } else if (clist) {
-    const uint32_t bin = upper_segment(coff, nbins, (uint64_t)run);
-    const uint2 r = clist[((uint64_t)bin << P) + (run - coff[bin])];
-    j = ((uint64_t)bin << P) + r.x;
-    jend = ((uint64_t)bin << P) + r.y;
+  } else if (runs) {
+    j = runs[run].x;
+    jend = runs[run].y;
   }
   if (j >= nsub) return;
   const uint64_t a = sb_off[j], n = sb_off[jend] - a;
@@ -799,18 +795,15 @@ static_assert(offsetof(SrSmem<uint64_t>, stagep) % 4 == 0 && offsetof(SrSmem<Key
 template <class KeyT, bool HASHED>
 __global__ void __launch_bounds__(SR_BLOCK, 2) sr_dedup_kernel(KeyT *T, uint8_t *TP, const uint64_t *sb_off,
                                                               uint64_t nsub, int P, int rest, uint32_t *cnt,
-                                                              const uint2 *clist, const uint64_t *coff, uint32_t nbins,
-                                                              uint32_t *ov, uint32_t *ov_cnt) {
+                                                              const uint2 *runs, uint32_t *ov, uint32_t *ov_cnt) {
   using C = SrCfg<KeyT>;
   extern __shared__ __align__(16) unsigned char sr_smem[];
   SrSmem<KeyT> &m = *reinterpret_cast<SrSmem<KeyT> *>(sr_smem);
   const unsigned tid = threadIdx.x;
   uint64_t j = blockIdx.x, jend = j + 1;
-  if (clist) {
-    const uint32_t bin = upper_segment(coff, nbins, (uint64_t)blockIdx.x);
-    const uint2 r = clist[((uint64_t)bin << P) + (blockIdx.x - coff[bin])];
-    j = ((uint64_t)bin << P) + r.x;
-    jend = ((uint64_t)bin << P) + r.y;
+  if (runs) {
+    j = runs[blockIdx.x].x;
+    jend = runs[blockIdx.x].y;
   }
   if (j >= nsub) return;
   const uint64_t a = sb_off[j], n64 = sb_off[jend] - a;
@@ -2018,40 +2011,38 @@ __global__ void wd_unpack_kernel(uint64_t *T, uint8_t *TP, const uint64_t *sb_of
   }
 }
 
-// Chunk plan of the sorted form: per bin, runs of consecutive
-// sub-buckets packed greedily up to cap keys and at most CS_BUCKETS
-// sub-buckets (the run's counting sort buckets a key by its sub-bucket's
-// place in the run first; sparse stretches of the key space -- canonical
-// k-mers starting with TTT... -- hold thousands of near-empty sub-buckets at
-// wide splits), a sub-bucket above cap keys being a run of its own, written as
-// (first, end) sub-bucket indices within the bin to clist[bin << P ...];
-// ccount[bin] = the bin's runs.
-// One warp per bin walks its runs one after another: the end of a run is the
-// last sub-bucket whose offset is within cap of the run's start, found by a
-// 32-way search of the offsets (in shared memory, relative to the bin's
-// start, when they fit).  A thread per bin stepping through the sub-buckets
-// took 0.41 ms for 128 bins of 2048.
-constexpr uint32_t CP_MAX = 8192;  // offsets kept in shared memory
+// Run plan of the sorted form: runs of consecutive sub-buckets packed
+// greedily up to cap keys, a sub-bucket above cap keys being a run of its own.
+// Stretches of up to 1024 sub-buckets (2^CP_BITS) of a bin are planned apart,
+// which also keeps a run to the CS_BUCKETS sub-buckets its counting sort tells
+// apart (sparse ranges of the key space -- canonical k-mers starting with
+// TTT... -- hold thousands of near-empty ones at wide splits).  The runs of
+// stretch q go to clist[q << bits ...] as first | end << 16, sub-buckets
+// within the stretch; ccount[q] = how many.
+// One warp per stretch walks its runs one after another: the end of a run is
+// the last sub-bucket whose offset is within cap of the run's start, found by
+// a 32-way search of the offsets (in shared memory, relative to the stretch's
+// start).  Whole bins a warp left the device idle where bins are few: 200 Mbp
+// in one bin, 2^16 sub-buckets, 17 ms.
+constexpr int CP_BITS = 10;
+static_assert(1u << CP_BITS <= CS_BUCKETS);
 constexpr int CP_BLOCK = 256;
-__global__ void __launch_bounds__(CP_BLOCK) cs_plan_kernel(const uint64_t *sb_off, uint32_t nbins, int P, uint32_t cap,
-                                                          uint2 *clist, uint32_t *ccount) {
-  __shared__ uint32_t s_off[CP_MAX + 1];
-  const uint32_t b = blockIdx.x, per = 1u << P;
-  const uint64_t *o = sb_off + ((uint64_t)b << P);
-  const uint64_t o0 = o[0];
-  const bool local = per <= CP_MAX && o[per] - o0 < (1ull << 32);
-  if (local)
-    for (uint32_t q = threadIdx.x; q <= per; q += CP_BLOCK) s_off[q] = (uint32_t)(o[q] - o0);
+__global__ void __launch_bounds__(CP_BLOCK) cs_plan_kernel(const uint64_t *sb_off, int bits, uint32_t cap, uint32_t *clist,
+                                                          uint32_t *ccount) {
+  __shared__ uint64_t s_off[(1u << CP_BITS) + 1];
+  const uint32_t b = blockIdx.x, per = 1u << bits;
+  const uint64_t *o = sb_off + ((uint64_t)b << bits);
+  for (uint32_t q = threadIdx.x; q <= per; q += CP_BLOCK) s_off[q] = o[q];
   __syncthreads();
   if (threadIdx.x >= 32) return;
-  auto at = [&](uint32_t q) -> uint64_t { return local ? (uint64_t)s_off[q] : o[q] - o0; };
+  auto at = [&](uint32_t q) -> uint64_t { return s_off[q]; };
   const unsigned lane = lane_id();
-  uint2 *out = clist + ((uint64_t)b << P);
+  uint32_t *out = clist + ((uint64_t)b << bits);
   uint32_t nc = 0, start = 0;
   while (start < per) {
     // the largest end in (start, lim] with at(end) <= at(start) + cap; start + 1 at least
     const uint64_t top = at(start) + cap;
-    uint32_t lo = start + 1, lim = min(per, start + CS_BUCKETS);  // at(lo) <= top or lo = start + 1
+    uint32_t lo = start + 1, lim = per;  // at(lo) <= top or lo = start + 1
     while (lo < lim) {
       const uint32_t step = (lim - lo + 31) / 32;
       const uint32_t q = lo + (lane + 1) * step;
@@ -2061,12 +2052,27 @@ __global__ void __launch_bounds__(CP_BLOCK) cs_plan_kernel(const uint64_t *sb_of
       lim = min(lim, lo + (c + 1) * step - 1);
       lo = next;
     }
-    if (lane == 0) out[nc] = make_uint2(start, lo);
+    if (lane == 0) out[nc] = start | lo << 16;
     nc++;
     start = lo;
   }
   if (lane == 0) ccount[b] = nc;
 }
+
+// The stretches' runs one after another, as sub-buckets [x, y): one warp per
+// stretch.
+__global__ void __launch_bounds__(CP_BLOCK) cs_runs_kernel(const uint32_t *clist, const uint64_t *coff, uint32_t nstretch,
+                                                          int bits, uint2 *runs) {
+  const uint32_t b = (blockIdx.x * CP_BLOCK + threadIdx.x) >> 5;
+  if (b >= nstretch) return;
+  const uint64_t o = coff[b];
+  const uint32_t n = (uint32_t)(coff[b + 1] - o), j0 = b << bits;  // (MAX_BINS << MSD_MAX_BITS sub-buckets fit)
+  for (uint32_t r = lane_id(); r < n; r += 32) {
+    const uint32_t x = clist[j0 + r];
+    runs[o + r] = make_uint2(j0 + (x & 0xFFFFu), j0 + (x >> 16));
+  }
+}
+static_assert((uint64_t)MAX_BINS << MSD_MAX_BITS <= 1ull << 28);
 
 // One warp per sub-bucket: copy its distinct keys to the dense array.
 template <class KeyT>
@@ -2280,25 +2286,27 @@ bool msd_sort_unique(KeyT *keys, KeyT *alt, uint64_t n, uint64_t max_bin, const 
     // sorted form (and 128-bit keys): consecutive small sub-buckets of a bin are packed into
     // one CTA's run (the top bits of canonical k-mers are skewed, so most
     // sub-buckets are far below the capacity the largest ones need)
-    const uint2 *clist = nullptr;
-    const uint64_t *coff = nullptr;
+    uint2 *runs = nullptr;
     uint64_t grid = nsub;
     if ((sorted || !W1) && P > 0) {
-      uint2 *cl = sc.clist.get<uint2>(nsub);
-      uint32_t *cc = sc.ccount.get<uint32_t>(nbins + 1);
-      uint64_t *co = sc.coff.get<uint64_t>(nbins + 1);
+      const int sbits = P < CP_BITS ? P : CP_BITS;
+      const uint32_t nstretch = (uint32_t)(nsub >> sbits);
+      uint32_t *cl = sc.clist.get<uint32_t>(nsub);
+      uint32_t *cc = sc.ccount.get<uint32_t>(nstretch + 1);
+      uint64_t *co = sc.coff.get<uint64_t>(nstretch + 1);
       // runs the rank dedup holds; also at most 2/3 of the block kernel's
       // capacity, whose shared-memory set (a power of two >= 1.5 n slots,
       // filled to 3/4 at most) then always holds one
       static_assert(SrCfg<uint64_t>::CAP <= cs_cap_for(false, true) * 2 / 3 && SrCfg<Key2>::CAP <= cs_cap_for(true, true) * 2 / 3);
-      cs_plan_kernel<<<nbins, CP_BLOCK, 0, s>>>(sb_off, nbins, P, SrCfg<KeyT>::CAP, cl, cc);
+      cs_plan_kernel<<<nstretch, CP_BLOCK, 0, s>>>(sb_off, sbits, SrCfg<KeyT>::CAP, cl, cc);
       CF1_LAUNCH_CHECK();
-      exclusive_scan_u32(cc, co, nbins, sc.scan_tmp, s);
-      CF1_CUDA(cudaMemcpyAsync(&rd.runs, co + nbins, sizeof(uint64_t), cudaMemcpyDeviceToHost, s));
+      exclusive_scan_u32(cc, co, nstretch, sc.scan_tmp, s);
+      CF1_CUDA(cudaMemcpyAsync(&rd.runs, co + nstretch, sizeof(uint64_t), cudaMemcpyDeviceToHost, s));
       CF1_CUDA(cudaStreamSynchronize(s));
       grid = rd.runs;
-      clist = cl;
-      coff = co;
+      runs = sc.runs.get<uint2>(grid);
+      cs_runs_kernel<<<(unsigned)ceil_div((uint64_t)nstretch * 32, CP_BLOCK), CP_BLOCK, 0, s>>>(cl, co, nstretch, sbits, runs);
+      CF1_LAUNCH_CHECK();
     }
     CF1_CUDA(cudaEventRecord(sc.ev[0], s));
     if (grp) {
@@ -2335,7 +2343,7 @@ bool msd_sort_unique(KeyT *keys, KeyT *alt, uint64_t n, uint64_t max_bin, const 
         gd_split_kernel<<<h_ov, GD_MOVE, 0, s>>>(T64, PT, sb_off, ov, PS, P, p1, U64, PU, sub_off, jl);
         CF1_LAUNCH_CHECK();
         kern<<<nov, CS_BLOCK, smem, s>>>(U, T, sub_off, nsub, shift, rest > 0 ? bits : 0, scnt, over, P, lb, PU, PT,
-                                         nullptr, nullptr, nbins, jl, nullptr, false);
+                                         nullptr, jl, nullptr, false);
         CF1_LAUNCH_CHECK();
         gd_gather_kernel<<<h_ov, GD_MOVE, 0, s>>>(U64, lo.with_pay ? lb.l0pay : nullptr, sb_off, ov, g, sub_off, scnt,
                                                    T64, cnt, keep, lo, p1);
@@ -2365,7 +2373,7 @@ bool msd_sort_unique(KeyT *keys, KeyT *alt, uint64_t n, uint64_t max_bin, const 
       }
       if (h_ov) {
         kern<<<h_ov, CS_BLOCK, smem, s>>>(T, U, sb_off, nsub, shift, rest > 0 ? bits : 0, cnt, over, P, lo, PT, PU,
-                                          nullptr, nullptr, nbins, ov, nullptr, !pk);
+                                          nullptr, ov, nullptr, !pk);
         CF1_LAUNCH_CHECK();
         CF1_CUDA(cudaEventRecord(sc.ev[1], s));
         finish();
@@ -2376,15 +2384,15 @@ bool msd_sort_unique(KeyT *keys, KeyT *alt, uint64_t n, uint64_t max_bin, const 
       const size_t ssm = sizeof(SrSmem<KeyT>);
       auto skern = hashed && !W1 ? sr_dedup_kernel<KeyT, !W1> : sr_dedup_kernel<KeyT, false>;
       CF1_CUDA(cudaFuncSetAttribute(skern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)ssm));
-      skern<<<(unsigned)grid, SR_BLOCK, ssm, s>>>(T, PT, sb_off, nsub, P, hashed ? 32 - P : rest > 0 ? rest : 0, cnt, clist,
-                                                 coff, nbins, ov, ovc);
+      skern<<<(unsigned)grid, SR_BLOCK, ssm, s>>>(T, PT, sb_off, nsub, P, hashed ? 32 - P : rest > 0 ? rest : 0, cnt, runs,
+                                                 ov, ovc);
       CF1_LAUNCH_CHECK();
       CF1_CUDA(cudaEventRecord(sc.ev[1], s));
       finish();
       const uint32_t h_ov = rd.overflow;
       if (h_ov) {
-        kern<<<h_ov, CS_BLOCK, smem, s>>>(T, U, sb_off, nsub, shift, rest > 0 ? bits : 0, cnt, over, P, lo, PT, PU, clist,
-                                          coff, nbins, nullptr, ov, true);
+        kern<<<h_ov, CS_BLOCK, smem, s>>>(T, U, sb_off, nsub, shift, rest > 0 ? bits : 0, cnt, over, P, lo, PT, PU, runs,
+                                          nullptr, ov, true);
         CF1_LAUNCH_CHECK();
         CF1_CUDA(cudaEventRecord(sc.ev[1], s));
         finish();

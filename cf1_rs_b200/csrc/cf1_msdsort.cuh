@@ -16,7 +16,7 @@ struct MsdRead {
 };
 
 struct MsdScratch {
-  DevBuf tile_off, hist, scan_tmp, sb_off, sb_off1, cnt, out_off, flag, clist, ccount, coff, ov, ovc;
+  DevBuf tile_off, hist, scan_tmp, sb_off, sb_off1, cnt, out_off, flag, clist, ccount, coff, runs, ov, ovc;
   // groups the group dedup left: their sub-buckets' offsets, counts, list and placed bytes
   DevBuf sub_off, sub_cnt, jlist, ov_pay;
   uint32_t last_overflow = 0;  // sub-buckets the last unsorted run left to the block kernel
