@@ -2074,15 +2074,15 @@ __global__ void __launch_bounds__(CP_BLOCK) cs_runs_kernel(const uint32_t *clist
 }
 static_assert((uint64_t)MAX_BINS << MSD_MAX_BITS <= 1ull << 28);
 
-// One warp per sub-bucket: copy its distinct keys to the dense array.
-template <class KeyT>
+// One warp per sub-bucket or 32 (see warp_units): copy their distinct keys to
+// the dense array.
+template <class KeyT, bool MANY>
 __global__ void cs_compact_kernel(const KeyT *T, const uint64_t *sb_off, const uint32_t *cnt, const uint64_t *out_off,
                                   uint64_t nsub, KeyT *dist) {
-  uint64_t j = ((uint64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
-  if (j >= nsub) return;
-  uint32_t c = cnt[j];
-  uint64_t a = sb_off[j], o = out_off[j];
-  for (uint32_t i = lane_id(); i < c; i += 32) dist[o + i] = T[a + i];
+  warp_units<MANY>(cnt, 0, nsub, [&](uint64_t j, uint32_t c) {
+    const uint64_t a = sb_off[j], o = out_off[j];
+    for (uint32_t i = lane_id(); i < c; i += 32) dist[o + i] = T[a + i];
+  });
 }
 
 __global__ void cs_bin_off_kernel(const uint64_t *out_off, uint32_t nbins, uint64_t per_bin, uint64_t *dist_off) {
@@ -2136,7 +2136,9 @@ void msd_compact(const KeyT *kept, uint64_t nsub, KeyT *dist, MsdScratch &sc, cu
       return;
     }
   }
-  cs_compact_kernel<KeyT><<<(unsigned)ceil_div(nsub * 32, 256), 256, 0, s>>>(
+  const bool many = many_units(nsub);
+  auto kern = many ? cs_compact_kernel<KeyT, true> : cs_compact_kernel<KeyT, false>;
+  kern<<<(unsigned)ceil_div(nsub, many ? 256 : 8), 256, 0, s>>>(
       kept, sc.sb_off.as<const uint64_t>(), sc.cnt.as<const uint32_t>(), sc.out_off.as<const uint64_t>(), nsub, dist);
   CF1_LAUNCH_CHECK();
 }

@@ -175,10 +175,10 @@ CF1_D void warp_copy_bytes(uint8_t *dst, const uint8_t *src, uint32_t n) {
   if (t < n) dst[t] = src[t];
 }
 
-// One warp per unit: each distinct key's side-set byte to its slot.
-// A learned bin's slot is the key's rank, which the dense layout already
-// gives; a BBHash bin probes level 0 first for PL_U keys per lane at once
-// (independent loads in flight: one probe after another would leave the
+// One warp per unit or 32 (see warp_units): each distinct key's side-set byte
+// to its slot.  A learned bin's slot is the key's rank, which the dense layout
+// already gives; a BBHash bin probes level 0 first for PL_U keys per lane at
+// once (independent loads in flight: one probe after another would leave the
 // warp waiting on each).  The ~12% of the keys level 0 did not place queue in
 // shared memory until a full warp of them walks the deeper levels at once:
 // walked where they were met, four lanes at a time, each step left the warp
@@ -189,85 +189,86 @@ struct PlQueue {
   uint64_t h[64];
   uint8_t pay[64];
 };
-template <class KeyT>
+template <class KeyT, bool MANY>
 __global__ void __launch_bounds__(PL_WARPS * 32) place_sides_kernel(MphfView<KeyT> m, const KeyT *kept, const KeyT *dense,
                                                           const uint8_t *kept_pay, const uint64_t *sb_off,
                                                           const uint32_t *cnt, const uint64_t *out_off, uint64_t j0,
                                                           uint64_t j1, int P, uint8_t *sides, uint32_t *err) {
   __shared__ PlQueue queues[PL_WARPS];
   PlQueue &pq = queues[threadIdx.x >> 5];
-  const uint64_t j = j0 + (((uint64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5);
-  if (j >= j1) return;
-  const uint32_t c = cnt[j], bin = (uint32_t)(j >> P);
-  const uint64_t a = sb_off[j], o = out_off[j], base = m.dist_off[bin], end = m.dist_off[bin + 1];
-  const bool ranked = m.learned && m.li.roots[bin].use_learned;
   const unsigned lane = lane_id(), lt = lanemask_lt();
   bool miss = false;
-  auto place = [&](uint64_t local, uint8_t p) {
-    const uint64_t slot = local == SLOT_NONE ? SLOT_NONE : base + local;
-    if (slot < end && slot >= base) sides[slot] = p;
-    else miss = true;
-  };
-  if (ranked) {
-    warp_copy_bytes(sides + o, kept_pay + a, c);
-  } else {
-    const BBMeta m0 = m.bb.levels ? m.bb.meta[bin] : BBMeta{};  // level 0 of this bin
-    uint32_t waiting = 0;
-    for (uint32_t i0 = 0; i0 < c; i0 += 32 * PL_U) {
-      uint64_t H[PL_U];
-      uint8_t pay[PL_U];
-      ulonglong2 e[PL_U];
-      uint32_t bit[PL_U];
+  warp_units<MANY>(cnt, j0, j1, [&](uint64_t j, uint32_t c) {
+    const uint32_t bin = (uint32_t)(j >> P);
+    const uint64_t a = sb_off[j], o = out_off[j], base = m.dist_off[bin], end = m.dist_off[bin + 1];
+    const bool ranked = m.learned && m.li.roots[bin].use_learned;
+    auto place = [&](uint64_t local, uint8_t p) {
+      const uint64_t slot = local == SLOT_NONE ? SLOT_NONE : base + local;
+      if (slot < end && slot >= base) sides[slot] = p;
+      else miss = true;
+    };
+    if (ranked) {
+      warp_copy_bytes(sides + o, kept_pay + a, c);
+    } else {
+      const BBMeta m0 = m.bb.levels ? m.bb.meta[bin] : BBMeta{};  // level 0 of this bin
+      uint32_t waiting = 0;
+      for (uint32_t i0 = 0; i0 < c; i0 += 32 * PL_U) {
+        uint64_t H[PL_U];
+        uint8_t pay[PL_U];
+        ulonglong2 e[PL_U];
+        uint32_t bit[PL_U];
 #pragma unroll
-      for (int u = 0; u < PL_U; u++) {
-        const uint32_t i = i0 + u * 32 + lane;
-        H[u] = 0;
-        pay[u] = 0;
-        if (i < c) {
-          H[u] = bb_key_hash(dense ? dense[o + i] : kept[a + i]);
-          pay[u] = kept_pay[a + i];
+        for (int u = 0; u < PL_U; u++) {
+          const uint32_t i = i0 + u * 32 + lane;
+          H[u] = 0;
+          pay[u] = 0;
+          if (i < c) {
+            H[u] = bb_key_hash(dense ? dense[o + i] : kept[a + i]);
+            pay[u] = kept_pay[a + i];
+          }
         }
-      }
 #pragma unroll
-      for (int u = 0; u < PL_U; u++) {
-        const uint32_t i = i0 + u * 32 + lane;
-        e[u] = make_ulonglong2(0ull, 0ull);
-        bit[u] = 0;
-        if (i < c && m0.nwords) {
-          const uint64_t pos = bb_pos(H[u], 0, m0.nwords);
-          e[u] = m.bb.AR[m0.word_off + (pos >> 6)];
-          bit[u] = (uint32_t)(pos & 63);
+        for (int u = 0; u < PL_U; u++) {
+          const uint32_t i = i0 + u * 32 + lane;
+          e[u] = make_ulonglong2(0ull, 0ull);
+          bit[u] = 0;
+          if (i < c && m0.nwords) {
+            const uint64_t pos = bb_pos(H[u], 0, m0.nwords);
+            e[u] = m.bb.AR[m0.word_off + (pos >> 6)];
+            bit[u] = (uint32_t)(pos & 63);
+          }
         }
-      }
 #pragma unroll
-      for (int u = 0; u < PL_U; u++) {
-        const bool in = i0 + u * 32 + lane < c, hit = (e[u].x >> bit[u]) & 1;
-        if (in && hit) {
-          uint64_t local = (uint32_t)(m0.rank_adj + (uint32_t)e[u].y + (uint32_t)popc64(e[u].x & ((1ull << bit[u]) - 1)));
-          if (m.bb.l1_slice_bits >= 0)  // sliced levels: the bin's slices before this one
-            local = (uint32_t)(local + m.bb.srank[0][((uint64_t)bin << m.bb.l1_slice_bits) +
-                                                     bb_slice(H[u], m.bb.l1_slice_bits)]);
-          place(local, pay[u]);
-        }
-        const unsigned later = __ballot_sync(FULL, in && !hit);
-        if (in && !hit) {  // the queue holds fewer than 32 here
-          const uint32_t q = waiting + (uint32_t)__popc(later & lt);
-          pq.h[q] = H[u];
-          pq.pay[q] = pay[u];
-        }
-        waiting += (uint32_t)__popc(later);
-        __syncwarp();
-        if (waiting >= 32) {
-          waiting -= 32;
-          place(m0.nwords ? bb_walk(m.bb, bin, pq.h[waiting + lane], 1, m.bb.levels) : SLOT_NONE,
-                pq.pay[waiting + lane]);
+        for (int u = 0; u < PL_U; u++) {
+          const bool in = i0 + u * 32 + lane < c, hit = (e[u].x >> bit[u]) & 1;
+          if (in && hit) {
+            uint64_t local = (uint32_t)(m0.rank_adj + (uint32_t)e[u].y + (uint32_t)popc64(e[u].x & ((1ull << bit[u]) - 1)));
+            if (m.bb.l1_slice_bits >= 0)  // sliced levels: the bin's slices before this one
+              local = (uint32_t)(local + m.bb.srank[0][((uint64_t)bin << m.bb.l1_slice_bits) +
+                                                       bb_slice(H[u], m.bb.l1_slice_bits)]);
+            place(local, pay[u]);
+          }
+          const unsigned later = __ballot_sync(FULL, in && !hit);
+          if (in && !hit) {  // the queue holds fewer than 32 here
+            const uint32_t q = waiting + (uint32_t)__popc(later & lt);
+            pq.h[q] = H[u];
+            pq.pay[q] = pay[u];
+          }
+          waiting += (uint32_t)__popc(later);
           __syncwarp();
+          if (waiting >= 32) {
+            waiting -= 32;
+            place(m0.nwords ? bb_walk(m.bb, bin, pq.h[waiting + lane], 1, m.bb.levels) : SLOT_NONE,
+                  pq.pay[waiting + lane]);
+            __syncwarp();
+          }
         }
       }
+      if (lane < waiting)
+        place(m0.nwords ? bb_walk(m.bb, bin, pq.h[lane], 1, m.bb.levels) : SLOT_NONE, pq.pay[lane]);
+      __syncwarp();  // the next unit's keys queue from the start again
     }
-    if (lane < waiting)
-      place(m0.nwords ? bb_walk(m.bb, bin, pq.h[lane], 1, m.bb.levels) : SLOT_NONE, pq.pay[lane]);
-  }
+  });
   if (__any_sync(FULL, miss) && lane == 0) atomicOr(err, (uint32_t)DEV_MPHF_MISS);
 }
 
@@ -419,8 +420,10 @@ void launch_place_sides(const MphfView<KeyT> &m, const KeyT *kept, const KeyT *d
                         const uint64_t *sb_off, const uint32_t *cnt, const uint64_t *out_off, uint64_t j0, uint64_t j1,
                         int P, uint8_t *sides, uint32_t *err, cudaStream_t s) {
   if (j1 <= j0) return;
-  place_sides_kernel<KeyT><<<(unsigned)ceil_div((j1 - j0) * 32, 256), 256, 0, s>>>(
-      m, kept, dense, kept_pay, sb_off, cnt, out_off, j0, j1, P, sides, err);
+  const bool many = many_units(j1 - j0);
+  auto kern = many ? place_sides_kernel<KeyT, true> : place_sides_kernel<KeyT, false>;
+  kern<<<(unsigned)ceil_div(j1 - j0, many ? 256 : 8), PL_WARPS * 32, 0, s>>>(m, kept, dense, kept_pay, sb_off, cnt, out_off,
+                                                                             j0, j1, P, sides, err);
   CF1_LAUNCH_CHECK();
 }
 
