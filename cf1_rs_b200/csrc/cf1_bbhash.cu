@@ -265,7 +265,7 @@ __global__ void __launch_bounds__(BF_BLOCK) bb_tail_kernel(const KeyT *rem0, Key
                                                            const uint64_t *cnt, uint32_t nbins, uint32_t l0,
                                                            ulonglong2 *AR, const uint64_t *off, uint64_t ar_base,
                                                            uint64_t ar_cap, const uint64_t *base, BBMeta *meta,
-                                                           uint32_t *levels, uint32_t *err) {
+                                                           unsigned long long *got, uint32_t *err) {
   extern __shared__ __align__(16) unsigned long long bf_bits[];  // set, col
   __shared__ uint32_t sm[BF_BLOCK / 32];
   const uint32_t b = blockIdx.x, tid = threadIdx.x;
@@ -352,7 +352,10 @@ __global__ void __launch_bounds__(BF_BLOCK) bb_tail_kernel(const KeyT *rem0, Key
     rem = out;
   }
   for (uint64_t w = used + tid; w < room; w += BF_BLOCK) AR[region + w] = make_ulonglong2(0ull, 0ull);
-  if (tid == 0) atomicMax(levels, l);
+  if (tid == 0) {  // the deepest level, and the entries in use
+    atomicMax(&got[0], (unsigned long long)l);
+    atomicAdd(&got[1], (unsigned long long)used);
+  }
 }
 
 // Keys whose bit did not survive go to the next level: each tile appends its
@@ -396,7 +399,7 @@ __global__ void __launch_bounds__(BB_BLOCK) bb_filter_kernel(const KeyT *rem, co
 template <class KeyT>
 void BBHashBuild<KeyT>::clear() {
   tail_words_ = nullptr;
-  total_words = 0;
+  total_words = used_words = dense_words = 0;
   levels = 0;
   bytes = 0;
   l1_slice_bits = -1;
@@ -465,18 +468,19 @@ void BBHashBuild<KeyT>::run_levels(uint32_t l, const KeyT *rem, const uint64_t *
     bb_room_kernel<<<(unsigned)ceil_div(nbins, 256), 256, 0, s>>>(cur, nbins, room);
     CF1_LAUNCH_CHECK();
     exclusive_scan_u64(room, off, nbins, scan_tmp_, s);
-    uint32_t *lv = lv_.get<uint32_t>(1);
-    CF1_CUDA(cudaMemcpyAsync(lv, &tail_from_, sizeof(uint32_t), cudaMemcpyHostToDevice, s));
+    unsigned long long *got = lv_.get<unsigned long long>(2);
+    CF1_CUDA(cudaMemcpyAsync(got, tail_from_, sizeof(tail_from_), cudaMemcpyHostToDevice, s));
     const size_t smem = 2 * BF_WORDS * sizeof(unsigned long long);
     CF1_CUDA(cudaFuncSetAttribute(bb_tail_kernel<KeyT>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
     bb_tail_kernel<KeyT><<<nbins, BF_BLOCK, smem, s>>>(rem, r0, r1, start, cur, nbins, l, ar_.as<ulonglong2>(), off,
                                                        total_words, ar_.cap / sizeof(ulonglong2), base_.as<uint64_t>(),
-                                                       meta_.as<BBMeta>(), lv, err);
+                                                       meta_.as<BBMeta>(), got, err);
     CF1_LAUNCH_CHECK();
     tail_words_ = off + nbins;
     levels = BB_MAX_LEVELS;  // until collect(): a walk ends at the first level a bin does not have
+    dense_words = total_words;
   };
-  tail_from_ = l;
+  tail_from_[0] = l;
   if (one_launch && expect <= BF_KEYS * nbins && largest <= BF_LARGEST) return tail();
   uint64_t *wcnt = wcnt_.as<uint64_t>(), *woff = woff_.as<uint64_t>();
   uint32_t *tile_off = tile_off_.as<uint32_t>();
@@ -493,7 +497,7 @@ void BBHashBuild<KeyT>::run_levels(uint32_t l, const KeyT *rem, const uint64_t *
     if (remaining == 0) break;
     if (one_launch && remaining <= BF_KEYS * nbins && ht[2] <= BF_LARGEST) {
       reserve_entries(total_words + bf_room(remaining) + nbins * (bf_room(1) + 1), total_words, s);
-      tail_from_ = l;
+      tail_from_[0] = l;
       return tail();
     }
     if (l >= BB_MAX_LEVELS) throw Error(CF1GPU_ERR_BIJECTION, "BBHash: keys left after the last level");
@@ -515,19 +519,20 @@ void BBHashBuild<KeyT>::run_levels(uint32_t l, const KeyT *rem, const uint64_t *
     rem = out;
   }
   levels = l;
+  used_words = dense_words = total_words;
   set_bytes();
 }
 
 template <class KeyT>
 void BBHashBuild<KeyT>::set_bytes() {
-  bytes = total_words * sizeof(ulonglong2) + (size_t)levels * nbins * sizeof(BBMeta) + 2 * srank_words * sizeof(uint32_t);
+  bytes = used_words * sizeof(ulonglong2) + (size_t)levels * nbins * sizeof(BBMeta) + 2 * srank_words * sizeof(uint32_t);
 }
 
 template <class KeyT>
 void BBHashBuild<KeyT>::collect_begin(uint64_t *got, cudaStream_t s) {
   if (!tail_words_) return;
   CF1_CUDA(cudaMemcpyAsync(&got[0], tail_words_, sizeof(uint64_t), cudaMemcpyDeviceToHost, s));
-  CF1_CUDA(cudaMemcpyAsync(&got[1], lv_.p, sizeof(uint32_t), cudaMemcpyDeviceToHost, s));
+  CF1_CUDA(cudaMemcpyAsync(&got[1], lv_.p, 2 * sizeof(uint64_t), cudaMemcpyDeviceToHost, s));
 }
 
 template <class KeyT>
@@ -535,6 +540,7 @@ void BBHashBuild<KeyT>::collect_end(const uint64_t *got) {
   if (!tail_words_) return;
   tail_words_ = nullptr;
   total_words += got[0];
+  used_words = dense_words + got[2];
   levels = std::max<uint32_t>((uint32_t)got[1], l1_slice_bits >= 0 ? 2 : 0);
   set_bytes();
 }

@@ -6,7 +6,9 @@ namespace cf1 {
 
 template <class KeyT>
 struct BBHashBuild {
-  uint64_t total_words = 0;        // entries of all levels
+  uint64_t total_words = 0;        // entries of all levels, with the room the last ones left
+  uint64_t dense_words = 0;        // those without gaps: the levels before the one-launch ones
+  uint64_t used_words = 0;         // entries some level has
   uint32_t levels = 0, nbins = 0;
   uint64_t bytes = 0;
   int l1_slice_bits = -1;          // see BBView
@@ -21,7 +23,7 @@ struct BBHashBuild {
   // other bins get no levels.  Synchronises the stream between the large
   // levels; the last ones run in one launch (bb_tail_kernel), whose entries and
   // deepest level collect_begin fetches and, after the stream's next wait,
-  // collect_end takes over (levels, total_words, bytes).  A device error goes
+  // collect_end takes over (levels, total_words, used_words, bytes).  A device error goes
   // to *err.
   // ws0/ws1 (optional, ws_cap keys each, not aliasing keys) hold the keys
   // still unplaced between levels; without them the builder allocates.
@@ -42,12 +44,12 @@ struct BBHashBuild {
                            const uint64_t *woff1, uint64_t words1, const uint32_t *placed1, const KeyT *surv,
                            const uint64_t *surv_off, const uint64_t *surv_cnt, uint64_t surv_total, uint64_t n_occ,
                            uint64_t max_bin, uint32_t *err, cudaStream_t s, KeyT *ws0 = nullptr, KeyT *ws1 = nullptr, uint64_t ws_cap = 0);
-  void collect_begin(uint64_t *got, cudaStream_t s);  // got: two words of page-locked memory
+  void collect_begin(uint64_t *got, cudaStream_t s);  // got: three words of page-locked memory
   void collect_end(const uint64_t *got);
   BBView view() const;
   void clear();
   const BBMeta *meta_device() const { return meta_.as<const BBMeta>(); }
-  // {bit word, level rank} entries of all levels (total_words of them)
+  // {bit word, level rank} entries of all levels (in total_words)
   const ulonglong2 *entries_device() const { return ar_.as<const ulonglong2>(); }
   // per-slice start ranks of sliced level l (srank_words of them)
   const uint32_t *srank_device(int l) const { return srank_[l].as<const uint32_t>(); }
@@ -65,7 +67,7 @@ struct BBHashBuild {
   // The entry array and the level buffers are kept across builds and grown on
   // demand, so a rebuild allocates nothing once sizes settle.
   DevBuf ar_, meta_, base_, rem_[2], cnt_[2], tot_, tile_off_, wcnt_, woff_, pc_, rtmp_, scan_tmp_, srank_[2], lv_;
-  uint32_t tail_from_ = 0;                  // first level of the one-launch tail (copied from here)
+  uint64_t tail_from_[2] = {0, 0};          // first level of the one-launch tail, no entries yet (copied from here)
   const uint64_t *tail_words_ = nullptr;    // device: its entries; nullptr: none pending
 
 };

@@ -63,7 +63,7 @@ size_t export_impl(cf1gpu_ctx *c, void *dst, size_t cap) {
   h.meta_off = off;
   off = align16(off + (uint64_t)NL * B * sizeof(BBMeta));
   h.ar_off = off;
-  h.ar_words = be.bb.total_words;
+  h.ar_words = be.bb.used_words;  // without the room between the last levels' blocks
   off = align16(off + h.ar_words * sizeof(ulonglong2));
   h.srank_off = off;
   h.srank_words = h.l1_slice_bits >= 0 ? be.bb.srank_words : 0;
@@ -86,8 +86,12 @@ size_t export_impl(cf1gpu_ctx *c, void *dst, size_t cap) {
   CF1_CUDA(cudaMemcpyAsync(d + h.dist_off_off, c->d_dist_off.p, (B + 1) * 8, cudaMemcpyDeviceToHost, s));
   if (NL)
     CF1_CUDA(cudaMemcpyAsync(d + h.meta_off, be.bb.meta_device(), (size_t)NL * B * sizeof(BBMeta), cudaMemcpyDeviceToHost, s));
-  if (h.ar_words)
-    CF1_CUDA(cudaMemcpyAsync(d + h.ar_off, be.bb.entries_device(), h.ar_words * sizeof(ulonglong2),
+  const uint64_t dense = be.bb.dense_words;
+  if (dense)
+    CF1_CUDA(cudaMemcpyAsync(d + h.ar_off, be.bb.entries_device(), dense * sizeof(ulonglong2), cudaMemcpyDeviceToHost, s));
+  std::vector<ulonglong2> tail(be.bb.total_words - dense);
+  if (!tail.empty())
+    CF1_CUDA(cudaMemcpyAsync(tail.data(), be.bb.entries_device() + dense, tail.size() * sizeof(ulonglong2),
                              cudaMemcpyDeviceToHost, s));
   for (int l = 0; l < 2 && h.srank_words; l++)
     CF1_CUDA(cudaMemcpyAsync(d + h.srank_off + l * h.srank_words * sizeof(uint32_t), be.bb.srank_device(l),
@@ -98,6 +102,18 @@ size_t export_impl(cf1gpu_ctx *c, void *dst, size_t cap) {
     CF1_CUDA(cudaMemcpyAsync(d + h.keys_off, c->d_dist.p, c->n_distinct * sizeof(KeyT), cudaMemcpyDeviceToHost, s));
   }
   CF1_CUDA(cudaStreamSynchronize(s));
+  if (!tail.empty()) {  // the last levels' blocks one after another
+    BBMeta *meta = reinterpret_cast<BBMeta *>(d + h.meta_off);
+    ulonglong2 *ar = reinterpret_cast<ulonglong2 *>(d + h.ar_off);
+    uint64_t at = dense;
+    for (uint64_t i = 0; i < (uint64_t)NL * B; i++) {
+      if (!meta[i].nwords || meta[i].word_off < dense) continue;
+      if (at + meta[i].nwords > h.ar_words) throw Error(CF1GPU_ERR_BIJECTION, "BBHash: more entries than counted");
+      std::memcpy(ar + at, tail.data() + (meta[i].word_off - dense), meta[i].nwords * sizeof(ulonglong2));
+      meta[i].word_off = at;
+      at += meta[i].nwords;
+    }
+  }
   return off;
 }
 

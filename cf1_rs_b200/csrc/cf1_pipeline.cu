@@ -39,7 +39,7 @@ struct Readback {
     uint64_t n_super, n_occ, n_kept;
   } u;
   cf1::MsdRead msd;
-  uint64_t bb[2];  // entries and deepest level of BBHash's last levels
+  uint64_t bb[3];  // BBHash's last levels: room, deepest level, entries in use
   uint64_t bins[3][MAX_BINS + 1];  // k-mer, record and slot offsets of the bins
 };
 
