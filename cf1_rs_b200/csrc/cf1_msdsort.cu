@@ -2341,7 +2341,9 @@ bool msd_sort_unique(KeyT *keys, KeyT *alt, uint64_t n, uint64_t max_bin, const 
         uint64_t *sub_off = sc.sub_off.get<uint64_t>(nsub + 1);
         uint32_t *scnt = sc.sub_cnt.get<uint32_t>(nsub + 1), *jl = sc.jlist.get<uint32_t>(nov);
         Level0Out lb = lo;
-        if (lo.with_pay) lb.l0pay = sc.ov_pay.get<uint8_t>(n + 16);
+        // the placed bytes go to PT, whose bytes of these groups have moved to
+        // PU: a sub-bucket's are the block kernel's scratch until its slice
+        lb.l0pay = PT;
         gd_split_kernel<<<h_ov, GD_MOVE, 0, s>>>(T64, PT, sb_off, ov, PS, P, p1, U64, PU, sub_off, jl);
         CF1_LAUNCH_CHECK();
         kern<<<nov, CS_BLOCK, smem, s>>>(U, T, sub_off, nsub, shift, rest > 0 ? bits : 0, scnt, over, P, lb, PU, PT,

@@ -17,8 +17,8 @@ struct MsdRead {
 
 struct MsdScratch {
   DevBuf tile_off, hist, scan_tmp, sb_off, sb_off1, cnt, out_off, flag, clist, ccount, coff, runs, ov, ovc;
-  // groups the group dedup left: their sub-buckets' offsets, counts, list and placed bytes
-  DevBuf sub_off, sub_cnt, jlist, ov_pay;
+  // groups the group dedup left: their sub-buckets' offsets, counts and list
+  DevBuf sub_off, sub_cnt, jlist;
   uint32_t last_overflow = 0;  // sub-buckets the last unsorted run left to the block kernel
   // The last run's units, 2^unit_bits per bin: what sb_off, cnt and out_off
   // have one entry for.  A unit is a sub-bucket, or a group of sub-buckets
