@@ -6,11 +6,8 @@
 // instead: the DMA of one chunk runs while several host threads copy the
 // other.  Page-locked, managed or device pointers are copied directly.
 #pragma once
-#include <atomic>
-#include <thread>
-#include <vector>
-
 #include "cf1_context.cuh"
+#include "cf1_hostcopier.h"
 
 namespace cf1 {
 
@@ -21,27 +18,6 @@ constexpr size_t IO_STAGE_MIN = 16u << 20;
 
 // True when CUDA knows nothing about the pointer: ordinary host memory.
 bool pageable(const void *p);
-
-// Host threads for one call's copies (they end with it); the calling thread
-// copies too.  Fewer are used when they cannot be created.
-class HostCopier {
- public:
-  explicit HostCopier(size_t total_bytes);
-  ~HostCopier();
-  HostCopier(const HostCopier &) = delete;
-  HostCopier &operator=(const HostCopier &) = delete;
-  void copy(void *dst, const void *src, size_t n);
-
- private:
-  void part(size_t i) const;
-  std::vector<std::thread> threads_;
-  std::atomic<uint64_t> epoch_{0};
-  std::atomic<size_t> left_{0};
-  std::atomic<bool> stop_{false};
-  char *dst_ = nullptr;
-  const char *src_ = nullptr;
-  size_t n_ = 0;
-};
 
 // bytes from the device to dst, in order after what is queued on the
 // context's stream; returns when they are there.

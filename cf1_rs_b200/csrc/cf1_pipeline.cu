@@ -1232,12 +1232,7 @@ void add_records(cf1gpu_ctx *c, const uint8_t *seqs, const uint64_t *off, size_t
       if (b == dst[i] + len + 1) h[dst[i] + len] = 'N';
     }
   };
-  if (nt == 1) work(0);
-  else {
-    std::vector<std::thread> th;
-    for (unsigned t = 0; t < nt; t++) th.emplace_back(work, t);
-    for (auto &x : th) x.join();
-  }
+  on_threads(nt, work);
   c->L = pos;
   c->uploaded = false;
 }
