@@ -2162,26 +2162,29 @@ int msd_prefix_bits(uint64_t max_bin_keys, bool sorted) {
   return p;
 }
 
-void msd_look_for_repeats(const uint64_t *keys, uint64_t n, const uint64_t *seg_off, uint32_t nbins, MsdScratch &sc,
-                          MsdRead &rd, cudaStream_t s) {
-  rd.repeats[0] = 0;
+void msd_look_for_repeats(const uint64_t *keys, uint64_t n, const uint64_t *seg_off, uint32_t nbins, uint64_t *got,
+                          MsdScratch &sc, cudaStream_t s) {
   // (bins past the widest split, on average, go without the group dedup anyway)
   if (n < RP_MIN || n / nbins > ((uint64_t)(GD_MAXSUB + 1) << MSD_MAX_BITS)) return;
   const uint64_t words = rp_words(n);
-  uint32_t *set = sc.hist.get<uint32_t>(2 * words + 8);  // free until the split
-  unsigned long long *got = reinterpret_cast<unsigned long long *>(set);
-  CF1_CUDA(cudaMemsetAsync(set, 0, (2 * words + 8) * sizeof(uint32_t), s));
-  rp_sample_kernel<<<RP_CTAS, RP_BLOCK, 0, s>>>(keys, seg_off, nbins, set + 8, set + 8 + words, got);
+  uint32_t *set = sc.hist.get<uint32_t>(2 * words);  // free until the split
+  CF1_CUDA(cudaMemsetAsync(set, 0, 2 * words * sizeof(uint32_t), s));
+  rp_sample_kernel<<<RP_CTAS, RP_BLOCK, 0, s>>>(keys, seg_off, nbins, set, set + words,
+                                               reinterpret_cast<unsigned long long *>(got));
   CF1_LAUNCH_CHECK();
-  CF1_CUDA(cudaMemcpyAsync(rd.repeats, got, sizeof(rd.repeats), cudaMemcpyDeviceToHost, s));
 }
 
-bool msd_lists_overflow(uint64_t max_bin, int P, const MsdRead &rd) {
-  if (!rd.repeats[0]) return false;
+bool msd_lists_overflow(const uint64_t *seg_off, uint32_t nbins, int P, const uint64_t *got) {
+  if (!got[0]) return false;
   const int g = gd_group_bits(P);
-  const double keys = (double)rd.repeats[0], copies = keys / (double)rd.repeats[1];
-  const double list = (double)rd.repeats[2] / keys * std::ldexp((double)max_bin, g - P);
-  return list + 1.5 * std::sqrt(list * copies) > (g <= 4 ? GdCfg<4>::MAXL : GdCfg<5>::MAXL);
+  const double keys = (double)got[0], copies = keys / (double)got[1];
+  uint64_t over = 0;
+  for (uint32_t b = 0; b < nbins; b++) {
+    const uint64_t occ = seg_off[b + 1] - seg_off[b];
+    const double list = (double)got[2] / keys * std::ldexp((double)occ, g - P);
+    if (list + 1.5 * std::sqrt(list * copies) > (g <= 4 ? GdCfg<4>::MAXL : GdCfg<5>::MAXL)) over += occ;
+  }
+  return over > (seg_off[nbins] - seg_off[0]) / 8;
 }
 
 template <class KeyT>

@@ -9,7 +9,6 @@ namespace cf1 {
 // caller's.
 struct MsdRead {
   uint64_t n_distinct, runs;
-  uint64_t repeats[3];  // msd_look_for_repeats: keys looked at, bits they set, keys that share theirs
   uint32_t overflow;  // units (unsorted) or runs (sorted) left to the block kernel
   uint32_t oversize;  // a sub-bucket fits nowhere
   uint32_t l0_err;    // Level0Out::err
@@ -88,13 +87,16 @@ struct Level0Out {
   uint32_t *uplaced = nullptr, *uplaced1 = nullptr;  // [units]
 };
 
-// How much the keys of the unsorted 64-bit form repeat, from a few bins, to
-// rd.repeats by the stream's next wait (repeats[0] = 0: not looked at), and whether the group dedup's lists then overflow on a split of P
-// bits: mean and 1.5 standard deviations of the largest bin's lists, the keys'
-// copies coming together.
-void msd_look_for_repeats(const uint64_t *keys, uint64_t n, const uint64_t *seg_off, uint32_t nbins, MsdScratch &sc,
-                          MsdRead &rd, cudaStream_t s);
-bool msd_lists_overflow(uint64_t max_bin, int P, const MsdRead &rd);
+// How much the keys of the unsorted 64-bit form repeat, from a few bins, added
+// to got (device, zeroed; it stays so for inputs not worth a look): keys looked
+// at, bits they set, keys that share theirs.  And from those, on the host,
+// whether an eighth of the keys (offsets seg_off) and more lie in bins where the
+// group dedup's lists overflow on a split of P bits: their mean and 1.5 standard
+// deviations do, the keys' copies coming together.
+constexpr uint32_t REPEATS = 3;
+void msd_look_for_repeats(const uint64_t *keys, uint64_t n, const uint64_t *seg_off, uint32_t nbins, uint64_t *got,
+                          MsdScratch &sc, cudaStream_t s);
+bool msd_lists_overflow(const uint64_t *seg_off, uint32_t nbins, int P, const uint64_t *got);
 
 // max_bin: the keys of the largest bin.
 // With dist = nullptr the distinct keys stay where the dedup left them, at

@@ -40,7 +40,8 @@ struct Readback {
   } u;
   cf1::MsdRead msd;
   uint64_t bb[3];  // BBHash's last levels: room, deepest level, entries in use
-  uint64_t bins[3][MAX_BINS + 1];  // k-mer, record and slot offsets of the bins
+  // k-mer offsets of the bins (and how much they repeat), their record and slot offsets
+  uint64_t bins[3][MAX_BINS + 1 + REPEATS];
 };
 
 // Small device counters of one run.
@@ -54,9 +55,10 @@ struct Small {
   uint32_t queues[8];
 };
 
+// The bins' k-mer offsets, and zeros after them for msd_look_for_repeats.
 __global__ void seg_gather_kernel(const uint64_t *kpre, const uint64_t *rec_off, uint32_t nbins, uint64_t *seg) {
   uint32_t b = blockIdx.x * blockDim.x + threadIdx.x;
-  if (b <= nbins) seg[b] = kpre[rec_off[b]];
+  if (b <= nbins + REPEATS) seg[b] = b <= nbins ? kpre[rec_off[b]] : 0;
 }
 
 // Bin sharding: records of the bins this shard keeps (b % shards == idx).
@@ -519,8 +521,8 @@ void run_impl(cf1gpu_ctx *c, StreamIO *io = nullptr, Step step = Step::FULL, con
   uint8_t *pay_alt = join3 ? c->d_pay_alt.get<uint8_t>(NO + 16) : nullptr;
   launch_expand<KeyT>(records, NS, kpre, W, k, keys, NO, L, batched ? &sm->queues[2] : nullptr, &sm->err, pctas, s,
                       pay);
-  uint64_t *seg = c->d_seg.get<uint64_t>(B + 1);
-  seg_gather_kernel<<<(unsigned)ceil_div(B + 1, 256), 256, 0, s>>>(kpre, rec_off, B, seg);
+  uint64_t *seg = c->d_seg.get<uint64_t>(B + 1 + REPEATS);
+  seg_gather_kernel<<<(unsigned)ceil_div(B + 1 + REPEATS, 256), 256, 0, s>>>(kpre, rec_off, B, seg);
   CF1_LAUNCH_CHECK();
   // the dense distinct-key array, allocated when a step writes it
   auto dist_buf = [&]() { return c->d_dist.get<KeyT>(NO + 1); };
@@ -528,8 +530,8 @@ void run_impl(cf1gpu_ctx *c, StreamIO *io = nullptr, Step step = Step::FULL, con
   const uint64_t *hseg = rb->bins[0];
   const bool grouped = !sorted && !c->wide && c->opts.mphf_mode == CF1GPU_MPHF_BBHASH;
   if constexpr (KOps<KeyT>::WORDS == 1)
-    if (grouped) msd_look_for_repeats(keys, NO, seg, B, be.msd, rb->msd, s);
-  CF1_CUDA(cudaMemcpyAsync(rb->bins[0], seg, (B + 1) * sizeof(uint64_t), cudaMemcpyDeviceToHost, s));
+    if (grouped) msd_look_for_repeats(keys, NO, seg, B, seg + B + 1, be.msd, s);
+  CF1_CUDA(cudaMemcpyAsync(rb->bins[0], seg, (B + 1 + REPEATS) * sizeof(uint64_t), cudaMemcpyDeviceToHost, s));
   CF1_CUDA(cudaStreamSynchronize(s));
   uint64_t max_bin = 0;
   for (uint32_t b = 0; b < B; b++) max_bin = std::max(max_bin, hseg[b + 1] - hseg[b]);
@@ -541,7 +543,7 @@ void run_impl(cf1gpu_ctx *c, StreamIO *io = nullptr, Step step = Step::FULL, con
   // 8.9 ms with most groups left to the block kernel, 4.3 / 3.7 / 3.4 on one bit
   // more; sequence that does not repeat loses by it, 2.97 against 3.35.)
   bool groups = true;
-  if (grouped && P0 >= 0 && msd_lists_overflow(max_bin, P0, rb->msd)) {
+  if (grouped && P0 >= 0 && msd_lists_overflow(hseg, B, P0, hseg + B + 1)) {
     if (P0 < 16) P0++;
     else groups = false;
   }
