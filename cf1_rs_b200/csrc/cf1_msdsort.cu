@@ -745,7 +745,7 @@ __global__ void __launch_bounds__(CS_BLOCK, SORTED ? 2 : 4) cs_sort_unique_kerne
 // ---------------------------------------------------------------- rank dedup
 // The sorted form's dedup, and that of 128-bit keys in the BBHash form
 // (HASHED): one CTA per run of consecutive sub-buckets of a bin (the plan's
-// chunks), at most SrCfg::CAP keys, held in registers.  A key's position is
+// runs), at most SrCfg::CAP keys, held in registers.  A key's position is
 // its distance from the run's start in the key range (HASHED: in the range of
 // the level-0 hash), scaled by a shift to NP = 8 CAP bits, so positions ascend
 // with the keys (with the hash):
@@ -1541,7 +1541,7 @@ int gd_group_bits(int P) { return P <= GD_BITS ? P : P - 4 <= GD_SPLIT ? 4 : GD_
 // 72% (69%) of a group's occurrences, and copies of a key always share their
 // bit, so groups near their capacity overflow it when most keys occur twice or
 // more (reads at any coverage, assemblies of one species).  One to four bins,
-// evenly spaced: their keys in one 64th of the hash range mark a bitmap of 8
+// evenly spaced, the next one that is not empty: their keys in one 64th of the hash range mark a bitmap of 8
 // bits an occurrence -- level 0's own density -- in global memory.  got: the
 // keys marked, the bits set, the keys that share their bit.
 constexpr uint32_t RP_CTAS = 512;  // of all bins
@@ -1555,7 +1555,9 @@ CF1_HD uint64_t rp_words(uint64_t occ) { return (occ >> (RP_BITS + 2)) + 1; }  /
 __global__ void __launch_bounds__(RP_BLOCK) rp_sample_kernel(const uint64_t *keys, const uint64_t *seg_off, uint32_t nbins,
                                                             uint32_t *set, uint32_t *col, unsigned long long *got) {
   const uint32_t nb = rp_bins(nbins), per = RP_CTAS / nb, i = blockIdx.x / per, part = blockIdx.x % per;
-  const uint32_t bin = (uint32_t)((2ull * i + 1) * nbins / (2 * nb));
+  uint32_t bin = (uint32_t)((2ull * i + 1) * nbins / (2 * nb));
+  // (a shard's bins are every shard_count-th one)
+  for (const uint32_t stop = (uint32_t)((i + 1ull) * nbins / nb); bin + 1 < stop && seg_off[bin + 1] == seg_off[bin];) bin++;
   const uint64_t a = seg_off[bin], e = seg_off[bin + 1];
   const uint32_t words = (uint32_t)((e - a) >> (RP_BITS + 2));
   if (!words) return;
@@ -1691,8 +1693,9 @@ __global__ void __launch_bounds__(256) gd_compact_kernel(const uint64_t *T, cons
 
 // ---------------------------------------------------------------- warp dedup
 // The unsorted (BBHash) form's dedup where sub-buckets are larger than the
-// width rule's (bins above 12.5 M keys, whose split is capped at 16 bits, or
-// a narrower split from the autotuner): one warp per sub-bucket and no block
+// width rule's (bins of 14.7 M keys and more, whose split is capped at 16 bits,
+// or a narrower split from the autotuner) and where sequence repeats at the
+// widest split: one warp per sub-bucket and no block
 // barriers: sub-buckets of a few hundred keys (the split of key *
 // KEY_SPREAD_MUL spreads them evenly), a private 512-slot open-addressing set
 // per warp in shared memory, and, with level 0 on, the sub-bucket's slice of

@@ -8,8 +8,9 @@ warps."""
 import numpy as np
 import pytest
 
+import cf1_rs_b200 as cg
 from oracle import oracle as o
-from tests.gpu_util import assert_parity
+from tests.gpu_util import assert_parity, sort_by_key
 
 pytestmark = pytest.mark.gpu
 
@@ -43,3 +44,24 @@ def test_tandem_arrays(unit):
     g, _ = assert_parity(seq, off, 31, num_bins=4)
     assert g.stats()["dedup_overflow"] > 0
     g.close()
+
+
+def test_a_shard_looks_at_its_own_bins():
+    """Shards 0 and 1 of 2 keep every second of six bins: each looks at one that
+    is its own."""
+    n = 17_800_000
+    unit = _random(n // 2, n)
+    seq, off = o.concat_records([unit] * 2)
+    ref = o.run(31, seq, off, nthreads=8, method=0)
+    keys, states = [], []
+    for shard in range(2):
+        with cg.Cf1Gpu(k=31, num_bins=6, shard_index=shard, shard_count=2) as g:
+            g.add_records(seq, off)
+            g.run()
+            st = g.stats()
+            assert st["sort_msd_bits"] == 15 and st["dedup_overflow"] == 0
+            k, s = g.dump_states()
+            keys.append(k)
+            states.append(s)
+    k, s = sort_by_key(np.concatenate(keys), np.concatenate(states))
+    assert np.array_equal(k, ref.keys) and np.array_equal(s, ref.states)
