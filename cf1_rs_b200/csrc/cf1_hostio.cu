@@ -5,13 +5,13 @@
 
 namespace cf1 {
 
-bool pageable(const void *p) {
+cudaMemoryType memory_type(const void *p) {
   cudaPointerAttributes a;
   if (cudaPointerGetAttributes(&a, p) != cudaSuccess) {
-    (void)cudaGetLastError();
-    return true;
+    (void)cudaGetLastError();  // not a pointer CUDA knows
+    return cudaMemoryTypeUnregistered;
   }
-  return a.type == cudaMemoryTypeUnregistered;
+  return a.type;
 }
 
 void copy_out(cf1gpu_ctx *c, void *dst, const void *dev, size_t bytes) {

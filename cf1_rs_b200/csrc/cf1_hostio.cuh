@@ -16,8 +16,9 @@ constexpr size_t IO_CHUNK = 4u << 20;  // bytes of a staging chunk
 // a context's first one ~10 ms, which 3 MB of state words never win back.
 constexpr size_t IO_STAGE_MIN = 16u << 20;
 
-// True when CUDA knows nothing about the pointer: ordinary host memory.
-bool pageable(const void *p);
+// What CUDA knows about the pointer: unregistered is ordinary host memory.
+cudaMemoryType memory_type(const void *p);
+inline bool pageable(const void *p) { return memory_type(p) == cudaMemoryTypeUnregistered; }
 
 // bytes from the device to dst, in order after what is queued on the
 // context's stream; returns when they are there.

@@ -945,15 +945,6 @@ void query_impl(cf1gpu_ctx *c, const uint64_t *keys, size_t n, uint64_t *slots) 
   CF1_CUDA(cudaStreamSynchronize(s));
 }
 
-bool page_locked(const void *p) {
-  cudaPointerAttributes a;
-  if (cudaPointerGetAttributes(&a, p) != cudaSuccess) {
-    (void)cudaGetLastError();  // not a pointer CUDA knows: pageable
-    return false;
-  }
-  return a.type == cudaMemoryTypeHost;
-}
-
 // dst[i]: the record's place in the concatenation (~0 for records below k
 // bases); end: the concatenation's length after the records.
 void intake_direct(cf1gpu_ctx *c, const uint8_t *seqs, const uint64_t *off, size_t n, const std::vector<uint64_t> &dst,
@@ -1211,7 +1202,7 @@ void add_records(cf1gpu_ctx *c, const uint8_t *seqs, const uint64_t *off, size_t
     pos += len + 1;
   }
   // page-locked records go straight to the device while nothing is staged
-  if (n && c->dev_valid == c->L && page_locked(seqs + off[0])) {
+  if (n && c->dev_valid == c->L && memory_type(seqs + off[0]) == cudaMemoryTypeHost) {
     intake_direct(c, seqs, off, n, dst, pos);
     c->uploaded = false;
     return;
