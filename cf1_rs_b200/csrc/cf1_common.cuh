@@ -256,6 +256,8 @@ static_assert(KEY_SPREAD_MUL * KEY_SPREAD_INV == 1, "KEY_SPREAD_INV inverts KEY_
 // occurrence's side-set byte has nibbles in {3, 5, 6, 9, F}:
 // each nibble is a 3-bit code (0 also has one; anything else, which no
 // occurrence gives, reads as F).
+// The expansion computes the codes themselves (contribution_code); pay_code,
+// byte to code, is what the host checks compare them with.
 constexpr uint64_t pay_nib_codes() {
   uint64_t t = 0;
   for (uint32_t v = 0; v < 16; v++) {

@@ -38,7 +38,9 @@ constexpr uint32_t LT_TILE = 16384;  // keys per CTA: the tile's set-up (segment
 constexpr uint32_t LT_MAX_SAMPLES = 4096;
 constexpr int H = LI_HIDDEN;
 
-// Adds one sample's MSE term (weight `scale`) and its gradient to g.
+// Adds one sample's MSE term (weight `scale`) and its gradient to g: the
+// diagnostic entry for any first layer (cf1gpu_learned_grad).  No run calls it;
+// the trainer forms its gradient from the ramps' sums (LiRamps below).
 // Parameter layout: w1[0,H) b1[H,2H) w2[2H,3H) b2[3H]; hidden units are
 // clipped ReLUs clamp(w1 x + b1, 0, 1) (li_act).  Queries evaluate the same
 // function on its piecewise-linear form (LIRoot, li_root_eval).

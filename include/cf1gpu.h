@@ -256,8 +256,9 @@ int cf1gpu_learned_stats(const cf1gpu_ctx *ctx, double out5[5]);
 
 /* Diagnostics: full-batch MSE loss and gradient of a learned-index root
  * (1 -> 16 clipped-ReLU clamp(w1 x + b1, 0, 1) -> 1, params = w1[16] b1[16]
- * w2[16] b2) over n samples, computed on `device` for any first layer (the
- * trainer's units tile [0, 1], which cf1gpu_learned_grad_q's code uses). */
+ * w2[16] b2) over n samples, computed on `device` for any first layer, by a
+ * kernel of its own that no run launches (the trainer's units tile [0, 1];
+ * its code is what cf1gpu_learned_grad_q runs). */
 int cf1gpu_learned_grad(int device, const float *params, const float *x, const float *t, size_t n, float *grad,
                         float *loss);
 
