@@ -1547,20 +1547,27 @@ int gd_group_bits(int P) { return P <= GD_BITS ? P : P - 4 <= GD_SPLIT ? 4 : GD_
 constexpr uint32_t RP_CTAS = 512;  // of all bins
 constexpr int RP_BITS = 6, RP_BLOCK = 512;
 constexpr uint64_t RP_RANGE = 37;  // any of the 64
-// Occurrences from which a look is taken: it costs ~10 us, and below that a run
+// Occurrences from which a look is taken: it costs 10-30 us, and below that a run
 // with most of its groups left to the block kernel takes under a millisecond.
 constexpr uint64_t RP_MIN = 8u << 20;
-CF1_HD uint32_t rp_bins(uint32_t nbins) { return nbins < 32 ? 1 : nbins < 64 ? 2 : 4; }  // at most 1/16 of the keys
+// Bins looked at: at most 1/16 of the keys, and two large ones tell as much as
+// four (200 Mbp in 128 bins, 24 us for four of 1.6 M).
+CF1_HD uint32_t rp_bins(uint64_t occ, uint32_t nbins) {
+  return nbins < 32 ? 1 : nbins < 64 || occ / nbins > (1u << 19) ? 2 : 4;
+}
 CF1_HD uint64_t rp_words(uint64_t occ) { return (occ >> (RP_BITS + 2)) + 1; }  // u32 words of occ keys' bits
 __global__ void __launch_bounds__(RP_BLOCK) rp_sample_kernel(const uint64_t *keys, const uint64_t *seg_off, uint32_t nbins,
-                                                            uint32_t *set, uint32_t *col, unsigned long long *got) {
-  const uint32_t nb = rp_bins(nbins), per = RP_CTAS / nb, i = blockIdx.x / per, part = blockIdx.x % per;
+                                                            uint32_t nb, uint32_t *set, uint32_t *col, unsigned long long *got) {
+  const uint32_t per = RP_CTAS / nb, i = blockIdx.x / per, part = blockIdx.x % per;
   uint32_t bin = (uint32_t)((2ull * i + 1) * nbins / (2 * nb));
   // (a shard's bins are every shard_count-th one)
   for (const uint32_t stop = (uint32_t)((i + 1ull) * nbins / nb); bin + 1 < stop && seg_off[bin + 1] == seg_off[bin];) bin++;
   const uint64_t a = seg_off[bin], e = seg_off[bin + 1];
   const uint32_t words = (uint32_t)((e - a) >> (RP_BITS + 2));
   if (!words) return;
+  __shared__ uint32_t sum[3];
+  if (threadIdx.x < 3) sum[threadIdx.x] = 0;
+  __syncthreads();
   uint32_t *s = set + (a >> (RP_BITS + 2)), *c = col + (a >> (RP_BITS + 2));
   uint32_t n = 0, bits = 0, shared = 0;
 #pragma unroll 8
@@ -1575,11 +1582,13 @@ __global__ void __launch_bounds__(RP_BLOCK) rp_sample_kernel(const uint64_t *key
   n = warp_sum(n);
   bits = warp_sum(bits);
   shared = warp_sum(shared);
-  if (lane_id() == 0 && n) {
-    atomicAdd(&got[0], (unsigned long long)n);
-    atomicAdd(&got[1], (unsigned long long)bits);
-    atomicAdd(&got[2], (unsigned long long)shared);
+  if (lane_id() == 0 && n) {  // (an atomic a warp on three addresses of global memory would take most of the kernel)
+    atomicAdd(&sum[0], n);
+    atomicAdd(&sum[1], bits);
+    atomicAdd(&sum[2], shared);
   }
+  __syncthreads();
+  if (threadIdx.x < 3 && sum[0]) atomicAdd(&got[threadIdx.x], (unsigned long long)sum[threadIdx.x]);
 }
 
 // Groups the dedup left: one CTA per listed group moves its keys (unpacked)
@@ -2172,7 +2181,7 @@ void msd_look_for_repeats(const uint64_t *keys, uint64_t n, const uint64_t *seg_
   const uint64_t words = rp_words(n);
   uint32_t *set = sc.hist.get<uint32_t>(2 * words);  // free until the split
   CF1_CUDA(cudaMemsetAsync(set, 0, 2 * words * sizeof(uint32_t), s));
-  rp_sample_kernel<<<RP_CTAS, RP_BLOCK, 0, s>>>(keys, seg_off, nbins, set, set + words,
+  rp_sample_kernel<<<RP_CTAS, RP_BLOCK, 0, s>>>(keys, seg_off, nbins, rp_bins(n, nbins), set, set + words,
                                                reinterpret_cast<unsigned long long *>(got));
   CF1_LAUNCH_CHECK();
 }
